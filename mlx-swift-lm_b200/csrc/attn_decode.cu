@@ -342,8 +342,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
 // ---------------------------------------------------------------------
 //
 // LIST runs the calls of one shape (the layers of a batched step, whose inputs are all in hand) as one
-// launch over their units laid end to end: a step of small layers is otherwise a chain of launches that
-// each cost their ramp, merge and tail (26 layers of the Gemma-3-1B shape: 383 us as 26 launches).
+// launch: a step of small layers is otherwise a chain of launches that each cost their ramp, merge and tail
+// (26 layers of the Gemma-3-1B shape: 383 us as 26 launches). Each call keeps the ranges it has as a launch of its
+// own, dealt to the resident CTAs in turn, so its outputs are the same bits: P is rounded to 16 bits, tokens that are
+// a range's maximum are exact, and longer ranges have fewer of those (one range per CTA over all calls: the error
+// against 64-bit sums rises by 3 .. 5 %). With several ranges per CTA a range must end without a wait: every warp
+// leaves its state in memory and walks on, and flat_list_merge_kernel does the merges of all units behind it. 26 layers
+// of the Gemma-3-1B shape (4 x 2048 tokens, rings of 512) and 8 layers of 8 x 8192 tokens, 32/8 heads, D 128, bf16:
+// 160 and 436 us with the merges inside (ticket, last CTA of the unit), 61 and 379 behind, 50 and 341 with the
+// descriptors handed over (FlatWork); one launch per call took 391 and 402.
+constexpr int FLAT_AHEAD = 4;   // segments of a list the producer may be ahead
 struct FlatLayer {
     CUtensorMap kmap, vmap;
     const void *q;
@@ -353,36 +361,41 @@ struct FlatLayer {
     int64_t kv_sb, kv_sh, kv_st;
     const void *new_k, *new_v;
     int64_t new_slot, nk_sb, nk_sh, nv_sb, nv_sh, T;
-    int64_t tile_first;   // flat tiles of the layers before this one
-    int32_t tiles;        // tiles per unit
+    int64_t part_first;        // row slots of the partials before this layer's
+    int32_t tiles, per, rem;   // tiles per unit; tiles per range of the call's own plan
+    int32_t nslots, first;     // partial slots per row; ranges of the layers before this one
 };
 struct FlatList {
-    int32_t n;
+    int32_t n, ranges;
     FlatLayer layer[KVC_LIST_MAX];
 };
 struct FlatSingle {
     CUtensorMap kmap, vmap;
 };
 
-// The unit that flat tile `x` falls in, and its arrays.
+// The range and the unit a CTA is at, and the unit's arrays.
 struct FlatSeg {
+    FlatPlan plan;
     const CUtensorMap *kmap, *vmap;
     const void *q, *new_k, *new_v;
     void *out;
     int64_t q_sb, o_sb;
     unsigned char *k_base, *v_base;
-    int64_t kv_sb, kv_sh, kv_st, new_slot, nk_sb, nk_sh, nv_sb, nv_sh, T, unit_x;
-    int layer, unit, hk, b, t0, n, tiles;
+    int64_t kv_sb, kv_sh, kv_st, new_slot, nk_sb, nk_sh, nv_sb, nv_sh, T, part_first;
+    int cta, layer, unit, hk, b, t0, n;
 };
 
+// Range `r` of the launch: its call and its tiles [x_lo, x_hi) of that call.
 template <bool LIST, typename LT>
-__device__ __forceinline__ void flat_locate(FlatSeg &g, const DecodeParams &p, const LT &list, int64_t x, int64_t x_hi) {
-    int64_t in = x;
+__device__ __forceinline__ void flat_range(FlatSeg &g, const DecodeParams &p, const LT &list, int r, int64_t &x_lo, int64_t &x_hi) {
+    g.plan = p.flat;
+    g.cta = r;
     if constexpr (LIST) {
-        while (g.layer + 1 < list.n && list.layer[g.layer + 1].tile_first <= x) ++g.layer;
+        while (g.layer + 1 < list.n && list.layer[g.layer + 1].first <= r) ++g.layer;
         const FlatLayer &l = list.layer[g.layer];
-        in -= l.tile_first;
-        g.tiles = l.tiles;
+        g.cta = r - l.first;
+        g.plan.tiles = l.tiles; g.plan.per = l.per; g.plan.rem = l.rem; g.plan.nslots = l.nslots;
+        g.part_first = l.part_first;
         g.kmap = &l.kmap; g.vmap = &l.vmap;
         g.q = l.q; g.out = l.out; g.q_sb = l.q_sb; g.o_sb = l.o_sb;
         g.k_base = l.k_base; g.v_base = l.v_base;
@@ -390,9 +403,7 @@ __device__ __forceinline__ void flat_locate(FlatSeg &g, const DecodeParams &p, c
         g.new_k = l.new_k; g.new_v = l.new_v; g.new_slot = l.new_slot;
         g.nk_sb = l.nk_sb; g.nk_sh = l.nk_sh; g.nv_sb = l.nv_sb; g.nv_sh = l.nv_sh;
         g.T = l.T;
-        g.unit = g.layer * p.B * p.Hkv;
     } else {
-        g.tiles = p.flat.tiles;
         g.kmap = &list.kmap; g.vmap = &list.vmap;
         g.q = p.q; g.out = p.out; g.q_sb = p.q_sb; g.o_sb = p.o_sb;
         g.k_base = p.k_base; g.v_base = p.v_base;
@@ -400,15 +411,50 @@ __device__ __forceinline__ void flat_locate(FlatSeg &g, const DecodeParams &p, c
         g.new_k = p.new_k; g.new_v = p.new_v; g.new_slot = p.new_slot;
         g.nk_sb = p.nk_sb; g.nk_sh = p.nk_sh; g.nv_sb = p.nv_sb; g.nv_sh = p.nv_sh;
         g.T = p.T;
-        g.unit = 0;
     }
-    const int u = (int)(in / g.tiles);
-    g.t0 = (int)(in % g.tiles);
-    g.n = (int)min((int64_t)(g.tiles - g.t0), x_hi - x);
-    g.unit += u;
-    g.hk = u % p.Hkv;
+    x_lo = flat_lo(g.plan, g.cta);
+    x_hi = flat_lo(g.plan, g.cta + 1);
+}
+
+// The unit that tile `x` of the call falls in (32-bit: a tile is 16 KB at least).
+__device__ __forceinline__ void flat_locate(FlatSeg &g, const DecodeParams &p, int64_t x, int64_t x_hi) {
+    const int u = (int)((uint32_t)x / (uint32_t)g.plan.tiles);
+    g.t0 = (int)x - u * g.plan.tiles;
+    g.n = (int)min((int64_t)(g.plan.tiles - g.t0), x_hi - x);
     g.b = u / p.Hkv;
-    g.unit_x = x - g.t0;
+    g.hk = u - g.b * p.Hkv;
+    g.unit = u;
+}
+
+__device__ __forceinline__ int flat_cta_of32(const FlatPlan &f, uint32_t x) {
+    const uint32_t big = (uint32_t)f.rem * (f.per + 1);
+    return x < big ? (int)(x / (uint32_t)(f.per + 1)) : f.rem + (int)((x - big) / (uint32_t)f.per);
+}
+
+// What the consumers need of a segment.
+struct FlatWork {
+    const unsigned char *q, *new_k, *new_v;   // the unit's query rows, and its new rows (null: stored already)
+    unsigned char *k_row, *v_row;             // where the new rows go
+    int64_t T, new_slot, part;                // part: first row slot of the segment's partials (lists)
+    int32_t t0, n, nslots, more;              // more: 0 ends a list
+    int32_t unit, hk, b, last;                // last: the segment ends its unit
+};
+template <typename T>
+__device__ __forceinline__ FlatWork flat_work(const FlatSeg &g, const DecodeParams &p) {
+    FlatWork w;
+    const int rep = p.Hq / p.Hkv;
+    w.q = (const unsigned char *)((const T *)g.q + g.b * g.q_sb + (int64_t)g.hk * rep * p.q_sh);
+    w.new_k = g.new_k ? (const unsigned char *)((const T *)g.new_k + g.b * g.nk_sb + g.hk * g.nk_sh) : nullptr;
+    w.new_v = (const unsigned char *)((const T *)g.new_v + g.b * g.nv_sb + g.hk * g.nv_sh);
+    const int64_t row = g.b * g.kv_sb + g.hk * g.kv_sh + g.new_slot * g.kv_st;
+    w.k_row = g.k_base + row;
+    w.v_row = g.v_base + row;
+    w.T = g.T; w.new_slot = g.new_slot;
+    w.t0 = g.t0; w.n = g.n;
+    w.unit = g.unit; w.hk = g.hk; w.b = g.b;
+    w.last = g.t0 + g.n == g.plan.tiles;
+    w.more = 1;
+    return w;
 }
 
 template <typename T, int D, int NSTAGE, bool LIST>
@@ -433,22 +479,27 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
     // Query rows of a segment's unit, brought in by the producer with one bulk copy (two buffers):
     // plain loads issued by the consumers while the tile stream saturates the memory system cost
     // several microseconds per segment.
-    uint64_t *qfull = (uint64_t *)(work + ((fp.red_rows * fp.nslots + 3) & ~3));   // keeps qbuf 16-byte aligned
-    uint64_t *qempty = qfull + 2;
-    unsigned char *qbuf = (unsigned char *)(qempty + 2);                      // [2][red_rows][D] elements
+    // Lists have no cross-warp buffer, and the producer hands the consumers a segment's descriptor with its query rows:
+    // worked out by every warp at a segment's start it was constant-cache misses and divisions between two tiles.
+    constexpr int NQ = LIST ? FLAT_AHEAD : 2;
+    uint64_t *qfull = LIST ? (uint64_t *)red_o : (uint64_t *)(work + ((fp.red_rows * fp.nslots + 3) & ~3));   // keeps qbuf 16-byte aligned
+    uint64_t *qempty = qfull + NQ;
+    unsigned char *qbuf = (unsigned char *)(qempty + NQ);                     // [NQ][red_rows][D] elements
+    FlatWork *works = (FlatWork *)(qbuf + (size_t)NQ * (p.Hq / p.Hkv) * p.L * D * 2);   // [NQ] (lists)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rep = p.Hq / p.Hkv;
     const int R = rep * p.L;
-    const int64_t x_lo = flat_lo(fp, blockIdx.x), x_hi = flat_lo(fp, blockIdx.x + 1);
     const uint32_t q_bytes = (uint32_t)R * D * 2;
+    int ranges = gridDim.x;
+    if constexpr (LIST) ranges = list.ranges;
 
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], CONSUMER_WARPS);
         }
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < NQ; ++s) {
             mbar_init(&qfull[s], 1);
             mbar_init(&qempty[s], CONSUMER_WARPS);
         }
@@ -475,8 +526,14 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             bool waited = !early;
             FlatSeg gs;
             gs.layer = 0;
-            for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
-                flat_locate<LIST>(gs, p, list, x, x_hi);
+            int r = blockIdx.x;
+            for (int64_t x = 0, x_hi = 0; ok; ++sg) {
+                if (x == x_hi) {
+                    if (r >= ranges) break;
+                    flat_range<LIST>(gs, p, list, r, x, x_hi);
+                    r += gridDim.x;
+                }
+                flat_locate(gs, p, x, x_hi);
                 const int t0 = gs.t0, n = gs.n, hk = gs.hk, b = gs.b;
                 int j_first = 0;
                 if (!waited) {
@@ -496,11 +553,21 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                     pdl_trigger();
                     waited = true;
                 }
-                if (p.q_bulk) {
-                    const int qb = sg & 1;
-                    if (sg >= 2) ok = mbar_wait(&qempty[qb], ((sg >> 1) - 1) & 1);
+                if (LIST || p.q_bulk) {
+                    const int qb = sg % NQ;
+                    if (sg >= NQ) ok = mbar_wait(&qempty[qb], ((sg / NQ) - 1) & 1);
                     if (!ok) break;
-                    mbar_expect_tx(&qfull[qb], q_bytes);
+                    if constexpr (LIST) {
+                        FlatWork w = flat_work<T>(gs, p);
+                        w.nslots = gs.plan.nslots;
+                        w.part = gs.part_first + ((int64_t)b * p.Hq + hk * rep) * w.nslots + gs.cta - flat_cta_of32(gs.plan, (uint32_t)(x - t0));
+                        works[qb] = w;
+                    }
+                    if (p.q_bulk) mbar_expect_tx(&qfull[qb], q_bytes);
+                    else mbar_arrive(&qfull[qb]);
+                }
+                if (p.q_bulk) {
+                    const int qb = sg % NQ;
                     bulk_load(qbuf + (size_t)qb * q_bytes, (const T *)gs.q + b * gs.q_sb + (int64_t)hk * rep * p.q_sh, q_bytes,
                               &qfull[qb]);
                 }
@@ -530,6 +597,14 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 }
                 x += n;
             }
+            if constexpr (LIST) {
+                const int qb = sg % NQ;
+                if (ok && sg >= NQ) ok = mbar_wait(&qempty[qb], ((sg / NQ) - 1) & 1);
+                if (ok) {
+                    works[qb].more = 0;
+                    mbar_arrive(&qfull[qb]);
+                }
+            }
             if (!ok) atomicExch(p.status, 9);
         }
         return;
@@ -553,17 +628,33 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
     int it = 0, sg = 0;
     FlatSeg gs;
     gs.layer = 0;
-    for (int64_t x = x_lo; x < x_hi; ++sg) {
-        flat_locate<LIST>(gs, p, list, x, x_hi);
-        const int t0 = gs.t0, n = gs.n, hk = gs.hk, b = gs.b, tiles = gs.tiles;
+    int64_t x = 0, x_hi = 0;
+    if constexpr (!LIST) flat_range<LIST>(gs, p, list, blockIdx.x, x, x_hi);
+    for (;; ++sg) {
+        FlatWork own;
+        const int qb = sg % NQ;
+        if constexpr (LIST) {
+            ok = ok && mbar_wait(&qfull[qb], (sg / NQ) & 1);
+            if (!ok) {
+                if (lane == 0) atomicExch(p.status, 13);
+                break;                                // no barrier is shared with the other warps here
+            }
+            if (!works[qb].more) break;
+        } else {
+            if (x >= x_hi) break;
+            flat_locate(gs, p, x, x_hi);
+            own = flat_work<T>(gs, p);
+        }
+        const FlatWork &w = LIST ? works[qb] : own;
+        const int t0 = w.t0, n = w.n;
         // Fused append: token T - 1 is not in the cache yet; the tiles are masked up to T - 2 and the
         // new row is scored from its source by warp 0 of the CTA that owns the unit's last tile.
-        const bool fused = gs.new_k != nullptr;
+        const bool fused = w.new_k != nullptr;
         // Appending at the end: the tiles are simply cut one token short. Replacing a row inside a
         // wrapped ring: every token is visible except that slot, which still holds the row it loses.
-        const bool ring = fused && gs.new_slot != gs.T - 1;
-        const int64_t t_cached = gs.T - ((fused && !ring) ? 2 : 1);
-        const int64_t hole = ring ? gs.new_slot : -1;
+        const bool ring = fused && w.new_slot != w.T - 1;
+        const int64_t t_cached = w.T - ((fused && !ring) ? 2 : 1);
+        const int64_t hole = ring ? w.new_slot : -1;
         int64_t row_limit[2];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -571,18 +662,15 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             const int l = r % p.L;
             row_limit[half] = (r < R) ? (p.causal ? min(t_cached, p.causal_offset + l) : t_cached) : -1;
         }
-        if (fused && warp == 0 && t0 + n == tiles && lane < 4) {
+        if (fused && warp == 0 && w.last && lane < 4) {
             // the new rows are consumed at the end of the segment: pull them towards L2 now
-            const char *kn = (const char *)((const T *)gs.new_k + b * gs.nk_sb + hk * gs.nk_sh);
-            const char *vn = (const char *)((const T *)gs.new_v + b * gs.nv_sb + hk * gs.nv_sh);
-            const char *line = ((lane & 1) ? vn : kn) + (lane >> 1) * 128;
+            const unsigned char *line = ((lane & 1) ? w.new_v : w.new_k) + (lane >> 1) * 128;
             if ((lane >> 1) * 128 < D * 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
         }
         uint32_t qa[KSTEPS][4];
         if (p.q_bulk) {
-            const int qb = sg & 1;
-            if (ok) {
-                ok = mbar_wait(&qfull[qb], (sg >> 1) & 1);
+            if (!LIST && ok) {
+                ok = mbar_wait(&qfull[qb], (sg / NQ) & 1);
                 if (!ok && lane == 0) atomicExch(p.status, 13);
             }
             const unsigned char *qs = qbuf + (size_t)qb * q_bytes;
@@ -600,7 +688,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 }
             }
             __syncwarp();
-            if (ok && lane == 0) mbar_arrive(&qempty[qb]);
+            if (!LIST && ok && lane == 0) mbar_arrive(&qempty[qb]);
         } else
 #pragma unroll
         for (int ks = 0; ks < KSTEPS; ++ks) {
@@ -611,8 +699,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 const int r = g + 8 * half;
                 uint32_t w0 = 0, w1 = 0;
                 if (r < R && !(KVC_SKIP_BITS(p) & 32)) {
-                    const int hq = hk * rep + r / p.L, l = r % p.L;
-                    const T *qp = (const T *)gs.q + b * gs.q_sb + hq * p.q_sh + l * p.q_sl + d0;
+                    const T *qp = (const T *)w.q + (int64_t)(r / p.L) * p.q_sh + (r % p.L) * p.q_sl + d0;
                     w0 = *(const uint32_t *)qp;
                     w1 = *(const uint32_t *)(qp + 2);
                 }
@@ -720,10 +807,9 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             if (lane == 0) mbar_arrive(&empty[s]);
         }
 
-        if (fused && warp == 0 && t0 + n == tiles && !(KVC_SKIP_BITS(p) & 32)) {
+        if (fused && warp == 0 && w.last && !(KVC_SKIP_BITS(p) & 32)) {
             // ---- the step's new token: score q . k_new, fold it into this warp's state, store the rows ----
-            const T *kn = (const T *)gs.new_k + b * gs.nk_sb + hk * gs.nk_sh;
-            const T *vn = (const T *)gs.new_v + b * gs.nv_sb + hk * gs.nv_sh;
+            const T *kn = (const T *)w.new_k, *vn = (const T *)w.new_v;
             float dot[2] = {0.f, 0.f};
 #pragma unroll
             for (int ks = 0; ks < KSTEPS; ++ks) {
@@ -758,23 +844,37 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 o_acc[nt][3] = o_acc[nt][3] * alpha[1] + pn[1] * vv.y;
             }
             // the append itself: rows of D elements, 16 bytes per lane
-            const int64_t row_off = b * gs.kv_sb + hk * gs.kv_sh + gs.new_slot * gs.kv_st;
             constexpr int CHUNKS = D * 2 / 16;
             for (int i = lane; i < 2 * CHUNKS; i += 32) {
                 const bool is_v = i >= CHUNKS;
                 const int ch = is_v ? i - CHUNKS : i;
                 const uint4 x = *(const uint4 *)((const unsigned char *)(is_v ? vn : kn) + ch * 16);
-                *(uint4 *)((is_v ? gs.v_base : gs.k_base) + row_off + ch * 16) = x;
+                *(uint4 *)((is_v ? w.v_row : w.k_row) + ch * 16) = x;
             }
         }
 
-        // ---- end of the segment: merge the four warps, publish the partial, maybe merge the unit ----
+        // ---- end of the segment ----
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             l_run[half] += __shfl_xor_sync(0xffffffffu, l_run[half], 1);
             l_run[half] += __shfl_xor_sync(0xffffffffu, l_run[half], 2);
         }
-        {
+        if constexpr (LIST) {
+            // this warp's state goes to its place in the partials; the merge kernel reads it
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int r = g + 8 * half;
+                if (r >= R) continue;
+                const int64_t at = (w.part + (int64_t)r * w.nslots) * CONSUMER_WARPS + warp;
+#pragma unroll
+                for (int nt = 0; nt < NT_O; ++nt)
+                    __stcg((float2 *)&p.o_part[at * D + 8 * nt + 2 * c], make_float2(o_acc[nt][2 * half], o_acc[nt][2 * half + 1]));
+                if (c == 0) __stcg(&p.ml_part[at], make_float2(m_run[half], l_run[half]));
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&qempty[qb]);      // descriptor and query rows may be replaced
+        } else {
+            // merge the four warps, publish the partial, maybe merge the unit
             float *wo = red_o + warp * fp.red_rows * RED_STRIDE;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
@@ -788,20 +888,77 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                     red_ml[(warp * fp.red_rows + r) * 2 + 1] = l_run[half];
                 }
             }
+            UnitOut u;
+            u.o_part = p.o_part; u.ml_part = p.ml_part; u.counters = p.counters;
+            u.out = p.out; u.out_dtype = p.out_dtype;
+            u.o_sb = p.o_sb; u.o_sh = p.o_sh; u.o_sl = p.o_sl;
+            u.o_signs = nullptr;
+            u.splits = 0; u.Hq = p.Hq; u.L = p.L;
+            if (!(KVC_SKIP_BITS(p) & 16))
+                segment_epilogue<D, CONSUMER_WARPS>(u, fp, red_o, red_ml, RED_STRIDE, work, is_last, w.unit, w.b, w.hk, rep, R);
         }
-        UnitOut u;
-        u.o_part = p.o_part; u.ml_part = p.ml_part; u.counters = p.counters;
-        // rows of the partials: the batches of the layers laid end to end
-        const int b_row = b + gs.layer * p.B;
-        u.out = (T *)gs.out - (int64_t)gs.layer * p.B * gs.o_sb;
-        u.out_dtype = p.out_dtype;
-        u.o_sb = gs.o_sb; u.o_sh = p.o_sh; u.o_sl = p.o_sl;
-        u.o_signs = nullptr;
-        u.splits = 0; u.Hq = p.Hq; u.L = p.L;
-        if (!(KVC_SKIP_BITS(p) & 16))
-            segment_epilogue<D, CONSUMER_WARPS>(u, fp, red_o, red_ml, RED_STRIDE, work, is_last, gs.unit, b_row, hk, rep, R,
-                                                gs.unit_x, gs.tiles);
         x += n;
+    }
+}
+
+// The merges of a list launch: x = unit over all calls, one thread an output element (latency is all there is to it).
+// First the warps of every range, then the ranges of the unit in
+// batches of eight: the operations and their order are those of segment_epilogue.
+template <typename T, int D>
+__global__ void __launch_bounds__(128)
+flat_list_merge_kernel(const __grid_constant__ FlatList list, const __grid_constant__ DecodeParams p) {
+    pdl_wait();
+    pdl_trigger();
+    const int units = p.B * p.Hkv, u = blockIdx.x % units, hk = u % p.Hkv, b = u / p.Hkv, rep = p.Hq / p.Hkv;
+    const FlatLayer &l = list.layer[blockIdx.x / units];
+    FlatPlan plan = p.flat;
+    plan.tiles = l.tiles; plan.per = l.per; plan.rem = l.rem;
+    const int64_t x = (int64_t)u * l.tiles;
+    const int expected = flat_cta_of(plan, x + l.tiles - 1) - flat_cta_of(plan, x) + 1;
+    const int i = blockIdx.y * 128 + threadIdx.x;
+    if (i < rep * D) {
+        const int r = i / D, d = i % D;
+        const int64_t at = (l.part_first + ((int64_t)b * p.Hq + hk * rep + r) * l.nslots) * CONSUMER_WARPS;
+        float m = -INFINITY, o = 0.f, lsum = 0.f;
+        for (int s0 = 0; s0 < expected; s0 += 8) {
+            float2 ml[8];
+            float ov[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool in = s0 + j < expected;
+                float2 wml[CONSUMER_WARPS];
+                float wo[CONSUMER_WARPS], wm = -INFINITY;
+#pragma unroll
+                for (int w = 0; w < CONSUMER_WARPS; ++w) {
+                    const int64_t a = at + (s0 + j) * CONSUMER_WARPS + w;
+                    wml[w] = in ? __ldcg(&p.ml_part[a]) : make_float2(-INFINITY, 0.f);
+                    wo[w] = in ? __ldcg(&p.o_part[a * D + d]) : 0.f;
+                    wm = fmaxf(wm, wml[w].x);
+                }
+                ov[j] = 0.f;
+                ml[j] = make_float2(wm, 0.f);
+#pragma unroll
+                for (int w = 0; w < CONSUMER_WARPS; ++w) {
+                    const float fw = (wml[w].x == -INFINITY) ? 0.f : fast_exp2(wml[w].x - wm);
+                    ov[j] = fmaf(wo[w], fw, ov[j]);
+                    ml[j].y = fmaf(wml[w].y, fw, ml[j].y);
+                }
+            }
+            float mb = m;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) mb = fmaxf(mb, (ml[j].y > 0.f) ? ml[j].x : -INFINITY);
+            const float keep = (m == -INFINITY) ? 0.f : fast_exp2(m - mb);
+            o *= keep;
+            lsum *= keep;
+            m = mb;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float fw = (ml[j].x == -INFINITY || ml[j].y <= 0.f) ? 0.f : fast_exp2(ml[j].x - m);
+                lsum = fmaf(ml[j].y, fw, lsum);
+                o = fmaf(ov[j], fw, o);
+            }
+        }
+        store_out(l.out, p.out_dtype, b * l.o_sb + (hk * rep + r) * p.o_sh + d, lsum > 0.f ? o / lsum : 0.f);
     }
 }
 
@@ -1333,6 +1490,11 @@ void launch_flat_typed(const std::conditional_t<LIST, FlatList, FlatSingle> &lis
     }
     KernelTimer timer(stream);
     KVC_CUDA(launch_pdl(attn_decode_flat_kernel<T, D, NSTAGE, LIST>, dim3(ctas), dim3(DEC_THREADS), smem, stream, list, p));
+    if constexpr (LIST) {
+        const int elems = p.Hq / p.Hkv * D;
+        KVC_CUDA(launch_pdl(flat_list_merge_kernel<T, D>, dim3(list.n * p.B * p.Hkv, (elems + 127) / 128), dim3(128), 0, stream, list, p));
+        ++g_launch_count;
+    }
     timer.stop();
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
@@ -1397,6 +1559,13 @@ FlatShape flat_shape(int sms, int D, int R, int64_t work, int64_t most_tiles) {
     return f;
 }
 
+// Shared memory of a list launch: ring, barriers, and FLAT_AHEAD segments' query rows and descriptors.
+size_t flat_list_smem(int D, int R) {
+    const int nstage = D == 64 ? 6 : 3;
+    return (size_t)nstage * 2 * (TILE_T * D * 2) + 2 * nstage * sizeof(uint64_t) + 64 + FLAT_AHEAD * (2 * sizeof(uint64_t) + (size_t)R * D * 2 + sizeof(FlatWork)) + 1024;
+}
+constexpr int64_t LIST_PARTIAL_BYTES = (int64_t)64 << 20;   // of a list launch's partials
+
 bool flat_new_rows_ok(const AttnArgs &a) {
     return a.L == 1 && a.mask.mode != KVC_MASK_CAUSAL && !((uintptr_t)a.new_k & 15) && !((uintptr_t)a.new_v & 15) &&
            (a.nk_sb * 2) % 16 == 0 && (a.nk_sh * 2) % 16 == 0 && (a.nv_sb * 2) % 16 == 0 && (a.nv_sh * 2) % 16 == 0;
@@ -1423,9 +1592,9 @@ int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t strea
     const int R = a0.Hq / a0.Hkv;
     const int64_t units = (int64_t)a0.B * a0.Hkv;
     if (R > 16 || n * units * (int64_t)sizeof(int) > COUNTER_BYTES) return 0;
-    static thread_local FlatList list;
-    list.n = n;
-    int64_t work = 0, most = 0;
+    static thread_local FlatList all, list;
+    const int sms = sm_count(a0.device);
+    const size_t smem = flat_list_smem(a0.D, R);
     bool q_bulk = true;
     for (int i = 0; i < n; ++i) {
         const AttnArgs &a = args[i];
@@ -1439,7 +1608,7 @@ int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t strea
         if (a.k.sb != a.v.sb || a.k.sh != a.v.sh || a.k.st != a.v.st) return 0;
         if (((uintptr_t)a.q & 3) || (a.q_sb & 1) || (a.q_sh & 1) || (a.q_sl & 1)) return 0;
         if (a.new_k && !flat_new_rows_ok(a)) return 0;
-        FlatLayer &l = list.layer[i];
+        FlatLayer &l = all.layer[i];
         if (!make_map(&l.kmap, a.k, a.D, a.T, a.Hkv, a.B) || !make_map(&l.vmap, a.v, a.D, a.T, a.Hkv, a.B)) return 0;
         l.q = a.q; l.out = a.out; l.q_sb = a.q_sb; l.o_sb = a.o_sb;
         l.k_base = (unsigned char *)a.k.data; l.v_base = (unsigned char *)a.v.data;
@@ -1449,46 +1618,60 @@ int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t strea
         l.nk_sb = a.nk_sb; l.nk_sh = a.nk_sh; l.nv_sb = a.nv_sb; l.nv_sh = a.nv_sh;
         l.T = a.T;
         l.tiles = (int32_t)((a.T + TILE_T - 1) / TILE_T);
-        l.tile_first = work;
-        work += units * l.tiles;
-        most = std::max<int64_t>(most, l.tiles);
+        const FlatShape own = flat_shape(sms, a.D, R, units * l.tiles, l.tiles);
+        if (!own.fits) return 0;
+        l.per = (int32_t)own.per; l.rem = (int32_t)own.rem;
+        l.nslots = (int32_t)own.nslots;
         q_bulk = q_bulk && a.q_sh == a.D && ((uintptr_t)a.q & 15) == 0 && (a.q_sb * 2) % 16 == 0;
     }
-    const FlatShape f = flat_shape(sm_count(a0.device), a0.D, R, work, most);
-    if (!f.fits) return 0;
     int *status = device_status_word(a0.device);
-    int *counters = counters_get(a0.device, stream, COUNTER_BYTES);
-    if (!status || !counters) return 0;
-    const int64_t qrows = (int64_t)n * a0.B * a0.Hq;
-    const size_t o_bytes = (size_t)qrows * f.nslots * a0.D * sizeof(float);
-    char *scratch = (char *)scratch_get(a0.device, o_bytes + (size_t)qrows * f.nslots * sizeof(float2) + 256, stream);
+    if (!status) return 0;
     DecodeParams p = {};
     p.out_dtype = a0.q_dtype;
     p.q_sh = a0.q_sh; p.q_sl = a0.q_sl; p.o_sh = a0.o_sh; p.o_sl = a0.o_sl;
-    p.o_part = (float *)scratch;
-    p.ml_part = (float2 *)(scratch + ((o_bytes + 255) / 256) * 256);
-    p.counters = counters; p.status = status;
+    p.status = status;
     p.B = a0.B; p.Hq = a0.Hq; p.Hkv = a0.Hkv; p.L = 1;
     p.splits = 1; p.row_blocks = 1;
     p.debug_skip = measure_skip_bits();
     p.scale_log2 = a0.scale * 1.4426950408889634f;
-    p.flat.tiles = (int)most;
-    p.flat.per = (int)f.per; p.flat.rem = (int)f.rem;
-    p.flat.nslots = (int)f.nslots; p.flat.red_rows = R;
+    p.flat.red_rows = R;   // the rest of the plan is each call's own
     p.q_bulk = q_bulk ? 1 : 0;
-#define KVC_FLATL(TT, DD, NS) launch_flat_typed<TT, DD, NS, true>(list, p, (int)f.ctas, f.smem, stream)
-    if (a0.q_dtype == KVC_BF16) {
-        if (a0.D == 64) KVC_FLATL(__nv_bfloat16, 64, 6);
-        else if (a0.D == 128) KVC_FLATL(__nv_bfloat16, 128, 3);
-        else KVC_FLATL(__nv_bfloat16, 256, 3);
-    } else {
-        if (a0.D == 64) KVC_FLATL(__half, 64, 6);
-        else if (a0.D == 128) KVC_FLATL(__half, 128, 3);
-        else KVC_FLATL(__half, 256, 3);
-    }
+    // as many calls a launch as the partials have room for
+    int launches = 0;
+    for (int from = 0; from < n;) {
+        int64_t ranges = 0, row_slots = 0;
+        list.n = 0;
+        for (; from < n; ++from) {
+            FlatLayer l = all.layer[from];
+            const int64_t rows = (int64_t)a0.B * a0.Hq * l.nslots;
+            if (list.n && (row_slots + rows) * CONSUMER_WARPS * a0.D * (int64_t)sizeof(float) > LIST_PARTIAL_BYTES) break;
+            l.first = (int32_t)ranges;
+            l.part_first = row_slots;
+            ranges += std::min<int64_t>((int64_t)sms * (a0.D <= 128 ? 2 : 1), units * l.tiles);
+            row_slots += rows;
+            list.layer[list.n++] = l;
+        }
+        list.ranges = (int32_t)ranges;
+        const int ctas = (int)std::min<int64_t>(ranges, (int64_t)sms * (a0.D <= 128 ? 2 : 1));
+        const size_t o_bytes = (size_t)row_slots * CONSUMER_WARPS * a0.D * sizeof(float);
+        char *scratch = (char *)scratch_get(a0.device, o_bytes + (size_t)row_slots * CONSUMER_WARPS * sizeof(float2) + 256, stream);
+        p.o_part = (float *)scratch;
+        p.ml_part = (float2 *)(scratch + ((o_bytes + 255) / 256) * 256);
+#define KVC_FLATL(TT, DD, NS) launch_flat_typed<TT, DD, NS, true>(list, p, ctas, smem, stream)
+        if (a0.q_dtype == KVC_BF16) {
+            if (a0.D == 64) KVC_FLATL(__nv_bfloat16, 64, 6);
+            else if (a0.D == 128) KVC_FLATL(__nv_bfloat16, 128, 3);
+            else KVC_FLATL(__nv_bfloat16, 256, 3);
+        } else {
+            if (a0.D == 64) KVC_FLATL(__half, 64, 6);
+            else if (a0.D == 128) KVC_FLATL(__half, 128, 3);
+            else KVC_FLATL(__half, 256, 3);
+        }
 #undef KVC_FLATL
+        launches += 2;
+    }
     g_last_chained_launch = g_launch_count;
-    return 1;
+    return launches;
 }
 
 namespace {

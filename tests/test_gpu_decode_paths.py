@@ -444,3 +444,31 @@ def test_f32_affine_decode_kernel_matches_oracle(kvc, oracle, cuda, bits, group,
         out = g.attention(q.to(cuda), k1.to(cuda), v1.to(cuda), D ** -0.5, mask)
         ref = oracle.attention_with_cache_update(to_oracle(q), to_oracle(k1), to_oracle(v1), o, D ** -0.5, mask)
         assert max_abs_diff(out, ref) <= TOL[torch.float32]
+
+
+@pytest.mark.parametrize("dtype,D,B,Hq,Hkv,lengths", [
+    (torch.bfloat16, 128, 8, 32, 8, [4097, 4097, 4097]),        # ranges of tens of tiles that cross units
+    (torch.float16, 64, 3, 8, 2, [1500, 64, 1500, 64]),         # fewer ranges than resident CTAs, one and many tiles
+    (torch.bfloat16, 256, 4, 4, 1, [2048] + [512] * 12),        # rings and a longer cache: each CTA takes several ranges
+    (torch.float16, 256, 1, 8, 2, [3000, 70]),                  # 47 ranges of a unit: six batches of eight in its merge
+])
+def test_batched_raw_step_gives_the_bits_of_the_calls_in_turn(kvc, cuda, dtype, D, B, Hq, Hkv, lengths):
+    """Calls that share a launch keep the ranges they have alone, so P (16 bits) meets the same maxima: equal bits."""
+    n = len(lengths)
+    caches = [kvc.RotatingKVCache(max_size=512, keep=0) if T == 512 else kvc.KVCacheSimple() for T in lengths]
+    for i, (c, T) in enumerate(zip(caches, lengths)):
+        c.update(*(seeded((B, Hkv, T, D), 10 * i + j, dtype).to(cuda) for j in (1, 2)))
+    copies = [c.copy() for c in caches]
+    q, k, v = ([seeded((B, h, 1, D), s + i, dtype).to(cuda) for i in range(n)] for h, s in ((Hq, 100), (Hkv, 200), (Hkv, 300)))
+    outs = [torch.empty_like(t) for t in q]
+    step = kvc.DecodeStep(caches, q, k, v, outs, D ** -0.5)
+    for turn in range(3):
+        kvc.launch_count(reset=True)
+        step.run()
+        if turn:                                       # the first step grows the linear caches
+            assert kvc.launch_count(reset=True) == 2   # the walk and the merges
+        for i, c in enumerate(copies):
+            assert torch.equal(outs[i], c.attention(q[i], k[i], v[i], D ** -0.5)), (turn, i)
+    for a, b in zip(caches, copies):
+        assert all(torch.equal(s, t) for s, t in zip(a.state, b.state))
+    assert kvc.lib().kvc_device_status() == 0
