@@ -1034,10 +1034,12 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
     constexpr int STAGE_BYTES = (PAIRS ? 4 : 2) * TILE_BYTES;      // K, V (, low halves of K, of V)
     // Query fragments in shared memory where registers are short (bytes of one half); NBK: 16-token blocks a warp
     // takes at a time. At D 256 an SM holds one warp per scheduler, so the chains of a step have to hide one another:
-    // two blocks give twice the independent MMAs and one maximum, one rescale for 32 tokens.
+    // two blocks give twice the independent MMAs. SMX: blocks that share a maximum and a rescale. One, where P is a
+    // single 16-bit value: tokens that are the maximum of their block are exact, and a maximum per 32 tokens leaves half
+    // as many (error against 64-bit sums + 0.4 % at 500 keys).
     constexpr bool Q_SHARED = PAIRS || D == 256;
     constexpr int QF_BYTES = Q_SHARED ? CONSUMER_WARPS * KSTEPS * 32 * 16 : 0;
-    constexpr int NBK = D == 256 && !PAIRS ? 2 : 1;
+    constexpr int NBK = D == 256 && !PAIRS ? 2 : 1, SMX = P_PAIR ? NBK : 1;
     unsigned char *qf = stages + (size_t)NSTAGE * STAGE_BYTES;
     uint64_t *full = (uint64_t *)(qf + (PAIRS ? 2 : 1) * QF_BYTES);
     uint64_t *empty = full + NSTAGE;
@@ -1239,89 +1241,93 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
                     }
                 }
                 const bool edge = t_blk + 16 * NBK - 1 > lim_min;  // warp-uniform
-                float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-                for (int j = 0; j < 2 * NBK; ++j) {
+                for (int u0 = 0; u0 < NBK; u0 += SMX) {
+                    float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int half = e >> 1;
-                        float v = sc[j][e] * score_scale;
-                        const int t = t_blk + j * 8 + 2 * c + (e & 1);
-                        if (MASKED) {
-                            if (bits_mask) {
-                                const int bit = (blk & 1) * 16 + j * 8 + 2 * c + (e & 1);
-                                if (!(((blk & 2 ? vis[half][1] : vis[half][0]) >> bit) & 1)) v = -INFINITY;
-                            } else if (t <= row_limit[half]) {
-                                v += mask_value(p.mask, row_mask[half] + t * p.mask.st);
+                    for (int j = 2 * u0; j < 2 * (u0 + SMX); ++j) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int half = e >> 1;
+                            float v = sc[j][e] * score_scale;
+                            const int t = t_blk + j * 8 + 2 * c + (e & 1);
+                            if (MASKED) {
+                                if (bits_mask) {
+                                    const int bit = (blk & 1) * 16 + j * 8 + 2 * c + (e & 1);
+                                    if (!(((blk & 2 ? vis[half][1] : vis[half][0]) >> bit) & 1)) v = -INFINITY;
+                                } else if (t <= row_limit[half]) {
+                                    v += mask_value(p.mask, row_mask[half] + t * p.mask.st);
+                                }
                             }
-                        }
-                        if (edge) v = (t <= row_limit[half]) ? v : -INFINITY;
-                        sc[j][e] = v;
-                        tmax[half] = fmaxf(tmax[half], v);
-                    }
-                }
-                float alpha[2];
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    tmax[half] = fmaxf(tmax[half], __shfl_xor_sync(0xffffffffu, tmax[half], 1));
-                    tmax[half] = fmaxf(tmax[half], __shfl_xor_sync(0xffffffffu, tmax[half], 2));
-                    const float m_new = fmaxf(m_run[half], tmax[half]);
-                    alpha[half] = (m_new == -INFINITY) ? 1.f : fast_exp2((m_run[half] - m_new) * log2_unit);
-                    m_run[half] = m_new;
-                }
-                uint32_t pa[NBK][4], pl[NBK][4];       // P, and what its rounding leaves
-#pragma unroll
-                for (int j = 0; j < 2 * NBK; ++j)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int half = e >> 1;
-                        sc[j][e] = (m_run[half] == -INFINITY) ? 0.f : fast_exp2((sc[j][e] - m_run[half]) * log2_unit);
-                    }
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    l_run[half] *= alpha[half];
-#pragma unroll
-                    for (int j = 0; j < 2 * NBK; ++j) l_run[half] += sc[j][2 * half] + sc[j][2 * half + 1];
-                }
-#pragma unroll
-                for (int u = 0; u < NBK; ++u)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float x = sc[2 * u + (i >> 1)][2 * (i & 1)], y = sc[2 * u + (i >> 1)][2 * (i & 1) + 1];
-                        pa[u][i] = MmaType<T>::pack(x, y);
-                        if constexpr (P_PAIR) {
-                            const float2 hi = MmaType<T>::unpack(pa[u][i]);
-                            pl[u][i] = MmaType<T>::pack(x - hi.x, y - hi.y);
+                            if (edge) v = (t <= row_limit[half]) ? v : -INFINITY;
+                            sc[j][e] = v;
+                            tmax[half] = fmaxf(tmax[half], v);
                         }
                     }
-                if (__any_sync(0xffffffffu, (alpha[0] != 1.f) | (alpha[1] != 1.f))) {
+                    float alpha[2];
 #pragma unroll
-                    for (int nt = 0; nt < NT_O; ++nt) {
-                        o_acc[nt][0] *= alpha[0];
-                        o_acc[nt][1] *= alpha[0];
-                        o_acc[nt][2] *= alpha[1];
-                        o_acc[nt][3] *= alpha[1];
+                    for (int half = 0; half < 2; ++half) {
+                        tmax[half] = fmaxf(tmax[half], __shfl_xor_sync(0xffffffffu, tmax[half], 1));
+                        tmax[half] = fmaxf(tmax[half], __shfl_xor_sync(0xffffffffu, tmax[half], 2));
+                        const float m_new = fmaxf(m_run[half], tmax[half]);
+                        alpha[half] = (m_new == -INFINITY) ? 1.f : fast_exp2((m_run[half] - m_new) * log2_unit);
+                        m_run[half] = m_new;
                     }
-                }
+                    uint32_t pa[SMX][4], pl[SMX][4];       // P, and what its rounding leaves
 #pragma unroll
-                for (int bx = 0; bx < BOXES; ++bx) {
+                    for (int j = 2 * u0; j < 2 * (u0 + SMX); ++j)
 #pragma unroll
-                    for (int cp = 0; cp < 4; ++cp) {
+                        for (int e = 0; e < 4; ++e) {
+                            const int half = e >> 1;
+                            sc[j][e] = (m_run[half] == -INFINITY) ? 0.f : fast_exp2((sc[j][e] - m_run[half]) * log2_unit);
+                        }
 #pragma unroll
-                        for (int u = 0; u < NBK; ++u) {
-                            const uint32_t va = vt_addr + bx * BOX_BYTES + boff + u * 16 * 128 + v_off[cp];
-                            uint32_t vf[4];
-                            ldmatrix_x4_trans(vf, va);
-                            MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pa[u], vf[0], vf[1]);
-                            MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa[u], vf[2], vf[3]);
+                    for (int half = 0; half < 2; ++half) {
+                        l_run[half] = fmaf(l_run[half], alpha[half], sc[2 * u0][2 * half]) + sc[2 * u0][2 * half + 1];
+#pragma unroll
+                        for (int j = 2 * u0 + 1; j < 2 * (u0 + SMX); ++j) l_run[half] = l_run[half] + sc[j][2 * half] + sc[j][2 * half + 1];
+                    }
+#pragma unroll
+                    for (int u = 0; u < SMX; ++u)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int j = 2 * (u0 + u) + (i >> 1);
+                            const float x = sc[j][2 * (i & 1)], y = sc[j][2 * (i & 1) + 1];
+                            pa[u][i] = MmaType<T>::pack(x, y);
                             if constexpr (P_PAIR) {
-                                MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pl[u], vf[0], vf[1]);
-                                MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pl[u], vf[2], vf[3]);
+                                const float2 hi = MmaType<T>::unpack(pa[u][i]);
+                                pl[u][i] = MmaType<T>::pack(x - hi.x, y - hi.y);
                             }
-                            if constexpr (PAIRS) {
-                                ldmatrix_x4_trans(vf, va + 2 * TILE_BYTES);
+                        }
+                    if (__any_sync(0xffffffffu, (alpha[0] != 1.f) | (alpha[1] != 1.f))) {
+#pragma unroll
+                        for (int nt = 0; nt < NT_O; ++nt) {
+                            o_acc[nt][0] *= alpha[0];
+                            o_acc[nt][1] *= alpha[0];
+                            o_acc[nt][2] *= alpha[1];
+                            o_acc[nt][3] *= alpha[1];
+                        }
+                    }
+#pragma unroll
+                    for (int bx = 0; bx < BOXES; ++bx) {
+#pragma unroll
+                        for (int cp = 0; cp < 4; ++cp) {
+#pragma unroll
+                            for (int u = 0; u < SMX; ++u) {
+                                const uint32_t va = vt_addr + bx * BOX_BYTES + boff + (u0 + u) * 16 * 128 + v_off[cp];
+                                uint32_t vf[4];
+                                ldmatrix_x4_trans(vf, va);
                                 MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pa[u], vf[0], vf[1]);
                                 MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa[u], vf[2], vf[3]);
+                                if constexpr (P_PAIR) {
+                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pl[u], vf[0], vf[1]);
+                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pl[u], vf[2], vf[3]);
+                                }
+                                if constexpr (PAIRS) {
+                                    ldmatrix_x4_trans(vf, va + 2 * TILE_BYTES);
+                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pa[u], vf[0], vf[1]);
+                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa[u], vf[2], vf[3]);
+                                }
                             }
                         }
                     }

@@ -535,3 +535,30 @@ def test_row_masked_by_the_lowest_value_is_an_average(kvc, cuda, dtype, mask_dty
     mean = v.double().mean(2).repeat_interleave(Hq // Hkv, 1)
     assert float((out[:, :, 3].double() - mean).abs().max()) <= 2.0 ** -9     # outputs below 1: half a bf16 spacing
     assert not out[:, :, 5].any() and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 256), (torch.float16, 256), (torch.bfloat16, 128)])
+def test_unmasked_chunk_takes_a_maximum_per_16_tokens(kvc, cuda, dtype, D):
+    """P rounds to 16 bits against the running maximum, and tokens that are it are exact: how many tokens share a
+    maximum is part of the result's precision. Emulated in 64 bits with 16 and with 32 tokens a step (one tile of 64
+    tokens, one split): the kernel's outputs are the first. What is left there is the store's rounding of sums that
+    agree to fp32; the two emulations differ by the rounding of P."""
+    B, Hq, Hkv, P, L = 4, 4, 1, 34, 30
+    k, v, q = (seeded((B, h, n, D), i, dtype) for h, n, i in ((Hkv, P + L, 1), (Hkv, P + L, 2), (Hq, L, 3)))
+    out = kvc.scaled_dot_product_attention(q.to(cuda), k.to(cuda), v.to(cuda), D ** -0.5, "causal").cpu()
+    s = (q.double() @ k.double().transpose(2, 3)) * D ** -0.5 * 1.4426950408889634
+    s = s.masked_fill(torch.arange(P + L)[None, :] > torch.arange(P, P + L)[:, None], -torch.inf)
+
+    def emulate(step):
+        m, l, o = torch.full((B, Hq, L, 1), -torch.inf, dtype=torch.float64), 0.0, 0.0
+        for t in range(0, P + L, step):
+            x = s[..., t:t + step]
+            m_new = torch.maximum(m, x.amax(-1, True))
+            a, p = torch.exp2(m - m_new), torch.exp2(x - m_new)
+            m, l, o = m_new, l * a + p.sum(-1, True), o * a + p.float().to(dtype).double() @ v[:, :, t:t + step].double()
+        return o / l
+    far = float((emulate(32) - emulate(16)).norm())
+    ref = emulate(16)
+    store = float((ref.float().to(dtype).double() - ref).norm())
+    assert float((out.double() - ref).norm()) <= 1.01 * store          # 32 tokens a step: hypot(store, far)
+    assert far > 0.3 * store
