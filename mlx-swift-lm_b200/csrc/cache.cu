@@ -12,14 +12,23 @@
 
 namespace kvc {
 
-// Set by the batched entry points around each layer's call: the cache of the layer launched just
-// before on the same stream (nullptr outside a batched call or for its first layer).
-static thread_local const kvc_cache *tl_batch_prev = nullptr;
-void set_batch_previous(const kvc_cache *prev) { tl_batch_prev = prev; }
+// Set by the batched entry points around each layer's call: the caches the launch just before works on,
+// on the same stream (none outside a batched call or for its first layer).
+static thread_local kvc_cache *const *tl_batch_prev = nullptr;
+static thread_local int tl_batch_prev_n = 0;
+void set_batch_previous(kvc_cache *const *prev, int n) {
+    tl_batch_prev = prev;
+    tl_batch_prev_n = n;
+}
 static thread_local bool tl_rope_previous = false;
 void set_rope_previous(bool rope) { tl_rope_previous = rope; }
-// The launch before this call's first one wrote no row of `c`: it belongs to another cache or turned q and k.
-static bool previous_spares(const kvc_cache *c) { return tl_rope_previous || (tl_batch_prev != nullptr && tl_batch_prev != c); }
+// The launch before this call's first one wrote no row of `c`: it belongs to other caches or turned q and k.
+static bool previous_spares(const kvc_cache *c) {
+    if (tl_rope_previous) return true;
+    for (int i = 0; i < tl_batch_prev_n; ++i)
+        if (tl_batch_prev[i] == c) return false;
+    return tl_batch_prev_n > 0;
+}
 
 int launch_attention(const AttnArgs &a, cudaStream_t stream);
 
@@ -1393,7 +1402,8 @@ void list_launch(ListKind kind, std::vector<ListedCall> &calls, cudaStream_t s) 
 // (their order does not matter then). Everything else is made one by one.
 void cache_attention_batch(kvc_cache *const *caches, int n, const kvc_tensor *q, const kvc_tensor *k, const kvc_tensor *v, float scale,
                            int32_t mask_mode, const kvc_tensor *outs, cudaStream_t s) {
-    struct HintReset { ~HintReset() { set_batch_previous(nullptr); } } hint_reset;
+    struct HintReset { ~HintReset() { set_batch_previous(nullptr, 0); } } hint_reset;
+    int last = 0, last_n = 0;     // the calls of the launch before: a list covers all of its caches
     for (int from = 0; from < n;) {
         const ListKind kind = list_kind(caches[from], q[from], k[from], v[from], outs[from], mask_mode);
         int to = from + 1;
@@ -1417,9 +1427,11 @@ void cache_attention_batch(kvc_cache *const *caches, int n, const kvc_tensor *q,
         if (to - from < 2 || (kind == ListKind::raw && !layers_of_one_model(caches + from, to - from))) {
             for (int i = from; i < to; ++i) {
                 // this call's launches follow the one before on the stream with nothing in between
-                set_batch_previous(i > 0 ? caches[i - 1] : nullptr);
+                set_batch_previous(caches + last, last_n);
                 cache_attention(caches[i], q[i], k[i], v[i], scale, mask_mode, nullptr, outs[i], s);
-                set_batch_previous(nullptr);
+                set_batch_previous(nullptr, 0);
+                last = i;
+                last_n = 1;
             }
             from = to;
             continue;
@@ -1433,6 +1445,8 @@ void cache_attention_batch(kvc_cache *const *caches, int n, const kvc_tensor *q,
             throw;
         }
         list_launch(kind, calls, s);
+        last = from;
+        last_n = to - from;
         from = to;
     }
 }

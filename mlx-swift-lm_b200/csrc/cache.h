@@ -183,9 +183,9 @@ AttnArgs make_attn_args(const kvc_tensor &q, const kvc_tensor &out, float scale,
                         const kvc_tensor *mask, int64_t T, int Hkv);
 KVSource raw_source(const kvc_tensor &t);
 
-// Batched entry points: names the cache whose kernels were launched just before the next
-// cache_attention call on the same stream (nullptr = unknown / none).
-void set_batch_previous(const kvc_cache *prev);
+// Batched entry points: the caches that the launch just before the next cache_attention call on the
+// same stream works on (n = 0: unknown / none). The array is read during that call only.
+void set_batch_previous(kvc_cache *const *prev, int n);
 // The launch before the next call's is the rotary kernel of its q and k.
 void set_rope_previous(bool rope);
 

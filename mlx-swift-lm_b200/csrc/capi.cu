@@ -1175,7 +1175,7 @@ kvc_status kvc_attention_batch(kvc_cache *const *caches, int32_t count, const kv
             };
             issue_inputs(0);
             int first = 0;
-            struct HintReset { ~HintReset() { kvc::set_batch_previous(nullptr); } } hint_reset;
+            struct HintReset { ~HintReset() { kvc::set_batch_previous(nullptr, 0); } } hint_reset;
             first = 0;
             for (size_t gi = 0; gi < group_end.size(); ++gi) {
                 KVC_CUDA(cudaStreamWaitEvent(s, pipe.events[2 + 2 * gi], 0));
@@ -1186,10 +1186,10 @@ kvc_status kvc_attention_batch(kvc_cache *const *caches, int32_t count, const kv
                     kvc_tensor tq = q[i], tk = k[i], tv = v[i], to = outs[i];
                     tq.data = dq; tk.data = dk; tv.data = dv; to.data = dout;
                     // layer i's launches follow layer i - 1's on the stream with nothing in between
-                    kvc::set_batch_previous(i > first ? caches[i - 1] : nullptr);
+                    kvc::set_batch_previous(i > first ? caches + (i - 1) : nullptr, i > first ? 1 : 0);
                     kvc::cache_attention(caches[i], tq, tk, tv, scale, mask_mode, nullptr, to, s);
                 }
-                kvc::set_batch_previous(nullptr);
+                kvc::set_batch_previous(nullptr, 0);
                 cudaEvent_t out_ready = pipe.events[3 + 2 * gi];
                 KVC_CUDA(cudaEventRecord(out_ready, s));
                 KVC_CUDA(cudaStreamWaitEvent(pipe.d2h, out_ready, 0));

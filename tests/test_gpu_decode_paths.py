@@ -472,3 +472,32 @@ def test_batched_raw_step_gives_the_bits_of_the_calls_in_turn(kvc, cuda, dtype, 
     for a, b in zip(caches, copies):
         assert all(torch.equal(s, t) for s, t in zip(a.state, b.state))
     assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("order", [[0, 1, 0], [0, 1, 2, 0], [0, 1, 0, 1, 0], [2, 0, 1, 1], list(range(33)) + [3, 40, 32]])
+@pytest.mark.parametrize("ring,P,D", [(False, 61, 128), (True, 60, 128), (False, 200, 64)])
+def test_batch_that_names_a_cache_again(kvc, cuda, order, ring, P, D):
+    """A call on a cache that an earlier launch of the batch has appended to sees that row: whatever launches the calls
+    share, outputs and caches are the bits of the calls made one by one with a wait between them."""
+    B, Hq, Hkv, n = 1, 8, 2, max(order) + 1
+    make = lambda: kvc.RotatingKVCache(max_size=64, keep=0) if ring else kvc.KVCacheSimple()
+    caches, alone = [make() for _ in range(n)], [make() for _ in range(n)]
+    for i in range(n):
+        k, v = (seeded((B, Hkv, P, D), 10 * i + j, torch.bfloat16).to(cuda) for j in (1, 2))
+        caches[i].update(k, v)
+        alone[i].update(k, v)
+    m = len(order)
+    # keys far along one direction and queries along it: each new row takes most of the weight, so a row missed shows
+    u = seeded((1, 1, 1, D), 5, torch.bfloat16).to(cuda)
+    for turn in range(20):
+        q = [u.expand(B, Hq, 1, D).contiguous() for _ in order]
+        k = [(u * (1 + 0.01 * (turn * m + i))).expand(B, Hkv, 1, D).contiguous() for i in range(m)]
+        v = [seeded((B, Hkv, 1, D), 1000 + turn * m + i, torch.bfloat16).to(cuda) for i in range(m)]
+        outs = [torch.empty_like(t) for t in q]
+        kvc.DecodeStep([caches[i] for i in order], q, k, v, outs, D ** -0.5).run()
+        for j, i in enumerate(order):
+            torch.cuda.synchronize()
+            assert torch.equal(outs[j], alone[i].attention(q[j], k[j], v[j], D ** -0.5)), (turn, j)
+    for a, b in zip(caches, alone):
+        assert a.offset == b.offset and all(torch.equal(s, t) for s, t in zip(a.state, b.state))
+    assert kvc.lib().kvc_device_status() == 0
