@@ -41,6 +41,15 @@ inline bool trace_dispatch() {
     return e && e[0] == '1';
 }
 
+// What a chunk on operand pairs takes beside its 16-bit rows: the low halves (k, q: null where the high ones are exact),
+// the factors that give scaled operands their size back (per query row; per (batch, KV head); null: 1; values always
+// have theirs), and the type of its output.
+struct ChunkLow {
+    const void *k, *v, *q;
+    const float *q_undo, *k_undo, *v_undo;
+    int32_t out_dtype;
+};
+
 namespace dev {
 
 constexpr uint32_t SPIN_LIMIT = 1u << 24;

@@ -76,9 +76,11 @@ struct DecodeParams {
     int64_t causal_offset;
     float scale_log2;  // scale * log2(e)
     MaskDesc mask;     // chunk kernel with an array mask
-    // chunk kernel on operand pairs: what the bf16 rows of q leave of the exact ones (same strides; null: nothing),
-    // whether the keys have such a half too
+    // chunk kernel on operand pairs: what the 16-bit rows of q leave of the exact ones (same strides; null: nothing),
+    // whether the keys have such a half too, and the factors that give the scaled operands their size back (per query
+    // row, per (batch, KV head) of the keys and of the values; null: 1)
     const void *q_low;
+    const float *q_undo, *k_undo, *v_undo;
     int32_t k_low;
 };
 
@@ -979,12 +981,17 @@ flat_list_merge_kernel(const __grid_constant__ FlatList list, const __grid_const
 // to the fragment rows with four shuffles. A 16-token block no row of the warp may see costs no MMA.
 // Additive masks are read where the scores are, and their scores stay in the natural domain (a row whose mask
 // is the type's lowest value throughout is a uniform average; times log2(e) that value would be -inf). These calls
-// ran in fp32 before, so P is a pair (its 16-bit rounding and what that leaves) and meets V in two MMAs.
+// ran in fp32 before, so P is a pair (its 16-bit rounding and what that leaves) and meets V in two MMAs. f16 pairs are carried
+// 2^10 up, clear of subnormals, and FOLD adds a step's tokens to the running sums by fp32 instructions: the MMA's own
+// accumulation rounds towards zero, and errors against 64-bit sums grew with the number of keys, by 0.02 % for f16
+// outputs at 30 000 (for bf16, whose store is eight times coarser, by 0.0006 % at 16 000: no fold there, it costs a fifth
+// of the time at D 256).
 // Six 512-token chunks of the Gemma-3-1B shape (4 x 4 heads, D 256, five rings of 512 and a global layer): 20.4 ms
 // on the general kernel, 0.407 ms here (0.487 with one 16-token block at a time).
 //
-// PAIRS (T bf16) takes q, K and V as pairs of bf16 arrays, high and low halves of fp32 values: products of
-// sixteen significant bits over the whole fp32 range (hi hi + lo hi + hi lo), for rows that are decoded from codes.
+// PAIRS takes q, K and V as pairs of arrays, high and low halves of fp32 values that were brought into the range of f16
+// by powers of two: products of 22 significant bits (hi hi + lo hi + hi lo; the small ones are summed apart), for rows
+// that are decoded from codes. T: f16, or bf16 for raw bf16 keys and their queries, which are exact as they are.
 // ---------------------------------------------------------------------
 
 // Bits of 32 mask bytes starting at p (any alignment), the first n of them inside the row.
@@ -1024,6 +1031,9 @@ template <typename T, int D, int NSTAGE, bool MASKED, bool PAIRS>
 __global__ void __launch_bounds__(DEC_THREADS, (D <= 128 ? 2 : 1))
 attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMaps, ChunkMaps> maps, const DecodeParams p) {
     constexpr bool P_PAIR = MASKED || PAIRS;
+    using VT = std::conditional_t<PAIRS, __half, T>;               // values and probabilities
+    constexpr bool FOLD = P_PAIR && std::is_same_v<VT, __half>;
+    constexpr float P_UP = P_PAIR && std::is_same_v<VT, __half> ? 1024.f : 1.f;
     constexpr int TILE_BYTES = TILE_T * D * 2;
     constexpr int BOXES = D / 64;
     constexpr int KSTEPS = D / 16;
@@ -1082,7 +1092,12 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
     // scores: log2 domain, or natural (log2_unit turns differences into log2) where values of a mask are added
     const bool bits_mask = MASKED && p.mask.dtype == KVC_BOOL && p.mask.st == 1;
     const float log2_unit = MASKED && !bits_mask ? 1.4426950408889634f : 1.f;
-    const float score_scale = MASKED && !bits_mask ? p.scale_log2 * 0.6931471805599453f : p.scale_log2;
+    float score_scale = MASKED && !bits_mask ? p.scale_log2 * 0.6931471805599453f : p.scale_log2;
+    float out_scale = 1.f / P_UP;
+    if constexpr (PAIRS) {
+        if (p.k_undo) score_scale *= p.k_undo[b * p.Hkv + hk];
+        out_scale *= p.v_undo[b * p.Hkv + hk];
+    }
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     float o_acc[NT_O][4];
 #pragma unroll
@@ -1128,6 +1143,14 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
         for (int o = 4; o <= 16; o <<= 1) {
             lim_max = max(lim_max, __shfl_xor_sync(0xffffffffu, lim_max, o));
             lim_min = min(lim_min, __shfl_xor_sync(0xffffffffu, lim_min, o));
+        }
+        float row_scale[2] = {score_scale, score_scale};
+        if (PAIRS && p.q_undo) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int r = min(r_warp + g + 8 * half, R - 1);
+                row_scale[half] *= p.q_undo[((int64_t)b * p.Hq + hk * rep + r / p.L) * p.L + r % p.L];
+            }
         }
         auto load_q = [&](const void *q, int ks, uint32_t (&f)[4]) {
             const int bx = ks / 4, ps = (ks >> 1) & 1, h = ks & 1;
@@ -1207,38 +1230,49 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
                 if (t_blk > lim_max) break;  // warp-uniform: nothing further in this tile is visible
                 if (MASKED && !((live >> blk) & ((1u << NBK) - 1u))) continue;
                 const uint32_t boff = blk * 16 * 128;
-                float sc[2 * NBK][4];
+                float sc[2 * NBK][4], rest[PAIRS ? 2 * NBK : 1][4];      // rest: the products with a low half
 #pragma unroll
-                for (int j = 0; j < 2 * NBK; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
-#pragma unroll
+                for (int j = 0; j < 2 * NBK; ++j) {
+                    sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
+                    if constexpr (PAIRS) rest[j][0] = rest[j][1] = rest[j][2] = rest[j][3] = 0.f;
+                }
+#pragma unroll(PAIRS ? 1 : BOXES)
                 for (int bx = 0; bx < BOXES; ++bx) {
 #pragma unroll
                     for (int ps = 0; ps < 2; ++ps) {
                         const int ks = bx * 4 + ps * 2;
                         const unsigned char *kp = kt + bx * BOX_BYTES + boff + k_off[ps];
-                        auto score = [&](const uint32_t (&f0)[4], const uint32_t (&f1)[4], const unsigned char *rows) {
+                        auto score = [&](float (&d)[2 * NBK][4], const uint32_t (&f0)[4], const uint32_t (&f1)[4], const unsigned char *rows) {
                             uint4 x[2 * NBK];
 #pragma unroll
                             for (int j = 0; j < 2 * NBK; ++j) x[j] = *(const uint4 *)(rows + j * 8 * 128);
 #pragma unroll
-                            for (int j = 0; j < 2 * NBK; ++j) MmaType<T>::mma(sc[j], f0, x[j].x, x[j].y);
+                            for (int j = 0; j < 2 * NBK; ++j) MmaType<T>::mma(d[j], f0, x[j].x, x[j].y);
 #pragma unroll
-                            for (int j = 0; j < 2 * NBK; ++j) MmaType<T>::mma(sc[j], f1, x[j].z, x[j].w);
+                            for (int j = 0; j < 2 * NBK; ++j) MmaType<T>::mma(d[j], f1, x[j].z, x[j].w);
                         };
                         if constexpr (Q_SHARED) {
                             const uint4 a0 = qh[ks * 32], a1 = qh[ks * 32 + 32];
                             const uint32_t f0[4] = {a0.x, a0.y, a0.z, a0.w}, f1[4] = {a1.x, a1.y, a1.z, a1.w};
-                            score(f0, f1, kp);
-                            if (PAIRS && p.k_low) score(f0, f1, kp + 2 * TILE_BYTES);
-                            if (PAIRS && p.q_low) {
-                                const uint4 b0 = ql[ks * 32], b1 = ql[ks * 32 + 32];
-                                const uint32_t e0[4] = {b0.x, b0.y, b0.z, b0.w}, e1[4] = {b1.x, b1.y, b1.z, b1.w};
-                                score(e0, e1, kp);
+                            score(sc, f0, f1, kp);
+                            if constexpr (PAIRS) {
+                                if (p.k_low) score(rest, f0, f1, kp + 2 * TILE_BYTES);
+                                if (p.q_low) {
+                                    const uint4 b0 = ql[ks * 32], b1 = ql[ks * 32 + 32];
+                                    const uint32_t e0[4] = {b0.x, b0.y, b0.z, b0.w}, e1[4] = {b1.x, b1.y, b1.z, b1.w};
+                                    score(rest, e0, e1, kp);
+                                }
                             }
                         } else {
-                            score(qa[ks], qa[ks + 1], kp);
+                            score(sc, qa[ks], qa[ks + 1], kp);
                         }
                     }
+                }
+                if constexpr (PAIRS) {
+#pragma unroll
+                    for (int j = 0; j < 2 * NBK; ++j)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) sc[j][e] += rest[j][e];
                 }
                 const bool edge = t_blk + 16 * NBK - 1 > lim_min;  // warp-uniform
 #pragma unroll
@@ -1249,7 +1283,7 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             const int half = e >> 1;
-                            float v = sc[j][e] * score_scale;
+                            float v = sc[j][e] * row_scale[half];
                             const int t = t_blk + j * 8 + 2 * c + (e & 1);
                             if (MASKED) {
                                 if (bits_mask) {
@@ -1292,41 +1326,60 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int j = 2 * (u0 + u) + (i >> 1);
-                            const float x = sc[j][2 * (i & 1)], y = sc[j][2 * (i & 1) + 1];
-                            pa[u][i] = MmaType<T>::pack(x, y);
+                            const float x = sc[j][2 * (i & 1)] * P_UP, y = sc[j][2 * (i & 1) + 1] * P_UP;
+                            pa[u][i] = MmaType<VT>::pack(x, y);
                             if constexpr (P_PAIR) {
-                                const float2 hi = MmaType<T>::unpack(pa[u][i]);
-                                pl[u][i] = MmaType<T>::pack(x - hi.x, y - hi.y);
+                                const float2 hi = MmaType<VT>::unpack(pa[u][i]);
+                                pl[u][i] = MmaType<VT>::pack(x - hi.x, y - hi.y);
                             }
                         }
-                    if (__any_sync(0xffffffffu, (alpha[0] != 1.f) | (alpha[1] != 1.f))) {
+                    if constexpr (!FOLD) {
+                        if (__any_sync(0xffffffffu, (alpha[0] != 1.f) | (alpha[1] != 1.f))) {
 #pragma unroll
-                        for (int nt = 0; nt < NT_O; ++nt) {
-                            o_acc[nt][0] *= alpha[0];
-                            o_acc[nt][1] *= alpha[0];
-                            o_acc[nt][2] *= alpha[1];
-                            o_acc[nt][3] *= alpha[1];
+                            for (int nt = 0; nt < NT_O; ++nt) {
+                                o_acc[nt][0] *= alpha[0];
+                                o_acc[nt][1] *= alpha[0];
+                                o_acc[nt][2] *= alpha[1];
+                                o_acc[nt][3] *= alpha[1];
+                            }
                         }
                     }
 #pragma unroll
                     for (int bx = 0; bx < BOXES; ++bx) {
 #pragma unroll
                         for (int cp = 0; cp < 4; ++cp) {
+                            const int nt = bx * 8 + 2 * cp;
+                            uint32_t vf[4];
+                            if constexpr (FOLD) {
+                                float part[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};   // this step's tokens
 #pragma unroll
-                            for (int u = 0; u < SMX; ++u) {
-                                const uint32_t va = vt_addr + bx * BOX_BYTES + boff + (u0 + u) * 16 * 128 + v_off[cp];
-                                uint32_t vf[4];
-                                ldmatrix_x4_trans(vf, va);
-                                MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pa[u], vf[0], vf[1]);
-                                MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa[u], vf[2], vf[3]);
-                                if constexpr (P_PAIR) {
-                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pl[u], vf[0], vf[1]);
-                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pl[u], vf[2], vf[3]);
+                                for (int u = 0; u < SMX; ++u) {
+                                    const uint32_t va = vt_addr + bx * BOX_BYTES + boff + (u0 + u) * 16 * 128 + v_off[cp];
+                                    if constexpr (PAIRS) {
+                                        ldmatrix_x4_trans(vf, va + 2 * TILE_BYTES);
+                                        MmaType<VT>::mma(part[0], pa[u], vf[0], vf[1]);
+                                        MmaType<VT>::mma(part[1], pa[u], vf[2], vf[3]);
+                                    }
+                                    ldmatrix_x4_trans(vf, va);
+                                    MmaType<VT>::mma(part[0], pl[u], vf[0], vf[1]);
+                                    MmaType<VT>::mma(part[1], pl[u], vf[2], vf[3]);
+                                    MmaType<VT>::mma(part[0], pa[u], vf[0], vf[1]);
+                                    MmaType<VT>::mma(part[1], pa[u], vf[2], vf[3]);
                                 }
-                                if constexpr (PAIRS) {
-                                    ldmatrix_x4_trans(vf, va + 2 * TILE_BYTES);
-                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pa[u], vf[0], vf[1]);
-                                    MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa[u], vf[2], vf[3]);
+#pragma unroll
+                                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e) o_acc[nt + i][e] = fmaf(o_acc[nt + i][e], alpha[e >> 1], part[i][e]);
+                            } else {
+#pragma unroll
+                                for (int u = 0; u < SMX; ++u) {
+                                    ldmatrix_x4_trans(vf, vt_addr + bx * BOX_BYTES + boff + (u0 + u) * 16 * 128 + v_off[cp]);
+                                    MmaType<T>::mma(o_acc[nt], pa[u], vf[0], vf[1]);
+                                    MmaType<T>::mma(o_acc[nt + 1], pa[u], vf[2], vf[3]);
+                                    if constexpr (P_PAIR) {
+                                        MmaType<T>::mma(o_acc[nt], pl[u], vf[0], vf[1]);
+                                        MmaType<T>::mma(o_acc[nt + 1], pl[u], vf[2], vf[3]);
+                                    }
                                 }
                             }
                         }
@@ -1350,7 +1403,7 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
             const int r = r_warp + g + 8 * half;
             if (r >= R) continue;
             if (p.splits == 1) {
-                const float inv = l_run[half] > 0.f ? 1.f / l_run[half] : 0.f;
+                const float inv = l_run[half] > 0.f ? out_scale / l_run[half] : 0.f;
                 const int hq = hk * rep + r / p.L, lq = r % p.L;
                 const int64_t base = b * p.o_sb + hq * p.o_sh + lq * p.o_sl;
 #pragma unroll
@@ -1363,7 +1416,7 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
 #pragma unroll
                 for (int nt = 0; nt < NT_O; ++nt)
                     __stcg((float2 *)&p.o_part[pbase * D + 8 * nt + 2 * c],
-                           make_float2(o_acc[nt][2 * half], o_acc[nt][2 * half + 1]));
+                           make_float2(o_acc[nt][2 * half] * out_scale, o_acc[nt][2 * half + 1] * out_scale));
                 if (c == 0) __stcg(&p.ml_part[pbase], make_float2(m_run[half], l_run[half]));
             }
         }
@@ -1570,7 +1623,7 @@ size_t flat_list_smem(int D, int R) {
     const int nstage = D == 64 ? 6 : 3;
     return (size_t)nstage * 2 * (TILE_T * D * 2) + 2 * nstage * sizeof(uint64_t) + 64 + FLAT_AHEAD * (2 * sizeof(uint64_t) + (size_t)R * D * 2 + sizeof(FlatWork)) + 1024;
 }
-constexpr int64_t LIST_PARTIAL_BYTES = (int64_t)64 << 20;   // of a list launch's partials
+constexpr int64_t LIST_PARTIAL_BYTES = (int64_t)32 << 20;   // of a list launch's partials
 
 bool flat_new_rows_ok(const AttnArgs &a) {
     return a.L == 1 && a.mask.mode != KVC_MASK_CAUSAL && !((uintptr_t)a.new_k & 15) && !((uintptr_t)a.new_v & 15) &&
@@ -1682,11 +1735,6 @@ int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t strea
 
 namespace {
 
-// Low halves of a call's bf16 operands (k, q: null where the high ones are exact), and the type of its output.
-struct ChunkLow {
-    const void *k, *v, *q;
-    int32_t out_dtype;
-};
 
 int launch_rows(const AttnArgs &a, const ChunkLow *low, cudaStream_t stream) {
     if (a.q_dtype != KVC_BF16 && a.q_dtype != KVC_F16) return 0;
@@ -1825,6 +1873,7 @@ int launch_rows(const AttnArgs &a, const ChunkLow *low, cudaStream_t stream) {
         p.out_dtype = low->out_dtype;
         p.q_low = low->q;
         p.k_low = low->k ? 1 : 0;
+        p.q_undo = low->q_undo; p.k_undo = low->k_undo; p.v_undo = low->v_undo;
     }
     const int units = (int)(bh * splits);
 
@@ -1840,12 +1889,18 @@ int launch_rows(const AttnArgs &a, const ChunkLow *low, cudaStream_t stream) {
                 return 0;
             pm.k = kmap; pm.v = vmap;
             // stages: two CTAs an SM up to D 128 (four 8 / 16 KB tiles a stage beside 16 / 32 KB of query fragments)
-#define KVC_CHP(DD, NS)                                                                               \
-    (masked ? launch_chunk_typed<__nv_bfloat16, DD, NS, true, true>(pm, p, ctas, stream)              \
-            : launch_chunk_typed<__nv_bfloat16, DD, NS, false, true>(pm, p, ctas, stream))
-            if (a.D == 64) KVC_CHP(64, 2);
-            else if (a.D == 128) KVC_CHP(128, 1);
-            else KVC_CHP(256, 1);
+#define KVC_CHP(TT, DD, NS)                                                               \
+    (masked ? launch_chunk_typed<TT, DD, NS, true, true>(pm, p, ctas, stream)             \
+            : launch_chunk_typed<TT, DD, NS, false, true>(pm, p, ctas, stream))
+            if (a.q_dtype == KVC_BF16) {
+                if (a.D == 64) KVC_CHP(__nv_bfloat16, 64, 2);
+                else if (a.D == 128) KVC_CHP(__nv_bfloat16, 128, 1);
+                else KVC_CHP(__nv_bfloat16, 256, 1);
+            } else {
+                if (a.D == 64) KVC_CHP(__half, 64, 2);
+                else if (a.D == 128) KVC_CHP(__half, 128, 1);
+                else KVC_CHP(__half, 256, 1);
+            }
 #undef KVC_CHP
             return 1;
         }
@@ -1886,11 +1941,7 @@ int launch_rows(const AttnArgs &a, const ChunkLow *low, cudaStream_t stream) {
 // Returns the number of kernels launched, or 0 when the call does not fit this path.
 int launch_attention_decode(const AttnArgs &a, cudaStream_t stream) { return launch_rows(a, nullptr, stream); }
 
-// A chunk over raw bf16 rows that are the high halves of exact ones (attention_chunk_rows_accepts has been asked).
-int launch_attention_chunk_pairs(const AttnArgs &a, const void *k_low, const void *v_low, const void *q_low, int32_t out_dtype,
-                                 cudaStream_t stream) {
-    const ChunkLow low = {k_low, v_low, q_low, out_dtype};
-    return launch_rows(a, &low, stream);
-}
+// A chunk over 16-bit rows that are the high halves of exact ones (attention_chunk_rows_accepts has been asked).
+int launch_attention_chunk_pairs(const AttnArgs &a, const ChunkLow &low, cudaStream_t stream) { return launch_rows(a, &low, stream); }
 
 }  // namespace kvc

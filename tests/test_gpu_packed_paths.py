@@ -562,3 +562,85 @@ def test_unmasked_chunk_takes_a_maximum_per_16_tokens(kvc, cuda, dtype, D):
     store = float((ref.float().to(dtype).double() - ref).norm())
     assert float((out.double() - ref).norm()) <= 1.01 * store          # 32 tokens a step: hypot(store, far)
     assert far > 0.3 * store
+
+
+def _rows64(oracle, state, kind, D):
+    """Keys and values that the arrays of a packed cache stand for, in 64 bits, in the basis of the callers' rows."""
+    dev = state[0].device
+
+    def unpack(w, bits):
+        return torch.from_numpy(oracle.unpack_low_bit(w.cpu().numpy().view(np.uint32), bits, D).astype(np.int64)).to(dev)
+
+    def affine(codes, scales, biases, bits):
+        s, b = (t.double().repeat_interleave(D // scales.shape[-1], -1) for t in (scales, biases))
+        return unpack(codes, bits).double() * s + b
+
+    def index(packed, norms, bits, seed):
+        h = torch.ones((1, 1), dtype=torch.float64, device=dev)
+        while h.shape[0] < D:
+            h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+        book, signs = (torch.from_numpy(a.astype(np.float64)).to(dev) for a in (oracle.codebook(D, bits), oracle.wht_signs(D, seed)))
+        return (book[unpack(packed, bits)] @ h) / D ** 0.5 * signs * norms.double().unsqueeze(-1)
+    if "group" in kind:
+        return affine(*state[:3], kind["bits"]), affine(*state[3:], kind["bits"])
+    kb, vb = kind["key_bits"], kind["value_bits"]
+    n = {0: 1, 8: 3}.get(kb, 2)
+    k = state[0].double() if kb == 0 else affine(*state[:3], 8) if kb == 8 else index(*state[:2], kb, 42)
+    return k, affine(*state[n:n + 3], vb) if kind.get("affine_values") else index(*state[n:n + 2], vb, 43)
+
+
+def _attention64(q, k, v, scale, allowed):
+    rep = q.shape[1] // k.shape[1]
+    k, v = (t.repeat_interleave(rep, 1) for t in (k, v))
+    return torch.softmax((q.double() @ k.transpose(2, 3) * scale).masked_fill(~allowed, -torch.inf), -1) @ v
+
+
+@pytest.mark.parametrize("kw,Hq,Hkv,D,P,L,gain", [
+    (dict(key_bits=4, value_bits=4, affine_values=True), 8, 2, 128, 3000, 100, 4.0),    # operand pairs
+    (dict(key_bits=8, value_bits=4), 8, 2, 128, 3000, 100, 4.0),
+    (dict(key_bits=0, value_bits=4), 8, 2, 128, 3000, 100, 1.0),
+    (dict(bits=4, group=64), 4, 1, 256, 3000, 100, 1.0),
+    (dict(key_bits=3, value_bits=4), 4, 1, 256, 3000, 100, 1.0),
+    (dict(key_bits=3, value_bits=3), 4, 4, 64, 500, 20, 1.0),
+])
+@pytest.mark.parametrize("size", [1.0, 2.0 ** -10])
+def test_chunks_on_operand_pairs_keep_single_precision(kvc, oracle, cuda, kw, Hq, Hkv, D, P, L, gain, size):
+    """f16 callers, one key channel in a hundred 20 times larger, and the same data a thousand times smaller: against
+    64-bit sums the outputs err by the store's rounding `ideal` and no more. 1.0005 * ideal leaves the arithmetic 0.03 *
+    ideal (errors add in quadrature), 2^-17 of the result, which is what single precision needs for scores near 50;
+    products of pairs of bf16 took 1.0034 .. 1.011."""
+    make = (lambda: kvc.QuantizedKVCache(kw["group"], kw["bits"])) if "group" in kw else \
+        (lambda: kvc.TurboQuantKVCache(bits=max(kw["key_bits"], kw["value_bits"]), **kw))
+    c = make()
+    g = torch.ones(D)
+    g[torch.randperm(D, generator=torch.Generator().manual_seed(3))[:max(1, D // 100)]] = 20.0
+    k, v, k1, v1, q = (seeded((2, h, n, D), s) for s, (h, n) in enumerate(((Hkv, P), (Hkv, P), (Hkv, L), (Hkv, L), (Hq, L))))
+    k, v, k1, v1, q = (t.half().to(cuda) for t in (k * g * size, v * size, k1 * g * size, v1 * size, q * gain))
+    (c.update_quantized if "group" in kw else c.encode_new_token)(k, v)
+    out = c.attention(q, k1, v1, D ** -0.5 / size, "causal")
+    K, V = _rows64(oracle, c.state, kw, D)
+    ref = _attention64(q, K, V, D ** -0.5 / size, torch.arange(P + L, device=cuda) <= torch.arange(P, P + L, device=cuda)[:, None])
+    ideal = float((ref.half().double() - ref).norm())
+    assert float((out.double() - ref).norm()) <= 1.0005 * ideal
+
+
+def test_small_probabilities_under_an_array_mask(kvc, cuda):
+    """16 000 keys at probabilities around 2^-26 beside one near 1 whose value row is zero: together they are the output.
+    f16 probabilities as they are would be zero there."""
+    B, H, D, P, L = 1, 2, 128, 16000, 4
+    u = seeded((1, 1, 1, D), 1)
+    u = u / u.norm()
+    k = (seeded((B, H, P + L, D), 2) * 0.02).half()
+    k[:, :, 7] = (u * 8.0).half()
+    v = (1.0 + 0.1 * seeded((B, H, P + L, D), 3)).half()
+    v[:, :, 7] = 0.0
+    q = (u * 2.25).expand(B, H, L, D).half().to(cuda)          # score of key 7: 18 nats, 26 powers of two
+    k, v = k.to(cuda), v.to(cuda)
+    c = kvc.KVCacheSimple()
+    c.update(k[:, :, :P], v[:, :, :P])
+    m = torch.arange(P + L, device=cuda) <= torch.arange(P, P + L, device=cuda)[:, None]
+    out = c.attention(q, k[:, :, P:], v[:, :, P:], 1.0, m)
+    ref = _attention64(q, k.double(), v.double(), 1.0, m)
+    # outputs around 2^-12, a subnormal of f16 begins at 2^-14: the store rounds to 2^-23 at most
+    assert float((out.double() - ref).abs().max()) <= 2.0 ** -23 * 1.01
+    assert float(ref.min()) > 2.0 ** -13
