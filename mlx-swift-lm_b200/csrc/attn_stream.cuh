@@ -12,8 +12,8 @@
 // group of up to eight rows costs half the MMAs and accumulators of the row-major orientation.
 //   * Keys go from the packed words into A fragments in registers: the order of the head dims inside an MMA
 //     is free as long as the query fragments use the same one, so lane (g, c) reads a contiguous piece of rows
-//     g and g + 8. Affine codes enter as exact integers and the scale / bias of a group is applied to the
-//     group's fp32 score (s * (q . c) + b * sum q); index keys enter as centroids (pair lookups in a table
+//     g and g + 8. Affine codes enter as exact integers around zero and the scale / bias of a group is applied to the
+//     group's fp32 score (s * (q . (c - m)) + (b + m s) * sum q); index keys enter as centroids (pair lookups in a table
 //     replicated per lane, no bank conflicts) and the row norm multiplies the fp32 score.
 //   * Values are unpacked 64 dims at a time into a private [16][64] f16 tile (16-byte chunks swizzled by the
 //     token) and read back transposed with ldmatrix. The row norm / group scale goes into P in fp32, the affine
@@ -174,18 +174,24 @@ __device__ __forceinline__ uint32_t pair_offset(const uint32_t (&w)[NW], int j, 
     return (x & MASK) | lane_bits;
 }
 
-// Two codes as one f16 pair whose BITS are the codes: the subnormals n * 2^-24, exact operands of the MMA (and
-// n * 2^-20 for the upper nibble of a byte), one logic operation or byte permute each. 4-bit words give the dims
-// (i, i + 4), i odd from the upper nibbles; 8-bit words (0, 1) and (2, 3).
+// Two codes n as the f16 pair n - 8 or n - 128, exact: 1024 + n (+ 16 n for the upper nibble of a byte) by one logic
+// operation or byte permute, then one f16 addition or fma. 4-bit words give the dims (i, i + 4), i odd from the upper
+// nibbles; 8-bit words (0, 1) and (2, 3). Codes left as the subnormals n * 2^-24 save the second instruction, but the
+// MMA aligns its products by their operands' exponents and cut the small ones short: with 4-bit values and 4 000 .. 8 000
+// keys f16 outputs erred by 0.06 .. 0.11 % more than those of the general kernel. Around zero, the codes' part of a sum
+// is no larger than the sum.
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, float b, float c) {
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), __float2half2_rn(b), __float2half2_rn(c));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
 __device__ __forceinline__ uint32_t code4(uint32_t w, int i) {
-    return ((i & 2) ? w >> 8 : w) & ((i & 1) ? 0x00F000F0u : 0x000F000Fu);
+    const uint32_t x = (((i & 2) ? w >> 8 : w) & ((i & 1) ? 0x00F000F0u : 0x000F000Fu)) | 0x64006400u;
+    return (i & 1) ? h2_fma(x, 0.0625f, -72.f) : h2_fma(x, 1.f, -1032.f);
 }
-__device__ __forceinline__ uint32_t code8(uint32_t w, int i) { return __byte_perm(w, 0u, i ? 0x4342 : 0x4140); }
-// dim within its chunk of eight that column j of an unpacked chunk holds, and the weight of that column's codes
+__device__ __forceinline__ uint32_t code8(uint32_t w, int i) { return h2_fma(__byte_perm(w, 0x64646464u, i ? 0x4342 : 0x4140), 1.f, -1152.f); }
+template <int KIND> constexpr float code_middle() { return KIND == SK_A4 ? 8.f : 128.f; }
+// dim within its chunk of eight that column j of an unpacked chunk holds
 template <int KIND> __device__ __forceinline__ constexpr int chunk_dim(int j) { return KIND == SK_A4 ? (j & 1) * 4 + (j >> 1) : j; }
-template <int KIND> __device__ __forceinline__ float code_unit(int j) {
-    return KIND == SK_A4 && (j & 2) ? 1048576.f : 16777216.f;
-}
 
 template <typename T> __device__ __forceinline__ float ld16(uint32_t a) {
     uint16_t r;
@@ -477,9 +483,8 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                     } else {
                         for (int j = 0; j < 4; ++j) e[j] = base + 4 * s + j;
                     }
-                    const float up = KK == SK_A4 ? 0.0625f : 1.f;     // upper nibbles weigh 16 times a lower one
                     qb[nb][0][u * UK + s][0] = MmaType<KT>::pack(qr[e[0]], qr[e[1]]);
-                    qb[nb][0][u * UK + s][1] = MmaType<KT>::pack(qr[e[2]] * up, qr[e[3]] * up);
+                    qb[nb][0][u * UK + s][1] = MmaType<KT>::pack(qr[e[2]], qr[e[3]]);
                     if constexpr (QP == 2) {
                         qb[nb][1][u * UK + s][0] = low_half2(qb[nb][0][u * UK + s][0], qr[e[0]], qr[e[1]]);
                         qb[nb][1][u * UK + s][1] = low_half2(qb[nb][0][u * UK + s][1], qr[e[2]], qr[e[3]]);
@@ -537,15 +542,21 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
             const int t0 = t_lo + blk * 16;
 
             // ---- scores: s[nb] = {(g, 2c), (g, 2c + 1), (g + 8, 2c), (g + 8, 2c + 1)} of (token, row), log2 domain ----
-            float s[NB][4];
+            // A chain of MMAs rounds towards zero at every step: raw rows take two short chains, index keys one for the
+            // high halves and one (s2) for the small products.
+            float s[NB][4], s2[NB][4];
 #pragma unroll
-            for (int nb = 0; nb < NB; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+            for (int nb = 0; nb < NB; ++nb) {
+                s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+                s2[nb][0] = s2[nb][1] = s2[nb][2] = s2[nb][3] = 0.f;
+            }
             auto mma_k = [&](float (&d)[NB][4], int ks, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
                 const uint32_t a[4] = {a0, a1, a2, a3};
 #pragma unroll
-                for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                    for (int i = 0; i < QP; ++i) MmaType<KT>::mma(d[nb], a, qb[nb][i][ks][0], qb[nb][i][ks][1]);
+                for (int nb = 0; nb < NB; ++nb) {
+                    MmaType<KT>::mma(d[nb], a, qb[nb][0][ks][0], qb[nb][0][ks][1]);
+                    if constexpr (QP == 2) MmaType<KT>::mma(s2[nb], a, qb[nb][1][ks][0], qb[nb][1][ks][1]);
+                }
             };
             if constexpr (K::RAW) {
 #pragma unroll
@@ -554,8 +565,12 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                     const uint4 x0 = lds128(kst + ((g * K::CH + (ch ^ key_xor<KK, D, UNIT>(g))) << 4));
                     const uint4 x1 = lds128(kst + (((g + 8) * K::CH + (ch ^ key_xor<KK, D, UNIT>(g + 8))) << 4));
                     mma_k(s, 2 * u, x0.x, x1.x, x0.y, x1.y);
-                    mma_k(s, 2 * u + 1, x0.z, x1.z, x0.w, x1.w);
+                    mma_k(s2, 2 * u + 1, x0.z, x1.z, x0.w, x1.w);
                 }
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[nb][e] += s2[nb][e];
             } else if constexpr (K::AFFINE) {
                 constexpr int PB = KU / 4 * K::BITS / 8;      // bytes of a lane's piece: 4, 8 or 16
                 constexpr int PW = PB / 4;
@@ -585,7 +600,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const uint32_t ad = kst + K::BLOCK + ((g + 8 * i) * p.groups_k + gr) * 2;
-                        const float sc = ld16<T>(ad) * 16777216.f, bb = ld16<T>(ad + K::SIDE);
+                        const float sc = ld16<T>(ad), bb = fmaf(sc, code_middle<KK>(), ld16<T>(ad + K::SIDE));
 #pragma unroll
                         for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -627,8 +642,12 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                     mma_k(s, q, lds32(o0), lds32(o1), lds32(o2), lds32(o3));
                     const uint32_t lo[4] = {lds32(o0 + K::TABLE), lds32(o1 + K::TABLE), lds32(o2 + K::TABLE), lds32(o3 + K::TABLE)};
 #pragma unroll
-                    for (int nb = 0; nb < NB; ++nb) MmaType<KT>::mma(s[nb], lo, qb[nb][0][q][0], qb[nb][0][q][1]);
+                    for (int nb = 0; nb < NB; ++nb) MmaType<KT>::mma(s2[nb], lo, qb[nb][0][q][0], qb[nb][0][q][1]);
                 }
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[nb][e] += s2[nb][e];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const float f = __uint_as_float(lds32(kst + K::BLOCK + (g + 8 * i) * 4));
@@ -761,7 +780,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                             const int u = (ps * 64 + mt * 16) / UNIT, gr = (u * p.groups_v) / NG;
                             const uint32_t a0 = vst + V::BLOCK + V::SIDE + (g * p.groups_v + gr) * 2, a1 = a0 + 16 * p.groups_v;
                             pack_p(vf[0][u], vf[1][u]);
-                            const float b0 = ld16<T>(a0), b1 = ld16<T>(a1);
+                            const float b0 = fmaf(vf[0][u], code_middle<VK>(), ld16<T>(a0)), b1 = fmaf(vf[1][u], code_middle<VK>(), ld16<T>(a1));
 #pragma unroll
                             for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -796,8 +815,8 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
         float *red_ml = red_o + ST_WARPS * rr_n * SH::RED_STRIDE;
         float *work = red_ml + ST_WARPS * rr_n * 2;
         __syncthreads();        // every warp has left the ring that the merge buffers overlay
-        // lane g holds columns g of the chunks of eight: its dim and the weight of its codes
-        const float undo = (V::AFFINE ? code_unit<VK>(g) : p.vcb_undo) / ST_PSCALE;
+        const float undo = (V::AFFINE ? 1.f : p.vcb_undo) / ST_PSCALE;
+        // lane g holds columns g of the chunks of eight: its dim
         const int gd = chunk_dim<VK>(g);
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb)

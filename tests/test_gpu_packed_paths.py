@@ -644,3 +644,31 @@ def test_small_probabilities_under_an_array_mask(kvc, cuda):
     # outputs around 2^-12, a subnormal of f16 begins at 2^-14: the store rounds to 2^-23 at most
     assert float((out.double() - ref).abs().max()) <= 2.0 ** -23 * 1.01
     assert float(ref.min()) > 2.0 ** -13
+
+
+@pytest.mark.parametrize("kw,Hq,Hkv,D,L", [
+    (dict(key_bits=4, value_bits=4, affine_values=True), 8, 2, 128, 1),
+    (dict(key_bits=4, value_bits=4, affine_values=True), 8, 2, 128, 4),     # two column blocks
+    (dict(bits=4, group=64), 4, 1, 256, 1),
+    (dict(bits=4, group=32), 4, 1, 256, 4),
+    (dict(bits=8, group=64), 4, 1, 256, 1),
+    (dict(key_bits=8, value_bits=4), 8, 2, 64, 1),
+    (dict(key_bits=3, value_bits=4, affine_values=True), 8, 2, 64, 4),
+])
+def test_stream_kernel_keeps_single_precision_over_affine_codes(kvc, oracle, cuda, kw, Hq, Hkv, D, L):
+    """f16 callers over 8 000 keys, where outputs are small beside the values: against 64-bit sums they err by the store's
+    rounding `ideal` alone. 1.0003 * ideal leaves the arithmetic 0.025 * ideal; codes that entered the MMA as subnormals
+    took 1.0006 .. 1.0011 (4 bits)."""
+    P = 8000
+    c = kvc.QuantizedKVCache(kw["group"], kw["bits"]) if "group" in kw else \
+        kvc.TurboQuantKVCache(bits=max(kw["key_bits"], kw["value_bits"]), **kw)
+    g = torch.ones(D)
+    g[torch.randperm(D, generator=torch.Generator().manual_seed(3))[:max(1, D // 100)]] = 20.0
+    k, v, k1, v1, q = (seeded((4, h, n, D), s) for s, (h, n) in enumerate(((Hkv, P), (Hkv, P), (Hkv, L), (Hkv, L), (Hq, L))))
+    k, v, k1, v1, q = (t.half().to(cuda) for t in (k * g, v, k1 * g, v1, q))
+    (c.update_quantized if "group" in kw else c.encode_new_token)(k, v)
+    out = c.attention(q, k1, v1, D ** -0.5, "causal" if L > 1 else "none")
+    K, V = _rows64(oracle, c.state, kw, D)
+    ref = _attention64(q, K, V, D ** -0.5, torch.arange(P + L, device=cuda) <= torch.arange(P, P + L, device=cuda)[:, None])
+    ideal = float((ref.half().double() - ref).norm())
+    assert float((out.double() - ref).norm()) <= 1.0003 * ideal
