@@ -1134,6 +1134,14 @@ static void turbo_compressed_attention(kvc_cache *c, const kvc_tensor &q, const 
     launch_attention(turbo_attn_args(c, q, k, scale, mask_mode, mask, out), s);
 }
 
+static bool fused_append_off() {
+    static const bool off = [] {
+        const char *e = std::getenv("KVC_FUSED_APPEND");
+        return e && e[0] == '0';
+    }();
+    return off;
+}
+
 void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v,
                      float scale, int32_t mask_mode, const kvc_tensor *mask, const kvc_tensor &out,
                      cudaStream_t s) {
@@ -1174,10 +1182,7 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
         default: {
             // Decode on a KVCacheSimple: the attention kernel appends the new row itself when it can
             // (one launch per layer); otherwise the append runs first as its own launch.
-            static const bool fuse_off = [] {
-                const char *e = std::getenv("KVC_FUSED_APPEND");
-                return e && e[0] == '0';
-            }();
+            const bool fuse_off = fused_append_off();
             if (!fuse_off && c->cfg.kind == KVC_KIND_SIMPLE && k.shape[2] == 1 && q.shape[2] == 1 && !c->open_round &&
                 mask_mode != KVC_MASK_ARRAY && k.stride[3] == 1 && v.stride[3] == 1 &&
                 (k.dtype == KVC_BF16 || k.dtype == KVC_F16)) {
@@ -1277,14 +1282,15 @@ enum class ListKind { none, raw, quantized, turbo };
 // append and the attention of the new rows.
 ListKind list_kind(const kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v, const kvc_tensor &out,
                    int32_t mask_mode) {
-    if (!c || c->open_round || mask_mode == KVC_MASK_ARRAY) return ListKind::none;
+    if (!c || c->open_round || (mask_mode != KVC_MASK_NONE && mask_mode != KVC_MASK_CAUSAL)) return ListKind::none;
     if (!plain4(q) || !plain4(k) || !plain4(v) || !plain4(out) || q.shape[2] != k.shape[2]) return ListKind::none;
     if (q.dtype != k.dtype || k.dtype != v.dtype || out.dtype != q.dtype || k.shape[1] < 1 || q.shape[1] % k.shape[1]) return ListKind::none;
     for (int i = 0; i < 4; ++i)
         if (q.shape[i] != out.shape[i] || (i != 1 && i != 2 && k.shape[i] != q.shape[i]) || k.shape[i] != v.shape[i]) return ListKind::none;
     switch (c->cfg.kind) {
         case KVC_KIND_SIMPLE:
-        case KVC_KIND_ROTATING: return k.shape[2] == 1 && (k.dtype == KVC_BF16 || k.dtype == KVC_F16) ? ListKind::raw : ListKind::none;
+        case KVC_KIND_ROTATING:
+            return !fused_append_off() && k.shape[2] == 1 && (k.dtype == KVC_BF16 || k.dtype == KVC_F16) ? ListKind::raw : ListKind::none;
         case KVC_KIND_QUANTIZED: return ListKind::quantized;
         case KVC_KIND_TURBO: return c->compressed ? ListKind::turbo : ListKind::none;
         default: return ListKind::none;

@@ -501,3 +501,20 @@ def test_batch_that_names_a_cache_again(kvc, cuda, order, ring, P, D):
     for a, b in zip(caches, alone):
         assert a.offset == b.offset and all(torch.equal(s, t) for s, t in zip(a.state, b.state))
     assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["raw", "affine"])
+def test_batch_refuses_and_is_told_what_a_call_alone_is(kvc, cuda, kind):
+    """A mask mode nobody knows is refused by calls that would share a launch as it is by one alone."""
+    def caches(n):
+        made = [kvc.KVCacheSimple() if kind == "raw" else kvc.QuantizedKVCache(64, 4) for _ in range(n)]
+        for c in made:
+            (c.update if kind == "raw" else c.update_quantized)(*(seeded((1, 2, 40, 128), j, torch.float16).to(cuda) for j in (1, 2)))
+        return made
+    t = [seeded((1, 4, 1, 128), 3, torch.float16).to(cuda)] + [seeded((1, 2, 1, 128), 4 + j, torch.float16).to(cuda) for j in (0, 1)]
+    statuses = []
+    for n in (1, 3):
+        made = caches(n)
+        step = kvc.DecodeStep(made, [t[0]] * n, [t[1]] * n, [t[2]] * n, [torch.empty_like(t[0]) for _ in range(n)], 0.1)
+        statuses.append(kvc.lib().kvc_attention_batch(step.handles, n, step.q, step.k, step.v, step.scale, 77, step.o, None, 0, 1))
+    assert statuses[0] == statuses[1] and (kind == "raw" or statuses[0] != 0)
