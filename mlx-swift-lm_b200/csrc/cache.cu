@@ -1392,11 +1392,14 @@ void list_launch(ListKind kind, std::vector<ListedCall> &calls, cudaStream_t s) 
     for (auto &l : calls) slots = slots && l.slot >= 0 && l.slot < l.attn.T;
     if (slots && launch_attention_list(args.data(), n, s) > 0) return;
     for (auto &l : calls) {
+        // growth copies and ring rebuilds of all calls were enqueued before the first of these launches
+        l.attn.stored_rows_settled = &l != &calls.front();
         if (launch_decode_or_zero(l.attn, l.slot, s) > 0) continue;
         append_pair(l.cache->k, l.cache->v, *l.k, *l.v, l.slot, s);
         AttnArgs a = l.attn;
         a.new_k = a.new_v = nullptr;
         a.new_slot = -1;
+        a.stored_rows_settled = false;
         launch_attention(a, s);
     }
 }

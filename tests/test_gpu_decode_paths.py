@@ -503,6 +503,26 @@ def test_batch_that_names_a_cache_again(kvc, cuda, order, ring, P, D):
     assert kvc.lib().kvc_device_status() == 0
 
 
+def test_batched_calls_that_do_not_fit_one_launch(kvc, cuda):
+    """A run of one kind with two head dims is made call by call: the same bits as alone."""
+    dims = [128, 64, 128, 64, 128]
+    caches = [kvc.KVCacheSimple(reserve_tokens=256) for _ in dims]
+    for i, (c, D) in enumerate(zip(caches, dims)):
+        c.update(*(seeded((2, 2, 130, D), 10 * i + j, torch.bfloat16).to(cuda) for j in (1, 2)))
+    alone = [c.copy() for c in caches]
+    for turn in range(8):
+        q, k, v = ([seeded((2, h, 1, D), 50 * turn + s + i, torch.bfloat16).to(cuda) for i, D in enumerate(dims)]
+                   for h, s in ((8, 100), (2, 200), (2, 300)))
+        outs = [torch.empty_like(t) for t in q]
+        kvc.DecodeStep(caches, q, k, v, outs, 0.1).run()
+        torch.cuda.synchronize()
+        for i, c in enumerate(alone):
+            assert torch.equal(outs[i], c.attention(q[i], k[i], v[i], 0.1)), (turn, i)
+            torch.cuda.synchronize()
+    for a, b in zip(caches, alone):
+        assert all(torch.equal(s, t) for s, t in zip(a.state, b.state))
+
+
 @pytest.mark.parametrize("kind", ["raw", "affine"])
 def test_batch_refuses_and_is_told_what_a_call_alone_is(kvc, cuda, kind):
     """A mask mode nobody knows is refused by calls that would share a launch as it is by one alone."""
