@@ -1266,6 +1266,7 @@ struct Span {
         lo = (uintptr_t)t.data;
         hi = lo + (uintptr_t)std::max<int64_t>(last, 0) * dtype_size(t.dtype);
     }
+    explicit Span(const Array4 &a) : lo((uintptr_t)a.ptr), hi((uintptr_t)a.ptr + a.bytes()) {}
     bool meets(const Span &o) const { return lo < o.hi && o.lo < hi; }
 };
 
@@ -1406,12 +1407,45 @@ void list_launch(ListKind kind, std::vector<ListedCall> &calls, cudaStream_t s) 
 
 }  // namespace
 
+// The arrays of the caches of a batch that some tensor of the batch may lie in (a view of cached rows given as new
+// ones): usually none, since callers' tensors come from elsewhere.
+struct NamedRows {
+    const kvc_cache *cache;
+    Span span;
+};
+static std::vector<NamedRows> rows_named_by(kvc_cache *const *caches, int n, const kvc_tensor *const (&tensors)[4]) {
+    uintptr_t lo = UINTPTR_MAX, hi = 0;
+    for (const kvc_tensor *t : tensors)
+        for (int i = 0; i < n; ++i) {
+            if (t[i].ndim < 1 || t[i].ndim > 4 || !t[i].data || !is_float_dtype(t[i].dtype)) continue;    // refused by its call
+            const Span sp(t[i]);
+            lo = std::min(lo, sp.lo);
+            hi = std::max(hi, sp.hi);
+        }
+    std::vector<NamedRows> out;
+    for (int i = 0; i < n; ++i) {
+        const kvc_cache *c = caches[i];
+        for (const Array4 *a : {&c->k, &c->v, &c->k_alt, &c->v_alt, &c->kq, &c->ks, &c->kb, &c->vq, &c->vs, &c->vb, &c->kp, &c->kn, &c->vp, &c->vn})
+            if (a->allocated() && (uintptr_t)a->ptr < hi && (uintptr_t)a->ptr + a->bytes() > lo) out.push_back({c, Span(*a)});
+    }
+    return out;
+}
+
 // What kvc_attention on each cache in turn would compute, in as few launches as the calls allow: consecutive
-// calls of one kind on different caches whose outputs feed no other call of the run are prepared together
-// (their order does not matter then). Everything else is made one by one.
+// calls of one kind on different caches, whose outputs feed no other call of the run and whose tensors lie in no
+// other call's cache, are prepared together (their order does not matter then). Everything else is made one by one.
 void cache_attention_batch(kvc_cache *const *caches, int n, const kvc_tensor *q, const kvc_tensor *k, const kvc_tensor *v, float scale,
                            int32_t mask_mode, const kvc_tensor *outs, cudaStream_t s) {
     struct HintReset { ~HintReset() { set_batch_previous(nullptr, 0); } } hint_reset;
+    const kvc_tensor *const tensors[4] = {q, k, v, outs};
+    const std::vector<NamedRows> named = rows_named_by(caches, n, tensors);
+    auto reads_cache_of = [&](int call, int other) {
+        for (const NamedRows &r : named)
+            if (r.cache == caches[other])
+                for (const kvc_tensor *t : tensors)
+                    if (r.span.meets(Span(t[call]))) return true;
+        return false;
+    };
     int last = 0, last_n = 0;     // the calls of the launch before: a list covers all of its caches
     for (int from = 0; from < n;) {
         const ListKind kind = list_kind(caches[from], q[from], k[from], v[from], outs[from], mask_mode);
@@ -1429,6 +1463,7 @@ void cache_attention_batch(kvc_cache *const *caches, int n, const kvc_tensor *q,
                 }
                 for (int i = from; i < to && apart; ++i)      // nor may it overwrite what an earlier call still reads
                     apart = !o.meets(Span(q[i])) && !o.meets(Span(k[i])) && !o.meets(Span(v[i]));
+                for (int i = from; i < to && apart && !named.empty(); ++i) apart = !reads_cache_of(to, i) && !reads_cache_of(i, to);
                 if (!apart) break;
                 written.push_back(o);
             }

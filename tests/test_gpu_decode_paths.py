@@ -538,3 +538,29 @@ def test_batch_refuses_and_is_told_what_a_call_alone_is(kvc, cuda, kind):
         step = kvc.DecodeStep(made, [t[0]] * n, [t[1]] * n, [t[2]] * n, [torch.empty_like(t[0]) for _ in range(n)], 0.1)
         statuses.append(kvc.lib().kvc_attention_batch(step.handles, n, step.q, step.k, step.v, step.scale, 77, step.o, None, 0, 1))
     assert statuses[0] == statuses[1] and (kind == "raw" or statuses[0] != 0)
+
+
+def test_batched_call_whose_new_rows_are_views_of_another_cache(kvc, cuda):
+    """Call 1 is given, as its new rows, the row that call 0 appends (a view of that cache); call 2's rows lie in a cache
+    that call 3 appends to. In turn, each call sees what the ones before it have written, and nothing of those after."""
+    B, Hq, Hkv, D, P = 1, 4, 2, 128, 100
+
+    def run(batched):
+        caches = [kvc.KVCacheSimple(reserve_tokens=256) for _ in range(4)]
+        for i, c in enumerate(caches):
+            c.update(*(seeded((B, Hkv, P, D), 10 * i + j, torch.bfloat16).to(cuda) for j in (1, 2)))
+        q = [seeded((B, Hq, 1, D), 50 + i, torch.bfloat16).to(cuda) for i in range(4)]
+        k, v = ([seeded((B, Hkv, 1, D), s + i, torch.bfloat16).to(cuda) for i in range(4)] for s in (60, 70))
+        for of, to in ((0, 1), (3, 2)):
+            caches[of].offset = P + 1
+            k[to], v[to] = (t[:, :, P:] for t in caches[of].state)
+            caches[of].offset = P
+        outs = [torch.empty_like(t) for t in q]
+        if batched:
+            kvc.DecodeStep(caches, q, k, v, outs, D ** -0.5).run(synchronize=True)
+        else:
+            for i, c in enumerate(caches):
+                c.attention(q[i], k[i], v[i], D ** -0.5, out=outs[i])
+                torch.cuda.synchronize()
+        return outs + [t.clone() for c in caches for t in c.state]
+    assert all(torch.equal(a, b) for a, b in zip(run(True), run(False)))
