@@ -267,17 +267,10 @@ def _from_pointer(ptr: int, nbytes: int, dtype, device):
     return _binding.wrap(ctypes.addressof(v), _device_index(_torch_mod.device(device))).view(dtype)
 
 
-_has_device = None
-
-
 def _stream_ptr(stream=None) -> int:
     if stream is not None:
         return int(stream.cuda_stream)
-    global _has_device
-    if _has_device is None:
-        _has_device = _torch_mod.cuda.is_available()
-    # host-only calls (file headers, empty caches) on a machine without a device take no stream
-    return _binding.current_stream() if _has_device else 0
+    return _binding.current_stream()    # 0 without a device: host-only calls (file headers, empty caches) take none
 
 
 def _stream_arg(stream):

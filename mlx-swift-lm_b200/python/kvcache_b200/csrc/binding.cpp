@@ -8,6 +8,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include "../../../../include/kvcache_b200.h"
@@ -45,8 +46,12 @@ bool describe(PyObject *o, kvc_tensor *out) {
     }
     const at::Tensor &t = THPVariable_Unpack(o);
     const int code = dtype_code(t.scalar_type());
-    if (code < 0 || t.dim() > KVC_MAX_DIMS) {
-        PyErr_Format(PyExc_KeyError, "tensor of an unsupported dtype or with more than %d dims", KVC_MAX_DIMS);
+    if (code < 0) {
+        PyErr_Format(PyExc_KeyError, "no library dtype for a tensor of %s", c10::toString(t.scalar_type()));
+        return false;
+    }
+    if (t.dim() > KVC_MAX_DIMS) {
+        PyErr_Format(PyExc_IndexError, "a tensor of %d dims: at most %d", (int)t.dim(), KVC_MAX_DIMS);
         return false;
     }
     *out = kvc_tensor{};
@@ -60,9 +65,11 @@ bool describe(PyObject *o, kvc_tensor *out) {
     return true;
 }
 
+// On a machine without a device there is no stream to ask for: the library's call says so by its status.
+void *current_stream() { return c10::cuda::device_count() > 0 ? (void *)c10::cuda::getCurrentCUDAStream().stream() : nullptr; }
+
 void *stream_arg(PyObject *o) {     // None: the current stream, else an address
-    if (o == Py_None) return (void *)c10::cuda::getCurrentCUDAStream().stream();
-    return PyLong_AsVoidPtr(o);
+    return o == Py_None ? current_stream() : PyLong_AsVoidPtr(o);
 }
 
 // What the three attention calls share: (..., q, k, v, scale, mode, mask, out, stream) from args[at] on.
@@ -210,7 +217,7 @@ PyObject *py_wrap(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 PyObject *py_current_stream(PyObject *, PyObject *) {
-    return guarded([&]() -> PyObject * { return PyLong_FromVoidPtr((void *)c10::cuda::getCurrentCUDAStream().stream()); });
+    return guarded([&]() -> PyObject * { return PyLong_FromVoidPtr(current_stream()); });
 }
 
 PyMethodDef methods[] = {
