@@ -23,13 +23,33 @@ if not os.path.exists(LIB_PATH):
         f"{LIB_PATH} is missing: build it with `python mlx-swift-lm_b200/build.py` "
         "(there is no CPU or PyTorch fallback for this library)")
 
-import torch as _torch_mod  # noqa: E402  (loaded first: _binding links against its libraries)
 
-try:
-    from . import _binding  # noqa: E402
-except ImportError as e:
-    raise ImportError(f"the binding module is missing or was built for another torch: build it with "
-                      f"`python mlx-swift-lm_b200/build.py` ({e})") from e
+class _WhenUsed:
+    """A module imported by its first use, which leaves it in the package's `name`. The C ABI, reached through lib(),
+    needs neither torch nor the binding module; calls that take tensors need both."""
+
+    def __init__(self, name, load):
+        self._name, self._load = name, load
+
+    def __getattr__(self, attr):
+        module = globals()[self._name] = self._load()
+        return getattr(module, attr)
+
+
+def _load_binding():
+    _torch()     # first: the binding links against its libraries
+    import importlib
+    try:
+        module = importlib.import_module("._binding", __name__)
+    except ImportError as e:
+        raise ImportError(f"the binding module is missing or was built for another torch: build it with "
+                          f"`python mlx-swift-lm_b200/build.py` ({e})") from e
+    module.init(*(ctypes.cast(f, ctypes.c_void_p).value for f in (_lib.kvc_attention, _lib.kvc_attention_rope, _lib.kvc_sdpa)))
+    return module
+
+
+_torch_mod = _WhenUsed("_torch_mod", lambda: _torch())
+_binding = _WhenUsed("_binding", _load_binding)
 
 _lib = ctypes.CDLL(LIB_PATH)
 
@@ -197,13 +217,6 @@ _lib.kvc_timing_enable.restype = None
 _lib.kvc_timing_read.argtypes = [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_int64), ctypes.c_int32]
 
 
-def _address(fn) -> int:
-    return ctypes.cast(fn, _vp).value
-
-
-_binding.init(_address(_lib.kvc_attention), _address(_lib.kvc_attention_rope), _address(_lib.kvc_sdpa))
-
-
 def lib() -> ctypes.CDLL:
     return _lib
 
@@ -231,7 +244,8 @@ def check(status: int) -> None:
 # ---------------------------------------------------------------------------
 
 def _torch():
-    return _torch_mod
+    import torch
+    return torch
 
 
 def _torch_dtype(code: int):
