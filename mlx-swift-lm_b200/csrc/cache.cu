@@ -244,20 +244,64 @@ Array4 Array4::share() {
     return *this;
 }
 
+namespace {
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) (void)cudaGetLastError();
+    return st == cudaStreamCaptureStatusActive;
+}
+// Calls on other streams while this thread captures one.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { KVC_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
+    ~OutsideCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+struct OwnStream {
+    cudaStream_t s = nullptr;
+    OwnStream() { KVC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
+    ~OwnStream() { (void)cudaStreamDestroy(s); }
+};
+}  // namespace
+
 void Array4::detach(int64_t keep_rows, cudaStream_t s) {
     if (!ptr || !shared) return;
+    bool last;
     {
         std::lock_guard<std::mutex> lock(shared->mu);
-        if (shared->holders == 1) {
-            // written in place from here on: behind what a holder that left may still be reading (its copy)
-            if (shared->left && shared->left_stream != s) KVC_CUDA(cudaStreamWaitEvent(s, shared->left, 0));
-            return;
-        }
+        last = shared->holders == 1;
     }
+    if (last) {
+        // Written in place from here on: behind what a holder that left may still be reading (its copy). A stream that
+        // is being captured takes no wait for work outside the capture, so the host waits there.
+        if (shared->left && shared->left_stream != s) {
+            if (capturing(s)) {
+                OutsideCapture outside;
+                KVC_CUDA(cudaEventSynchronize(shared->left));
+            } else {
+                KVC_CUDA(cudaStreamWaitEvent(s, shared->left, 0));
+            }
+        }
+        if (shared->left) (void)cudaEventDestroy(shared->left);
+        delete shared;
+        shared = nullptr;
+        return;
+    }
+    const int64_t rows = std::min(keep_rows, cap);
     Array4 own;
-    own.alloc(B, H, cap, W, dtype, s, std::min(keep_rows, cap));
-    copy_rows(*this, 0, own, 0, std::min(keep_rows, cap), s);
-    release(s);
+    if (capturing(s)) {
+        // Memory allocated and copied by the captured stream would belong to the graph: the copy is made now, on a stream
+        // of its own. (What the graph builds on has completed when its capture begins.)
+        OutsideCapture outside;
+        OwnStream side;
+        own.alloc(B, H, cap, W, dtype, side.s, rows);
+        copy_rows(*this, 0, own, 0, rows, side.s);
+        release(side.s);
+        KVC_CUDA(cudaStreamSynchronize(side.s));
+    } else {
+        own.alloc(B, H, cap, W, dtype, s, rows);
+        copy_rows(*this, 0, own, 0, rows, s);
+        release(s);
+    }
     *this = own;
 }
 

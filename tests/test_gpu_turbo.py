@@ -417,3 +417,39 @@ def test_tensor_core_verify_kernel_with_calibrated_keys(kvc, oracle, cuda, capfd
     ref = oracle.attention_with_cache_update(to_oracle(q2), to_oracle(k2), to_oracle(v2), o, D ** -0.5, "causal")
     assert worst_excess(out, ref, dtype) <= 0
     assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("converted_is", ["alive", "gone"])
+def test_source_of_a_conversion_can_be_captured(kvc, cuda, converted_is):
+    """A cache whose rows a converted one holds, or held, still takes its steps under stream capture, and a replay after
+    the converted cache has rewritten and freed its rows reads its own."""
+    D, P = 128, 100
+    k = seeded((1, 2, P, D), 1, torch.bfloat16).to(cuda)
+    q, k1, v1 = (seeded((1, h, 1, D), s, torch.bfloat16).to(cuda) for h, s in ((4, 2), (2, 3), (2, 4)))
+    s, plain = kvc.KVCacheSimple(reserve_tokens=256), kvc.KVCacheSimple(reserve_tokens=256)
+    s.update(k, -k)
+    plain.update(k, -k)
+    out = torch.empty_like(q)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        s.attention(q, k1, v1, 0.1, out=out)        # warm: workspaces of this stream
+    torch.cuda.synchronize()
+    s.trim(1)
+    t = s.to_turbo(4, 4)
+    if converted_is == "gone":
+        t.encode_new_token(k1, v1)
+        del t
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        s.attention(q, k1, v1, 0.1, out=out)
+    if converted_is == "alive":
+        t.encode_new_token(k1, v1)                  # frees what the two shared
+        filler = [torch.full((1 << 20,), 7.0, device=cuda) for _ in range(4)]
+    expect = plain.attention(q, k1, v1, 0.1)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, expect)
+    assert torch.equal(s.state[0], plain.state[0]) and torch.equal(s.state[1], plain.state[1])
