@@ -208,6 +208,7 @@ void Array4::alloc(int64_t b, int64_t h, int64_t c, int64_t w, int32_t dt, cudaS
     // kernels copy full stages of up to 256 tokens, and a stage must never reach past the (batch, head) slab
     B = b; H = h; cap = round_up(std::max<int64_t>(c, 1), 256); W = w; dtype = dt;
     shared = nullptr;
+    borrowed = false;
     ptr = dev_alloc(bytes(), s);
     if (written == 0) KVC_CUDA(cudaMemsetAsync(ptr, 0, bytes(), s));
     else if (written > 0) zero_rows(*this, written, cap - written, s);
@@ -241,7 +242,9 @@ Array4 Array4::share() {
     if (!shared) shared = new SharedRows();
     std::lock_guard<std::mutex> lock(shared->mu);
     ++shared->holders;
-    return *this;
+    Array4 other = *this;
+    other.borrowed = true;
+    return other;
 }
 
 namespace {
@@ -263,7 +266,7 @@ struct OwnStream {
 };
 }  // namespace
 
-void Array4::detach(int64_t keep_rows, cudaStream_t s) {
+void Array4::detach(int64_t keep_rows, int64_t need, cudaStream_t s) {
     if (!ptr || !shared) return;
     bool last;
     {
@@ -286,19 +289,19 @@ void Array4::detach(int64_t keep_rows, cudaStream_t s) {
         shared = nullptr;
         return;
     }
-    const int64_t rows = std::min(keep_rows, cap);
+    const int64_t rows = std::min(keep_rows, cap), room = borrowed ? std::max(need, rows) : cap;
     Array4 own;
     if (capturing(s)) {
         // Memory allocated and copied by the captured stream would belong to the graph: the copy is made now, on a stream
         // of its own. (What the graph builds on has completed when its capture begins.)
         OutsideCapture outside;
         OwnStream side;
-        own.alloc(B, H, cap, W, dtype, side.s, rows);
+        own.alloc(B, H, room, W, dtype, side.s, rows);
         copy_rows(*this, 0, own, 0, rows, side.s);
         release(side.s);
         KVC_CUDA(cudaStreamSynchronize(side.s));
     } else {
-        own.alloc(B, H, cap, W, dtype, s, rows);
+        own.alloc(B, H, room, W, dtype, s, rows);
         copy_rows(*this, 0, own, 0, rows, s);
         release(s);
     }
@@ -454,8 +457,9 @@ static void linear_update(kvc_cache *c, const kvc_tensor &k, const kvc_tensor &v
         KVC_REQUIRE(k.shape[0] == c->k.B && k.shape[1] == c->k.H && k.shape[3] == c->k.W &&
                         v.shape[3] == c->v.W && k.dtype == c->k.dtype,
                     "update: new keys/values do not match the cached shape or dtype");
-        c->k.detach(c->offset, s);
-        c->v.detach(c->offset, s);
+        const int64_t room = std::max<int64_t>(c->cfg.reserve_tokens, round_up(c->offset + S, step));
+        c->k.detach(c->offset, room, s);
+        c->v.detach(c->offset, room, s);
         c->k.ensure(c->offset + S, c->offset, step, s);
         c->v.ensure(c->offset + S, c->offset, step, s);
     }
@@ -1065,7 +1069,7 @@ static void turbo_ensure_compressed(kvc_cache *c, int64_t need, int64_t keep_row
     for (Array4 *a : {&c->kp, &c->kn, &c->vp, &c->vn, &c->kq, &c->ks, &c->kb, &c->vq, &c->vs, &c->vb})
         if (a->allocated()) a->ensure(need, keep_rows, step, s);
     if (c->raw_key && c->k.allocated()) {
-        c->k.detach(keep_rows, s);
+        c->k.detach(keep_rows, need, s);
         c->k.ensure(need, keep_rows, step, s);
     }
 }
@@ -1077,8 +1081,10 @@ static void turbo_compress_raw(kvc_cache *c, cudaStream_t s) {
     KVC_REQUIRE(c->v.W == c->k.W, "TurboQuant: key and value head dims must match");
     ensure_codecs(c, D, s);
     // whole 256-row steps, like the reference's allocations: the decode kernels stream whole stages; with
-    // room for the token whose attention asked for the compression
-    const int64_t cap = round_up(std::max<int64_t>(std::max<int64_t>(c->cfg.reserve_tokens, c->k.cap), c->offset + 1), 256);
+    // room for the token whose attention asked for the compression, and for what this cache's own raw rows had room for
+    // (rows shared with the cache it was converted from have that one's capacity)
+    const int64_t own = c->k.borrowed ? 0 : c->k.cap;
+    const int64_t cap = round_up(std::max<int64_t>(std::max<int64_t>(c->cfg.reserve_tokens, own), c->offset + 1), 256);
     turbo_alloc_compressed(c, c->k.B, c->k.H, D, c->k.dtype, cap, s, c->offset);
     kvc_tensor kt = c->k.view(c->offset), vt = c->v.view(c->offset);
     if (c->raw_key) {

@@ -26,6 +26,7 @@ struct SharedRows {
 struct Array4 {
     void *ptr = nullptr;
     SharedRows *shared = nullptr;
+    bool borrowed = false;      // shared by a conversion: the capacity is that of the cache converted from
     int32_t dtype = KVC_BF16;
     int64_t B = 0, H = 0, cap = 0, W = 0;
 
@@ -40,9 +41,10 @@ struct Array4 {
     // be finite); the caller writes rows [0, written) itself. -1: the caller zeroes with zero_tails.
     void alloc(int64_t b, int64_t h, int64_t c, int64_t w, int32_t dt, cudaStream_t s, int64_t written = 0);
     void release(cudaStream_t s);
-    // Another holder of the same rows; whoever writes first takes a copy (detach).
+    // Another holder of the same rows; whoever writes first takes a copy (detach), a borrower one of room for `need`
+    // rows, the lender one as large as what it had.
     Array4 share();
-    void detach(int64_t keep_rows, cudaStream_t s);
+    void detach(int64_t keep_rows, int64_t need, cudaStream_t s);
     // Grow to at least `need` token rows, preserving the first `keep_rows`.
     void ensure(int64_t need, int64_t keep_rows, int64_t step, cudaStream_t s);
     kvc_tensor view(int64_t tokens, int64_t first = 0) const;

@@ -453,3 +453,19 @@ def test_source_of_a_conversion_can_be_captured(kvc, cuda, converted_is):
         torch.cuda.synchronize()
         assert torch.equal(out, expect)
     assert torch.equal(s.state[0], plain.state[0]) and torch.equal(s.state[1], plain.state[1])
+
+
+@pytest.mark.parametrize("key_bits", [4, 8, 0])
+def test_converted_cache_is_as_large_as_its_tokens(kvc, cuda, key_bits):
+    """What the source had reserved is not allocated again, compressed or (raw keys) as a copy; the source keeps it."""
+    k = seeded((1, 2, 100, 128), 1, torch.bfloat16).to(cuda)
+    s, plain = kvc.KVCacheSimple(reserve_tokens=65536), kvc.TurboQuantKVCache(bits=4, key_bits=key_bits, value_bits=4)
+    s.update(k, -k)
+    plain.update(k, -k)
+    before = s.memory_bytes
+    t = s.to_turbo(key_bits, 4)
+    for c in (t, plain):
+        c.encode_new_token(k[:, :, :1], k[:, :, :1])
+    assert t.memory_bytes == plain.memory_bytes
+    s.update(k, -k)
+    assert s.memory_bytes == before
