@@ -287,8 +287,13 @@ int launch_attention_chunk_packed_pairs(const AttnArgs &a, cudaStream_t stream) 
     const size_t per_b = kv * (k_in_place ? 2 : k_raw ? 3 : 4) + (q_in_place ? 0 : k_turbo ? 2 * q : q) + (v_turbo ? 2 * q : 0) + 2 * heads + rows_f;
     if (per_b > PAIR_SCRATCH_LIMIT) return 0;
     const int fit = (int)std::min<size_t>({(size_t)a.B, PAIR_SCRATCH_LIMIT / per_b, (size_t)32767});
-    const int nslices = (a.B + fit - 1) / fit, slice = (a.B + nslices - 1) / nslices;
-    const PoolRows rows{dev_alloc((size_t)slice * per_b, stream), stream};
+    const int nslices = (a.B + fit - 1) / fit;
+    int slice = (a.B + nslices - 1) / nslices;
+    // a device too full for the rows of one sequence leaves the call to the general kernel, which needs its partials only
+    void *memory = dev_try_alloc((size_t)slice * per_b, stream);
+    while (!memory && slice > 1) memory = dev_try_alloc((size_t)(slice = (slice + 1) / 2) * per_b, stream);
+    if (!memory) return 0;
+    const PoolRows rows{memory, stream};
     int launches = 0;
     for (int b0 = 0; b0 < a.B; b0 += slice) {
         const int nb = std::min(slice, a.B - b0);

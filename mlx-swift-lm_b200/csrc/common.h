@@ -60,6 +60,7 @@ inline bool is_float_dtype(int32_t dt) { return dt == KVC_F32 || dt == KVC_F16 |
 // device memory: stream-ordered allocations from the device's default pool.
 // ---------------------------------------------------------------------
 void *dev_alloc(size_t bytes, cudaStream_t stream);
+void *dev_try_alloc(size_t bytes, cudaStream_t stream);   // nullptr where the device has no room
 void dev_free(void *ptr, cudaStream_t stream);
 // Scratch that grows on demand, one arena per (device, stream), reused by every
 // attention call enqueued on that stream (split-K partials).

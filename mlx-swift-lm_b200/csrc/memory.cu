@@ -67,6 +67,18 @@ void *dev_alloc(size_t bytes, cudaStream_t stream) {
     return p;
 }
 
+void *dev_try_alloc(size_t bytes, cudaStream_t stream) {
+    ensure_pool(current_device());
+    void *p = nullptr;
+    const cudaError_t e = cudaMallocAsync(&p, bytes, stream);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    KVC_CUDA(e);
+    return p;
+}
+
 void dev_free(void *ptr, cudaStream_t stream) {
     if (!ptr) return;
     cudaError_t e = cudaFreeAsync(ptr, stream);

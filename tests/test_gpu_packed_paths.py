@@ -1,6 +1,10 @@
 """The TMA-staged tensor-core decode kernels over packed caches (affine codes,
 TurboQuant indices) against the oracle, driven through the cache objects the
 way attentionWithCacheUpdate drives them."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -672,3 +676,35 @@ def test_stream_kernel_keeps_single_precision_over_affine_codes(kvc, oracle, cud
     ref = _attention64(q, K, V, D ** -0.5, torch.arange(P + L, device=cuda) <= torch.arange(P, P + L, device=cuda)[:, None])
     ideal = float((ref.half().double() - ref).norm())
     assert float((out.double() - ref).norm()) <= 1.0003 * ideal
+
+
+def test_chunk_on_operand_pairs_on_a_full_device(kvc, cuda):
+    """A chunk whose decoded rows the device has no room for runs on the general kernel instead of failing."""
+    code = """
+import torch, kvcache_b200 as kvc
+torch.manual_seed(0)
+c = kvc.QuantizedKVCache(64, 4, reserve_tokens=40960)
+for _ in range(10):
+    k, v = torch.randn(2, 1, 8, 4000, 256, dtype=torch.half, device="cuda")
+    c.update_quantized(k, v)
+q, k, v = (torch.randn(1, h, 70, 256, dtype=torch.half, device="cuda") for h in (8, 8, 8))
+out = torch.empty_like(q)
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+hold = torch.empty(torch.cuda.mem_get_info()[0] - (300 << 20), dtype=torch.uint8, device="cuda")
+launches, outs = [], []
+for step in range(2):
+    kvc.launch_count(reset=True)
+    c.attention(q, k, v, 0.0625, "causal", out=out)
+    torch.cuda.synchronize()
+    launches.append(kvc.launch_count(reset=True))
+    outs.append(out.clone())
+    c.trim(70)
+    del hold
+    torch.cuda.empty_cache()
+    hold = None
+assert launches[0] == 3 and launches[1] == 4, launches
+assert float((outs[0].float() - outs[1].float()).abs().max()) < 2e-3
+"""
+    env = dict(os.environ, PYTHONPATH=os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlx-swift-lm_b200", "python"))
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
