@@ -441,16 +441,21 @@ struct FlatWork {
     int32_t t0, n, nslots, more;              // more: 0 ends a list
     int32_t unit, hk, b, last;                // last: the segment ends its unit
 };
+// Its new rows and where they go (read by the warp that appends, at the segment's end).
+template <typename T>
+__device__ __forceinline__ void flat_new_rows(FlatWork &w, const FlatSeg &g) {
+    w.new_k = (const unsigned char *)((const T *)g.new_k + g.b * g.nk_sb + g.hk * g.nk_sh);
+    w.new_v = (const unsigned char *)((const T *)g.new_v + g.b * g.nv_sb + g.hk * g.nv_sh);
+    const int64_t row = g.b * g.kv_sb + g.hk * g.kv_sh + g.new_slot * g.kv_st;
+    w.k_row = g.k_base + row;
+    w.v_row = g.v_base + row;
+}
 template <typename T>
 __device__ __forceinline__ FlatWork flat_work(const FlatSeg &g, const DecodeParams &p) {
     FlatWork w;
     const int rep = p.Hq / p.Hkv;
     w.q = (const unsigned char *)((const T *)g.q + g.b * g.q_sb + (int64_t)g.hk * rep * p.q_sh);
-    w.new_k = g.new_k ? (const unsigned char *)((const T *)g.new_k + g.b * g.nk_sb + g.hk * g.nk_sh) : nullptr;
-    w.new_v = (const unsigned char *)((const T *)g.new_v + g.b * g.nv_sb + g.hk * g.nv_sh);
-    const int64_t row = g.b * g.kv_sb + g.hk * g.kv_sh + g.new_slot * g.kv_st;
-    w.k_row = g.k_base + row;
-    w.v_row = g.v_base + row;
+    w.new_k = (const unsigned char *)g.new_k;
     w.T = g.T; w.new_slot = g.new_slot;
     w.t0 = g.t0; w.n = g.n;
     w.unit = g.unit; w.hk = g.hk; w.b = g.b;
@@ -561,6 +566,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                     if (!ok) break;
                     if constexpr (LIST) {
                         FlatWork w = flat_work<T>(gs, p);
+                        if (gs.new_k) flat_new_rows<T>(w, gs);
                         w.nslots = gs.plan.nslots;
                         w.part = gs.part_first + ((int64_t)b * p.Hq + hk * rep) * w.nslots + gs.cta - flat_cta_of32(gs.plan, (uint32_t)(x - t0));
                         works[qb] = w;
@@ -666,7 +672,10 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
         }
         if (fused && warp == 0 && w.last && lane < 4) {
             // the new rows are consumed at the end of the segment: pull them towards L2 now
-            const unsigned char *line = ((lane & 1) ? w.new_v : w.new_k) + (lane >> 1) * 128;
+            FlatWork rows;
+            if constexpr (!LIST) flat_new_rows<T>(rows, gs);
+            const FlatWork &nr = LIST ? w : rows;
+            const unsigned char *line = ((lane & 1) ? nr.new_v : nr.new_k) + (lane >> 1) * 128;
             if ((lane >> 1) * 128 < D * 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
         }
         uint32_t qa[KSTEPS][4];
@@ -811,7 +820,10 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
 
         if (fused && warp == 0 && w.last && !(KVC_SKIP_BITS(p) & 32)) {
             // ---- the step's new token: score q . k_new, fold it into this warp's state, store the rows ----
-            const T *kn = (const T *)w.new_k, *vn = (const T *)w.new_v;
+            FlatWork rows;
+            if constexpr (!LIST) flat_new_rows<T>(rows, gs);
+            const FlatWork &nr = LIST ? w : rows;
+            const T *kn = (const T *)nr.new_k, *vn = (const T *)nr.new_v;
             float dot[2] = {0.f, 0.f};
 #pragma unroll
             for (int ks = 0; ks < KSTEPS; ++ks) {
@@ -851,7 +863,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 const bool is_v = i >= CHUNKS;
                 const int ch = is_v ? i - CHUNKS : i;
                 const uint4 x = *(const uint4 *)((const unsigned char *)(is_v ? vn : kn) + ch * 16);
-                *(uint4 *)((is_v ? w.v_row : w.k_row) + ch * 16) = x;
+                *(uint4 *)((is_v ? nr.v_row : nr.k_row) + ch * 16) = x;
             }
         }
 
