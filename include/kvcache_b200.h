@@ -621,9 +621,11 @@ int64_t    kvc_launch_count(int32_t reset);
  * with host != 0, kvc_attention_host) on caches[i] with q[i], k[i], v[i],
  * outs[i] for i in [0, count). This is the loop over layers of
  * TokenIterator.step (Evaluate.swift:905-916) as a native caller would run it;
- * mask arrays are not supported here. Every call gives what it would give on its
- * own: calls on different caches whose buffers do not overlap may share launches. synchronize != 0 waits for the stream
- * once at the end. */
+ * mask arrays are not supported here. Caches and outputs are as if the calls were
+ * made one after another. Calls on different caches whose buffers do not overlap may
+ * share launches: over raw caches with the same bits, over packed caches equal up to
+ * the rounding of the output type (another order of the sums). synchronize != 0 waits
+ * for the stream once at the end. */
 kvc_status kvc_attention_batch(kvc_cache *const *caches, int32_t count, const kvc_tensor *queries,
                                const kvc_tensor *keys, const kvc_tensor *values, float scale,
                                int32_t mask_mode, const kvc_tensor *outs, void *stream,

@@ -351,7 +351,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
 // against 64-bit sums rises by 3 .. 5 %). With several ranges per CTA a range must end without a wait: every warp
 // leaves its state in memory and walks on, and flat_list_merge_kernel does the merges of all units behind it. 26 layers
 // of the Gemma-3-1B shape (4 x 2048 tokens, rings of 512) and 8 layers of 8 x 8192 tokens, 32/8 heads, D 128, bf16:
-// 160 and 436 us with the merges inside (ticket, last CTA of the unit), 61 and 379 behind, 50 and 341 with the
+// 160 and 436 us with the merges inside (ticket, last CTA of the unit), 61 and 379 behind, 47 and 350 with the
 // descriptors handed over (FlatWork); one launch per call took 391 and 402.
 constexpr int FLAT_AHEAD = 4;   // segments of a list the producer may be ahead
 struct FlatLayer {

@@ -1,10 +1,11 @@
 // Decode attention over every pair of K / V representations a 16-bit caller can hold (raw rows, affine
 // 4- / 8-bit codes, 2- / 3- / 4-bit codebook indices, mixed: raw or affine keys with index values, index
-// keys with affine values), head dims 64 / 128 / 256, up to 64 query rows per KV head, and lists of
-// independent affine caches.
+// keys with affine values; raw keys with raw values have kernels of their own), head dims 64 / 128 / 256, up to 64 query
+// rows per KV head, and lists of calls of one shape.
 //
 // What bounds it: instruction issue and the shared-memory pipe for the packed layouts, HBM for the wide ones.
-// Split: every WARP is on its own. It walks 16-token blocks of the CTA's token range (blocks w, w + 8, ...),
+// Split: every WARP is on its own. It walks 16-token blocks of the CTA's token range (every fifth to twelfth:
+// as many as the CTA has warps),
 // keeps a private ring of packed blocks in shared memory that its own lanes fill with 16-byte cp.async copies
 // (a block of 16 rows is one contiguous piece of each array; bytes past the last token are zero-filled, so no
 // padding of the arrays is asked for), and no barrier is taken until the segment ends. The token side sits on
@@ -22,7 +23,7 @@
 //     bits) and a product is the three MMAs hi hi + lo hi + hi lo (two where one side is exact). The MMAs are not what
 //     bounds the kernel; the second table lookup of each centroid pair is the price.
 //     8 layers x 4 sequences x 4099 tokens, 32/8 heads, D 128, 8-bit keys / 4-bit values, f16: 2521 us on the general
-//     kernel, 111 us here; 80 us with single f16 operands, which no longer err by the store's rounding alone.
+//     kernel, 114 us here; 80 us with single f16 operands, which no longer err by the store's rounding alone.
 //   * The running reference is only moved when a score (with its value factor) passes it by more than 2^3.
 // Work is cut into equal ranges of 64-token tiles per resident CTA (FlatPlan), units that cross a CTA boundary
 // are merged by segment_epilogue.
@@ -326,7 +327,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
         const char *kd = (const char *)ks.data + bi * ks.sb + sg.hk * ks.sh;
         const char *vd = (const char *)vs.data + bi * vs.sb + sg.hk * vs.sh;
         const char *ksc = K::RAW ? nullptr : (const char *)ks.scales + bi * ks.gsb + sg.hk * ks.gsh;
-        const char *vsc = V::RAW ? nullptr : (const char *)vs.scales + bi * vs.gsb + sg.hk * vs.gsh;
+        const char *vsc = (const char *)vs.scales + bi * vs.gsb + sg.hk * vs.gsh;
         const char *kbi = K::AFFINE ? (const char *)ks.biases + bi * ks.gsb + sg.hk * ks.gsh : nullptr;
         const char *vbi = V::AFFINE ? (const char *)vs.biases + bi * vs.gsb + sg.hk * vs.gsh : nullptr;
         const int k_side = K::AFFINE ? 2 * p.groups_k : 4, v_side = V::AFFINE ? 2 * p.groups_v : 4;   // bytes per token
@@ -342,10 +343,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
             }
         };
         auto value_place = [](int i) {
-            if constexpr (V::RAW) {          // tile form: [64-dim box][token][128 bytes], chunks swizzled by the token
-                const int tok = i / V::CH, ch = i % V::CH;
-                return (ch >> 3) * 2048 + tok * 128 + (((ch & 7) ^ (tok & 7)) << 4);
-            } else if constexpr (!V::POW2) return i << 4;
+            if constexpr (!V::POW2) return i << 4;
             else {
                 const int tok = i / V::CH, ch = i % V::CH;
                 return (tok * V::CH + (ch ^ value_xor<VK, D>(tok))) << 4;
@@ -371,7 +369,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
             };
             if (!K::RAW) claim(ksc, k_side, K::BLOCK);
             if (K::AFFINE) claim(kbi, k_side, K::BLOCK + K::SIDE);
-            if (!V::RAW) claim(vsc, v_side, K::STAGE + V::BLOCK);
+            claim(vsc, v_side, K::STAGE + V::BLOCK);
             if (V::AFFINE) claim(vbi, v_side, K::STAGE + V::BLOCK + V::SIDE);
         }
         const char *k_lane = kd + (int64_t)t_lo * K::RB + lane * 16, *v_lane = vd + (int64_t)t_lo * V::RB + lane * 16;
