@@ -237,6 +237,8 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
     if (affine && (a.q_signs || a.o_signs || a.q_calib || a.k.dtype != a.q_dtype || a.v.dtype != a.q_dtype)) return 0;
     if (!source_ok(a.k, a.D, turbo) || !source_ok(a.v, a.D, turbo)) return 0;
     if (a.T < 1 || a.T > (int64_t)1 << 30 || a.B < 1) return 0;
+    // the rows are written out for this call alone: for less work than this the kernels that decode in their tile loop
+    if (a.L < 64 || (int64_t)a.B * a.Hq * ((a.L + 127) / 128) < sm_count(a.device) / 2) return 0;
 
     // the contraction as the tcgen05 kernel would see it: raw K / V of the query dtype, contiguous
     AttnArgs r = a;

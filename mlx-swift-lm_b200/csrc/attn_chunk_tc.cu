@@ -1,23 +1,31 @@
 // Prefill / long verify chunks over raw K/V on the 5th-generation tensor cores (tcgen05 + TMEM).
 //
 // attentionWithCacheUpdate's scaledDotProductAttention call (AttentionUtils.swift:87-93) for a chunk
-// of L query positions per head: one CTA takes 128 consecutive positions of one query head and walks
-// the 128-key tiles it can see.
+// of L query positions per head. The query rows of a KV head's group are cut into tiles of up to 128
+// rows, position-major (a tile is `lb` positions x `hb` heads of the group: an odd group wastes no row
+// block and a tile's causal limits lie close together). A unit is TWO neighbouring row tiles, A and B,
+// which share every K and V tile.
 //
-//   warp 0      TMA producer: the Q block once, then K and V tiles into two slots each (K one tile ahead)
-//   warp 1      owns the TMEM allocation; lane 0 issues the MMAs:
-//                 S_j = Q K_j^T          (A = Q, B = K_j, both K-major)      -> TMEM S buffer j % 2
-//                 O_j = P_j V_j          (A = P_j from shared memory, B = V_j MN-major) -> TMEM O buffer j % 2
-//   warps 2..5  softmax: thread = query row = TMEM lane. S_j comes out of TMEM in one round trip (128
-//               registers), row maximum, exponentials, P_j written as the next MMA's A operand in
-//               shared memory (two P tiles, so that tile j + 1 never waits for O_j to have read
-//               P_j); the rescale factor of the tile goes to the correction warps
-//   warps 6..9  correction: thread = query row. O_j comes out of TMEM and is folded into the row's
-//               register accumulator, o = o * alpha_j + O_j; normalisation and the store at the end
+//   warps 0..3  softmax of tile A, warps 4..7 of tile B: thread = query row = TMEM lane. The 128 scores of a
+//               key tile come out of TMEM in one round trip, row maximum, exponentials, and P goes back into
+//               TMEM over the scores' own columns, where the O product reads it as its A operand
+//   warp 8      TMA producer: Q tiles per unit, K and V tiles into one ring
+//   warp 9      owns the TMEM allocation and issues the MMAs in the order
+//                 O_A += P_A(j) V_j | S_A = Q_A K_{j+1}^T | O_B += P_B(j) V_j | S_B = Q_B K_{j+1}^T
+//               so that one tile's products run while the other tile's softmax does
 //
-// Every O_j is a fresh product (no accumulation in TMEM), so the running-maximum rescale never has to
-// touch TMEM. S_{j+1} is issued before O_j: the tensor cores work on the next scores while the
-// softmax warps are busy with the current ones, and the correction warps trail by one product.
+// O accumulates in TMEM, in the reference that the row's exponents are taken against. The scores of tile j + 1 are
+// issued behind the O product of tile j, so when they arrive O is settled and the softmax threads may multiply it; they
+// do so under their exponentials, which wait for the special-function unit. Two forms:
+//   the reference is the row's running maximum, which moves at most once per 128 keys (PARTS = 1);
+//   it is the largest score of every 128 / PARTS keys, also where that is below the row's (PARTS = 2 or 4): the largest
+//   probability of each part is exactly 1 and loses nothing to the 16-bit store, so the errors against 64-bit sums are
+//   4 ... 10 % smaller (bf16 and f16, 128 ... 16 000 keys), for O products in parts with a rescale between them.
+//
+// Units are handed out whole, in rounds of one per SM; what is left over is laid end to end and cut into equal ranges,
+// or few units are cut into pieces (a cut unit leaves fp32 partials, and the CTA that finishes it merges them).
+//
+// TMEM columns: S_A / P_A at 0, S_B / P_B at 128, O_A at 256, O_B at 384.
 //
 // Shared-memory operand layout (what TMA's 128-byte swizzle writes): a box is 128 rows x 128 bytes
 // (64 elements), 16-byte chunk c of row r at chunk c ^ (r & 7); a 128 x 128 tile is two boxes (Q, K and
@@ -29,8 +37,10 @@
 // Every wait is bounded; a wait that runs out sets the device status word, the CTA drains and frees
 // its TMEM.
 #include <atomic>
+#include <climits>
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -46,330 +56,651 @@ using namespace dev;
 
 using namespace tc;
 
+constexpr int CT_THREADS = 384;
+// registers a thread: 384 * 168 at launch = 256 * 216 (softmax) + 128 * 72 (the warps that issue copies and MMAs)
+constexpr int CT_REGS_SOFTMAX = 216, CT_REGS_ISSUE = 72;
+// The reference of a part is never further below the row's largest score than this, so that O and the sums stay far
+// from overflow.
+constexpr float CT_SPAN_LOG2 = 24.f;
 
 struct ChunkTcParams {
     void *out;
     int64_t o_sb, o_sh, o_sl;
-    int32_t B, Hq, Hkv, L;
+    int32_t B, rep, Hkv, L;
     int64_t T;
-    int32_t row_blocks;
+    int32_t hb, lb;             // heads and positions of a row tile (hb * lb <= 128)
+    int32_t head_tiles;         // row tiles side by side over the group's heads
+    int32_t row_tiles;          // row tiles of a (batch, KV head)
+    int32_t units;              // ... and units: pairs of row tiles
     int32_t causal;
     int64_t causal_offset;
     float scale_log2;
+    // units end to end over all (batch, KV head): CTA c walks units c, c + grid, ... of the first waves * grid, then the
+    // key tiles [c * per + min(c, rem), ...) of the rest (the tail), whose units are cut where the ranges end
+    int32_t all_units, waves;
+    int32_t ranges, per, rem;   // ranges = 0: no tail
+    int32_t pieces;             // not 0: every unit is cut into this many pieces, one CTA each (no rounds, no tail)
+    int32_t group_tiles;        // key tiles of the units of a (batch, KV head)
+    int32_t tail_base;          // ... of those before the tail's first unit in its own group
+    float *o_part;              // [CTA][first / last segment][A / B][D / 4][128 rows][4]
+    float2 *ml_part;            // [CTA][first / last segment][A / B][128 rows] (reference, sum)
+    int *tickets;               // [unit of the tail][A / B], zeroed before the launch
     int *status;
 };
 
-enum : int {
-    BAR_Q = 0,
-    BAR_K_FULL = 1,                         // [TC_STAGES]
-    BAR_K_EMPTY = BAR_K_FULL + TC_STAGES,   // [TC_STAGES] free once the S product has read the tile
-    BAR_V_FULL = BAR_K_EMPTY + TC_STAGES,   // [TC_STAGES]
-    BAR_V_EMPTY = BAR_V_FULL + TC_STAGES,   // [TC_STAGES] free once the O product has read the tile
-    BAR_S_FULL = BAR_V_EMPTY + TC_STAGES,   // [2]
-    BAR_S_EMPTY = BAR_S_FULL + 2,           // [2]
-    BAR_P_FULL = BAR_S_EMPTY + 2,           // [2]
-    BAR_P_EMPTY = BAR_P_FULL + 2,           // [2]
-    BAR_O_FULL = BAR_P_EMPTY + 2,           // [2]
-    BAR_O_EMPTY = BAR_O_FULL + 2,           // [2]
-    BAR_A_FULL = BAR_O_EMPTY + 2,           // [2] rescale factors of a tile written
-    BAR_A_EMPTY = BAR_A_FULL + 2,           // [2] ... and read
-    BAR_L_FULL = BAR_A_EMPTY + 2,           // row sums written
-    BAR_COUNT = BAR_L_FULL + 1
+template <int D> constexpr int ct_stages() { return D == 128 ? 5 : 10; }
+
+template <int STAGES> struct Bars {
+    enum : int {
+        Q_FULL = 0,                        // [2] row tile A / B
+        Q_EMPTY = Q_FULL + 2,              // [2] free once the unit's last S product has read the tile
+        RING_FULL = Q_EMPTY + 2,           // [STAGES] K_0, V_0, K_1, V_1, ...
+        RING_EMPTY = RING_FULL + STAGES,   // [STAGES]
+        S_FULL = RING_EMPTY + STAGES,      // [2]
+        P_FULL = S_FULL + 2,               // [4][2] the probabilities of a part of the tile, O in their reference
+        O_PART = P_FULL + 8,               // [2] the O product of a part other than the last is done
+        O_FULL = O_PART + 2,               // [2] the segment's last O product is done
+        GROUP = O_FULL + 2,                // [2] the 128 threads of a softmax group meet
+        COUNT = GROUP + 2
+    };
 };
 
-template <typename T, int D>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+// The pair of row tiles of a unit, and its key tiles. Units of a (batch, KV head) are counted from the last positions
+// to the first: with a causal mask the long units go first.
+__device__ __host__ inline int ct_pair_of(const ChunkTcParams &p, int unit) { return p.units - 1 - unit % p.units; }
+__device__ __host__ inline int ct_unit_tiles(const ChunkTcParams &p, int unit) {
+    if (!p.causal) return (int)((p.T + TC_KEYS - 1) / TC_KEYS);
+    const int pair = ct_pair_of(p, unit), last_tile = 2 * pair + 1 < p.row_tiles ? 2 * pair + 1 : p.row_tiles - 1;
+    const int64_t end = (int64_t)(last_tile / p.head_tiles + 1) * p.lb;
+    const int64_t keys = p.causal_offset + (end < p.L ? end : p.L);
+    return (int)(((keys < p.T ? keys : p.T) + TC_KEYS - 1) / TC_KEYS);
+}
+
+// A CTA's work in segments, one per unit it touches.
+struct CtSegment {
+    int unit;
+    int t0, t1, n;     // its key tiles, and the unit's
+    int has_b;         // the unit has two row tiles
+};
+constexpr int CT_MAX_SEGMENTS = 40;
+
+__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z, int u, int v) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(u), "r"(v)
+        : "memory");
+}
+
+// True in one lane of a converged warp. The MMA warp runs its loop with all lanes and picks the lane only around the
+// instructions themselves: under a branch on the lane number every descriptor takes the slow way from vector to uniform
+// registers (70 ... 100 cycles per product, against the 64 the tensor core needs for it).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+
+// One wait of a whole warp: all its threads carry on, or none does.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
+// Two fp32 operations an instruction.
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack_f2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// 32 output columns of a row as 16-bit values.
+template <typename T> __device__ __forceinline__ void store_row32(T *dst, const float *o, float inv) {
+#pragma unroll
+    for (int c8 = 0; c8 < 4; ++c8) {
+        uint4 v;
+        v.x = pack_pair<T>(o[c8 * 8 + 0] * inv, o[c8 * 8 + 1] * inv);
+        v.y = pack_pair<T>(o[c8 * 8 + 2] * inv, o[c8 * 8 + 3] * inv);
+        v.z = pack_pair<T>(o[c8 * 8 + 4] * inv, o[c8 * 8 + 5] * inv);
+        v.w = pack_pair<T>(o[c8 * 8 + 6] * inv, o[c8 * 8 + 7] * inv);
+        *(uint4 *)(dst + c8 * 8) = v;
+    }
+}
+
+template <typename T, int D, int PARTS>
+__global__ void __launch_bounds__(CT_THREADS, 1)
 attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
-                     const __grid_constant__ CUtensorMap vmap, const ChunkTcParams p) {
+                     const __grid_constant__ CUtensorMap vmap, const __grid_constant__ ChunkTcParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    // parts in which a tile's probabilities are handed over; with one reference for all of them, the first 96 keys and the
+    // rest (their O product runs under the other exponentials; 64 keys: 3 % slower)
+    constexpr int HANDS = PARTS == 1 ? 2 : PARTS;
+    auto key_of = [](int part) constexpr { return PARTS == 1 ? (part == 0 ? 0 : part == 1 ? 96 : TC_KEYS) : part * (TC_KEYS / PARTS); };
+    constexpr int STAGES = ct_stages<D>();
+    using BAR = Bars<STAGES>;
     constexpr int NBOX = D / 64;                               // boxes of 64 head dims per Q / K / V tile
-    constexpr int QKV_TILE = NBOX * TC_BOX;                    // bytes of a 128-row tile of D head dims
-    unsigned char *sq = base;                                  // Q block
-    unsigned char *skv = sq + QKV_TILE;                        // ring: stage s = K tile | V tile
-    uint64_t *bars = (uint64_t *)(skv + TC_STAGES * 2 * QKV_TILE);
-    uint32_t *tmem_slot = (uint32_t *)(bars + BAR_COUNT);
-    float *s_alpha = (float *)(tmem_slot + 4);                 // [2][128] rescale factor of tile j for each row
-    float *s_lsum = s_alpha + 2 * TC_ROWS;                     // [128] final row sums
+    constexpr int TILE = NBOX * TC_BOX;                        // bytes of a 128-row tile of D head dims
+    unsigned char *sq = base;                                  // Q tiles A, B
+    unsigned char *ring = sq + 2 * TILE;
+    uint64_t *bars = (uint64_t *)(ring + STAGES * TILE);
+    uint32_t *tmem_slot = (uint32_t *)(bars + BAR::COUNT);
+    int *s_segments = (int *)(tmem_slot + 1);
+    int *s_ticket = s_segments + 1;                            // [2]
+    CtSegment *s_seg = (CtSegment *)(s_ticket + 2);            // [CT_MAX_SEGMENTS]
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // unit = (batch, KV head, row block, query head of the group): the CTAs that share K/V are neighbours
-    const int rep = p.Hq / p.Hkv;
-    int u = blockIdx.x;
-    const int hr = u % rep; u /= rep;
-    // with a causal mask the late row blocks see the most keys: they go first, the short ones fill the tail
-    const int rb = p.row_blocks - 1 - (u % p.row_blocks); u /= p.row_blocks;
-    const int hk = u % p.Hkv;
-    const int b = u / p.Hkv;
-    const int hq = hk * rep + hr;
-    const int l0 = rb * TC_ROWS;
-    // keys this block can see: up to the last row's limit
-    const int64_t last_l = min((int64_t)p.L - 1, (int64_t)l0 + TC_ROWS - 1);
-    const int64_t keys = p.causal ? min(p.T, p.causal_offset + last_l + 1) : p.T;
-    const int n_tiles = (int)((keys + TC_KEYS - 1) / TC_KEYS);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be the same in all lanes: a role's addresses stay in uniform registers
 
     if (tid == 0) {
-        mbar_init(&bars[BAR_Q], 1);
-        for (int s = 0; s < TC_STAGES; ++s) {
-            mbar_init(&bars[BAR_K_FULL + s], 1);
-            mbar_init(&bars[BAR_K_EMPTY + s], 1);
-            mbar_init(&bars[BAR_V_FULL + s], 1);
-            mbar_init(&bars[BAR_V_EMPTY + s], 1);
+        for (int w = 0; w < 2; ++w) {
+            mbar_init(&bars[BAR::Q_FULL + w], 1);
+            mbar_init(&bars[BAR::Q_EMPTY + w], 1);
+            mbar_init(&bars[BAR::S_FULL + w], 1);
+            for (int h = 0; h < 4; ++h) mbar_init(&bars[BAR::P_FULL + 2 * h + w], 128);
+            mbar_init(&bars[BAR::O_PART + w], 1);
+            mbar_init(&bars[BAR::O_FULL + w], 1);
+            mbar_init(&bars[BAR::GROUP + w], 128);
         }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars[BAR_S_FULL + s], 1);
-            mbar_init(&bars[BAR_S_EMPTY + s], 128);
-            mbar_init(&bars[BAR_O_FULL + s], 1);
-            mbar_init(&bars[BAR_O_EMPTY + s], 128);
-        }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars[BAR_A_FULL + s], 128);
-            mbar_init(&bars[BAR_A_EMPTY + s], 128);
-        }
-        mbar_init(&bars[BAR_L_FULL], 128);
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars[BAR_P_FULL + s], 128);
-            mbar_init(&bars[BAR_P_EMPTY + s], 1);
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&bars[BAR::RING_FULL + s], 1);
+            mbar_init(&bars[BAR::RING_EMPTY + s], 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    __syncthreads();
     if (warp == 1) {
+        // the segments of the CTA
+        if (lane < 3) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)(lane == 0 ? &qmap : lane == 1 ? &kmap : &vmap)) : "memory");
+        const int c = blockIdx.x;
+        int segments = 0;
+        auto add = [&](int unit, int t0, int t1, int n) {
+            if (lane == 0) {
+                CtSegment &g = s_seg[segments];
+                g.unit = unit;
+                g.t0 = t0; g.t1 = t1; g.n = n;
+                g.has_b = 2 * ct_pair_of(p, unit) + 1 < p.row_tiles;
+            }
+            ++segments;
+        };
+        if (p.pieces > 0) {
+            const int unit = c / p.pieces, piece = c % p.pieces, n = ct_unit_tiles(p, unit);
+            add(unit, n * piece / p.pieces, n * (piece + 1) / p.pieces, n);
+        }
+        for (int r = 0; r < p.waves; ++r) {
+            const int unit = r * (int)gridDim.x + c;
+            if (unit < p.all_units) {
+                const int n = ct_unit_tiles(p, unit);
+                add(unit, 0, n, n);
+            }
+        }
+        if (c < p.ranges) {
+            // the unit of the range's first tile: its group by division, the unit by a scan over the group's
+            const int pos = p.tail_base + c * p.per + min(c, p.rem);
+            int unit = (p.waves * (int)gridDim.x / p.units + pos / p.group_tiles) * p.units, t = pos % p.group_tiles;
+            for (int e = 0; e < p.units; e += 32) {
+                const int n = e + lane < p.units ? ct_unit_tiles(p, unit + e + lane) : 0;
+                int upto = n;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d) upto += o;
+                }
+                const unsigned past = __ballot_sync(0xffffffffu, upto > t);
+                if (past) {
+                    const int at = __ffs(past) - 1;
+                    unit += e + at;
+                    t -= __shfl_sync(0xffffffffu, upto - n, at);
+                    break;
+                }
+                t -= __shfl_sync(0xffffffffu, upto, 31);
+            }
+            int left = p.per + (c < p.rem ? 1 : 0);
+            while (left > 0 && segments < CT_MAX_SEGMENTS) {
+                const int n = ct_unit_tiles(p, unit);
+                add(unit, t, min(n, t + left), n);
+                left -= n - t;
+                t = 0;
+                ++unit;
+            }
+        }
+        if (lane == 0) *s_segments = segments;
+    }
+    // rows of a Q tile that no copy writes are zero
+    for (int i = tid; i < 2 * NBOX * (TC_ROWS - p.hb * p.lb) * 8; i += CT_THREADS) {
+        const int chunk = i & 7, box = (i >> 3) % (2 * NBOX), row = (i >> 3) / (2 * NBOX) + p.hb * p.lb;
+        *(uint4 *)(sq + box * TC_BOX + row * 128 + chunk * 16) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    // the first copies are on their way while the others wait for the TMEM columns
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TC_TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    if (warp != 8) {
+        tc_fence_before();
+        asm volatile("bar.sync 1, %0;" ::"n"(CT_THREADS - 32) : "memory");
+        tc_fence_after();
+    }
+    const uint32_t tmem = warp == 8 ? 0u : *tmem_slot;       // (nothing of the producer's)
+    const int segments = *s_segments;
     pdl_wait();  // everything below reads what earlier kernels on the stream wrote
 
-    if (warp == 0) {
-        // ---------------- producer ----------------
-        if (lane == 0) {
+    if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CT_REGS_ISSUE));
+        if (warp == 8 && lane == 0) {
+            // ---------------- producer ----------------
             bool ok = true;
-            mbar_expect_tx(&bars[BAR_Q], QKV_TILE);
+            uint32_t slot = 0, round = 0, q_used[2] = {0, 0};
+            auto load_tile = [&](const CUtensorMap *map, int t, int hk, int b) {
+                if (round > 0 && !mbar_wait(&bars[BAR::RING_EMPTY + slot], (round - 1) & 1)) return false;
+                unsigned char *dst = ring + (size_t)slot * TILE;
+                mbar_expect_tx(&bars[BAR::RING_FULL + slot], TILE);
 #pragma unroll
-            for (int bx = 0; bx < NBOX; ++bx) tma_load_4d(sq + bx * TC_BOX, &qmap, &bars[BAR_Q], bx * 64, l0, hq, b);
-            // A K slot is free as soon as its score product is done, a V slot only after the output
-            // product one tile later: K runs one tile ahead of V so that neither waits for the other.
-            auto load_k = [&](int j) {
-                const int s = j % TC_STAGES;
-                if (j >= TC_STAGES && !mbar_wait(&bars[BAR_K_EMPTY + s], ((j / TC_STAGES) - 1) & 1)) return false;
-                unsigned char *kt = skv + (size_t)s * 2 * QKV_TILE;
-                mbar_expect_tx(&bars[BAR_K_FULL + s], QKV_TILE);
-#pragma unroll
-                for (int bx = 0; bx < NBOX; ++bx) tma_load_4d(kt + bx * TC_BOX, &kmap, &bars[BAR_K_FULL + s], bx * 64, j * TC_KEYS, hk, b);
+                for (int bx = 0; bx < NBOX; ++bx) tma_load_4d(dst + bx * TC_BOX, map, &bars[BAR::RING_FULL + slot], bx * 64, t * TC_KEYS, hk, b);
+                if (++slot == STAGES) {
+                    slot = 0;
+                    ++round;
+                }
                 return true;
             };
-            auto load_v = [&](int j) {
-                const int s = j % TC_STAGES;
-                if (j >= TC_STAGES && !mbar_wait(&bars[BAR_V_EMPTY + s], ((j / TC_STAGES) - 1) & 1)) return false;
-                unsigned char *vt = skv + (size_t)s * 2 * QKV_TILE + QKV_TILE;
-                mbar_expect_tx(&bars[BAR_V_FULL + s], QKV_TILE);
+            for (int sg = 0; ok && sg < segments; ++sg) {
+                const CtSegment g = s_seg[sg];
+                const int group = g.unit / p.units, hk = group % p.Hkv, b = group / p.Hkv;
+                ok = load_tile(&kmap, g.t0, hk, b);
+                for (int i = 0; ok && i <= g.has_b; ++i) {
+                    if (q_used[i] > 0) ok = mbar_wait(&bars[BAR::Q_EMPTY + i], (q_used[i] - 1) & 1);
+                    if (!ok) break;
+                    ++q_used[i];
+                    const int rt = 2 * ct_pair_of(p, g.unit) + i;
+                    mbar_expect_tx(&bars[BAR::Q_FULL + i], (uint32_t)(p.hb * p.lb * 128 * NBOX));
 #pragma unroll
-                for (int bx = 0; bx < NBOX; ++bx) tma_load_4d(vt + bx * TC_BOX, &vmap, &bars[BAR_V_FULL + s], bx * 64, j * TC_KEYS, hk, b);
-                return true;
-            };
-            if (n_tiles > 0) ok = load_k(0);
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                if (j + 1 < n_tiles) ok = load_k(j + 1);
-                if (ok) ok = load_v(j);
+                    for (int bx = 0; bx < NBOX; ++bx)
+                        tma_load_5d(sq + i * TILE + bx * TC_BOX, &qmap, &bars[BAR::Q_FULL + i], bx * 64, (rt % p.head_tiles) * p.hb,
+                                    (rt / p.head_tiles) * p.lb, hk, b);
+                }
+                for (int t = g.t0; ok && t < g.t1; ++t) {
+                    if (t > g.t0) ok = load_tile(&kmap, t, hk, b);
+                    if (ok) ok = load_tile(&vmap, t, hk, b);
+                }
             }
             if (!ok) atomicExch(p.status, 21);
-        }
-    } else if (warp == 1) {
-        // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        } else if (warp == 9) {
+            // ---------------- MMA issue ----------------
             // instruction descriptor: f32 accumulator (bits 4-5 = 1), A and B formats (bits 7-9 and 10-12:
             // 0 = f16, 1 = bf16), B major at bit 16 (1 = MN-major), N / 8 at bits 17-22, M / 16 at 24-28
-            constexpr uint32_t FMT = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+            constexpr uint32_t FMT = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
             constexpr uint32_t IDESC = (1u << 4) | (FMT << 7) | (FMT << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
             // the O product has N = D columns
             constexpr uint32_t IDESC_PV = (1u << 4) | (FMT << 7) | (FMT << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((128u >> 4) << 24);
             // Descriptors differ only in the start-address field (16-byte units): a box is 1024 units, a
             // k-step inside a box row 2, 16 keys of the MN-major V tile 128.
             const uint64_t q_desc = umma_desc(smem_u32(sq), 16, 1024);
-            const uint64_t k_desc = umma_desc(smem_u32(skv), 16, 1024);
-            const uint64_t v_desc = umma_desc(smem_u32(skv) + QKV_TILE, 16384, 1024);
-            bool ok = mbar_wait(&bars[BAR_Q], 0);
-            auto issue_s = [&](int j) {
-                const int s = j % TC_STAGES;
-                if (!mbar_wait(&bars[BAR_K_FULL + s], (j / TC_STAGES) & 1)) return false;
-                if (j >= 2 && !mbar_wait(&bars[BAR_S_EMPTY + (j & 1)], ((j >> 1) - 1) & 1)) return false;
-                tc_fence_after();
-                const uint64_t kd = k_desc + (uint64_t)(s * (2 * QKV_TILE / 16));
-                const uint32_t d_addr = tmem + (uint32_t)(j & 1) * 128u;
-#pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint64_t off = (uint64_t)((ks >> 2) * (TC_BOX / 16) + (ks & 3) * 2);
-                    umma_f16(d_addr, q_desc + off, kd + off, IDESC, ks > 0 ? 1u : 0u);
+            const uint64_t k_desc = umma_desc(smem_u32(ring), 16, 1024);
+            const uint64_t v_desc = umma_desc(smem_u32(ring), 16384, 1024);
+            bool ok = true;
+            uint32_t k_slot = 0, k_par = 0, v_slot = 1, v_par = 0;   // ring entries of the next K and V tile
+            uint32_t q_par = 0, p_par = 0;                           // bit i: row tile i
+            auto step2 = [](uint32_t &slot, uint32_t &par) {
+                slot += 2;
+                if (slot >= (uint32_t)STAGES) {
+                    slot -= STAGES;
+                    par ^= 1;
                 }
-                umma_commit(&bars[BAR_S_FULL + (j & 1)]);
-                umma_commit(&bars[BAR_K_EMPTY + s]);
-                return true;
             };
-            if (ok) ok = issue_s(0);
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                if (j + 1 < n_tiles) ok = issue_s(j + 1);
-                if (!ok) break;
-                const int s = j % TC_STAGES;
-                ok = mbar_wait(&bars[BAR_V_FULL + s], (j / TC_STAGES) & 1);
-                if (ok) ok = mbar_wait(&bars[BAR_P_FULL + (j & 1)], (j >> 1) & 1);
-                if (ok && j >= 1) ok = mbar_wait(&bars[BAR_O_EMPTY], (j - 1) & 1);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t vd = v_desc + (uint64_t)(s * (2 * QKV_TILE / 16));
-                // TMEM columns: S_0, S_1 at 0, 128; O at 256 (one accumulator: it is folded away long before the
-                // next O product is due); P_0, P_1 at 384, 448, written there by the softmax warps and read as
-                // the A operand (16 keys = 8 columns per product)
-                const uint32_t o_addr = tmem + 256u;
-                const uint32_t p_addr = tmem + 384u + (uint32_t)(j & 1) * 64u;
+            // One step takes the O products of a key tile and the S products of the next one, which may open the next segment.
+            int sg = 0, left = 0;                    // the segment of the next S products, and its tiles still to come
+            bool o_here = false, o_first = false, o_b = false, b = false;   // *b: the unit has a row tile B
+            while (ok) {
+                const bool opens = left == 0 && sg < segments;
+                o_b = b;
+                if (opens) {
+                    left = s_seg[sg].t1 - s_seg[sg].t0;
+                    b = s_seg[sg].has_b != 0;
+                    ++sg;
+                }
+                const bool s_here = left > 0, s_last = left == 1, o_last = o_here && (opens || !s_here);
+                if (!o_here && !s_here) break;
+                if (o_here) ok = warp_wait(&bars[BAR::RING_FULL + v_slot], v_par);
+                if (ok && s_here) ok = warp_wait(&bars[BAR::RING_FULL + k_slot], k_par);
+                const uint64_t kd = k_desc + (uint64_t)(k_slot * (TILE / 16)), vd = v_desc + (uint64_t)(v_slot * (TILE / 16));
+                auto o_part = [&](uint32_t i, auto which) {
+                    constexpr int h = decltype(which)::value, FROM = key_of(h) / 16, TO = key_of(h + 1) / 16;
+                    if (ok) ok = warp_wait(&bars[BAR::P_FULL + 2 * h + i], (p_par >> i) & 1);
+                    if (!ok) return;
+                    tc_fence_after();
+                    if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < TC_KEYS / 16; ++ks)
-                    umma_f16_ts(o_addr, p_addr + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_PV, ks > 0 ? 1u : 0u);
-                umma_commit(&bars[BAR_O_FULL]);
-                umma_commit(&bars[BAR_P_EMPTY + (j & 1)]);
-                umma_commit(&bars[BAR_V_EMPTY + s]);
+                        for (int ks = FROM; ks < TO; ++ks)
+                            umma_f16_ts(tmem + 256u + i * 128u, tmem + i * 128u + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_PV,
+                                        (o_first && ks == 0) ? 0u : 1u);
+                        if (PARTS > 1) umma_commit(&bars[BAR::O_PART + i]);
+                    }
+                    __syncwarp();
+                };
+                // (a part waits for the rescale behind the one before: the other row tile's part runs meanwhile)
+                if (PARTS > 1 && o_here) {
+                    o_part(0, std::integral_constant<int, 0>());
+                    if (o_b) o_part(1, std::integral_constant<int, 0>());
+                }
+                if (PARTS == 4 && o_here) {
+                    o_part(0, std::integral_constant<int, 1>());
+                    if (o_b) o_part(1, std::integral_constant<int, 1>());
+                    o_part(0, std::integral_constant<int, 2>());
+                    if (o_b) o_part(1, std::integral_constant<int, 2>());
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    if (!ok) break;
+                    const bool o_i = o_here && (i == 0 || o_b), s_i = s_here && (i == 0 || b);
+                    if (s_i && opens) {
+                        ok = warp_wait(&bars[BAR::Q_FULL + i], (q_par >> i) & 1);
+                        q_par ^= 1u << i;
+                    }
+                    if (o_i) {
+                        if (PARTS == 1) o_part(i, std::integral_constant<int, 0>());
+                        if (ok) ok = warp_wait(&bars[BAR::P_FULL + 2 * (HANDS - 1) + i], (p_par >> i) & 1);
+                        p_par ^= 1u << i;
+                    }
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t s_addr = tmem + i * 128u;
+                        if (o_i) {
+#pragma unroll
+                            for (int ks = key_of(HANDS - 1) / 16; ks < TC_KEYS / 16; ++ks)
+                                umma_f16_ts(tmem + 256u + i * 128u, s_addr + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_PV, 1u);
+                            if (o_last) umma_commit(&bars[BAR::O_FULL + i]);
+                        }
+                        if (s_i) {
+                            const uint64_t qd = q_desc + (uint64_t)(i * (TILE / 16));
+#pragma unroll
+                            for (int ks = 0; ks < D / 16; ++ks) {
+                                const uint64_t off = (uint64_t)((ks >> 2) * (TC_BOX / 16) + (ks & 3) * 2);
+                                umma_f16(s_addr, qd + off, kd + off, IDESC, ks > 0 ? 1u : 0u);
+                            }
+                            umma_commit(&bars[BAR::S_FULL + i]);
+                            if (s_last) umma_commit(&bars[BAR::Q_EMPTY + i]);
+                        }
+                        if (i == 1) {
+                            if (o_here) umma_commit(&bars[BAR::RING_EMPTY + v_slot]);
+                            if (s_here) umma_commit(&bars[BAR::RING_EMPTY + k_slot]);
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (o_here) step2(v_slot, v_par);
+                if (s_here) step2(k_slot, k_par);
+                o_here = s_here;
+                o_first = opens;
+                if (s_here) --left;
             }
             if (!ok) atomicExch(p.status, 22);
         }
-    } else if (warp < 6) {
-        // ---------------- softmax: thread = row ----------------
+    } else {
+        // ---------------- softmax and output: thread = row ----------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CT_REGS_SOFTMAX));
+        const int i = warp >> 2;                            // row tile A / B
         const int quarter = warp & 3;                       // the TMEM lanes this warp may touch
         const int row = quarter * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-        const int64_t l = (int64_t)l0 + row;
-        const int64_t limit = p.causal ? min(p.T - 1, p.causal_offset + l) : p.T - 1;   // last visible key
-        const int64_t block_min_limit = p.causal ? min(p.T - 1, p.causal_offset + l0) : p.T - 1;
-        float m_run = -INFINITY, l_run = 0.f;
+        const uint32_t s_addr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)i * 128u;
+        const uint32_t o_addr = s_addr + 256u;
+        const int row_l = row / p.hb, row_h = row % p.hb;
+        const uint64_t scale2 = pack_f2(p.scale_log2, p.scale_log2);
+        uint32_t s_par = 0, o_par = 0, g_par = 0, h_par = 0;
         bool ok = true;
-        for (int j = 0; j < n_tiles; ++j) {
-            ok = mbar_wait(&bars[BAR_S_FULL + (j & 1)], (j >> 1) & 1);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t s_addr = lane_addr + (uint32_t)(j & 1) * 128u;
-            uint32_t raw[TC_KEYS];
+        for (int sg = 0; ok && sg < segments; ++sg) {
+            const CtSegment w = s_seg[sg];
+            if (i == 1 && !w.has_b) continue;
+            const int rt = 2 * ct_pair_of(p, w.unit) + i;
+            const int l0 = (rt / p.head_tiles) * p.lb;
+            const int l = l0 + row_l, h = (rt % p.head_tiles) * p.hb + row_h;
+            const bool valid = row < p.hb * p.lb && l < p.L && h < p.rep;
+            const int limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l) : p.T - 1);     // last visible key
+            const int tile_limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l0) : p.T - 1);
+            float m_top = -INFINITY, m_ref = -INFINITY, l_run = 0.f;   // largest score, reference of O and of l_run
+            for (int t = w.t0; t < w.t1; ++t) {
+                ok = warp_wait(&bars[BAR::S_FULL + i], s_par);
+                if (!ok) break;
+                s_par ^= 1;
+                tc_fence_after();
+                uint32_t raw[TC_KEYS];
 #pragma unroll
-            for (int cb = 0; cb < 4; ++cb) tmem_ld32_issue(s_addr + cb * 32, raw + cb * 32);
-            tmem_ld_wait();
-            // the scores are in registers: the S buffer is free for tile j + 2
-            tc_fence_before();
-            mbar_arrive(&bars[BAR_S_EMPTY + (j & 1)]);
-            const int64_t key0 = (int64_t)j * TC_KEYS;
-            if (key0 + TC_KEYS - 1 > block_min_limit) {   // some row of the block loses keys in this tile
-#pragma unroll
-                for (int i = 0; i < TC_KEYS; ++i)
-                    if (key0 + i > limit) raw[i] = 0xff800000u;   // -inf
-            }
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int i = 0; i < TC_KEYS; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(raw[i]));
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            const float m_new = fmaxf(m_run, mx * p.scale_log2);
-            const float alpha = (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - m_new);
-            const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
-            // hand the tile's rescale factor to the correction warps
-            if (j >= 2) ok = mbar_wait(&bars[BAR_A_EMPTY + (j & 1)], ((j >> 1) - 1) & 1);
-            if (!ok) break;
-            s_alpha[(j & 1) * TC_ROWS + row] = alpha;
-            mbar_arrive(&bars[BAR_A_FULL + (j & 1)]);
-            // this P tile is free once the O product of two tiles ago has read it
-            if (j >= 2) ok = mbar_wait(&bars[BAR_P_EMPTY + (j & 1)], ((j >> 1) - 1) & 1);
-            if (!ok) break;
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int kc = 0; kc < TC_KEYS / 8; ++kc) {   // 16-byte chunk (8 keys) of the row
-                float e[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    e[i] = fast_exp2(fmaf(__uint_as_float(raw[kc * 8 + i]), p.scale_log2, neg_m));   // exp2(-inf) = 0
-                    sum4[i & 3] += e[i];
-                }
-                // the probabilities as pairs, kept in the registers the scores came in (entry 4 kc + q of the
-                // packed row: always behind the scores still to be read)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) raw[kc * 4 + q] = pack_pair<T>(e[2 * q], e[2 * q + 1]);
-                // P_j goes into TMEM (this thread's lane), where the O product reads it as its A operand
-                if (kc == 7) tmem_st32_issue(lane_addr + 384u + (uint32_t)(j & 1) * 64u, raw);
-            }
-            tmem_st32_issue(lane_addr + 384u + (uint32_t)(j & 1) * 64u + 32u, raw + 32);
-            tmem_st_wait();
-            tc_fence_before();
-            mbar_arrive(&bars[BAR_P_FULL + (j & 1)]);
-            l_run = l_run * alpha + (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-            m_run = m_new;
-        }
-        if (ok) {
-            s_lsum[row] = l_run;
-            mbar_arrive(&bars[BAR_L_FULL]);
-        } else {
-            atomicExch(p.status, 23);
-        }
-    } else {
-        // ---------------- correction: thread = row ----------------
-        const int quarter = warp & 3;
-        const int row = quarter * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + 256u;
-        const int64_t l = (int64_t)l0 + row;
-        float o_acc[D];
-#pragma unroll
-        for (int i = 0; i < D; ++i) o_acc[i] = 0.f;
-        bool ok = true;
-        for (int j = 0; j < n_tiles; ++j) {
-            ok = mbar_wait(&bars[BAR_A_FULL + (j & 1)], (j >> 1) & 1);
-            if (!ok) break;
-            const float alpha = s_alpha[(j & 1) * TC_ROWS + row];
-            mbar_arrive(&bars[BAR_A_EMPTY + (j & 1)]);
-            ok = mbar_wait(&bars[BAR_O_FULL], j & 1);
-            if (!ok) break;
-            tc_fence_after();
-#pragma unroll
-            for (int half = 0; half < D / 64; ++half) {
-                uint32_t raw[64];
-                tmem_ld32_issue(lane_addr + half * 64, raw);
-                tmem_ld32_issue(lane_addr + half * 64 + 32, raw + 32);
+                for (int cb = 0; cb < 4; ++cb) tmem_ld32_issue(s_addr + cb * 32, raw + cb * 32);
                 tmem_ld_wait();
+                if (t * TC_KEYS + TC_KEYS - 1 > tile_limit) {   // some row of the tile loses keys here
+                    const int last = limit - t * TC_KEYS;
 #pragma unroll
-                for (int i = 0; i < 64; ++i) o_acc[half * 64 + i] = fmaf(o_acc[half * 64 + i], alpha, __uint_as_float(raw[i]));
+                    for (int k = 0; k < TC_KEYS; ++k)
+                        if (k > last) raw[k] = 0xff800000u;   // -inf
+                }
+                float ref[PARTS], alpha[PARTS];
+#pragma unroll
+                for (int part = 0; part < PARTS; ++part) {
+                    constexpr int KEYS = TC_KEYS / PARTS;
+                    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                    for (int k = part * KEYS; k < (part + 1) * KEYS; k += 2)
+                        mx4[(k >> 1) & 3] = fmaxf(mx4[(k >> 1) & 3], fmaxf(__uint_as_float(raw[k]), __uint_as_float(raw[k + 1])));
+                    const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+                    m_top = fmaxf(m_top, mx);
+                    ref[part] = PARTS > 1 ? fmaxf(mx, m_top - CT_SPAN_LOG2) : m_top;
+                    alpha[part] = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - ref[part]);
+                    m_ref = ref[part];
+                }
+                // O is settled when the scores are there: they came behind the O products of the tile before
+                auto hand_over = [&](auto which) {
+                    constexpr int h = decltype(which)::value, FROM = key_of(h), TO = key_of(h + 1), part = PARTS == 1 ? 0 : h;
+                    const bool first = h == 0, move = (first ? t > w.t0 : PARTS > 1) && __any_sync(0xffffffffu, alpha[part] != 1.f);
+                    const uint64_t alpha2 = pack_f2(alpha[part], alpha[part]);
+                    constexpr int CH = PARTS == 1 ? 32 : 16;   // columns of O at a time (16: 3 % slower with one reference)
+                    uint32_t o[CH];
+                    auto o_load = [&](int cb) {
+                        if constexpr (CH == 32) tmem_ld32_issue(o_addr + cb * CH, o);
+                        else tmem_ld16_issue(o_addr + cb * CH, o);
+                    };
+                    auto o_store = [&](int cb) {
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int k = 0; k < CH; k += 2) {
+                            float lo, hi;
+                            unpack_f2(mul_f2(pack_f2(__uint_as_float(o[k]), __uint_as_float(o[k + 1])), alpha2), lo, hi);
+                            o[k] = __float_as_uint(lo);
+                            o[k + 1] = __float_as_uint(hi);
+                        }
+                        if constexpr (CH == 32) tmem_st32_issue(o_addr + cb * CH, o);
+                        else tmem_st16_issue(o_addr + cb * CH, o);
+                    };
+                    const float neg_m = ref[part] == -INFINITY ? 0.f : -ref[part];   // exp2(-inf) = 0
+                    const uint64_t neg2 = pack_f2(neg_m, neg_m);
+                    uint64_t sum[2] = {0, 0};
+#pragma unroll
+                    for (int k0 = FROM; k0 < TO; k0 += CH) {
+                        // a rescale of O runs under the exponentials: they wait for the special-function unit
+                        if (first && move && k0 < D) o_load(k0 / CH);
+#pragma unroll
+                        for (int k = k0; k < k0 + CH; k += 2) {
+                            float e0, e1;
+                            unpack_f2(fma_f2(pack_f2(__uint_as_float(raw[k]), __uint_as_float(raw[k + 1])), scale2, neg2), e0, e1);
+                            e0 = fast_exp2(e0);
+                            e1 = fast_exp2(e1);
+                            sum[(k >> 1) & 1] = add_f2(sum[(k >> 1) & 1], pack_f2(e0, e1));
+                            // the probabilities as pairs, kept in the registers the scores came in
+                            raw[k >> 1] = pack_pair<T>(e0, e1);
+                        }
+                        if (first && move && k0 < D) o_store(k0 / CH);
+                    }
+                    if (!first && PARTS > 1) {
+                        if (ok) ok = warp_wait(&bars[BAR::O_PART + i], h_par);
+                        h_par ^= 1;
+                        tc_fence_after();
+                    }
+                    if (move)
+#pragma unroll
+                        for (int cb = first ? TO / CH : 0; cb < D / CH; ++cb) {
+                            o_load(cb);
+                            o_store(cb);
+                        }
+#pragma unroll
+                    for (int c = FROM / 2; c < TO / 2; c += 16) tmem_st16_issue(s_addr + c, raw + c);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    mbar_arrive(&bars[BAR::P_FULL + 2 * h + i]);
+                    float s0, s1, s2, s3;
+                    unpack_f2(sum[0], s0, s1);
+                    unpack_f2(sum[1], s2, s3);
+                    l_run = fmaf(l_run, first || PARTS > 1 ? alpha[part] : 1.f, (s0 + s1) + (s2 + s3));
+                };
+                hand_over(std::integral_constant<int, 0>());
+                hand_over(std::integral_constant<int, 1>());
+                if (PARTS == 4) {
+                    hand_over(std::integral_constant<int, PARTS == 4 ? 2 : 0>());
+                    hand_over(std::integral_constant<int, PARTS == 4 ? 3 : 0>());
+                }
+                if (!ok) break;
             }
-            tc_fence_before();
-            mbar_arrive(&bars[BAR_O_EMPTY]);
-        }
-        if (ok) ok = mbar_wait(&bars[BAR_L_FULL], 0);
-        if (!ok) {
-            atomicExch(p.status, 24);
-        } else if (l < p.L) {
-            const float l_sum = s_lsum[row];
+            if (!ok) break;
+            ok = warp_wait(&bars[BAR::O_FULL + i], o_par);
+            if (!ok) break;
+            o_par ^= 1;
+            tc_fence_after();
+            const int group = w.unit / p.units, hk = group % p.Hkv, b = group / p.Hkv;
+            T *dst = (T *)p.out + b * p.o_sb + (int64_t)(hk * p.rep + h) * p.o_sh + (int64_t)l * p.o_sl;
+            if (w.t0 == 0 && w.t1 == w.n) {
+                const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+#pragma unroll 1
+                for (int cb = 0; cb < D / 32; ++cb) {
+                    float o[32];
+                    tmem_ld32(o_addr + cb * 32, o);
+                    if (valid) store_row32<T>(dst + cb * 32, o, inv);
+                }
+                continue;
+            }
+            // ---- the unit is cut: leave a partial; the CTA that leaves the last one merges them ----
+            const int c = blockIdx.x;
+            {
+                const int64_t slot = ((int64_t)c * 2 + (sg == p.waves ? 0 : 1)) * 2 + i;
+                float4 *po = (float4 *)p.o_part + slot * (D / 4) * TC_ROWS + row;
+#pragma unroll 1
+                for (int cb = 0; cb < D / 32; ++cb) {
+                    float o[32];
+                    tmem_ld32(o_addr + cb * 32, o);
+#pragma unroll
+                    for (int c4 = 0; c4 < 8; ++c4) po[(cb * 8 + c4) * TC_ROWS] = make_float4(o[c4 * 4], o[c4 * 4 + 1], o[c4 * 4 + 2], o[c4 * 4 + 3]);
+                }
+                p.ml_part[slot * TC_ROWS + row] = make_float2(m_ref, l_run);
+            }
+            __threadfence();
+            mbar_arrive(&bars[BAR::GROUP + i]);
+            ok = warp_wait(&bars[BAR::GROUP + i], g_par);
+            if (!ok) break;
+            g_par ^= 1;
+            // the CTAs c0 ... c1 that own pieces of the unit: [x, x + n) of the tail
+            int c0, c1;
+            bool starts = true;   // the unit opens its first CTA's range
+            if (p.pieces > 0) {
+                c0 = w.unit * p.pieces;
+                c1 = c0 + p.pieces - 1;
+            } else {
+                int x = c * p.per + min(c, p.rem) - s_seg[p.waves].t0;
+                for (int k = p.waves; k < sg; ++k) x += s_seg[k].n;
+                const int big = p.rem * (p.per + 1);
+                auto cta_of = [&](int f) { return f < big ? f / (p.per + 1) : p.rem + (f - big) / p.per; };
+                c0 = cta_of(x);
+                c1 = cta_of(x + w.n - 1);
+                starts = x == c0 * p.per + min(c0, p.rem);
+            }
+            if (row == 0) s_ticket[i] = atomicAdd(&p.tickets[(w.unit - p.waves * (int)gridDim.x) * 2 + i], 1);
+            mbar_arrive(&bars[BAR::GROUP + i]);
+            ok = warp_wait(&bars[BAR::GROUP + i], g_par);
+            if (!ok) break;
+            g_par ^= 1;
+            if (s_ticket[i] != c1 - c0) continue;
+            __threadfence();
+            auto slot_of = [&](int cc) { return ((int64_t)cc * 2 + (cc == c0 && !starts ? 1 : 0)) * 2 + i; };
+            // two partials at a time: sixteen vectors of a thread in flight
+            constexpr int AT_ONCE = 2;
+            float m = -INFINITY, l_sum = 0.f;
+            auto ml_of = [&](int cc) {
+                return cc <= c1 ? __ldcg(&p.ml_part[slot_of(cc) * TC_ROWS + row]) : make_float2(-INFINITY, 0.f);
+            };
+            for (int cc = c0; cc <= c1; cc += AT_ONCE) {
+                float2 ml[AT_ONCE];
+#pragma unroll
+                for (int j = 0; j < AT_ONCE; ++j) ml[j] = ml_of(cc + j);
+#pragma unroll
+                for (int j = 0; j < AT_ONCE; ++j) {
+                    const float m_new = fmaxf(m, ml[j].x);
+                    if (m_new != -INFINITY) l_sum = l_sum * fast_exp2(m - m_new) + ml[j].y * fast_exp2(ml[j].x - m_new);
+                    m = m_new;
+                }
+            }
             const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
-            T *dst = (T *)p.out + b * p.o_sb + hq * p.o_sh + l * p.o_sl;
+#pragma unroll 1
+            for (int cb = 0; cb < D / 32; ++cb) {
+                float acc[32];
 #pragma unroll
-            for (int c8 = 0; c8 < D / 8; ++c8) {
-                uint4 w;
-                w.x = pack_pair<T>(o_acc[c8 * 8 + 0] * inv, o_acc[c8 * 8 + 1] * inv);
-                w.y = pack_pair<T>(o_acc[c8 * 8 + 2] * inv, o_acc[c8 * 8 + 3] * inv);
-                w.z = pack_pair<T>(o_acc[c8 * 8 + 4] * inv, o_acc[c8 * 8 + 5] * inv);
-                w.w = pack_pair<T>(o_acc[c8 * 8 + 6] * inv, o_acc[c8 * 8 + 7] * inv);
-                *(uint4 *)(dst + c8 * 8) = w;
+                for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+#pragma unroll 1
+                for (int cc = c0; cc <= c1; cc += AT_ONCE) {
+                    float4 v[AT_ONCE][8];
+                    float f[AT_ONCE];
+#pragma unroll
+                    for (int j = 0; j < AT_ONCE; ++j) {
+                        const float4 *po = (const float4 *)p.o_part + slot_of(cc + j) * (D / 4) * TC_ROWS + row;
+                        f[j] = ml_of(cc + j).x;
+#pragma unroll
+                        for (int c4 = 0; c4 < 8; ++c4) v[j][c4] = cc + j <= c1 ? __ldcg(&po[(cb * 8 + c4) * TC_ROWS]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int j = 0; j < AT_ONCE; ++j) {
+                        f[j] = f[j] == -INFINITY ? 0.f : fast_exp2(f[j] - m);
+#pragma unroll
+                        for (int c4 = 0; c4 < 8; ++c4) {
+                            acc[c4 * 4 + 0] = fmaf(v[j][c4].x, f[j], acc[c4 * 4 + 0]);
+                            acc[c4 * 4 + 1] = fmaf(v[j][c4].y, f[j], acc[c4 * 4 + 1]);
+                            acc[c4 * 4 + 2] = fmaf(v[j][c4].z, f[j], acc[c4 * 4 + 2]);
+                            acc[c4 * 4 + 3] = fmaf(v[j][c4].w, f[j], acc[c4 * 4 + 3]);
+                        }
+                    }
+                }
+                if (valid) store_row32<T>(dst + cb * 32, acc, inv);
             }
         }
+        if (!ok) atomicExch(p.status, 23);
     }
     // all roles meet here; TMEM goes back whatever happened
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 9) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
     }
 }
 
-template <typename T, int D>
-bool launch_tc_typed(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkTcParams &p, int ctas,
-                     cudaStream_t stream) {
-    const size_t smem = (size_t)(D / 64) * TC_BOX * (1 + 2 * TC_STAGES) + BAR_COUNT * sizeof(uint64_t) + 64 +
-                        3 * TC_ROWS * sizeof(float) + 1024;
+template <typename T, int D, int PARTS>
+bool launch_tc_as(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkTcParams &p, int ctas,
+                  cudaStream_t stream) {
+    const size_t smem = (size_t)(D / 64) * TC_BOX * (2 + ct_stages<D>()) + Bars<ct_stages<D>()>::COUNT * sizeof(uint64_t) + 16 +
+                        CT_MAX_SEGMENTS * sizeof(CtSegment) + 1024;
+    static_assert((D / 64) * TC_BOX * (2 + ct_stages<D>()) + Bars<ct_stages<D>()>::COUNT * 8 + 16 + CT_MAX_SEGMENTS * sizeof(CtSegment) + 1024 <= 232448,
+                  "more shared memory than a CTA may have");
     // 0 = not yet, 1 = ready, -1 = refused; distinct handles may call from distinct host threads
     static std::atomic<int> configured[64];
     const int dev = current_device();
@@ -377,23 +708,62 @@ bool launch_tc_typed(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUt
     int state = configured[dev].load(std::memory_order_acquire);
     if (state == 0) {
         // setting the attribute twice from two racing threads is harmless; the result is the same
-        const cudaError_t e = cudaFuncSetAttribute(attn_chunk_tc_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_chunk_tc_kernel<T, D, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) (void)cudaGetLastError();
         state = e == cudaSuccess ? 1 : -1;
         configured[dev].store(state, std::memory_order_release);
     }
     if (state < 0) return false;
     KernelTimer timer(stream);
-    KVC_CUDA(launch_pdl(attn_chunk_tc_kernel<T, D>, dim3(ctas), dim3(TC_THREADS), smem, stream, qmap, kmap, vmap, p));
+    KVC_CUDA(launch_pdl(attn_chunk_tc_kernel<T, D, PARTS>, dim3(ctas), dim3(CT_THREADS), smem, stream, qmap, kmap, vmap, p));
     timer.stop();
     ++g_launch_count;
     return true;
 }
 
+template <typename T, int D>
+bool launch_tc_typed(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkTcParams &p, int ctas, int parts,
+                     cudaStream_t stream) {
+    if (parts == 4) return launch_tc_as<T, D, 4>(qmap, kmap, vmap, p, ctas, stream);
+    return parts == 2 ? launch_tc_as<T, D, 2>(qmap, kmap, vmap, p, ctas, stream) : launch_tc_as<T, D, 1>(qmap, kmap, vmap, p, ctas, stream);
+}
+
+// Queries [B, Hq, L, D] as (dim, head of the group, position, KV head, batch): a box is hb heads x lb positions of 64 dims.
+bool make_query_map(CUtensorMap *map, const AttnArgs &a, int rep, int hb, int lb) {
+    EncodeTiledFn fn = encode_tiled_tc();
+    if (!fn) return false;
+    const int64_t row = a.q_sl * 2, head = a.Hq > 1 ? a.q_sh * 2 : row;
+    const cuuint64_t dims[5] = {(cuuint64_t)a.D, (cuuint64_t)rep, (cuuint64_t)a.L, (cuuint64_t)a.Hkv, (cuuint64_t)a.B};
+    const cuuint64_t strides[4] = {(cuuint64_t)head, (cuuint64_t)row, (cuuint64_t)(head * rep), (cuuint64_t)(a.B > 1 ? a.q_sb * 2 : head)};
+    const cuuint32_t box[5] = {64, (cuuint32_t)hb, (cuuint32_t)lb, 1, 1};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUtensorMapDataType dt = a.q_dtype == KVC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    return fn(map, dt, 5, const_cast<void *>(a.q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Device memory for the length of one call, in stream order (inside a capture: of the graph). Null where there is no room.
+struct CallMemory {
+    void *ptr = nullptr;
+    cudaStream_t stream;
+    CallMemory(size_t bytes, cudaStream_t s) : stream(s) {
+        if (bytes > 0) ptr = dev_try_alloc(bytes, s);
+    }
+    ~CallMemory() { dev_free(ptr, stream); }   // nothing for a null pointer
+    CallMemory(const CallMemory &) = delete;
+    CallMemory &operator=(const CallMemory &) = delete;
+};
+
+// 128-row blocks of the call's query rows, head by head.
+int64_t row_blocks_of(const AttnArgs &a) { return (int64_t)a.B * a.Hq * ((a.L + TC_ROWS - 1) / TC_ROWS); }
+
+// Fewer blocks than half the part holds, or few positions.
+bool few_blocks(const AttnArgs &a) { return row_blocks_of(a) < sm_count(a.device) / 2 || a.L < 64; }
+
 }  // namespace
 
-// Returns 1 when the call was taken (head dim 64 or 128, f16 / bf16 raw K and V, no array mask, enough
-// 128-row blocks to fill the part), 0 otherwise. KVC_CHUNK_TC=0 turns the path off.
+// Returns 1 when the call was taken (head dim 64 or 128, f16 / bf16 raw K and V, no array mask), 0 otherwise.
+// KVC_CHUNK_TC=0 turns the path off.
 bool attention_chunk_tc_accepts(const AttnArgs &a) {
     static const bool off = [] {
         const char *e = std::getenv("KVC_CHUNK_TC");
@@ -403,13 +773,16 @@ bool attention_chunk_tc_accepts(const AttnArgs &a) {
     if ((a.D != 128 && a.D != 64) || (a.q_dtype != KVC_BF16 && a.q_dtype != KVC_F16)) return false;
     if (a.k.kind != SRC_RAW || a.v.kind != SRC_RAW || a.k.dtype != a.q_dtype || a.v.dtype != a.q_dtype) return false;
     if (a.mask.mode == KVC_MASK_ARRAY || a.q_signs || a.o_signs || a.q_calib || a.new_k || a.q_rot || a.o_rot) return false;
-    if (a.Hkv <= 0 || a.Hq % a.Hkv || a.T < 1 || a.T > (int64_t)1 << 30 || a.L < 64) return false;
+    if (a.Hkv <= 0 || a.Hq % a.Hkv || a.T < 1 || a.T > (int64_t)1 << 30) return false;
+    // Up to 64 rows of a KV head's group the decode and verify kernels do less work on rows that are not there; from there on
+    // (8 of 32 heads, D 128, behind 4 096 keys) 64 positions take 38 us here and 82 on the mma.sync chunk kernel, 128 of 16
+    // sequences 0.6 of its time. (More than 128 heads of a group at few positions leave a row tile nearly empty.)
+    const int64_t rep = a.Hq / a.Hkv;
+    if (a.L < 64 && (rep * a.L <= 64 || rep > TC_ROWS)) return false;
+    // (one tile of that kernel's keys: its maximum per 16 of them is the more precise one, and little is left to gain)
+    if (few_blocks(a) && a.T <= 64) return false;
     if (a.mask.mode == KVC_MASK_CAUSAL && a.mask.causal_offset < 0) return false;
-    const int64_t row_blocks = ((int64_t)a.L + TC_ROWS - 1) / TC_ROWS;
-    const int64_t ctas = (int64_t)a.B * a.Hq * row_blocks;
-    // a CTA owns an SM (its TMEM and 193 KB of shared memory): fewer blocks than half the part run
-    // better on the split-K kernel
-    if (ctas < sm_count(a.device) / 2 || ctas > (int64_t)1 << 30) return false;
+    if (row_blocks_of(a) > (int64_t)1 << 30) return false;
     if (!strides_fit(a.q, a.D, a.q_sl, a.q_sh, a.q_sb, a.Hq, a.B)) return false;
     if (!strides_fit(a.k.data, a.D, a.k.st, a.k.sh, a.k.sb, a.Hkv, a.B) || !strides_fit(a.v.data, a.D, a.v.st, a.v.sh, a.v.sb, a.Hkv, a.B))
         return false;
@@ -419,31 +792,112 @@ bool attention_chunk_tc_accepts(const AttnArgs &a) {
 
 int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     if (!attention_chunk_tc_accepts(a)) return 0;
-    const int64_t row_blocks = ((int64_t)a.L + TC_ROWS - 1) / TC_ROWS;
-    const int64_t ctas = (int64_t)a.B * a.Hq * row_blocks;
     int *status = device_status_word(a.device);
     if (!status) return 0;
-    CUtensorMap qmap, kmap, vmap;
-    if (!make_map_tc(&qmap, a.q, a.q_dtype, a.D, a.L, a.Hq, a.B, a.q_sl, a.q_sh, a.q_sb)) return 0;
-    if (!make_map_tc(&kmap, a.k.data, a.k.dtype, a.D, a.T, a.Hkv, a.B, a.k.st, a.k.sh, a.k.sb)) return 0;
-    if (!make_map_tc(&vmap, a.v.data, a.v.dtype, a.D, a.T, a.Hkv, a.B, a.v.st, a.v.sh, a.v.sb)) return 0;
     ChunkTcParams p = {};
     p.out = a.out;
     p.o_sb = a.o_sb; p.o_sh = a.o_sh; p.o_sl = a.o_sl;
-    p.B = a.B; p.Hq = a.Hq; p.Hkv = a.Hkv; p.L = a.L; p.T = a.T;
-    p.row_blocks = (int)row_blocks;
+    p.B = a.B; p.rep = a.Hq / a.Hkv; p.Hkv = a.Hkv; p.L = a.L; p.T = a.T;
     p.causal = a.mask.mode == KVC_MASK_CAUSAL ? 1 : 0;
     p.causal_offset = a.mask.causal_offset;
     p.scale_log2 = a.scale * 1.4426950408889634f;
     p.status = status;
+    // a row tile holds all heads of the group at 128 / rep positions, or 128 positions of one head: the one with fewer tiles
+    const int64_t one_head = (int64_t)p.rep * ((a.L + TC_ROWS - 1) / TC_ROWS);
+    p.hb = 1; p.lb = TC_ROWS;
+    if (p.rep <= TC_ROWS && (a.L + TC_ROWS / p.rep - 1) / (TC_ROWS / p.rep) <= one_head) {
+        p.hb = p.rep;
+        p.lb = TC_ROWS / p.rep;
+    }
+    p.head_tiles = p.rep / p.hb;
+    const int64_t row_tiles = (int64_t)p.head_tiles * ((a.L + p.lb - 1) / p.lb);
+    if (row_tiles > (int64_t)1 << 20) return 0;
+    p.row_tiles = (int)row_tiles;
+    p.units = (p.row_tiles + 1) / 2;
+    const int64_t groups = (int64_t)a.B * a.Hkv;
+    int64_t group_tiles = 0;
+    int most = 0, least = INT_MAX;
+    for (int u = 0; u < p.units; ++u) {
+        const int n = ct_unit_tiles(p, u);
+        group_tiles += n;
+        most = std::max(most, n);
+        least = std::min(least, n);
+    }
+    if (groups * p.units > (int64_t)1 << 28) return 0;
+    p.all_units = (int)(groups * p.units);
+
+    CUtensorMap qmap, kmap, vmap;
+    if (!make_query_map(&qmap, a, p.rep, p.hb, p.lb)) return 0;
+    if (!make_map_tc(&kmap, a.k.data, a.k.dtype, a.D, a.T, a.Hkv, a.B, a.k.st, a.k.sh, a.k.sb)) return 0;
+    if (!make_map_tc(&vmap, a.v.data, a.v.dtype, a.D, a.T, a.Hkv, a.B, a.v.st, a.v.sh, a.v.sb)) return 0;
+
+    // How the units are handed out, judged by the key tiles of the busiest SM (a CTA's start takes about three tiles' time,
+    // the change of a unit one, writing a partial two, merging one a half):
+    //   whole units in rounds, one per SM, or, where units differ much, a CTA for each;
+    //   few units: all cut into the same number of pieces, a CTA for each piece;
+    //   equal ranges of all units end to end: evenest, but the CTAs are spread over all of K and V at once, so only where
+    //     those stay in L2 (8 x 8 heads of 8 704 keys, 285 MB: 2.1 GB came from HBM in a launch);
+    //   whole units in rounds, so that neighbours share their K and V tiles, and equal ranges of what is left.
+    constexpr int64_t L2_BYTES = (int64_t)64 << 20;
+    const int64_t sms = sm_count(a.device), units = p.all_units, flat = groups * group_tiles, average = (flat + units - 1) / units;
+    const bool settled = groups * a.T * a.D * 4 <= L2_BYTES;
+    const int64_t rounds = (units + sms - 1) / sms;
+    const bool even = least * 4 >= most * 3 && rounds <= CT_MAX_SEGMENTS;
+    const int64_t waves = settled ? 0 : units / sms;
+    const int64_t tail = settled ? flat : (units - waves * sms) * average, per = (tail + sms - 1) / sms;   // (exact length below)
+    const int64_t pieces = std::min<int64_t>(sms / units, least / 2);
+    const int64_t whole = even ? 3 + rounds * (average + 1) : std::max<int64_t>(most, rounds * average) + 3 * rounds;
+    const int64_t cut = 3 + waves * (most + 1) + per + 3 + (most / std::max<int64_t>(per, 1) + 2) / 2;
+    const int64_t apart = pieces > 1 ? 3 + (most + pieces - 1) / pieces + 2 + pieces / 2 : INT64_MAX;
+    int64_t tail_tiles = 0, ranges = 0;
+    if (apart < whole && apart <= cut) {
+        ranges = units * pieces;
+    } else if (cut < whole && waves + 2 < CT_MAX_SEGMENTS) {
+        tail_tiles = flat;
+        for (int64_t u = 0; u < waves * sms; ++u) tail_tiles -= ct_unit_tiles(p, (int)(u % p.units));
+        ranges = std::max<int64_t>(1, std::min<int64_t>(sms, tail_tiles / 4));
+        if (tail_tiles < 1 || tail_tiles > (int64_t)1 << 29 || group_tiles > (int64_t)1 << 29 ||
+            tail_tiles / ranges / least + 2 > CT_MAX_SEGMENTS - waves)
+            ranges = 0;
+    }
+    const size_t part = (size_t)ranges * 4 * TC_ROWS;
+    const size_t o_bytes = part * a.D * sizeof(float), ml_bytes = part * sizeof(float2);
+    const size_t t_bytes = (size_t)(tail_tiles > 0 ? units - waves * sms : units) * 2 * sizeof(int);
+    CallMemory mem(ranges > 0 ? o_bytes + ml_bytes + t_bytes : 0, stream);
+    int64_t ctas = even ? std::min(units, sms) : units;
+    p.waves = even ? (int)rounds : 1;
+    if (mem.ptr) {
+        p.o_part = (float *)mem.ptr;
+        p.ml_part = (float2 *)((char *)mem.ptr + o_bytes);
+        p.tickets = (int *)((char *)p.ml_part + ml_bytes);
+        KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
+        if (tail_tiles > 0) {
+            ctas = waves > 0 ? sms : ranges;
+            p.waves = (int)waves;
+            p.ranges = (int)ranges;
+            p.per = (int)(tail_tiles / ranges);
+            p.rem = (int)(tail_tiles % ranges);
+            p.group_tiles = (int)group_tiles;
+            for (int64_t u = waves * sms / p.units * p.units; u < waves * sms; ++u) p.tail_base += ct_unit_tiles(p, (int)u);
+        } else {
+            ctas = ranges;
+            p.waves = 0;
+            p.pieces = (int)pieces;
+        }
+    }
+    // Small calls take a finer reference: they spend their time on the start, the partials and the merge, and the mma.sync
+    // chunk kernel that takes them otherwise errs by little (a running maximum per 16 keys, in splits of 64 keys and up).
+    const int parts = few_blocks(a) ? (a.T < 2048 ? 4 : 2) : 1;
     bool taken;
     if (a.D == 128)
-        taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 128>(qmap, kmap, vmap, p, (int)ctas, stream)
-                                      : launch_tc_typed<__half, 128>(qmap, kmap, vmap, p, (int)ctas, stream);
+        taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 128>(qmap, kmap, vmap, p, (int)ctas, parts, stream)
+                                      : launch_tc_typed<__half, 128>(qmap, kmap, vmap, p, (int)ctas, parts, stream);
     else
-        taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 64>(qmap, kmap, vmap, p, (int)ctas, stream)
-                                      : launch_tc_typed<__half, 64>(qmap, kmap, vmap, p, (int)ctas, stream);
-    if (taken && trace_dispatch()) fprintf(stderr, "[kvc] chunk_tc: %lld CTAs of 128 rows\n", (long long)ctas);
+        taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 64>(qmap, kmap, vmap, p, (int)ctas, parts, stream)
+                                      : launch_tc_typed<__half, 64>(qmap, kmap, vmap, p, (int)ctas, parts, stream);
+    if (taken && trace_dispatch())
+        fprintf(stderr, "[kvc] chunk_tc: %lld units of two row tiles (%d heads x %d positions), %lld CTAs, %d rounds, ranges of %d tiles, %d pieces, %d references a tile\n",
+                (long long)units, p.hb, p.lb, (long long)ctas, p.waves, p.per, p.pieces, parts);
     return taken ? 1 : 0;
 }
 
