@@ -63,58 +63,80 @@ struct MatParams {
     void *k_out, *v_out;        // [B, H, T, D] contiguous
     int32_t B, H, D;
     int64_t T;
-    int32_t turbo;
 };
 
-// One thread = eight consecutive head dims of one token of K or V (blockIdx.z = 2 * b + which).
+// One thread = eight consecutive head dims of MAT_ROWS tokens of K or V (blockIdx.z = 2 * b + which).
 // T: dtype of the affine scales / biases; TO: dtype of the rows written (T for affine, f16 for TurboQuant).
-template <typename T, typename TO>
+// Bound by the 16-bit rows it writes. The loads of its tokens are all in flight before the first is used, and a centroid
+// is looked up in a table with a copy for every lane (no bank conflicts; indexed in the launch's parameters, lanes that
+// differ take turns). Four layers of a 512-token chunk behind 8 192 tokens, 4 sequences, 64/8 heads, K 3- / V 4-bit
+// indices: 3.23 -> 2.91 ms for the calls; 4-bit affine rows behind 4 096 tokens: 606 -> 600 us.
+constexpr int MAT_ROWS = 4;
+template <typename T, typename TO, int D, bool TURBO>
 __global__ void __launch_bounds__(256) materialize_kernel(const __grid_constant__ MatParams p) {
+    constexpr int PER_ROW = D / 8, STEP = 256 / PER_ROW;
+    __shared__ float table[TURBO ? 16 * 32 : 1];
     const int which = blockIdx.z & 1, b = blockIdx.z >> 1, h = blockIdx.y;
     const MatSource &s = which ? p.v : p.k;
-    const int per_row = p.D / 8;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.T * per_row) return;
-    const int64_t t = i / per_row;
-    const int d0 = (int)(i % per_row) * 8;
-    const uint32_t *row = s.codes + b * s.sb + h * s.sh + t * s.st;
-    float x[8];
-    if (!p.turbo) {
-        const int g = d0 / s.group;
-        const int64_t gi = b * s.gsb + h * s.gsh + t * s.gst + g;
-        const float sc = to_f32<T>(((const T *)s.scales)[gi]), bi = to_f32<T>(((const T *)s.biases)[gi]);
-        if (s.bits == 4) {
-            const uint32_t w = row[d0 / 8];
+    const int lane = threadIdx.x & 31, d0 = ((int)threadIdx.x % PER_ROW) * 8;
+    const int64_t t0 = (int64_t)blockIdx.x * (STEP * MAT_ROWS) + (int)threadIdx.x / PER_ROW;
+    const uint32_t *row0 = s.codes + b * s.sb + h * s.sh;
+    const int64_t g0 = b * s.gsb + h * s.gsh;
+    uint32_t w[MAT_ROWS][2];
+    float f0[MAT_ROWS], f1[MAT_ROWS];
+    const int bit0 = d0 * s.bits, w0 = bit0 >> 5, words = (D * s.bits + 31) / 32;
+    const bool second = TURBO ? w0 + 1 < words : s.bits == 8;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = fmaf(sc, (float)((w >> (4 * j)) & 15u), bi);
-        } else if (s.bits == 8) {
-            const uint32_t w0 = row[d0 / 4], w1 = row[d0 / 4 + 1];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                x[j] = fmaf(sc, (float)((w0 >> (8 * j)) & 255u), bi);
-                x[4 + j] = fmaf(sc, (float)((w1 >> (8 * j)) & 255u), bi);
+    for (int r = 0; r < MAT_ROWS; ++r) {
+        const int64_t t = t0 + r * STEP;
+        w[r][0] = w[r][1] = 0u;
+        f0[r] = f1[r] = 0.f;
+        if (t < p.T) {
+            const uint32_t *row = row0 + t * s.st + w0;
+            w[r][0] = row[0];
+            if (second) w[r][1] = row[1];
+            if (TURBO) {
+                f0[r] = s.norms[g0 + t * s.gst];
+            } else {
+                const int64_t gi = g0 + t * s.gst + d0 / s.group;
+                f0[r] = to_f32<T>(((const T *)s.scales)[gi]);
+                f1[r] = to_f32<T>(((const T *)s.biases)[gi]);
             }
-        } else {  // 2 bits
-            const uint32_t w = row[d0 / 16] >> ((d0 % 16) * 2);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = fmaf(sc, (float)((w >> (2 * j)) & 3u), bi);
         }
-    } else {
-        // indices are a low-bit-first stream of `bits` per dim; eight of them start at bit d0 * bits
-        const float nrm = s.norms[b * s.gsb + h * s.gsh + t * s.gst];
-        const int bit0 = d0 * s.bits, w0 = bit0 >> 5, sh = bit0 & 31;
-        const int words = (p.D * s.bits + 31) / 32;
-        uint64_t win = row[w0];
-        if (w0 + 1 < words) win |= (uint64_t)row[w0 + 1] << 32;
-        win >>= sh;
-        const uint32_t m = (1u << s.bits) - 1u;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = fminf(fmaxf(nrm * s.codebook[(uint32_t)(win >> (j * s.bits)) & m], -65504.f), 65504.f);
     }
-    uint4 o;
-    o.x = pack2<TO>(x[0], x[1]); o.y = pack2<TO>(x[2], x[3]); o.z = pack2<TO>(x[4], x[5]); o.w = pack2<TO>(x[6], x[7]);
-    TO *out = (TO *)(which ? p.v_out : p.k_out) + (((int64_t)b * p.H + h) * p.T + t) * p.D + d0;
-    *(uint4 *)out = o;
+    if (TURBO) {
+        for (int i = threadIdx.x; i < 16 * 32; i += 256) table[i] = s.codebook[i >> 5];
+        __syncthreads();
+    }
+    TO *out = (TO *)(which ? p.v_out : p.k_out) + (((int64_t)b * p.H + h) * p.T) * D + d0;
+    const int shift = bit0 & 31;
+    const uint32_t m = (1u << s.bits) - 1u;
+#pragma unroll
+    for (int r = 0; r < MAT_ROWS; ++r) {
+        const int64_t t = t0 + r * STEP;
+        if (t >= p.T) break;
+        float x[8];
+        // codes are a low-bit-first stream of `bits` per dim
+        const uint64_t win = (w[r][0] | (uint64_t)w[r][1] << 32) >> shift;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t code = (uint32_t)(win >> (j * s.bits)) & m;
+            if (TURBO) x[j] = fminf(fmaxf(f0[r] * table[code * 32 + lane], -65504.f), 65504.f);
+            else x[j] = fmaf(f0[r], (float)code, f1[r]);
+        }
+        uint4 o;
+        o.x = pack2<TO>(x[0], x[1]); o.y = pack2<TO>(x[2], x[3]); o.z = pack2<TO>(x[4], x[5]); o.w = pack2<TO>(x[6], x[7]);
+        *(uint4 *)(out + t * D) = o;
+    }
+}
+
+template <typename T, bool TURBO> void materialize(const MatParams &p, cudaStream_t stream) {
+    const int per_block = 256 / (p.D / 8) * MAT_ROWS;
+    const dim3 grid((unsigned)((p.T + per_block - 1) / per_block), (unsigned)p.H, (unsigned)(2 * p.B));
+    if (p.D == 128) materialize_kernel<T, T, 128, TURBO><<<grid, 256, 0, stream>>>(p);
+    else materialize_kernel<T, T, 64, TURBO><<<grid, 256, 0, stream>>>(p);
+    KVC_CUDA(cudaGetLastError());
+    ++g_launch_count;
 }
 
 struct RotParams {
@@ -284,14 +306,9 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
         mp.v = to_mat(a.v, b0);
         mp.k_out = k_out; mp.v_out = v_out;
         mp.B = nb; mp.H = a.Hkv; mp.D = a.D; mp.T = a.T;
-        mp.turbo = turbo ? 1 : 0;
-        const int64_t per_head = a.T * (a.D / 8);
-        const dim3 grid((unsigned)((per_head + 255) / 256), (unsigned)a.Hkv, (unsigned)(2 * nb));
-        if (turbo) materialize_kernel<__half, __half><<<grid, 256, 0, stream>>>(mp);
-        else if (a.q_dtype == KVC_BF16) materialize_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>(mp);
-        else materialize_kernel<__half, __half><<<grid, 256, 0, stream>>>(mp);
-        KVC_CUDA(cudaGetLastError());
-        ++g_launch_count;
+        if (turbo) materialize<__half, true>(mp, stream);
+        else if (a.q_dtype == KVC_BF16) materialize<__nv_bfloat16, false>(mp, stream);
+        else materialize<__half, false>(mp, stream);
         ++launches;
 
         AttnArgs call = r;
