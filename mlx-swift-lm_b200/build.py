@@ -29,7 +29,7 @@ SOURCES = [
     "attn_turbo.cu", "attn_turbo_v4.cu",
     "attn_f32.cu", "attn_stream.cu", "attn_stream_bf16_64.cu", "attn_stream_bf16_128.cu", "attn_stream_bf16_256.cu",
     "attn_stream_f16_64.cu", "attn_stream_f16_128.cu", "attn_stream_f16_256.cu",
-    "attn_chunk_packed.cu", "attn_chunk_tc.cu", "attn_chunk_mat.cu", "attn_chunk_pairs.cu", "attn_verify_tc.cu",
+    "attn_chunk_packed.cu", "attn_chunk_tc.cu", "attn_chunk_one_tc.cu", "attn_chunk_mat.cu", "attn_chunk_pairs.cu", "attn_verify_tc.cu",
     "attn_dispatch.cu",
     "cache.cu",
     "round.cu",

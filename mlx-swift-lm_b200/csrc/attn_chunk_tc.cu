@@ -124,64 +124,6 @@ struct CtSegment {
 };
 constexpr int CT_MAX_SEGMENTS = 40;
 
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z, int u, int v) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(u), "r"(v)
-        : "memory");
-}
-
-// True in one lane of a converged warp. The MMA warp runs its loop with all lanes and picks the lane only around the
-// instructions themselves: under a branch on the lane number every descriptor takes the slow way from vector to uniform
-// registers (70 ... 100 cycles per product, against the 64 the tensor core needs for it).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-    return one != 0;
-}
-
-// One wait of a whole warp: all its threads carry on, or none does.
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
-}
-
-// Two fp32 operations an instruction.
-__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack_f2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// 32 output columns of a row as 16-bit values.
-template <typename T> __device__ __forceinline__ void store_row32(T *dst, const float *o, float inv) {
-#pragma unroll
-    for (int c8 = 0; c8 < 4; ++c8) {
-        uint4 v;
-        v.x = pack_pair<T>(o[c8 * 8 + 0] * inv, o[c8 * 8 + 1] * inv);
-        v.y = pack_pair<T>(o[c8 * 8 + 2] * inv, o[c8 * 8 + 3] * inv);
-        v.z = pack_pair<T>(o[c8 * 8 + 4] * inv, o[c8 * 8 + 5] * inv);
-        v.w = pack_pair<T>(o[c8 * 8 + 6] * inv, o[c8 * 8 + 7] * inv);
-        *(uint4 *)(dst + c8 * 8) = v;
-    }
-}
-
 template <typename T, int D, int PARTS>
 __global__ void __launch_bounds__(CT_THREADS, 1)
 attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
@@ -727,32 +669,6 @@ bool launch_tc_typed(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUt
     if (parts == 4) return launch_tc_as<T, D, 4>(qmap, kmap, vmap, p, ctas, stream);
     return parts == 2 ? launch_tc_as<T, D, 2>(qmap, kmap, vmap, p, ctas, stream) : launch_tc_as<T, D, 1>(qmap, kmap, vmap, p, ctas, stream);
 }
-
-// Queries [B, Hq, L, D] as (dim, head of the group, position, KV head, batch): a box is hb heads x lb positions of 64 dims.
-bool make_query_map(CUtensorMap *map, const AttnArgs &a, int rep, int hb, int lb) {
-    EncodeTiledFn fn = encode_tiled_tc();
-    if (!fn) return false;
-    const int64_t row = a.q_sl * 2, head = a.Hq > 1 ? a.q_sh * 2 : row;
-    const cuuint64_t dims[5] = {(cuuint64_t)a.D, (cuuint64_t)rep, (cuuint64_t)a.L, (cuuint64_t)a.Hkv, (cuuint64_t)a.B};
-    const cuuint64_t strides[4] = {(cuuint64_t)head, (cuuint64_t)row, (cuuint64_t)(head * rep), (cuuint64_t)(a.B > 1 ? a.q_sb * 2 : head)};
-    const cuuint32_t box[5] = {64, (cuuint32_t)hb, (cuuint32_t)lb, 1, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const CUtensorMapDataType dt = a.q_dtype == KVC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    return fn(map, dt, 5, const_cast<void *>(a.q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// Device memory for the length of one call, in stream order (inside a capture: of the graph). Null where there is no room.
-struct CallMemory {
-    void *ptr = nullptr;
-    cudaStream_t stream;
-    CallMemory(size_t bytes, cudaStream_t s) : stream(s) {
-        if (bytes > 0) ptr = dev_try_alloc(bytes, s);
-    }
-    ~CallMemory() { dev_free(ptr, stream); }   // nothing for a null pointer
-    CallMemory(const CallMemory &) = delete;
-    CallMemory &operator=(const CallMemory &) = delete;
-};
 
 // 128-row blocks of the call's query rows, head by head.
 int64_t row_blocks_of(const AttnArgs &a) { return (int64_t)a.B * a.Hq * ((a.L + TC_ROWS - 1) / TC_ROWS); }

@@ -131,6 +131,23 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return r;
 }
 
+// Bits of 32 mask bytes starting at p (any alignment), the first n of them inside the row.
+__device__ __forceinline__ uint32_t mask_bits32(const uint8_t *p, int n) {
+    if (n <= 0) return 0;
+    n = min(n, 32);
+    const uint32_t *w = (const uint32_t *)((uintptr_t)p & ~(uintptr_t)3);
+    const int sh = (int)((uintptr_t)p & 3) * 8, words = (n + (sh >> 3) + 3) >> 2;   // only words that hold a byte of the row
+    uint32_t bits = 0, cur = __ldg(w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t nxt = i + 1 < words ? __ldg(w + i + 1) : 0u;
+        const uint32_t b = __vcmpne4(__funnelshift_r(cur, nxt, sh), 0u) & 0x08040201u;
+        bits |= ((b | b >> 8 | b >> 16 | b >> 24) & 15u) << (4 * i);
+        cur = nxt;
+    }
+    return n == 32 ? bits : bits & ((1u << n) - 1u);
+}
+
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])

@@ -1006,23 +1006,6 @@ flat_list_merge_kernel(const __grid_constant__ FlatList list, const __grid_const
 // that are decoded from codes. T: f16, or bf16 for raw bf16 keys and their queries, which are exact as they are.
 // ---------------------------------------------------------------------
 
-// Bits of 32 mask bytes starting at p (any alignment), the first n of them inside the row.
-__device__ __forceinline__ uint32_t mask_bits32(const uint8_t *p, int n) {
-    if (n <= 0) return 0;
-    n = min(n, 32);
-    const uint32_t *w = (const uint32_t *)((uintptr_t)p & ~(uintptr_t)3);
-    const int sh = (int)((uintptr_t)p & 3) * 8, words = (n + (sh >> 3) + 3) >> 2;   // only words that hold a byte of the row
-    uint32_t bits = 0, cur = __ldg(w);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t nxt = i + 1 < words ? __ldg(w + i + 1) : 0u;
-        const uint32_t b = __vcmpne4(__funnelshift_r(cur, nxt, sh), 0u) & 0x08040201u;
-        bits |= ((b | b >> 8 | b >> 16 | b >> 24) & 15u) << (4 * i);
-        cur = nxt;
-    }
-    return n == 32 ? bits : bits & ((1u << n) - 1u);
-}
-
 __device__ __forceinline__ float mask_value(const MaskDesc &m, int64_t i) {
     switch (m.dtype) {
         case KVC_BOOL: return ((const uint8_t *)m.data)[i] ? 0.f : -INFINITY;

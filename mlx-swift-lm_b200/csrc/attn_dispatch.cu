@@ -16,6 +16,7 @@ int launch_attention_stream_list(const AttnArgs *args, int n, cudaStream_t strea
 int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t stream);
 int launch_attention_chunk_packed(const AttnArgs &a, cudaStream_t stream);
 int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream);
+int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream);
 int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream);
 int launch_attention_chunk_packed_pairs(const AttnArgs &a, cudaStream_t stream);
 int launch_attention_verify_tc_raw(const AttnArgs &a, cudaStream_t stream);
@@ -34,7 +35,9 @@ bool force_general() {
 
 int launch_attention(const AttnArgs &a, cudaStream_t stream) {
     if (!force_general()) {
-        int n = launch_attention_chunk_tc(a, stream);   // long chunks over raw caches: tcgen05 kernel
+        int n = launch_attention_chunk_tc(a, stream);   // chunks over raw caches: tcgen05 kernel
+        if (n > 0) return n;
+        n = launch_attention_chunk_one(a, stream);   // ... under boolean array masks, and at head dim 256
         if (n > 0) return n;
         n = launch_attention_verify_tc_raw(a, stream);   // verify rounds of 17 ... 64 rows per KV head over raw caches
         if (n > 0) return n;

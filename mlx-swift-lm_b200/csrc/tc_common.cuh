@@ -7,6 +7,7 @@
 
 #include "attn_common.cuh"
 #include "common.h"
+#include "f32x2.cuh"
 
 namespace kvc {
 namespace tc {
@@ -114,7 +115,41 @@ template <> __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float l
     return r;
 }
 
-// Barrier slots in shared memory.
+__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z, int u, int v) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(u), "r"(v)
+        : "memory");
+}
+
+// True in one lane of a converged warp. The MMA warp runs its loop with all lanes and picks the lane only around the
+// instructions themselves: under a branch on the lane number every descriptor takes the slow way from vector to uniform
+// registers (70 ... 100 cycles per product, against the 64 the tensor core needs for it).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+
+// One wait of a whole warp: all its threads carry on, or none does.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
+// 32 output columns of a row as 16-bit values.
+template <typename T> __device__ __forceinline__ void store_row32(T *dst, const float *o, float inv) {
+#pragma unroll
+    for (int c8 = 0; c8 < 4; ++c8) {
+        uint4 v;
+        v.x = pack_pair<T>(o[c8 * 8 + 0] * inv, o[c8 * 8 + 1] * inv);
+        v.y = pack_pair<T>(o[c8 * 8 + 2] * inv, o[c8 * 8 + 3] * inv);
+        v.z = pack_pair<T>(o[c8 * 8 + 4] * inv, o[c8 * 8 + 5] * inv);
+        v.w = pack_pair<T>(o[c8 * 8 + 6] * inv, o[c8 * 8 + 7] * inv);
+        *(uint4 *)(dst + c8 * 8) = v;
+    }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -132,16 +167,16 @@ inline EncodeTiledFn encode_tiled_tc() {
     return fn;
 }
 
-// [B, H, rows, D] view, element strides (inner 1): boxes of 128 rows x 64 elements, 128-byte swizzle,
+// [B, H, rows, D] view, element strides (inner 1): boxes of box_rows rows x 64 elements, 128-byte swizzle,
 // rows beyond `rows` read as zero.
 inline bool make_map_tc(CUtensorMap *map, const void *data, int32_t dtype, int D, int64_t rows, int H, int B, int64_t s_row,
-                 int64_t s_h, int64_t s_b) {
+                 int64_t s_h, int64_t s_b, int box_rows = 128) {
     EncodeTiledFn fn = encode_tiled_tc();
     if (!fn) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)rows, (cuuint64_t)H, (cuuint64_t)B};
     const cuuint64_t strides[3] = {(cuuint64_t)s_row * 2, (cuuint64_t)(H > 1 ? s_h : s_row * rows) * 2,
                                    (cuuint64_t)(B > 1 ? s_b : (H > 1 ? s_h * H : s_row * rows)) * 2};
-    const cuuint32_t box[4] = {64, 128, 1, 1};
+    const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUtensorMapDataType dt = dtype == KVC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     return fn(map, dt, 4, const_cast<void *>(data), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -156,7 +191,31 @@ inline bool strides_fit(const void *data, int D, int64_t s_row, int64_t s_h, int
     return true;
 }
 
-// Returns false when the device does not grant the kernel its shared memory (the caller falls back to
-// the mma.sync chunk kernel).
+// Queries [B, Hq, L, D] as (dim, head of the group, position, KV head, batch): a box is hb heads x lb positions of 64 dims.
+inline bool make_query_map(CUtensorMap *map, const AttnArgs &a, int rep, int hb, int lb) {
+    EncodeTiledFn fn = encode_tiled_tc();
+    if (!fn) return false;
+    const int64_t row = a.q_sl * 2, head = a.Hq > 1 ? a.q_sh * 2 : row;
+    const cuuint64_t dims[5] = {(cuuint64_t)a.D, (cuuint64_t)rep, (cuuint64_t)a.L, (cuuint64_t)a.Hkv, (cuuint64_t)a.B};
+    const cuuint64_t strides[4] = {(cuuint64_t)head, (cuuint64_t)row, (cuuint64_t)(head * rep), (cuuint64_t)(a.B > 1 ? a.q_sb * 2 : head)};
+    const cuuint32_t box[5] = {64, (cuuint32_t)hb, (cuuint32_t)lb, 1, 1};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUtensorMapDataType dt = a.q_dtype == KVC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    return fn(map, dt, 5, const_cast<void *>(a.q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Device memory for the length of one call, in stream order (inside a capture: of the graph). Null where there is no room.
+struct CallMemory {
+    void *ptr = nullptr;
+    cudaStream_t stream;
+    CallMemory(size_t bytes, cudaStream_t s) : stream(s) {
+        if (bytes > 0) ptr = dev_try_alloc(bytes, s);
+    }
+    ~CallMemory() { dev_free(ptr, stream); }   // nothing for a null pointer
+    CallMemory(const CallMemory &) = delete;
+    CallMemory &operator=(const CallMemory &) = delete;
+};
+
 }  // namespace tc
 }  // namespace kvc

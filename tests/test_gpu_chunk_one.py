@@ -1,0 +1,71 @@
+"""The tcgen05 chunk kernel that keeps P as pairs: boolean array masks, and head dim 256."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(cuda, dtype, B, Hq, Hkv, D, L, T, seed=1):
+    def rand(i, *shape):
+        return torch.randn(shape, generator=torch.Generator(cuda).manual_seed(seed + i), device=cuda).to(dtype)
+    return rand(0, B, Hq, L, D), rand(1, B, Hkv, T, D), rand(2, B, Hkv, T, D)
+
+
+def _check(kvc, capfd, q, k, v, mask, seen):
+    """Against plain fp32 attention; P is exact to 2^-16 (pairs), so what is left is the store: half a spacing of the output,
+    and 2^-14 of the largest value for P, the exponentials and sums in another order."""
+    dtype, rep, scale = q.dtype, q.shape[1] // k.shape[1], q.shape[-1] ** -0.5
+    kr, vr = (x.float().repeat_interleave(rep, 1) for x in (k, v))
+    s = ((q.float() @ kr.transpose(-1, -2)) * scale).masked_fill(~seen, float("-inf"))
+    ref = torch.nan_to_num(torch.softmax(s, -1), nan=0.0) @ vr
+    out = kvc.scaled_dot_product_attention(q, k, v, scale, mask)
+    torch.cuda.synchronize()
+    assert "chunk_one" in capfd.readouterr().err
+    store = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert ((out.float() - ref).abs() <= store * ref.abs() + 2.0 ** -14 * v.abs().max()).all()
+    assert not out[~seen.expand_as(s).any(-1)].any()
+    assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,Hq,Hkv,D,L,T,window", [
+    (4, 4, 1, 256, 512, 1023, 512),     # sliding window, its tiles shared among pieces
+    (1, 16, 16, 64, 70, 300, 100),      # one head a row tile; two CTAs an SM
+    (2, 28, 4, 128, 37, 65, 30),        # one key past the calls of the mma.sync kernel; 126 rows a row tile
+    (1, 8, 1, 256, 20, 4097, 64),       # most tiles unseen: pieces with nothing to do
+    (9, 32, 8, 128, 129, 200, 128),     # more row tiles than places: no pieces
+])
+def test_window_masks(kvc, cuda, capfd, monkeypatch, dtype, B, Hq, Hkv, D, L, T, window):
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    q, k, v = _case(cuda, dtype, B, Hq, Hkv, D, L, T)
+    i, j = torch.arange(T - L, T, device=cuda)[:, None], torch.arange(T, device=cuda)[None]
+    seen = (j <= i) & (j > i - window)
+    _check(kvc, capfd, q, k, v, seen, seen)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("form", ["heads", "batch", "odd rows"])
+def test_masks_of_any_form(kvc, cuda, capfd, monkeypatch, D, form):
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    B, Hq, Hkv, L, T = 2, 6, 2, 75, 333
+    q, k, v = _case(cuda, torch.bfloat16, B, Hq, Hkv, D, L, T)
+    shape = {"heads": (1, Hq, L, T + 3), "batch": (B, 1, L, T + 3), "odd rows": (L, T + 3)}[form]
+    m = torch.rand(shape, generator=torch.Generator(cuda).manual_seed(7), device=cuda) < 0.3
+    m[..., 5, :] = False                      # a position that sees nothing
+    m[..., 64:192] = False                    # tiles that nobody sees
+    m = m[..., 3:]                            # rows that begin anywhere
+    _check(kvc, capfd, q, k, v, m, m)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,Hq,Hkv,L,T,mask", [
+    (1, 4, 1, 512, 2048, "causal"), (3, 8, 8, 66, 127, "none"), (1, 2, 1, 129, 129, "causal"), (2, 4, 1, 17, 3000, "causal"),
+])
+def test_head_dim_256(kvc, cuda, capfd, monkeypatch, dtype, B, Hq, Hkv, L, T, mask):
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    q, k, v = _case(cuda, dtype, B, Hq, Hkv, 256, L, T)
+    seen = torch.ones(L, T, dtype=torch.bool, device=cuda)
+    if mask == "causal":
+        seen = seen.tril(T - L)
+    _check(kvc, capfd, q, k, v, mask, seen)
+    _check(kvc, capfd, q.transpose(1, 2).contiguous().transpose(1, 2), k, v, mask, seen)
