@@ -9,6 +9,7 @@
 //   * sums run sequentially over a lane's own elements, then over the xor
 //     butterfly 16, 8, 4, 2, 1 across lanes.
 #include "common.h"
+#include "f32x2.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1076,32 +1077,51 @@ template <int D> __device__ __forceinline__ float tree_sum(float (&p)[16 / (D / 
 template <int D>
 __device__ __forceinline__ float rotate_wide(const float (&sg)[16], int l, float (&v)[16]) {
     constexpr int E = D / 32, RUNS = 16 / E, LPR = D / 16;
-    float p[RUNS];
+    using namespace dev;
+    uint64_t x[8];                                   // dims 2i and 2i + 1
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = pack_f2(v[2 * i], v[2 * i + 1]);
+    float sq[16], p[RUNS];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) unpack_f2(mul_f2(x[i], x[i]), sq[2 * i], sq[2 * i + 1]);
 #pragma unroll
     for (int j = 0; j < RUNS; ++j) {
-        p[j] = __fmul_rn(v[j * E], v[j * E]);
+        p[j] = sq[j * E];
 #pragma unroll
-        for (int i = 1; i < E; ++i) p[j] = __fadd_rn(p[j], __fmul_rn(v[j * E + i], v[j * E + i]));
+        for (int i = 1; i < E; ++i) p[j] = __fadd_rn(p[j], sq[j * E + i]);
     }
     const float norm = __fsqrt_rn(tree_sum<D>(p));
     const float inv_norm = (norm > 1e-8f) ? __frcp_rn(norm) : 0.0f;
+    const uint64_t inv2 = pack_f2(inv_norm, inv_norm), minus = pack_f2(-1.f, -1.f);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], __fmul_rn(inv_norm, sg[i]));
+    for (int i = 0; i < 8; ++i) {
+        x[i] = mul_f2(x[i], mul_f2(inv2, pack_f2(sg[2 * i], sg[2 * i + 1])));
+        float lo, hi;
+        unpack_f2(x[i], lo, hi);
+        x[i] = pack_f2(__fadd_rn(lo, hi), __fsub_rn(lo, hi));
+    }
 #pragma unroll
-    for (int st = 1; st < 16; st <<= 1)
+    for (int st = 1; st < 8; st <<= 1)               // (dims 2 st apart)
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
+        for (int i = 0; i < 8; ++i)
             if ((i & st) == 0) {
-                const float lo = v[i], hi = v[i + st];
-                v[i] = __fadd_rn(lo, hi);
-                v[i + st] = __fsub_rn(lo, hi);
+                const uint64_t lo = x[i], hi = x[i + st];
+                x[i] = add_f2(lo, hi);
+                x[i + st] = fma_f2(hi, minus, lo);
             }
 #pragma unroll
     for (int m = 1; m < LPR; m <<= 1) {
         const float sign = (l & m) ? -1.f : 1.f;
+        const uint64_t sign2 = pack_f2(sign, sign);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __fmaf_rn(v[i], sign, __shfl_xor_sync(0xffffffffu, v[i], m));
+        for (int i = 0; i < 8; ++i) {
+            float lo, hi;
+            unpack_f2(x[i], lo, hi);
+            x[i] = fma_f2(x[i], sign2, pack_f2(__shfl_xor_sync(0xffffffffu, lo, m), __shfl_xor_sync(0xffffffffu, hi, m)));
+        }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) unpack_f2(x[i], v[2 * i], v[2 * i + 1]);
     return norm;
 }
 
@@ -1120,8 +1140,17 @@ __device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a,
     float (&v)[16] = rot;
     load_row_elems<T, 16>(src, v);
     const float norm = rotate_wide<D>(sg, l, v);
+    float place[16];                                 // cell of a value, before it is brought into the table
+    {
+        using namespace dev;
+        const uint64_t dim2 = pack_f2(inv_sqrt_dim, inv_sqrt_dim), scale2 = pack_f2(cells.scale, cells.scale), shift2 = pack_f2(cells.shift, cells.shift);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], inv_sqrt_dim);
+        for (int i = 0; i < 16; i += 2) {
+            const uint64_t x = mul_f2(pack_f2(v[i], v[i + 1]), dim2);
+            unpack_f2(x, v[i], v[i + 1]);
+            if (!CAL) unpack_f2(fma_f2(x, scale2, shift2), place[i], place[i + 1]);
+        }
+    }
     float stored = norm;
     uint32_t w[2] = {0u, 0u};
     constexpr int PER = BITS * 16 > 32 ? 32 / BITS : 16;    // codes per word (3 bits: ten, and the straddling one below)
@@ -1134,7 +1163,7 @@ __device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a,
             cal = a.calib[l * 16 + i];
             x = __fdiv_rn(x, cal);
         }
-        const float u = fminf(fmaxf(__fmaf_rn(x, cells.scale, cells.shift), CELL_MAGIC), CELL_MAGIC + 63.f);
+        const float u = fminf(fmaxf(CAL ? __fmaf_rn(x, cells.scale, cells.shift) : place[i], CELL_MAGIC), CELL_MAGIC + 63.f);
         const float2 e = cell[(__float_as_uint(u) & 63u) * 16];
         const uint32_t idx = __float_as_uint(e.y) + (x > e.x ? 1u : 0u);
         if constexpr (BITS == 3) bits3 = (bits3 << 3) | idx;
@@ -1195,16 +1224,24 @@ struct CalibSums {
     }
     __device__ __forceinline__ void add_row(const float (&rot)[16]) {
         ++rows;
+        using namespace dev;
+        auto both = [](float x) { return pack_f2(x, x); };
+        auto add = [&](int w, int i, uint64_t y, float down, float up) {
+            const uint64_t t = fma_f2(y, both(down), both(CELL_MAGIC));
+            const uint64_t r = add_f2(fma_f2(add_f2(t, both(-CELL_MAGIC)), both(up), y), both(CELL_MAGIC));
+            float t0, t1, r0, r1;
+            unpack_f2(t, t0, t1);
+            unpack_f2(r, r0, r1);
+            top[w][i] += __float_as_uint(t0);
+            top[w][i + 1] += __float_as_uint(t1);
+            rest[w][i] += __float_as_uint(r0);
+            rest[w][i + 1] += __float_as_uint(r1);
+        };
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            auto add = [&](int w, float y, float down, float up) {
-                const float t = __fmaf_rn(y, down, CELL_MAGIC);
-                const float r = __fmaf_rn(__fsub_rn(t, CELL_MAGIC), up, y);
-                top[w][i] += __float_as_uint(t);
-                rest[w][i] += __float_as_uint(__fadd_rn(r, CELL_MAGIC));
-            };
-            add(0, __fmul_rn(rot[i], 1073741824.0f), 6.103515625e-5f, -16384.f);                             // 2^30, parts of 2^14
-            add(1, __fmul_rn(__fmul_rn(rot[i], rot[i]), 68719476736.0f), 1.52587890625e-5f, -65536.f);       // 2^36, parts of 2^16
+        for (int i = 0; i < 16; i += 2) {
+            const uint64_t x = pack_f2(rot[i], rot[i + 1]);
+            add(0, i, mul_f2(x, both(1073741824.0f)), 6.103515625e-5f, -16384.f);                  // 2^30, parts of 2^14
+            add(1, i, mul_f2(mul_f2(x, x), both(68719476736.0f)), 1.52587890625e-5f, -65536.f);    // 2^36, parts of 2^16
         }
     }
 };
