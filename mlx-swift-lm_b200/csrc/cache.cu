@@ -81,19 +81,23 @@ void copy_rows(const Array4 &src, int64_t src_first, Array4 &dst, int64_t dst_fi
     launch_gather(g, s);
 }
 
-void gather_rows(const Array4 &src, Array4 &dst, const std::vector<GatherSeg> &segs, cudaStream_t s) {
+// The rows `segs` selects (in that order) of K and V, to the front of other arrays.
+void gather_rows(const Array4 &k, Array4 &k_dst, const Array4 &v, Array4 &v_dst, const std::vector<GatherSeg> &segs, cudaStream_t s) {
     if (segs.size() > 4) fail(KVC_ERR_INTERNAL, "ring re-order produced more than 4 segments");
-    GatherArgs g;
-    g.src = src.ptr;
-    g.dst = dst.ptr;
-    g.s_sb = src.sb(); g.s_sh = src.sh(); g.s_st = src.st();
-    g.d_sb = dst.sb(); g.d_sh = dst.sh(); g.d_st = dst.st();
-    g.B = (int)src.B; g.H = (int)src.H; g.W = (int)src.W;
-    g.esize = (int)src.esize();
-    g.nseg = (int)segs.size();
-    for (size_t i = 0; i < segs.size(); ++i) g.seg[i] = segs[i];
-    g.dst_start = 0;
-    launch_gather(g, s);
+    auto args = [&](const Array4 &src, const Array4 &dst) {
+        GatherArgs g;
+        g.src = src.ptr;
+        g.dst = dst.ptr;
+        g.s_sb = src.sb(); g.s_sh = src.sh(); g.s_st = src.st();
+        g.d_sb = dst.sb(); g.d_sh = dst.sh(); g.d_st = dst.st();
+        g.B = (int)src.B; g.H = (int)src.H; g.W = (int)src.W;
+        g.esize = (int)src.esize();
+        g.nseg = (int)segs.size();
+        for (size_t i = 0; i < segs.size(); ++i) g.seg[i] = segs[i];
+        g.dst_start = 0;
+        return g;
+    };
+    launch_gather_pair(args(k, k_dst), args(v, v_dst), s);
 }
 
 // Append the rows of `t` ([B, H, S, W], any strides) to `dst` at token `pos`.
@@ -183,8 +187,7 @@ void rot_rebuild(kvc_cache *c, const std::vector<GatherSeg> &segs, int64_t extra
     const int64_t need = std::max<int64_t>(std::max<int64_t>(n + extra_cap, c->cfg.max_size), c->k.cap);
     ensure_like(c->k_alt, c->k, need, s);
     ensure_like(c->v_alt, c->v, need, s);
-    gather_rows(c->k, c->k_alt, segs, s);
-    gather_rows(c->v, c->v_alt, segs, s);
+    gather_rows(c->k, c->k_alt, c->v, c->v_alt, segs, s);
     std::swap(c->k, c->k_alt);
     std::swap(c->v, c->v_alt);
     c->len = n;
@@ -595,8 +598,7 @@ void cache_maybe_trim_front(kvc_cache *c, cudaStream_t s) {
         seg_push(keep, drop, chunk);
         ensure_like(c->k_alt, c->k, std::max<int64_t>(chunk, c->k.cap), s);
         ensure_like(c->v_alt, c->v, std::max<int64_t>(chunk, c->v.cap), s);
-        gather_rows(c->k, c->k_alt, keep, s);
-        gather_rows(c->v, c->v_alt, keep, s);
+        gather_rows(c->k, c->k_alt, c->v, c->v_alt, keep, s);
         std::swap(c->k, c->k_alt);
         std::swap(c->v, c->v_alt);
     }
@@ -2134,8 +2136,7 @@ void cache_logical_view(kvc_cache *c, int64_t tail, cudaStream_t s, kvc_tensor *
     }
     ensure_like(c->k_view, c->k, std::max<int64_t>(n, c->cfg.max_size), s);
     ensure_like(c->v_view, c->v, std::max<int64_t>(n, c->cfg.max_size), s);
-    gather_rows(c->k, c->k_view, segs, s);
-    gather_rows(c->v, c->v_view, segs, s);
+    gather_rows(c->k, c->k_view, c->v, c->v_view, segs, s);
     if (ok) *ok = c->k_view.view(n);
     if (ov) *ov = c->v_view.view(n);
 }

@@ -200,6 +200,8 @@ void launch_append(const AppendArgs &a, cudaStream_t stream);
 // return false when the calls do not fit: the caller then makes them one by one.
 bool launch_append_list(const AppendArgs *args, int n, cudaStream_t stream);
 void launch_gather(const GatherArgs &a, cudaStream_t stream);
+// K and V of one mapping, in one launch where they have one shape.
+void launch_gather_pair(const GatherArgs &k, const GatherArgs &v, cudaStream_t stream);
 
 // Bytes [from, pitch) of every plane of a few arrays, zeroed in one launch.
 struct ZeroTails {
