@@ -13,7 +13,7 @@
 // works through its range unit by unit. In a CTA:
 //   warp 0      loads the group's queries once (TMA, 128 rows x D, rows past the group zero; rotated for
 //               TurboQuant, column-permuted for the affine codec, as they are for raw caches)
-//   warp 1      owns TMEM; lane 0 issues S_j = Q' K_j^T (two tiles ahead) and O_j = P_j V_j
+//   warp 1      owns TMEM and issues S_j = Q' K_j^T (two tiles ahead) and O_j = P_j V_j
 //   warps 4, 5  softmax: thread = query row = TMEM lane 0..63 (a group has at most 64 rows here, and a warp
 //               reaches the TMEM lanes 32 * (warp % 4) ...): scores to probabilities, row sums
 //   warps 8, 9, 12, 13  correction: thread = (query row, half of the dims), folds O_j into the row's
@@ -181,7 +181,8 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     float *s_lsum = s_alpha + 4 * TC_ROWS;                     // [128]
     float *s_mfin = s_lsum + TC_ROWS;                          // [128]
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be the same in all lanes
     const int rep = p.Hq / p.Hkv;
     const int n_all = (int)((p.T + TC_KEYS - 1) / TC_KEYS);
     // The key tiles of all units laid end to end are cut into equal ranges, one per CTA (so that every SM has
@@ -259,8 +260,8 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             tma_load_4d(sq + TC_BOX, &qmap, &bars[VB_Q], 64, 0, unit, 0);
         }
     } else if (warp == 1) {
-        // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        // ---------------- MMA issue: all lanes walk, one issues ----------------
+        {
             // operand formats at bits 7-9 (A) and 10-12 (B): 0 = f16, 1 = bf16
             constexpr uint32_t FMT = std::is_same<TP, __nv_bfloat16>::value ? 1u : 0u;
             constexpr uint32_t IDESC = (1u << 4) | (FMT << 7) | (FMT << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
@@ -268,21 +269,24 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             const uint64_t q_desc = umma_desc(smem_u32(sq), 16, 1024);
             const uint64_t k_desc = umma_desc(smem_u32(skv), 16, 1024);
             const uint64_t v_desc = umma_desc(smem_u32(skv) + VT_TILE, 16384, 1024);
-            bool ok = mbar_wait(&bars[VB_Q], 0);
+            bool ok = warp_wait(&bars[VB_Q], 0);
             auto issue_s = [&](int j) {
                 const int s = j & 1;
-                if (!mbar_wait(&bars[VB_K_FULL + s], (j >> 1) & 1)) return false;
-                if (j >= 2 && !mbar_wait(&bars[VB_S_EMPTY + s], ((j >> 1) - 1) & 1)) return false;
+                if (!warp_wait(&bars[VB_K_FULL + s], (j >> 1) & 1)) return false;
+                if (j >= 2 && !warp_wait(&bars[VB_S_EMPTY + s], ((j >> 1) - 1) & 1)) return false;
                 tc_fence_after();
                 const uint64_t kd = k_desc + (uint64_t)(s * (2 * VT_TILE / 16));
                 const uint32_t d_addr = tmem + (uint32_t)s * 128u;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint64_t off = (uint64_t)((ks >> 2) * (TC_BOX / 16) + (ks & 3) * 2);
-                    umma_f16(d_addr, q_desc + off, kd + off, IDESC, ks > 0 ? 1u : 0u);
+                    for (int ks = 0; ks < D / 16; ++ks) {
+                        const uint64_t off = (uint64_t)((ks >> 2) * (TC_BOX / 16) + (ks & 3) * 2);
+                        umma_f16(d_addr, q_desc + off, kd + off, IDESC, ks > 0 ? 1u : 0u);
+                    }
+                    umma_commit(&bars[VB_S_FULL + s]);
+                    umma_commit(&bars[VB_K_EMPTY + s]);
                 }
-                umma_commit(&bars[VB_S_FULL + s]);
-                umma_commit(&bars[VB_K_EMPTY + s]);
+                __syncwarp();
                 return true;
             };
             // TMEM columns: S_0, S_1 at 0, 128; O at 256; P_0, P_1 at 384, 448. The S product runs two tiles ahead
@@ -294,21 +298,24 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 if (j + 2 < n_tiles) ok = issue_s(j + 2);
                 if (!ok) break;
                 const int s = j & 1;
-                ok = mbar_wait(&bars[VB_V_FULL + s], (j >> 1) & 1);
-                if (ok) ok = mbar_wait(&bars[VB_P_FULL + s], (j >> 1) & 1);
-                if (ok && j >= 1) ok = mbar_wait(&bars[VB_O_EMPTY], (j - 1) & 1);
+                ok = warp_wait(&bars[VB_V_FULL + s], (j >> 1) & 1);
+                if (ok) ok = warp_wait(&bars[VB_P_FULL + s], (j >> 1) & 1);
+                if (ok && j >= 1) ok = warp_wait(&bars[VB_O_EMPTY], (j - 1) & 1);
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t vd = v_desc + (uint64_t)(s * (2 * VT_TILE / 16));
                 const uint32_t o_addr = tmem + 256u;
                 // P_j is read from TMEM, where the softmax warps wrote it (16 keys = 8 columns per product)
                 const uint32_t p_addr = tmem + 384u + (uint32_t)s * 64u;
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < TC_KEYS / 16; ++ks)
-                    umma_f16_ts(o_addr, p_addr + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_PV, ks > 0 ? 1u : 0u);
-                umma_commit(&bars[VB_O_FULL]);
-                umma_commit(&bars[VB_P_EMPTY + s]);
-                umma_commit(&bars[VB_V_EMPTY + s]);
+                    for (int ks = 0; ks < TC_KEYS / 16; ++ks)
+                        umma_f16_ts(o_addr, p_addr + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_PV, ks > 0 ? 1u : 0u);
+                    umma_commit(&bars[VB_O_FULL]);
+                    umma_commit(&bars[VB_P_EMPTY + s]);
+                    umma_commit(&bars[VB_V_EMPTY + s]);
+                }
+                __syncwarp();
             }
             // the commits of the last two tiles nobody else waits for: they must have arrived before the barriers
             // are set up again for the next segment
@@ -316,7 +323,7 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 const int jl = n_tiles - back;
                 if (jl < 0) break;
                 const int s = jl & 1, par = (jl >> 1) & 1;
-                ok = mbar_wait(&bars[VB_K_EMPTY + s], par) && mbar_wait(&bars[VB_V_EMPTY + s], par) && mbar_wait(&bars[VB_P_EMPTY + s], par);
+                ok = warp_wait(&bars[VB_K_EMPTY + s], par) && warp_wait(&bars[VB_V_EMPTY + s], par) && warp_wait(&bars[VB_P_EMPTY + s], par);
             }
             if (!ok) atomicExch(p.status, 26);
         }
