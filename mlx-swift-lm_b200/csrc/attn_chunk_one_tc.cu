@@ -193,7 +193,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 before = t;
             }
             if (ok && before >= 0) ok = load_tile(&vmap, before);
-            if (!ok) atomicExch(p.status, 26);
+            if (!ok) atomicExch(p.status, 16);
         }
     } else if (warp == 5) {
         // ---------------- MMA issue (descriptors: attn_chunk_tc.cu) ----------------
@@ -253,7 +253,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             ++n;
         }
         if (ok && n > 0) issue_o(n - 1, true);
-        if (!ok) atomicExch(p.status, 27);
+        if (!ok) atomicExch(p.status, 17);
     } else {
         // ---------------- softmax and output: thread = row ----------------
         const int row = warp * 32 + lane;
@@ -411,7 +411,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 }
             }
         }
-        if (!ok) atomicExch(p.status, 28);
+        if (!ok) atomicExch(p.status, 18);
     }
     // all roles meet here; TMEM goes back whatever happened
     tc_fence_before();
@@ -497,9 +497,20 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
     const int64_t row_tiles = (int64_t)p.head_tiles * ((a.L + p.lb - 1) / p.lb), units = (int64_t)a.B * a.Hkv * row_tiles;
     if (row_tiles > (int64_t)1 << 20 || units > (int64_t)1 << 24) return 0;
     p.row_tiles = (int)row_tiles;
-    // pieces while SMs are free for them and each has a few key tiles; at most eight partials for the CTA that merges
+    // Pieces where places are free for them and they pay, in tiles' time (1.7 us at head dim 256): writing a partial costs
+    // the merging CTA about two and a half, merging one more than one. A mask is taken to hide half of the tiles. (64 row
+    // tiles of 10 visible tiles, D 256: 25 us whole, 30 as two pieces; calls of one row tile of 71, 4 heads: 43 us in eight, 47 in five.)
     const int64_t slots = (int64_t)sm_count(a.device) * (a.D == 256 ? 1 : 2), n = (a.T + ON_KEYS - 1) / ON_KEYS;
-    int64_t pieces = std::max<int64_t>(1, std::min<int64_t>({slots / units, n / 3, 8}));
+    const double visible = masked ? 0.5 * n : n;
+    int64_t pieces = 1;
+    double least = visible;
+    for (int64_t s = 2; s <= 8 && units * s <= slots && s * 3 <= n; ++s) {
+        const double time = visible / s + 2.5 + 1.2 * s;
+        if (time < least) {
+            least = time;
+            pieces = s;
+        }
+    }
     const int64_t most = ON_LIVE_WORDS * 32;
     if ((n + pieces - 1) / pieces > most) return 0;
 
