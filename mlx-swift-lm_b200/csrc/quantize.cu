@@ -1024,7 +1024,8 @@ turbo_encode_vec_kernel(TurboEncodeArgs ka, TurboEncodeArgs va, float inv_sqrt_d
 // cells are not, whatever the rounding of the map (the host builds the cells with the same fused multiply-add).
 // Sums run over the fixed tree (D / 32 neighbouring dims left to right, then the exchanges 16, 8, 4, 2, 1, of
 // which the last ones stay inside a lane), so norms and codes are the bits of turbo_encode_kernel.
-// 2 x 131072 rows of D 128 bf16, 4 bits: 96 us before.
+// 2 x 131072 rows of D 128 bf16, 4 bits: 96 us before. Products and sums take two dims an instruction (f32x2.cuh): keys with
+// the calibration statistic 43.3 -> 41.1 us, values 33 -> 30.
 // ---------------------------------------------------------------------
 struct EncodeCells {
     float scale, shift;      // cell = round(x * scale) + shift, as the low bits of fma(x, scale, shift)
