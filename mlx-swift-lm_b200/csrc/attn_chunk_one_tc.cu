@@ -474,7 +474,7 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
     if (masked ? (a.mask.dtype != KVC_BOOL || a.mask.st != 1 || !a.mask.data) : a.D != 256) return 0;
     if (a.mask.mode == KVC_MASK_CAUSAL && a.mask.causal_offset < 0) return 0;
     // up to 64 keys: one tile of the mma.sync chunk kernel, whose maximum per 16 of them is as precise
-    if (a.Hkv <= 0 || a.Hq % a.Hkv || a.T <= 64 || a.T > (int64_t)1 << 30) return 0;
+    if (a.B < 1 || a.L < 1 || a.Hq < 1 || a.Hkv <= 0 || a.Hq % a.Hkv || a.T <= 64 || a.T > (int64_t)1 << 30) return 0;
     const int64_t rep = a.Hq / a.Hkv;
     if (a.L < 64 && (rep * a.L <= 64 || rep > TC_ROWS)) return 0;
     if (!strides_fit(a.q, a.D, a.q_sl, a.q_sh, a.q_sb, a.Hq, a.B)) return 0;
