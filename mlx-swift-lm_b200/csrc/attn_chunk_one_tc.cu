@@ -473,6 +473,7 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
     const bool masked = a.mask.mode == KVC_MASK_ARRAY;
     if (masked ? (a.mask.dtype != KVC_BOOL || a.mask.st != 1 || !a.mask.data) : a.D != 256) return 0;
     if (a.mask.mode == KVC_MASK_CAUSAL && a.mask.causal_offset < 0) return 0;
+    if (!(a.scale > 0.f)) return 0;   // as in attn_chunk_tc.cu: hidden keys are -inf before the scale meets them
     // up to 64 keys: one tile of the mma.sync chunk kernel, whose maximum per 16 of them is as precise
     if (a.B < 1 || a.L < 1 || a.Hq < 1 || a.Hkv <= 0 || a.Hq % a.Hkv || a.T <= 64 || a.T > (int64_t)1 << 30) return 0;
     const int64_t rep = a.Hq / a.Hkv;

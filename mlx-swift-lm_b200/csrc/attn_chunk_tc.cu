@@ -690,6 +690,9 @@ bool attention_chunk_tc_accepts(const AttnArgs &a) {
     if (a.k.kind != SRC_RAW || a.v.kind != SRC_RAW || a.k.dtype != a.q_dtype || a.v.dtype != a.q_dtype) return false;
     if (a.mask.mode == KVC_MASK_ARRAY || a.q_signs || a.o_signs || a.q_calib || a.new_k || a.q_rot || a.o_rot) return false;
     if (a.B < 1 || a.L < 1 || a.Hq < 1 || a.Hkv <= 0 || a.Hq % a.Hkv || a.T < 1 || a.T > (int64_t)1 << 30) return false;
+    // hidden keys are -inf before the scale meets them, and the maximum is taken there too: positive scales only (the mma.sync
+    // chunk kernel multiplies first)
+    if (!(a.scale > 0.f)) return false;
     // Up to 64 rows of a KV head's group the decode and verify kernels do less work on rows that are not there; from there on
     // (8 of 32 heads, D 128, behind 4 096 keys) 64 positions take 38 us here and 82 on the mma.sync chunk kernel, 128 of 16
     // sequences 0.6 of its time. (More than 128 heads of a group at few positions leave a row tile nearly empty.)
