@@ -884,6 +884,7 @@ int launch_attention_verify_tc(const AttnArgs &a, cudaStream_t stream) {
     if (a.k.kind != SRC_TURBO || a.v.kind != SRC_TURBO || !a.q_signs || !a.o_signs || a.q_rot || a.o_rot) return 0;
     if (a.mask.mode == KVC_MASK_ARRAY || a.new_k) return 0;
     if (a.mask.mode == KVC_MASK_CAUSAL && a.mask.causal_offset < 0) return 0;
+    if (!(a.scale > 0.f)) return 0;           // hidden keys are -inf before the scale meets them, and so is the maximum taken
     const int kb = a.k.bits, vb = a.v.bits;
     if (vb != 4 || kb < 2 || kb > 4) return 0;
     if (kb == 4 && std::memcmp(a.k.codebook, a.v.codebook, sizeof(a.k.codebook)) != 0) return 0;   // 4-bit keys read the value pair table
@@ -1024,6 +1025,7 @@ int launch_attention_verify_tc_affine(const AttnArgs &a, cudaStream_t stream) {
     if (a.k.kind != SRC_AFFINE || a.v.kind != SRC_AFFINE || a.q_signs || a.o_signs || a.q_rot || a.o_rot || a.q_calib) return 0;
     if (a.mask.mode == KVC_MASK_ARRAY || a.new_k) return 0;
     if (a.mask.mode == KVC_MASK_CAUSAL && a.mask.causal_offset < 0) return 0;
+    if (!(a.scale > 0.f)) return 0;           // hidden keys are -inf before the scale meets them, and so is the maximum taken
     if ((a.k.bits != 4 && a.k.bits != 8) || a.v.bits != a.k.bits || a.k.group != 64 || a.v.group != 64) return 0;
     if (a.k.dtype != a.v.dtype || (a.k.dtype != KVC_BF16 && a.k.dtype != KVC_F16)) return 0;
     if (a.Hkv <= 0 || a.Hq % a.Hkv || a.T < 1 || a.T > (int64_t)1 << 30) return 0;
@@ -1136,6 +1138,7 @@ int launch_attention_verify_tc_raw(const AttnArgs &a, cudaStream_t stream) {
     if (a.k.kind != SRC_RAW || a.v.kind != SRC_RAW || a.k.dtype != a.q_dtype || a.v.dtype != a.q_dtype) return 0;
     if (a.mask.mode == KVC_MASK_ARRAY || a.q_signs || a.o_signs || a.q_calib || a.new_k || a.q_rot || a.o_rot) return 0;
     if (a.mask.mode == KVC_MASK_CAUSAL && a.mask.causal_offset < 0) return 0;
+    if (!(a.scale > 0.f)) return 0;           // hidden keys are -inf before the scale meets them, and so is the maximum taken
     if (a.Hkv <= 0 || a.Hq % a.Hkv || a.T < 1 || a.T > (int64_t)1 << 30) return 0;
     const int rep = a.Hq / a.Hkv, R = rep * a.L;
     if (R <= 16 || R > 64) return 0;          // up to 16 rows: the decode kernels

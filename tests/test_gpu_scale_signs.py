@@ -34,6 +34,8 @@ BOUND = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
     (2, 8, 2, 128, 300, 333, "window"),
     (1, 4, 1, 256, 20, 333, "window"),
     (1, 4, 1, 256, 70, 333, "causal"),
+    (2, 32, 8, 128, 6, 333, "causal"),     # verify rounds
+    (1, 4, 1, 128, 6, 333, "none"),
 ])
 def test_chunks(kvc, cuda, dtype, scale, B, Hq, Hkv, D, L, T, mask):
     q, k, v = (torch.randn((B, h, n, D), generator=torch.Generator(cuda).manual_seed(i), device=cuda).to(dtype)
@@ -46,9 +48,9 @@ def test_chunks(kvc, cuda, dtype, scale, B, Hq, Hkv, D, L, T, mask):
 
 @pytest.mark.parametrize("make", ["affine", "turbo"])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
-@pytest.mark.parametrize("L", [64, 300])
-def test_packed_prompt_chunks(kvc, cuda, make, scale, L):
-    """Rows that would be written out for the tcgen05 kernel. 8-bit codes: half a step of a group's range in the values, and as
+@pytest.mark.parametrize("L", [6, 64, 300])
+def test_packed_caches(kvc, cuda, make, scale, L):
+    """Verify rounds and prompt chunks. 8-bit codes: half a step of a group's range in the values, and as
     much again for the keys; 4-bit centroids err by a tenth of a value, averaged over the keys like the values themselves."""
     B, Hq, Hkv, D, P = 4, 32, 8, 128, 269
     c = kvc.QuantizedKVCache(64, 8) if make == "affine" else kvc.TurboQuantKVCache(bits=4, key_bits=4, value_bits=4)
