@@ -31,6 +31,7 @@
 namespace kvc {
 
 int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream);
+int launch_attention_decode(const AttnArgs &a, cudaStream_t stream);
 bool attention_chunk_tc_accepts(const AttnArgs &a);
 
 namespace {
@@ -330,7 +331,8 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
             call.q = q_out;
             call.q_sb = rp.o_sb; call.q_sh = rp.o_sh; call.q_sl = rp.o_sl;
         }
-        const int n = launch_attention_chunk_tc(call, stream);
+        int n = launch_attention_chunk_tc(call, stream);
+        if (n <= 0) n = launch_attention_decode(call, stream);   // no memory for its sums: the mma.sync chunk kernel
         if (n <= 0) fail(KVC_ERR_INTERNAL, "the tensor-core chunk kernel refused a call it had accepted");
         launches += n;
         if (turbo) {

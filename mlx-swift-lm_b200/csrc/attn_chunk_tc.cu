@@ -22,6 +22,10 @@
 //   probability of each part is exactly 1 and loses nothing to the 16-bit store, so the errors against 64-bit sums are
 //   4 ... 10 % smaller (bf16 and f16, 128 ... 16 000 keys), for O products in parts with a rescale between them.
 //
+// The tensor core adds towards zero: a sum of n keys in one accumulator loses 6e-9 n of itself (values of one sign), which
+// outgrows the rounding of an f16 output within a few thousand keys. After `fold` key tiles the softmax threads therefore add
+// O to fp32 sums of their own, behind O in TMEM at head dim 64 and in memory at 128, and the next O product starts from nothing.
+//
 // Units are handed out whole, in rounds of one per SM; what is left over is laid end to end and cut into equal ranges,
 // or few units are cut into pieces (a cut unit leaves fp32 partials, and the CTA that finishes it merges them).
 //
@@ -82,6 +86,8 @@ struct ChunkTcParams {
     int32_t pieces;             // not 0: every unit is cut into this many pieces, one CTA each (no rounds, no tail)
     int32_t group_tiles;        // key tiles of the units of a (batch, KV head)
     int32_t tail_base;          // ... of those before the tail's first unit in its own group
+    int32_t fold;               // key tiles of a segment between two folds
+    float *o_fold;              // [CTA][A / B][D / 4][128 rows][4] (head dim 128)
     float *o_part;              // [CTA][first / last segment][A / B][D / 4][128 rows][4]
     float2 *ml_part;            // [CTA][first / last segment][A / B][128 rows] (reference, sum)
     int *tickets;               // [unit of the tail][A / B], zeroed before the launch
@@ -308,6 +314,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
             };
             // One step takes the O products of a key tile and the S products of the next one, which may open the next segment.
             int sg = 0, left = 0;                    // the segment of the next S products, and its tiles still to come
+            int since = 0;                           // S products behind the last fold
             bool o_here = false, o_first = false, o_b = false, b = false;   // *b: the unit has a row tile B
             while (ok) {
                 const bool opens = left == 0 && sg < segments;
@@ -390,7 +397,8 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 if (o_here) step2(v_slot, v_par);
                 if (s_here) step2(k_slot, k_par);
                 o_here = s_here;
-                o_first = opens;
+                since = opens || since == p.fold - 1 ? 0 : since + 1;
+                o_first = since == 0;
                 if (s_here) --left;
             }
             if (!ok) atomicExch(p.status, 22);
@@ -417,11 +425,17 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
             const int limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l) : p.T - 1);     // last visible key
             const int tile_limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l0) : p.T - 1);
             float m_top = -INFINITY, m_ref = -INFINITY, l_run = 0.f;   // largest score, reference of O and of l_run
+            int since = -1;                                            // tiles behind the last fold
+            FoldedSums<D> sums(o_addr, (float4 *)p.o_fold + ((int64_t)blockIdx.x * 2 + i) * (D / 4) * TC_ROWS + row);
             for (int t = w.t0; t < w.t1; ++t) {
                 ok = warp_wait(&bars[BAR::S_FULL + i], s_par);
                 if (!ok) break;
                 s_par ^= 1;
                 tc_fence_after();
+                if (++since == p.fold) {
+                    sums.fold(m_ref);
+                    since = 0;
+                }
                 uint32_t raw[TC_KEYS];
 #pragma unroll
                 for (int cb = 0; cb < 4; ++cb) tmem_ld32_issue(s_addr + cb * 32, raw + cb * 32);
@@ -449,7 +463,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 // O is settled when the scores are there: they came behind the O products of the tile before
                 auto hand_over = [&](auto which) {
                     constexpr int h = decltype(which)::value, FROM = key_of(h), TO = key_of(h + 1), part = PARTS == 1 ? 0 : h;
-                    const bool first = h == 0, move = (first ? t > w.t0 : PARTS > 1) && __any_sync(0xffffffffu, alpha[part] != 1.f);
+                    const bool first = h == 0, move = (first ? since > 0 : PARTS > 1) && __any_sync(0xffffffffu, alpha[part] != 1.f);
                     const uint64_t alpha2 = pack_f2(alpha[part], alpha[part]);
                     constexpr int CH = PARTS == 1 ? 32 : 16;   // columns of O at a time (16: 3 % slower with one reference)
                     uint32_t o[CH];
@@ -529,7 +543,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
 #pragma unroll 1
                 for (int cb = 0; cb < D / 32; ++cb) {
                     float o[32];
-                    tmem_ld32(o_addr + cb * 32, o);
+                    sums.total(cb, m_ref, o);
                     if (valid) store_row32<T>(dst + cb * 32, o, inv);
                 }
                 continue;
@@ -538,14 +552,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
             const int c = blockIdx.x;
             {
                 const int64_t slot = ((int64_t)c * 2 + (sg == p.waves ? 0 : 1)) * 2 + i;
-                float4 *po = (float4 *)p.o_part + slot * (D / 4) * TC_ROWS + row;
-#pragma unroll 1
-                for (int cb = 0; cb < D / 32; ++cb) {
-                    float o[32];
-                    tmem_ld32(o_addr + cb * 32, o);
-#pragma unroll
-                    for (int c4 = 0; c4 < 8; ++c4) po[(cb * 8 + c4) * TC_ROWS] = make_float4(o[c4 * 4], o[c4 * 4 + 1], o[c4 * 4 + 2], o[c4 * 4 + 3]);
-                }
+                sums.leave(m_ref, (float4 *)p.o_part + slot * (D / 4) * TC_ROWS + row);
                 p.ml_part[slot * TC_ROWS + row] = make_float2(m_ref, l_run);
             }
             __threadfence();
@@ -777,19 +784,11 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
         ranges = std::max<int64_t>(1, std::min<int64_t>(sms, tail_tiles / 4));
         if (tail_tiles < 1 || tail_tiles > (int64_t)1 << 29 || group_tiles > (int64_t)1 << 29 ||
             tail_tiles / ranges / least + 2 > CT_MAX_SEGMENTS - waves)
-            ranges = 0;
+            tail_tiles = ranges = 0;
     }
-    const size_t part = (size_t)ranges * 4 * TC_ROWS;
-    const size_t o_bytes = part * a.D * sizeof(float), ml_bytes = part * sizeof(float2);
-    const size_t t_bytes = (size_t)(tail_tiles > 0 ? units - waves * sms : units) * 2 * sizeof(int);
-    CallMemory mem(ranges > 0 ? o_bytes + ml_bytes + t_bytes : 0, stream);
-    int64_t ctas = even ? std::min(units, sms) : units;
-    p.waves = even ? (int)rounds : 1;
-    if (mem.ptr) {
-        p.o_part = (float *)mem.ptr;
-        p.ml_part = (float2 *)((char *)mem.ptr + o_bytes);
-        p.tickets = (int *)((char *)p.ml_part + ml_bytes);
-        KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
+    int64_t ctas, longest;                                       // ... and the most key tiles of a segment
+    size_t o_bytes, ml_bytes, t_bytes, fold_bytes;
+    auto lay_out = [&] {
         if (tail_tiles > 0) {
             ctas = waves > 0 ? sms : ranges;
             p.waves = (int)waves;
@@ -798,12 +797,39 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
             p.rem = (int)(tail_tiles % ranges);
             p.group_tiles = (int)group_tiles;
             for (int64_t u = waves * sms / p.units * p.units; u < waves * sms; ++u) p.tail_base += ct_unit_tiles(p, (int)u);
-        } else {
+            longest = waves > 0 ? most : std::min(most, p.per + 1);
+        } else if (ranges > 0) {
             ctas = ranges;
-            p.waves = 0;
             p.pieces = (int)pieces;
+            longest = (most + pieces - 1) / pieces;
+        } else {
+            ctas = even ? std::min(units, sms) : units;
+            p.waves = even ? (int)rounds : 1;
+            longest = most;
         }
+        // (in memory a fold costs a key tile's time: 512 f16 keys 323 us where no folds take 267, 768 about 300, and the kernel
+        // that folded every tile in registers 311; 512 x 8 x 32 heads behind 3 584 keys)
+        p.fold = fold_keys(a.q_dtype) * (a.D == 128 ? 3 : 2) / 2 / TC_KEYS;
+        const size_t part = (size_t)ranges * 4 * TC_ROWS;
+        o_bytes = part * a.D * sizeof(float);
+        ml_bytes = part * sizeof(float2);
+        t_bytes = ranges > 0 ? (size_t)(tail_tiles > 0 ? units - waves * sms : units) * 2 * sizeof(int) : 0;
+        fold_bytes = a.D == 128 && longest > p.fold ? (size_t)ctas * 2 * TC_ROWS * a.D * sizeof(float) : 0;
+        return fold_bytes + o_bytes + ml_bytes + t_bytes;
+    };
+    const ChunkTcParams uncut = p;
+    CallMemory mem(lay_out(), stream);
+    if (!mem.ptr && ranges > 0) {                                // no room: whole units
+        p = uncut;
+        tail_tiles = ranges = 0;
+        lay_out();
     }
+    if (!mem.ptr && fold_bytes > 0) return 0;
+    p.o_fold = (float *)mem.ptr;
+    p.o_part = (float *)((char *)mem.ptr + fold_bytes);
+    p.ml_part = (float2 *)((char *)p.o_part + o_bytes);
+    p.tickets = (int *)((char *)p.ml_part + ml_bytes);
+    if (ranges > 0) KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
     // Small calls take a finer reference: they spend their time on the start, the partials and the merge, and the mma.sync
     // chunk kernel that takes them otherwise errs by little (a running maximum per 16 keys, in splits of 64 keys and up).
     const int parts = few_blocks(a) ? (a.T < 2048 ? 4 : 2) : 1;

@@ -137,6 +137,86 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
 
+// Keys whose products the tensor core may add up before the sums go on in fp32 instructions. It adds towards zero, and a sum of
+// n keys loses 6e-9 n of itself (values of one sign; about half of that for values around zero): 3e-6 of an f16 output, which
+// is rounded by 2e-4, and 2.5e-5 of a bf16 one, rounded by eight times that, so that errors against 64 bits grow by 0.01 %.
+inline int fold_keys(int32_t dtype) { return dtype == KVC_F16 ? 512 : 4096; }
+
+__device__ __forceinline__ void add4_global(float4 *p, float x, float y, float z, float w) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+
+// The fp32 sums a softmax thread (a row) folds its D columns of O into, in a reference of their own. Behind O in TMEM where
+// there is room, otherwise in memory that only this thread touches: [column / 4][128 rows] of float4, added to where they lie
+// (no load to wait for) unless the reference has left them far behind.
+template <int D> struct FoldedSums {
+    static constexpr bool IN_TMEM = D == 64;
+    uint32_t o;
+    float4 *sums;
+    float m = -INFINITY;                 // their reference
+    bool any = false;
+    __device__ __forceinline__ FoldedSums(uint32_t o_addr, float4 *memory) : o(o_addr), sums(memory) {}
+    // 32 columns of O and of the sums, in the reference m_o
+    __device__ __forceinline__ void total(int cb, float m_o, float (&x)[32]) {
+        tmem_ld32(o + cb * 32, x);
+        if (!any) return;
+        const float f = m == -INFINITY ? 0.f : fast_exp2(m - m_o);
+        if constexpr (IN_TMEM) {
+            float s[32];
+            tmem_ld32(o + D + cb * 32, s);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) x[k] = fmaf(s[k], f, x[k]);
+        } else
+#pragma unroll
+        for (int c4 = 0; c4 < 8; ++c4) {
+            const float4 y = __ldcg(&sums[(cb * 8 + c4) * TC_ROWS]);
+            x[c4 * 4 + 0] = fmaf(y.x, f, x[c4 * 4 + 0]);
+            x[c4 * 4 + 1] = fmaf(y.y, f, x[c4 * 4 + 1]);
+            x[c4 * 4 + 2] = fmaf(y.z, f, x[c4 * 4 + 2]);
+            x[c4 * 4 + 3] = fmaf(y.w, f, x[c4 * 4 + 3]);
+        }
+    }
+    // ... all of them to memory of the same layout
+    __device__ __forceinline__ void leave(float m_o, float4 *to) {
+#pragma unroll 1
+        for (int cb = 0; cb < D / 32; ++cb) {
+            float x[32];
+            total(cb, m_o, x);
+#pragma unroll
+            for (int c4 = 0; c4 < 8; ++c4) __stcg(&to[(cb * 8 + c4) * TC_ROWS], make_float4(x[c4 * 4], x[c4 * 4 + 1], x[c4 * 4 + 2], x[c4 * 4 + 3]));
+        }
+    }
+    // All threads of a warp; O is settled, and the product after it starts from nothing.
+    __device__ __forceinline__ void fold(float m_o) {
+        if (IN_TMEM) {
+#pragma unroll 1
+            for (int cb = 0; cb < D / 32; ++cb) {
+                float x[32];
+                uint32_t bits[32];
+                total(cb, m_o, x);
+#pragma unroll
+                for (int k = 0; k < 32; ++k) bits[k] = __float_as_uint(x[k]);
+                tmem_st32_issue(o + D + cb * 32, bits);
+            }
+            tmem_st_wait();
+            m = m_o;
+        } else if (!any || __any_sync(0xffffffffu, !(m_o - m <= 64.f))) {
+            leave(m_o, sums);
+            m = m_o;
+        } else {
+            const float f = fast_exp2(m_o - m);
+#pragma unroll 2
+            for (int cb = 0; cb < D / 32; ++cb) {
+                float x[32];
+                tmem_ld32(o + cb * 32, x);
+#pragma unroll
+                for (int c4 = 0; c4 < 8; ++c4) add4_global(&sums[(cb * 8 + c4) * TC_ROWS], x[c4 * 4] * f, x[c4 * 4 + 1] * f, x[c4 * 4 + 2] * f, x[c4 * 4 + 3] * f);
+            }
+        }
+        any = true;
+    }
+};
+
 // 32 output columns of a row as 16-bit values.
 template <typename T> __device__ __forceinline__ void store_row32(T *dst, const float *o, float inv) {
 #pragma unroll

@@ -84,3 +84,31 @@ def test_chunk_with_cut_units_can_be_captured(kvc, cuda):
         graph.replay()
         torch.cuda.synchronize()
         assert np.array_equal(out.view(torch.int16).cpu(), kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, "causal").view(torch.int16).cpu())
+
+
+def _bias(out, ref):
+    """How far the outputs lie from 64-bit ones towards zero (negative) or away from it, of their mean size."""
+    return ((out.double() - ref) * ref.sign()).mean().item() / ref.abs().mean().item()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,L,T", [
+    (1, 80, 8, 64, 70000),       # equal ranges of all units
+    (1, 148, 148, 70, 9000),     # whole units
+    (8, 32, 8, 21, 9000),        # pieces of a unit
+])
+def test_sums_over_long_contexts(kvc, cuda, capfd, monkeypatch, D, B, Hq, Hkv, L, T):
+    """f16 sums of one sign: the tensor core adds towards zero and alone loses 6e-9 of them a key, 5e-5 over 9 000; folded into fp32
+    sums every 512 or 768 keys they lose 3e-6 or 4.5e-6. The stores' rounding averages out over the outputs (four sigma are allowed)."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    q, k, v = (torch.randn((B, h, n, D), generator=torch.Generator(cuda).manual_seed(i), device=cuda) for i, (h, n) in enumerate(((Hq, L), (Hkv, T), (Hkv, T))))
+    q, k, v = q.half(), k.half(), (v + 1).half()
+    out = kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, "causal")
+    torch.cuda.synchronize()
+    assert "chunk_tc" in capfd.readouterr().err
+    rep, seen = Hq // Hkv, torch.arange(T, device=cuda) <= torch.arange(T - L, T, device=cuda)[:, None]
+    ref = torch.stack([torch.stack([torch.softmax((q[b, h].double() @ k[b, h // rep].double().T * D ** -0.5).masked_fill_(~seen, float("-inf")), -1)
+                                    @ v[b, h // rep].double() for h in range(Hq)]) for b in range(B)])
+    assert abs(_bias(out, ref)) <= 4.5e-6 + 4 * 2.2e-4 * out.numel() ** -0.5
+    assert ((out.double() - ref).norm() / ref.norm()).item() <= 2.0 ** -11
+    assert kvc.lib().kvc_device_status() == 0
