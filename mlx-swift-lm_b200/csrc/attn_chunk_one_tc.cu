@@ -17,6 +17,9 @@
 // on, so that a window's run of visible tiles is shared evenly. Under an array mask the CTA first reads the mask of its
 // rows and tiles and leaves out the tiles no row sees.
 //
+// Every `fold` tiles O goes on in fp32 sums, as in attn_chunk_tc.cu (masked f16 outputs: errors against 64 bits + 0.5 % at 32 000
+// keys without it, in eight pieces).
+//
 // What bounds it: the chain S -> softmax -> O of one row tile; the two products take 1 800 cycles of a tile at head dim
 // 256 (768 for S, whose 64 columns are bound by shared-memory reads, 1 024 for both halves of P).
 //
@@ -58,7 +61,8 @@ struct ChunkOneParams {
     int64_t causal_offset;
     float scale_log2;
     MaskDesc mask;
-    float *o_part;                           // [unit][piece][D / 4][128 rows][4]
+    int32_t fold;                            // key tiles of a CTA between two folds
+    float *o_part;                           // [unit][piece][D / 4][128 rows][4]: partials, and (head dim 128 and 256) the folded sums until then
     float2 *ml_part;                         // [unit][piece][128 rows] (reference, sum)
     int *tickets;                            // [unit], zeroed before the launch
     int *status;
@@ -205,6 +209,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         const uint64_t v_desc = umma_desc(smem_u32(ring), ON_BOX, 1024);
         bool ok = true;
         uint32_t slot = 0, par = 0, n = 0;   // ring entry; S products issued
+        int since = 0;                       // O products behind the last fold
         auto next = [&] {
             if (++slot == (uint32_t)STAGES) {
                 slot = 0;
@@ -224,12 +229,13 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 #pragma unroll
                     for (int ks = 0; ks < ON_KEYS / 16; ++ks)
                         umma_f16_ts(tmem + O_COL, p_addr + (uint32_t)(low * 32 + ks * 8), vd + (uint64_t)(ks * 128), IDESC_PV,
-                                    (j == 0 && low == 1 && ks == 0) ? 0u : 1u);
+                                    (since == 0 && low == 1 && ks == 0) ? 0u : 1u);
                 umma_commit(&bars[BAR::O_DONE]);
                 if (last) umma_commit(&bars[BAR::O_LAST]);
                 umma_commit(&bars[BAR::RING_EMPTY + slot]);
             }
             __syncwarp();
+            since = since == p.fold - 1 ? 0 : since + 1;
             next();
         };
         for (int c = 0; ok && c < mine; ++c) {
@@ -264,7 +270,10 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         const uint8_t *mrow = MASKED && valid ? mask_row(h, l) : nullptr;
         float m_run = -INFINITY, l_run = 0.f;
         uint32_t n = 0;
+        int since = -1;                      // tiles behind the last fold
         bool ok = true;
+        float4 *part = (float4 *)p.o_part + ((int64_t)unit * p.pieces + piece) * (D / 4) * TC_ROWS + row;
+        FoldedSums<D> sums(o_addr, part);
         for (int c = 0; c < mine; ++c) {
             if (!live(c)) continue;
             const int key0 = (piece + c * p.pieces) * ON_KEYS;
@@ -297,6 +306,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 mx4[(k >> 1) & 3] = fmaxf(mx4[(k >> 1) & 3], fmaxf(__uint_as_float(raw[k]), __uint_as_float(raw[k + 1])));
             const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
             const float alpha = m_run == m_new ? 1.f : fast_exp2(m_run - m_new);   // exp2(-inf) = 0
+            const float m_old = m_run;
             m_run = m_new;
             const float neg_m = m_new == -INFINITY ? 0.f : -m_new;
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -312,11 +322,16 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 low[k >> 1] = pack_pair<T>(e0 * P_UP - f.x, e1 * P_UP - f.y);
                 raw[k >> 1] = high;
             }
-            if (n > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+            const bool fold = ++since == p.fold;
+            if (n > 0 && (fold || __any_sync(0xffffffffu, alpha != 1.f))) {
                 ok = warp_wait(&bars[BAR::O_DONE], (n - 1) & 1);   // (not a phase too early: the product before
                                                                      // it was done when these scores came)
                 if (!ok) break;
                 tc_fence_after();
+                if (fold) {
+                    sums.fold(m_old);
+                    since = 0;
+                } else
 #pragma unroll 2
                 for (int cb = 0; cb < D / 32; ++cb) {
                     uint32_t o[32];
@@ -341,7 +356,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             T *dst = (T *)p.out + b * p.o_sb + (int64_t)(hk * p.rep + h) * p.o_sh + (int64_t)l * p.o_sl;
             auto o_of = [&](int cb, float (&o)[32]) {
                 if (n > 0) {
-                    tmem_ld32(o_addr + cb * 32, o);
+                    sums.total(cb, m_run, o);
                 } else {
 #pragma unroll
                     for (int k = 0; k < 32; ++k) o[k] = 0.f;
@@ -357,16 +372,14 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 }
             } else {
                 // ---- leave a partial; the CTA that leaves the last one of the unit merges them ----
-                const int64_t slot = (int64_t)unit * p.pieces + piece;
-                float4 *po = (float4 *)p.o_part + slot * (D / 4) * TC_ROWS + row;
 #pragma unroll 1
                 for (int cb = 0; cb < D / 32; ++cb) {
                     float o[32];
                     o_of(cb, o);
 #pragma unroll
-                    for (int c4 = 0; c4 < 8; ++c4) po[(cb * 8 + c4) * TC_ROWS] = make_float4(o[c4 * 4], o[c4 * 4 + 1], o[c4 * 4 + 2], o[c4 * 4 + 3]);
+                    for (int c4 = 0; c4 < 8; ++c4) __stcg(&part[(cb * 8 + c4) * TC_ROWS], make_float4(o[c4 * 4], o[c4 * 4 + 1], o[c4 * 4 + 2], o[c4 * 4 + 3]));
                 }
-                p.ml_part[slot * TC_ROWS + row] = make_float2(m_run, l_run);
+                p.ml_part[((int64_t)unit * p.pieces + piece) * TC_ROWS + row] = make_float2(m_run, l_run);
                 __threadfence();
                 mbar_arrive(&bars[BAR::GROUP]);
                 ok = warp_wait(&bars[BAR::GROUP], 0);
@@ -520,18 +533,21 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
     if (!make_map_tc(&kmap, a.k.data, a.k.dtype, a.D, a.T, a.Hkv, a.B, a.k.st, a.k.sh, a.k.sb, ON_KEYS)) return 0;
     if (!make_map_tc(&vmap, a.v.data, a.v.dtype, a.D, a.T, a.Hkv, a.B, a.v.st, a.v.sh, a.v.sb, ON_KEYS)) return 0;
 
+    p.fold = fold_keys(a.q_dtype) / ON_KEYS;
+    const bool folds = (n + pieces - 1) / pieces > p.fold;
     const size_t part = (size_t)units * pieces * TC_ROWS;
     const size_t o_bytes = part * a.D * sizeof(float), ml_bytes = part * sizeof(float2), t_bytes = (size_t)units * sizeof(int);
-    CallMemory mem(pieces > 1 ? o_bytes + ml_bytes + t_bytes : 0, stream);
-    p.pieces = 1;
-    if (mem.ptr) {
-        p.pieces = (int)pieces;
-        p.o_part = (float *)mem.ptr;
+    CallMemory mem(pieces > 1 ? o_bytes + ml_bytes + t_bytes : folds && a.D > 64 ? o_bytes : 0, stream);
+    if (!mem.ptr && (pieces > 1 || (folds && a.D > 64))) {   // no room: whole units that need no sums in memory, or the mma.sync kernel
+        if (n > most || (n > p.fold && a.D > 64)) return 0;
+        pieces = 1;
+    }
+    p.pieces = (int)pieces;
+    p.o_part = (float *)mem.ptr;
+    if (pieces > 1) {
         p.ml_part = (float2 *)((char *)mem.ptr + o_bytes);
         p.tickets = (int *)((char *)p.ml_part + ml_bytes);
         KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
-    } else if (n > most) {
-        return 0;
     }
     const int ctas = (int)(units * p.pieces);
     const bool taken = a.q_dtype == KVC_BF16 ? launch_one<__nv_bfloat16>(qmap, kmap, vmap, p, a.D, masked, ctas, stream)

@@ -69,3 +69,25 @@ def test_head_dim_256(kvc, cuda, capfd, monkeypatch, dtype, B, Hq, Hkv, L, T, ma
         seen = seen.tril(T - L)
     _check(kvc, capfd, q, k, v, mask, seen)
     _check(kvc, capfd, q.transpose(1, 2).contiguous().transpose(1, 2), k, v, mask, seen)
+
+
+@pytest.mark.parametrize("D,mask", [(64, "array"), (128, "array"), (256, "array"), (256, "causal")])
+@pytest.mark.parametrize("B,Hq,Hkv,L,T", [
+    (1, 4, 1, 64, 70000),        # pieces
+    (1, 160, 160, 70, 9000),     # whole units
+])
+def test_sums_over_long_contexts(kvc, cuda, capfd, monkeypatch, D, mask, B, Hq, Hkv, L, T):
+    """f16 sums of one sign: the tensor core adds towards zero and alone loses 6e-9 of them a key, 5e-5 over 9 000; folded into fp32
+    sums every 512 keys they lose 3e-6. The stores' rounding averages out over the outputs (four sigma are allowed)."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    q, k, v = _case(cuda, torch.float32, B, Hq, Hkv, D, L, T)
+    q, k, v = q.half(), k.half(), (v + 1).half()
+    seen = torch.arange(T, device=cuda) <= torch.arange(T - L, T, device=cuda)[:, None]
+    out = kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, seen if mask == "array" else mask)
+    torch.cuda.synchronize()
+    assert "chunk_one" in capfd.readouterr().err
+    ref = torch.stack([torch.softmax((q[0, h].double() @ k[0, h * Hkv // Hq].double().T * D ** -0.5).masked_fill_(~seen, float("-inf")), -1)
+                       @ v[0, h * Hkv // Hq].double() for h in range(Hq)])
+    assert abs(((out[0].double() - ref) * ref.sign()).mean().item()) <= (3e-6 + 4 * 2.2e-4 * out.numel() ** -0.5) * ref.abs().mean().item()
+    assert ((out[0].double() - ref).norm() / ref.norm()).item() <= 2.0 ** -11
+    assert kvc.lib().kvc_device_status() == 0
