@@ -830,9 +830,10 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     p.ml_part = (float2 *)((char *)p.o_part + o_bytes);
     p.tickets = (int *)((char *)p.ml_part + ml_bytes);
     if (ranges > 0) KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
-    // Small calls take a finer reference: they spend their time on the start, the partials and the merge, and the mma.sync
-    // chunk kernel that takes them otherwise errs by little (a running maximum per 16 keys, in splits of 64 keys and up).
-    const int parts = few_blocks(a) ? (a.T < 2048 ? 4 : 2) : 1;
+    // Small calls take a finer reference: the mma.sync chunk kernel that takes them otherwise errs by little (a running maximum per
+    // 16 keys, in up to 64 splits of 64 keys and up: four references are as precise below 16 384 keys, two from there on; behind
+    // 4 000 keys two err by 3 % more).
+    const int parts = few_blocks(a) ? (a.T < 16384 ? 4 : 2) : 1;
     bool taken;
     if (a.D == 128)
         taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 128>(qmap, kmap, vmap, p, (int)ctas, parts, stream)
