@@ -511,15 +511,17 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
     const int64_t row_tiles = (int64_t)p.head_tiles * ((a.L + p.lb - 1) / p.lb), units = (int64_t)a.B * a.Hkv * row_tiles;
     if (row_tiles > (int64_t)1 << 20 || units > (int64_t)1 << 24) return 0;
     p.row_tiles = (int)row_tiles;
-    // Pieces where places are free for them and they pay, in tiles' time (1.7 us at head dim 256): writing a partial costs
-    // the merging CTA about two and a half, merging one more than one. A mask is taken to hide half of the tiles. (64 row
-    // tiles of 10 visible tiles, D 256: 25 us whole, 30 as two pieces; calls of one row tile of 71, 4 heads: 43 us in eight, 47 in five.)
-    const int64_t slots = (int64_t)sm_count(a.device) * (a.D == 256 ? 1 : 2), n = (a.T + ON_KEYS - 1) / ON_KEYS;
+    // Pieces where places are free for them and they pay, in tiles' time (1.7 us): a partial costs the merging CTA two and a half
+    // to write and 1.2 to merge at head dim 256 (0.3 at 64). A mask is taken to hide half of the tiles. Two CTAs on an SM take 1.6
+    // times as long for a tile. (64 row tiles of 10 visible tiles, D 256: 25 us whole, 30 as two pieces. One row tile of four heads
+    // behind 40 000 keys, all visible: 149 us in 8 pieces, 62 in 32 at D 64; 178 in 8, 118 in 16, 104 in 24 at D 256. 8 row tiles
+    // behind 16 000, D 64: 64 us in 8, 40 in 16, 48 in 24.)
+    const int64_t sms = sm_count(a.device), slots = sms * (a.D == 256 ? 1 : 2), n = (a.T + ON_KEYS - 1) / ON_KEYS;
     const double visible = masked ? 0.5 * n : n;
     int64_t pieces = 1;
     double least = visible;
-    for (int64_t s = 2; s <= 8 && units * s <= slots && s * 3 <= n; ++s) {
-        const double time = visible / s + 2.5 + 1.2 * s;
+    for (int64_t s = 2; s <= 64 && units * s <= slots && s * 3 <= n; ++s) {
+        const double time = visible / s * (units * s > sms ? 1.6 : 1.0) + 2.5 + 1.2 * s * a.D / 256;
         if (time < least) {
             least = time;
             pieces = s;
