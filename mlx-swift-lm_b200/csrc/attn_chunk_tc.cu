@@ -757,24 +757,33 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     if (!make_map_tc(&kmap, a.k.data, a.k.dtype, a.D, a.T, a.Hkv, a.B, a.k.st, a.k.sh, a.k.sb)) return 0;
     if (!make_map_tc(&vmap, a.v.data, a.v.dtype, a.D, a.T, a.Hkv, a.B, a.v.st, a.v.sh, a.v.sb)) return 0;
 
+    // Small calls take a finer reference: the mma.sync chunk kernel that takes them otherwise errs by little (a running maximum per
+    // 16 keys, in up to 64 splits of 64 keys and up: four references are as precise below 16 384 keys, two from there on; behind
+    // 4 000 keys two err by 3 % more).
+    const int parts = few_blocks(a) ? (a.T < 16384 ? 4 : 2) : 1;
+
     // How the units are handed out, judged by the key tiles of the busiest SM (a CTA's start takes about three tiles' time,
-    // the change of a unit one, writing a partial two, merging one a half):
+    // the change of a unit one or two, writing a partial two, merging one a half, the memory for them and its cleared tickets
+    // three, or two of the longer ones with finer references):
     //   whole units in rounds, one per SM, or, where units differ much, a CTA for each;
     //   few units: all cut into the same number of pieces, a CTA for each piece;
     //   equal ranges of all units end to end: evenest, but the CTAs are spread over all of K and V at once, so only where
     //     those stay in L2 (8 x 8 heads of 8 704 keys, 285 MB: 2.1 GB came from HBM in a launch);
     //   whole units in rounds, so that neighbours share their K and V tiles, and equal ranges of what is left.
+    // (D 128, 160 units of 1 ... 3 tiles: 19 us whole, 34 in ranges; 48 of 5 or 6, D 64: 17 whole, 21 in pieces; 40 of 16: 38
+    // whole, 33 in pieces, 37 in ranges; 64 of 254: 494, 261, 236.)
     constexpr int64_t L2_BYTES = (int64_t)64 << 20;
     const int64_t sms = sm_count(a.device), units = p.all_units, flat = groups * group_tiles, average = (flat + units - 1) / units;
     const bool settled = groups * a.T * a.D * 4 <= L2_BYTES;
     const int64_t rounds = (units + sms - 1) / sms;
     const bool even = least * 4 >= most * 3 && rounds <= CT_MAX_SEGMENTS;
     const int64_t waves = settled ? 0 : units / sms;
-    const int64_t tail = settled ? flat : (units - waves * sms) * average, per = (tail + sms - 1) / sms;   // (exact length below)
+    const int64_t tail = settled ? flat : (units - waves * sms) * average, per = std::max<int64_t>(4, (tail + sms - 1) / sms);   // (exact length below)
     const int64_t pieces = std::min<int64_t>(sms / units, least / 2);
+    const int64_t set_up = 3 + (parts == 1 ? 3 : 2);
     const int64_t whole = even ? 3 + rounds * (average + 1) : std::max<int64_t>(most, rounds * average) + 3 * rounds;
-    const int64_t cut = 3 + waves * (most + 1) + per + 3 + (most / std::max<int64_t>(per, 1) + 2) / 2;
-    const int64_t apart = pieces > 1 ? 3 + (most + pieces - 1) / pieces + 2 + pieces / 2 : INT64_MAX;
+    const int64_t cut = set_up + waves * (most + 1) + per + 2 * (per / average) + 3 + (most / per + 2) / 2;
+    const int64_t apart = pieces > 1 ? set_up + (most + pieces - 1) / pieces + 2 + pieces / 2 : INT64_MAX;
     int64_t tail_tiles = 0, ranges = 0;
     if (apart < whole && apart <= cut) {
         ranges = units * pieces;
@@ -830,10 +839,6 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     p.ml_part = (float2 *)((char *)p.o_part + o_bytes);
     p.tickets = (int *)((char *)p.ml_part + ml_bytes);
     if (ranges > 0) KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
-    // Small calls take a finer reference: the mma.sync chunk kernel that takes them otherwise errs by little (a running maximum per
-    // 16 keys, in up to 64 splits of 64 keys and up: four references are as precise below 16 384 keys, two from there on; behind
-    // 4 000 keys two err by 3 % more).
-    const int parts = few_blocks(a) ? (a.T < 16384 ? 4 : 2) : 1;
     bool taken;
     if (a.D == 128)
         taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 128>(qmap, kmap, vmap, p, (int)ctas, parts, stream)
