@@ -527,7 +527,7 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
             pieces = s;
         }
     }
-    const int64_t most = ON_LIVE_WORDS * 32;
+    const int64_t most = masked ? ON_LIVE_WORDS * 32 : n;   // a bit for every tile under a mask
     if ((n + pieces - 1) / pieces > most) return 0;
 
     CUtensorMap qmap, kmap, vmap;
