@@ -260,8 +260,10 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
     if (affine && (a.q_signs || a.o_signs || a.q_calib || a.k.dtype != a.q_dtype || a.v.dtype != a.q_dtype)) return 0;
     if (!source_ok(a.k, a.D, turbo) || !source_ok(a.v, a.D, turbo)) return 0;
     if (a.T < 1 || a.T > (int64_t)1 << 30 || a.B < 1) return 0;
-    // the rows are written out for this call alone: for less work than this the kernels that decode in their tile loop
-    if (a.L < 64 || (int64_t)a.B * a.Hq * ((a.L + 127) / 128) < sm_count(a.device) / 2) return 0;
+    // The rows are written out for this call alone: for less work than this the kernels that decode in their tile loop. Asked of every
+    // slice too, so that all sequences of a call are computed alike.
+    auto enough = [&](int64_t B) { return a.L >= 64 && B * a.Hq * ((a.L + 127) / 128) >= sm_count(a.device) / 2; };
+    if (!enough(a.B)) return 0;
 
     // the contraction as the tcgen05 kernel would see it: raw K / V of the query dtype, contiguous
     AttnArgs r = a;
@@ -284,14 +286,14 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
     const size_t q_per_b = turbo ? (size_t)a.Hq * a.L * a.D * es : 0;
     const size_t per_b = kv_per_b + q_per_b + 512;
     if (per_b > MAT_SCRATCH_LIMIT) return 0;
-    // whole sequences per slice, the slices as even as they come; every slice must still fill the part
+    // whole sequences per slice, the slices as even as they come
     const int fit = (int)std::min<size_t>((size_t)a.B, MAT_SCRATCH_LIMIT / per_b);
     const int nslices = (a.B + fit - 1) / fit;
     const int slice = (a.B + nslices - 1) / nslices;
     {
         AttnArgs probe = r;
         probe.B = a.B - (nslices - 1) * slice;   // the last, smallest slice
-        if (probe.B < 1 || !attention_chunk_tc_accepts(probe)) return 0;
+        if (probe.B < 1 || !enough(probe.B) || !attention_chunk_tc_accepts(probe)) return 0;
         probe.B = slice;
         if (!attention_chunk_tc_accepts(probe)) return 0;
     }

@@ -708,3 +708,21 @@ assert float((outs[0].float() - outs[1].float()).abs().max()) < 2e-3
 """
     env = dict(os.environ, PYTHONPATH=os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mlx-swift-lm_b200", "python"))
     subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
+
+
+def test_sequences_of_a_call_take_one_kernel(kvc, cuda, capfd, monkeypatch):
+    """Rows written out for a chunk are limited to a few GB at a time. Where a last slice of the batch would be too small to be worth it,
+    no sequence of the call is treated that way: equal sequences have equal outputs."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    B, Hq, Hkv, D, P, L = 3, 32, 8, 128, 262144, 64
+    c = kvc.QuantizedKVCache(64, 4, reserve_tokens=P + L)
+    g = torch.Generator(cuda).manual_seed(1)
+    rand = lambda h, n: torch.randn((1, h, n, D), generator=g, device=cuda).to(torch.bfloat16).expand(B, h, n, D).contiguous()
+    for _ in range(0, P, 32768):
+        c.update_quantized(rand(Hkv, 32768), rand(Hkv, 32768))
+    capfd.readouterr()
+    out = c.attention(rand(Hq, L), rand(Hkv, L), rand(Hkv, L), D ** -0.5, "causal")
+    torch.cuda.synchronize()
+    assert "rows written out" not in capfd.readouterr().err
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+    assert kvc.lib().kvc_device_status() == 0
