@@ -26,7 +26,8 @@
 // TMEM columns: S_0 / P_0 at 0, S_1 / P_1 at 64, O behind them. Operand layouts as in attn_chunk_tc.cu, with K / V boxes
 // of 64 rows (8 192 bytes).
 //
-// Every wait is bounded; a wait that runs out sets the device status word, the CTA drains and frees its TMEM.
+// Every wait is bounded; a wait that runs out sets the device status word, the CTA waits (bounded too) for its copies and
+// products in flight and frees its TMEM.
 #include <atomic>
 #include <cuda.h>
 
@@ -81,7 +82,8 @@ template <int STAGES> struct OneBars {
         O_DONE = P_FULL + 2,             // every O product
         O_LAST = O_DONE + 1,             // the last one
         GROUP = O_LAST + 1,              // the softmax threads meet
-        COUNT = GROUP + 1
+        DRAIN = GROUP + 1,               // the products of a CTA that gave up are done
+        COUNT = DRAIN + 1
     };
 };
 
@@ -130,6 +132,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         mbar_init(&bars[BAR::O_DONE], 1);
         mbar_init(&bars[BAR::O_LAST], 1);
         mbar_init(&bars[BAR::GROUP], 128);
+        mbar_init(&bars[BAR::DRAIN], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 4 && lane < 3) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)(lane == 0 ? &qmap : lane == 1 ? &kmap : &vmap)) : "memory");
@@ -183,11 +186,13 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 return true;
             };
             int before = -1;
+            bool q_loaded = false;
             for (int c = 0; ok && c < mine; ++c) {
                 if (!live(c)) continue;
                 const int t = piece + c * p.pieces;
                 ok = load_tile(&kmap, t);
                 if (before < 0) {
+                    q_loaded = true;
                     mbar_expect_tx(&bars[BAR::Q_FULL], (uint32_t)(p.hb * p.lb * 128 * NBOX));
 #pragma unroll
                     for (int bx = 0; bx < NBOX; ++bx) tma_load_5d(sq + bx * TC_BOX, &qmap, &bars[BAR::Q_FULL], bx * 64, h0, l0, hk, b);
@@ -197,7 +202,11 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 before = t;
             }
             if (ok && before >= 0) ok = load_tile(&vmap, before);
-            if (!ok) atomicExch(p.status, 16);
+            if (!ok) {
+                atomicExch(p.status, 16);
+                drain_copies(&bars[BAR::RING_FULL], STAGES, slot, round);
+                if (q_loaded) (void)mbar_wait(&bars[BAR::Q_FULL], 0);
+            }
         }
     } else if (warp == 5) {
         // ---------------- MMA issue (descriptors: attn_chunk_tc.cu) ----------------
@@ -259,7 +268,10 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             ++n;
         }
         if (ok && n > 0) issue_o(n - 1, true);
-        if (!ok) atomicExch(p.status, 17);
+        if (!ok) {
+            atomicExch(p.status, 17);
+            drain_products(&bars[BAR::DRAIN]);
+        }
     } else {
         // ---------------- softmax and output: thread = row ----------------
         const int row = warp * 32 + lane;

@@ -38,8 +38,8 @@
 // groups are 1024 bytes apart; the MN-major V tile advances 2048 bytes per 16 keys, its two 64-dim
 // halves are 16384 bytes apart (leading offset) and its 8-key groups 1024 bytes (stride offset).
 //
-// Every wait is bounded; a wait that runs out sets the device status word, the CTA drains and frees
-// its TMEM.
+// Every wait is bounded; a wait that runs out sets the device status word, the CTA waits (bounded too) for its copies and
+// products in flight and frees its TMEM.
 #include <atomic>
 #include <climits>
 #include <cuda.h>
@@ -107,7 +107,8 @@ template <int STAGES> struct Bars {
         O_PART = P_FULL + 8,               // [2] the O product of a part other than the last is done
         O_FULL = O_PART + 2,               // [2] the segment's last O product is done
         GROUP = O_FULL + 2,                // [2] the 128 threads of a softmax group meet
-        COUNT = GROUP + 2
+        DRAIN = GROUP + 2,                 // the products of a CTA that gave up are done
+        COUNT = DRAIN + 1
     };
 };
 
@@ -165,6 +166,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
             mbar_init(&bars[BAR::O_FULL + w], 1);
             mbar_init(&bars[BAR::GROUP + w], 128);
         }
+        mbar_init(&bars[BAR::DRAIN], 1);
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&bars[BAR::RING_FULL + s], 1);
             mbar_init(&bars[BAR::RING_EMPTY + s], 1);
@@ -288,7 +290,12 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     if (ok) ok = load_tile(&vmap, t, hk, b);
                 }
             }
-            if (!ok) atomicExch(p.status, 21);
+            if (!ok) {
+                atomicExch(p.status, 21);
+                drain_copies(&bars[BAR::RING_FULL], STAGES, slot, round);
+                for (int i = 0; i < 2; ++i)
+                    if (q_used[i] > 0) (void)mbar_wait(&bars[BAR::Q_FULL + i], (q_used[i] - 1) & 1);
+            }
         } else if (warp == 9) {
             // ---------------- MMA issue ----------------
             // instruction descriptor: f32 accumulator (bits 4-5 = 1), A and B formats (bits 7-9 and 10-12:
@@ -401,7 +408,10 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 o_first = since == 0;
                 if (s_here) --left;
             }
-            if (!ok) atomicExch(p.status, 22);
+            if (!ok) {
+                atomicExch(p.status, 22);
+                drain_products(&bars[BAR::DRAIN]);
+            }
         }
     } else {
         // ---------------- softmax and output: thread = row ----------------

@@ -137,6 +137,21 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
 
+// After a wait that ran out. Producer lane: the copies into a ring whose next entry is `slot` in its use number `round` have
+// arrived (the last use of every entry).
+__device__ __forceinline__ void drain_copies(uint64_t *full, uint32_t stages, uint32_t slot, uint32_t round) {
+    for (uint32_t s = 0; s < stages; ++s) {
+        const uint32_t uses = round + (s < slot ? 1u : 0u);
+        if (uses > 0) (void)mbar_wait(&full[s], (uses - 1) & 1);
+    }
+}
+// The warp that issues products: all of them are done (`bar`: used here alone).
+__device__ __forceinline__ void drain_products(uint64_t *bar) {
+    if (elect_one()) umma_commit(bar);
+    __syncwarp();
+    (void)warp_wait(bar, 0);
+}
+
 // Keys whose products the tensor core may add up before the sums go on in fp32 instructions. It adds towards zero, and a sum of
 // n keys loses 6e-9 n of itself (values of one sign; about half of that for values around zero): 3e-6 of an f16 output, which
 // is rounded by 2e-4, and 2.5e-5 of a bf16 one, rounded by eight times that, so that errors against 64 bits grow by 0.01 %.
