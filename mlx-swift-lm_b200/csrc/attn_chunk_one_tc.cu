@@ -285,7 +285,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         int since = -1;                      // tiles behind the last fold
         bool ok = true;
         float4 *part = (float4 *)p.o_part + ((int64_t)unit * p.pieces + piece) * (D / 4) * TC_ROWS + row;
-        FoldedSums<D> sums(o_addr, part);
+        FoldedSums<D, D == 64> sums(o_addr, part);
         for (int c = 0; c < mine; ++c) {
             if (!live(c)) continue;
             const int key0 = (piece + c * p.pieces) * ON_KEYS;

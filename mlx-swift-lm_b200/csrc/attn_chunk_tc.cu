@@ -4,15 +4,16 @@
 // of L query positions per head. The query rows of a KV head's group are cut into tiles of up to 128
 // rows, position-major (a tile is `lb` positions x `hb` heads of the group: an odd group wastes no row
 // block and a tile's causal limits lie close together). A unit is TWO neighbouring row tiles, A and B,
-// which share every K and V tile.
+// which share every K and V tile, or, where the tiles do not fill the SMs (SINGLE), one.
 //
 //   warps 0..3  softmax of tile A, warps 4..7 of tile B: thread = query row = TMEM lane. The 128 scores of a
 //               key tile come out of TMEM in one round trip, row maximum, exponentials, and P goes back into
 //               TMEM over the scores' own columns, where the O product reads it as its A operand
-//   warp 8      TMA producer: Q tiles per unit, K and V tiles into one ring
-//   warp 9      owns the TMEM allocation and issues the MMAs in the order
+//   warp 8 (4)  TMA producer: Q tiles per unit, K and V tiles into one ring
+//   warp 9 (5)  owns the TMEM allocation and issues the MMAs in the order
 //                 O_A += P_A(j) V_j | S_A = Q_A K_{j+1}^T | O_B += P_B(j) V_j | S_B = Q_B K_{j+1}^T
-//               so that one tile's products run while the other tile's softmax does
+//               so that one tile's products run while the other tile's softmax does. A single row tile has B's buffer for
+//               its scores too, S of tile j + 1 comes before O += P(j) V(j), and there are no warps 4..7
 //
 // O accumulates in TMEM, in the reference that the row's exponents are taken against. The scores of tile j + 1 are
 // issued behind the O product of tile j, so when they arrive O is settled and the softmax threads may multiply it; they
@@ -24,12 +25,13 @@
 //
 // The tensor core adds towards zero: a sum of n keys in one accumulator loses 6e-9 n of itself (values of one sign), which
 // outgrows the rounding of an f16 output within a few thousand keys. After `fold` key tiles the softmax threads therefore add
-// O to fp32 sums of their own, behind O in TMEM at head dim 64 and in memory at 128, and the next O product starts from nothing.
+// O to fp32 sums of their own, behind O in TMEM or, for pairs at head dim 128, in memory, and the next O product starts from
+// nothing.
 //
 // Units are handed out whole, in rounds of one per SM; what is left over is laid end to end and cut into equal ranges,
 // or few units are cut into pieces (a cut unit leaves fp32 partials, and the CTA that finishes it merges them).
 //
-// TMEM columns: S_A / P_A at 0, S_B / P_B at 128, O_A at 256, O_B at 384.
+// TMEM columns: S_A / P_A at 0, S_B / P_B at 128, O_A at 256, O_B at 384. (Single: S_0 / P_0, S_1 / P_1, O, folded sums.)
 //
 // Shared-memory operand layout (what TMA's 128-byte swizzle writes): a box is 128 rows x 128 bytes
 // (64 elements), 16-byte chunk c of row r at chunk c ^ (r & 7); a 128 x 128 tile is two boxes (Q, K and
@@ -60,8 +62,9 @@ using namespace dev;
 
 using namespace tc;
 
-constexpr int CT_THREADS = 384;
-// registers a thread: 384 * 168 at launch = 256 * 216 (softmax) + 128 * 72 (the warps that issue copies and MMAs)
+// Pairs: registers a thread: 384 * 168 at launch = 256 * 216 (softmax) + 128 * 72 (the warps that issue copies and MMAs). A single
+// row tile has half the softmax warps, and registers enough as launched.
+template <bool SINGLE> constexpr int ct_threads() { return SINGLE ? 192 : 384; }
 constexpr int CT_REGS_SOFTMAX = 216, CT_REGS_ISSUE = 72;
 // The reference of a part is never further below the row's largest score than this, so that O and the sums stay far
 // from overflow.
@@ -70,12 +73,13 @@ constexpr float CT_SPAN_LOG2 = 24.f;
 struct ChunkTcParams {
     void *out;
     int64_t o_sb, o_sh, o_sl;
-    int32_t B, rep, Hkv, L;
+    int32_t rep, Hkv, L;
     int64_t T;
+    int32_t wide;               // row tiles a unit
     int32_t hb, lb;             // heads and positions of a row tile (hb * lb <= 128)
     int32_t head_tiles;         // row tiles side by side over the group's heads
     int32_t row_tiles;          // row tiles of a (batch, KV head)
-    int32_t units;              // ... and units: pairs of row tiles
+    int32_t units;              // ... and units of one or two row tiles
     int32_t causal;
     int64_t causal_offset;
     float scale_log2;
@@ -87,7 +91,7 @@ struct ChunkTcParams {
     int32_t group_tiles;        // key tiles of the units of a (batch, KV head)
     int32_t tail_base;          // ... of those before the tail's first unit in its own group
     int32_t fold;               // key tiles of a segment between two folds
-    float *o_fold;              // [CTA][A / B][D / 4][128 rows][4] (head dim 128)
+    float *o_fold;              // [CTA][A / B][D / 4][128 rows][4] (pairs at head dim 128)
     float *o_part;              // [CTA][first / last segment][A / B][D / 4][128 rows][4]
     float2 *ml_part;            // [CTA][first / last segment][A / B][128 rows] (reference, sum)
     int *tickets;               // [unit of the tail][A / B], zeroed before the launch
@@ -112,27 +116,30 @@ template <int STAGES> struct Bars {
     };
 };
 
-// The pair of row tiles of a unit, and its key tiles. Units of a (batch, KV head) are counted from the last positions
+// The first row tile of a unit, and its key tiles. Units of a (batch, KV head) are counted from the last positions
 // to the first: with a causal mask the long units go first.
-__device__ __host__ inline int ct_pair_of(const ChunkTcParams &p, int unit) { return p.units - 1 - unit % p.units; }
+__device__ __host__ inline int ct_first_of(const ChunkTcParams &p, int unit) { return p.wide * (p.units - 1 - unit % p.units); }
 __device__ __host__ inline int ct_unit_tiles(const ChunkTcParams &p, int unit) {
     if (!p.causal) return (int)((p.T + TC_KEYS - 1) / TC_KEYS);
-    const int pair = ct_pair_of(p, unit), last_tile = 2 * pair + 1 < p.row_tiles ? 2 * pair + 1 : p.row_tiles - 1;
+    const int first = ct_first_of(p, unit), last_tile = first + p.wide <= p.row_tiles ? first + p.wide - 1 : p.row_tiles - 1;
     const int64_t end = (int64_t)(last_tile / p.head_tiles + 1) * p.lb;
     const int64_t keys = p.causal_offset + (end < p.L ? end : p.L);
     return (int)(((keys < p.T ? keys : p.T) + TC_KEYS - 1) / TC_KEYS);
 }
 
-// A CTA's work in segments, one per unit it touches.
+// A CTA's work in segments, one per unit it touches. (What takes divisions is worked out once, before the wait for the launch
+// ahead: on short calls the producer's first copy and the stores waited for it.)
 struct CtSegment {
     int unit;
     int t0, t1, n;     // its key tiles, and the unit's
     int has_b;         // the unit has two row tiles
+    int hk, b;         // KV head and sequence
+    int l0[2], h0[2];  // first position and head of the row tiles
 };
 constexpr int CT_MAX_SEGMENTS = 40;
 
-template <typename T, int D, int PARTS>
-__global__ void __launch_bounds__(CT_THREADS, 1)
+template <typename T, int D, int PARTS, bool SINGLE>
+__global__ void __launch_bounds__(ct_threads<SINGLE>(), 1)
 attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                      const __grid_constant__ CUtensorMap vmap, const __grid_constant__ ChunkTcParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -153,6 +160,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
     int *s_ticket = s_segments + 1;                            // [2]
     CtSegment *s_seg = (CtSegment *)(s_ticket + 2);            // [CT_MAX_SEGMENTS]
 
+    constexpr int THREADS = ct_threads<SINGLE>(), PRODUCER = SINGLE ? 4 : 8, ISSUER = PRODUCER + 1;   // (warps)
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be the same in all lanes: a role's addresses stay in uniform registers
 
@@ -183,7 +191,15 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 CtSegment &g = s_seg[segments];
                 g.unit = unit;
                 g.t0 = t0; g.t1 = t1; g.n = n;
-                g.has_b = 2 * ct_pair_of(p, unit) + 1 < p.row_tiles;
+                const int group = unit / p.units, rt = ct_first_of(p, unit);
+                g.has_b = !SINGLE && rt + 1 < p.row_tiles;
+                g.b = group / p.Hkv;
+                g.hk = group - g.b * p.Hkv;
+                for (int i = 0; i < (SINGLE ? 1 : 2); ++i) {
+                    const int row_block = (rt + i) / p.head_tiles;
+                    g.l0[i] = row_block * p.lb;
+                    g.h0[i] = (rt + i - row_block * p.head_tiles) * p.hb;
+                }
             }
             ++segments;
         };
@@ -231,30 +247,30 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
         if (lane == 0) *s_segments = segments;
     }
     // rows of a Q tile that no copy writes are zero
-    for (int i = tid; i < 2 * NBOX * (TC_ROWS - p.hb * p.lb) * 8; i += CT_THREADS) {
+    for (int i = tid; i < 2 * NBOX * (TC_ROWS - p.hb * p.lb) * 8; i += THREADS) {
         const int chunk = i & 7, box = (i >> 3) % (2 * NBOX), row = (i >> 3) / (2 * NBOX) + p.hb * p.lb;
         *(uint4 *)(sq + box * TC_BOX + row * 128 + chunk * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     // the first copies are on their way while the others wait for the TMEM columns
-    if (warp == 9) {
+    if (warp == ISSUER) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TC_TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (warp != 8) {
+    if (warp != PRODUCER) {
         tc_fence_before();
-        asm volatile("bar.sync 1, %0;" ::"n"(CT_THREADS - 32) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(THREADS - 32) : "memory");
         tc_fence_after();
     }
-    const uint32_t tmem = warp == 8 ? 0u : *tmem_slot;       // (nothing of the producer's)
+    const uint32_t tmem = warp == PRODUCER ? 0u : *tmem_slot;       // (nothing of the producer's)
     const int segments = *s_segments;
     pdl_wait();  // everything below reads what earlier kernels on the stream wrote
 
-    if (warp >= 8) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CT_REGS_ISSUE));
-        if (warp == 8 && lane == 0) {
+    if (warp >= PRODUCER) {
+        if constexpr (!SINGLE) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CT_REGS_ISSUE));
+        if (warp == PRODUCER && lane == 0) {
             // ---------------- producer ----------------
             bool ok = true;
             uint32_t slot = 0, round = 0, q_used[2] = {0, 0};
@@ -271,19 +287,17 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 return true;
             };
             for (int sg = 0; ok && sg < segments; ++sg) {
-                const CtSegment g = s_seg[sg];
-                const int group = g.unit / p.units, hk = group % p.Hkv, b = group / p.Hkv;
+                const CtSegment &g = s_seg[sg];
+                const int hk = g.hk, b = g.b;
                 ok = load_tile(&kmap, g.t0, hk, b);
                 for (int i = 0; ok && i <= g.has_b; ++i) {
                     if (q_used[i] > 0) ok = mbar_wait(&bars[BAR::Q_EMPTY + i], (q_used[i] - 1) & 1);
                     if (!ok) break;
                     ++q_used[i];
-                    const int rt = 2 * ct_pair_of(p, g.unit) + i;
                     mbar_expect_tx(&bars[BAR::Q_FULL + i], (uint32_t)(p.hb * p.lb * 128 * NBOX));
 #pragma unroll
                     for (int bx = 0; bx < NBOX; ++bx)
-                        tma_load_5d(sq + i * TILE + bx * TC_BOX, &qmap, &bars[BAR::Q_FULL + i], bx * 64, (rt % p.head_tiles) * p.hb,
-                                    (rt / p.head_tiles) * p.lb, hk, b);
+                        tma_load_5d(sq + i * TILE + bx * TC_BOX, &qmap, &bars[BAR::Q_FULL + i], bx * 64, g.h0[i], g.l0[i], hk, b);
                 }
                 for (int t = g.t0; ok && t < g.t1; ++t) {
                     if (t > g.t0) ok = load_tile(&kmap, t, hk, b);
@@ -296,7 +310,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 for (int i = 0; i < 2; ++i)
                     if (q_used[i] > 0) (void)mbar_wait(&bars[BAR::Q_FULL + i], (q_used[i] - 1) & 1);
             }
-        } else if (warp == 9) {
+        } else if (warp == ISSUER) {
             // ---------------- MMA issue ----------------
             // instruction descriptor: f32 accumulator (bits 4-5 = 1), A and B formats (bits 7-9 and 10-12:
             // 0 = f16, 1 = bf16), B major at bit 16 (1 = MN-major), N / 8 at bits 17-22, M / 16 at 24-28
@@ -319,11 +333,82 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     par ^= 1;
                 }
             };
+            if constexpr (SINGLE) {
+                // One step takes the S product of a key tile, into the buffer its predecessor does not use, and the O product of
+                // that predecessor.
+                int sg = 0, left = 0, since = 0;     // the segment of the next S product, its tiles still to come; S products behind the last fold
+                bool o_here = false, o_first = false;
+                for (uint32_t n = 0; ok; ++n) {
+                    const bool opens = left == 0 && sg < segments;
+                    if (opens) {
+                        left = s_seg[sg].t1 - s_seg[sg].t0;
+                        ++sg;
+                    }
+                    const bool s_here = left > 0, o_last = o_here && (opens || !s_here);
+                    if (!o_here && !s_here) break;
+                    if (s_here) {
+                        ok = warp_wait(&bars[BAR::RING_FULL + k_slot], k_par);
+                        if (ok && opens) {
+                            ok = warp_wait(&bars[BAR::Q_FULL], q_par);
+                            q_par ^= 1;
+                        }
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint64_t kd = k_desc + (uint64_t)(k_slot * (TILE / 16));
+                        if (elect_one()) {
+#pragma unroll
+                            for (int ks = 0; ks < D / 16; ++ks) {
+                                const uint64_t off = (uint64_t)((ks >> 2) * (TC_BOX / 16) + (ks & 3) * 2);
+                                umma_f16(tmem + (n & 1) * 128u, q_desc + off, kd + off, IDESC, ks > 0 ? 1u : 0u);
+                            }
+                            umma_commit(&bars[BAR::S_FULL + (n & 1)]);
+                            if (left == 1) umma_commit(&bars[BAR::Q_EMPTY]);
+                            umma_commit(&bars[BAR::RING_EMPTY + k_slot]);
+                        }
+                        __syncwarp();
+                        step2(k_slot, k_par);
+                    }
+                    if (o_here) {
+                        const uint32_t buf = (n - 1) & 1, par = ((n - 1) >> 1) & 1;
+                        ok = warp_wait(&bars[BAR::RING_FULL + v_slot], v_par);
+                        const uint64_t vd = v_desc + (uint64_t)(v_slot * (TILE / 16));
+                        auto o_part = [&](auto which) {
+                            constexpr int h = decltype(which)::value, FROM = key_of(h) / 16, TO = key_of(h + 1) / 16;
+                            if (ok) ok = warp_wait(&bars[BAR::P_FULL + 2 * h + buf], par);
+                            if (!ok) return;
+                            tc_fence_after();
+                            if (elect_one()) {
+#pragma unroll
+                                for (int ks = FROM; ks < TO; ++ks)
+                                    umma_f16_ts(tmem + 256u, tmem + buf * 128u + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_PV,
+                                                (o_first && ks == 0) ? 0u : 1u);
+                                if (PARTS > 1 || h == HANDS - 1) umma_commit(&bars[BAR::O_PART]);
+                                if (h == HANDS - 1) {
+                                    if (o_last) umma_commit(&bars[BAR::O_FULL]);
+                                    umma_commit(&bars[BAR::RING_EMPTY + v_slot]);
+                                }
+                            }
+                            __syncwarp();
+                        };
+                        o_part(std::integral_constant<int, 0>());
+                        o_part(std::integral_constant<int, 1>());
+                        if constexpr (HANDS == 4) {
+                            o_part(std::integral_constant<int, 2>());
+                            o_part(std::integral_constant<int, 3>());
+                        }
+                        step2(v_slot, v_par);
+                    }
+                    o_here = s_here;
+                    since = opens || since == p.fold - 1 ? 0 : since + 1;
+                    o_first = since == 0;
+                    if (s_here) --left;
+                }
+            }
             // One step takes the O products of a key tile and the S products of the next one, which may open the next segment.
             int sg = 0, left = 0;                    // the segment of the next S products, and its tiles still to come
             int since = 0;                           // S products behind the last fold
             bool o_here = false, o_first = false, o_b = false, b = false;   // *b: the unit has a row tile B
-            while (ok) {
+            while (!SINGLE && ok) {
                 const bool opens = left == 0 && sg < segments;
                 o_b = b;
                 if (opens) {
@@ -415,34 +500,42 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
         }
     } else {
         // ---------------- softmax and output: thread = row ----------------
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CT_REGS_SOFTMAX));
+        if constexpr (!SINGLE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CT_REGS_SOFTMAX));
         const int i = warp >> 2;                            // row tile A / B
         const int quarter = warp & 3;                       // the TMEM lanes this warp may touch
         const int row = quarter * 32 + lane;
-        const uint32_t s_addr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)i * 128u;
-        const uint32_t o_addr = s_addr + 256u;
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16), o_addr = lanes + 256u + (uint32_t)i * 128u;
+        uint32_t buf = i, s_addr = lanes + buf * 128u;       // S / P buffer: the row tile's own, or both in turn
         const int row_l = row / p.hb, row_h = row % p.hb;
         const uint64_t scale2 = pack_f2(p.scale_log2, p.scale_log2);
         uint32_t s_par = 0, o_par = 0, g_par = 0, h_par = 0;
         bool ok = true;
         for (int sg = 0; ok && sg < segments; ++sg) {
-            const CtSegment w = s_seg[sg];
+            const CtSegment &w = s_seg[sg];
             if (i == 1 && !w.has_b) continue;
-            const int rt = 2 * ct_pair_of(p, w.unit) + i;
-            const int l0 = (rt / p.head_tiles) * p.lb;
-            const int l = l0 + row_l, h = (rt % p.head_tiles) * p.hb + row_h;
+            const int l0 = w.l0[i], l = l0 + row_l, h = w.h0[i] + row_h;
             const bool valid = row < p.hb * p.lb && l < p.L && h < p.rep;
             const int limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l) : p.T - 1);     // last visible key
             const int tile_limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l0) : p.T - 1);
             float m_top = -INFINITY, m_ref = -INFINITY, l_run = 0.f;   // largest score, reference of O and of l_run
             int since = -1;                                            // tiles behind the last fold
-            FoldedSums<D> sums(o_addr, (float4 *)p.o_fold + ((int64_t)blockIdx.x * 2 + i) * (D / 4) * TC_ROWS + row);
+            FoldedSums<D, SINGLE || D == 64> sums(o_addr, (float4 *)p.o_fold + ((int64_t)blockIdx.x * 2 + i) * (D / 4) * TC_ROWS + row);
             for (int t = w.t0; t < w.t1; ++t) {
-                ok = warp_wait(&bars[BAR::S_FULL + i], s_par);
+                ok = warp_wait(&bars[BAR::S_FULL + buf], s_par);
                 if (!ok) break;
-                s_par ^= 1;
+                if (!SINGLE) s_par ^= 1;
                 tc_fence_after();
+                // one row tile: the scores come while the O product of the tile before may be under way
+                bool settled = !SINGLE || t == w.t0;
+                auto settle = [&] {
+                    ok = warp_wait(&bars[BAR::O_PART], h_par);
+                    h_par ^= 1;
+                    tc_fence_after();
+                    settled = true;
+                };
                 if (++since == p.fold) {
+                    if (!settled) settle();
+                    if (!ok) break;
                     sums.fold(m_ref);
                     since = 0;
                 }
@@ -470,7 +563,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     alpha[part] = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - ref[part]);
                     m_ref = ref[part];
                 }
-                // O is settled when the scores are there: they came behind the O products of the tile before
+                // O is settled when the scores of a pair are there: they came behind the O products of the tile before
                 auto hand_over = [&](auto which) {
                     constexpr int h = decltype(which)::value, FROM = key_of(h), TO = key_of(h + 1), part = PARTS == 1 ? 0 : h;
                     const bool first = h == 0, move = (first ? since > 0 : PARTS > 1) && __any_sync(0xffffffffu, alpha[part] != 1.f);
@@ -496,6 +589,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     const float neg_m = ref[part] == -INFINITY ? 0.f : -ref[part];   // exp2(-inf) = 0
                     const uint64_t neg2 = pack_f2(neg_m, neg_m);
                     uint64_t sum[2] = {0, 0};
+                    if (SINGLE && first && !settled) settle();
 #pragma unroll
                     for (int k0 = FROM; k0 < TO; k0 += CH) {
                         // a rescale of O runs under the exponentials: they wait for the special-function unit
@@ -527,7 +621,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     for (int c = FROM / 2; c < TO / 2; c += 16) tmem_st16_issue(s_addr + c, raw + c);
                     tmem_st_wait();
                     tc_fence_before();
-                    mbar_arrive(&bars[BAR::P_FULL + 2 * h + i]);
+                    mbar_arrive(&bars[BAR::P_FULL + 2 * h + buf]);
                     float s0, s1, s2, s3;
                     unpack_f2(sum[0], s0, s1);
                     unpack_f2(sum[1], s2, s3);
@@ -540,14 +634,19 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     hand_over(std::integral_constant<int, PARTS == 4 ? 3 : 0>());
                 }
                 if (!ok) break;
+                if (SINGLE) {
+                    s_par ^= buf;
+                    buf ^= 1;
+                    s_addr = lanes + buf * 128u;
+                }
             }
             if (!ok) break;
+            if (SINGLE) h_par ^= 1;                          // (the last O product: the wait below)
             ok = warp_wait(&bars[BAR::O_FULL + i], o_par);
             if (!ok) break;
             o_par ^= 1;
             tc_fence_after();
-            const int group = w.unit / p.units, hk = group % p.Hkv, b = group / p.Hkv;
-            T *dst = (T *)p.out + b * p.o_sb + (int64_t)(hk * p.rep + h) * p.o_sh + (int64_t)l * p.o_sl;
+            T *dst = (T *)p.out + w.b * p.o_sb + (int64_t)(w.hk * p.rep + h) * p.o_sh + (int64_t)l * p.o_sl;
             if (w.t0 == 0 && w.t1 == w.n) {
                 const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
 #pragma unroll 1
@@ -647,13 +746,13 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
     // all roles meet here; TMEM goes back whatever happened
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == ISSUER) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
     }
 }
 
-template <typename T, int D, int PARTS>
+template <typename T, int D, int PARTS, bool SINGLE>
 bool launch_tc_as(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkTcParams &p, int ctas,
                   cudaStream_t stream) {
     const size_t smem = (size_t)(D / 64) * TC_BOX * (2 + ct_stages<D>()) + Bars<ct_stages<D>()>::COUNT * sizeof(uint64_t) + 16 +
@@ -667,24 +766,31 @@ bool launch_tc_as(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtens
     int state = configured[dev].load(std::memory_order_acquire);
     if (state == 0) {
         // setting the attribute twice from two racing threads is harmless; the result is the same
-        const cudaError_t e = cudaFuncSetAttribute(attn_chunk_tc_kernel<T, D, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_chunk_tc_kernel<T, D, PARTS, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) (void)cudaGetLastError();
         state = e == cudaSuccess ? 1 : -1;
         configured[dev].store(state, std::memory_order_release);
     }
     if (state < 0) return false;
     KernelTimer timer(stream);
-    KVC_CUDA(launch_pdl(attn_chunk_tc_kernel<T, D, PARTS>, dim3(ctas), dim3(CT_THREADS), smem, stream, qmap, kmap, vmap, p));
+    KVC_CUDA(launch_pdl(attn_chunk_tc_kernel<T, D, PARTS, SINGLE>, dim3(ctas), dim3(ct_threads<SINGLE>()), smem, stream, qmap, kmap, vmap, p));
     timer.stop();
     ++g_launch_count;
     return true;
 }
 
+template <typename T, int D, bool SINGLE>
+bool launch_tc_parts(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkTcParams &p, int ctas, int parts,
+                     cudaStream_t stream) {
+    if (parts == 4) return launch_tc_as<T, D, 4, SINGLE>(qmap, kmap, vmap, p, ctas, stream);
+    return parts == 2 ? launch_tc_as<T, D, 2, SINGLE>(qmap, kmap, vmap, p, ctas, stream) : launch_tc_as<T, D, 1, SINGLE>(qmap, kmap, vmap, p, ctas, stream);
+}
+
 template <typename T, int D>
 bool launch_tc_typed(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkTcParams &p, int ctas, int parts,
                      cudaStream_t stream) {
-    if (parts == 4) return launch_tc_as<T, D, 4>(qmap, kmap, vmap, p, ctas, stream);
-    return parts == 2 ? launch_tc_as<T, D, 2>(qmap, kmap, vmap, p, ctas, stream) : launch_tc_as<T, D, 1>(qmap, kmap, vmap, p, ctas, stream);
+    return p.wide == 1 ? launch_tc_parts<T, D, true>(qmap, kmap, vmap, p, ctas, parts, stream)
+                       : launch_tc_parts<T, D, false>(qmap, kmap, vmap, p, ctas, parts, stream);
 }
 
 // 128-row blocks of the call's query rows, head by head.
@@ -733,7 +839,7 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     ChunkTcParams p = {};
     p.out = a.out;
     p.o_sb = a.o_sb; p.o_sh = a.o_sh; p.o_sl = a.o_sl;
-    p.B = a.B; p.rep = a.Hq / a.Hkv; p.Hkv = a.Hkv; p.L = a.L; p.T = a.T;
+    p.rep = a.Hq / a.Hkv; p.Hkv = a.Hkv; p.L = a.L; p.T = a.T;
     p.causal = a.mask.mode == KVC_MASK_CAUSAL ? 1 : 0;
     p.causal_offset = a.mask.causal_offset;
     p.scale_log2 = a.scale * 1.4426950408889634f;
@@ -749,18 +855,8 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     const int64_t row_tiles = (int64_t)p.head_tiles * ((a.L + p.lb - 1) / p.lb);
     if (row_tiles > (int64_t)1 << 20) return 0;
     p.row_tiles = (int)row_tiles;
-    p.units = (p.row_tiles + 1) / 2;
     const int64_t groups = (int64_t)a.B * a.Hkv;
-    int64_t group_tiles = 0;
-    int most = 0, least = INT_MAX;
-    for (int u = 0; u < p.units; ++u) {
-        const int n = ct_unit_tiles(p, u);
-        group_tiles += n;
-        most = std::max(most, n);
-        least = std::min(least, n);
-    }
-    if (groups * p.units > (int64_t)1 << 28) return 0;
-    p.all_units = (int)(groups * p.units);
+    if (groups * p.row_tiles > (int64_t)1 << 28) return 0;
 
     CUtensorMap qmap, kmap, vmap;
     if (!make_query_map(&qmap, a, p.rep, p.hb, p.lb)) return 0;
@@ -782,65 +878,106 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     //   whole units in rounds, so that neighbours share their K and V tiles, and equal ranges of what is left.
     // (D 128, 160 units of 1 ... 3 tiles: 19 us whole, 34 in ranges; 48 of 5 or 6, D 64: 17 whole, 21 in pieces; 40 of 16: 38
     // whole, 33 in pieces, 37 in ranges; 64 of 254: 494, 261, 236.)
+    // All of it for units of two row tiles and of one, whose key tiles take 0.6 of the time, or more where the references of a tile
+    // follow one another (D 128, us in pairs and one by one: 8 heads x 400 positions behind 695 keys 29.1, 19.5; 512 behind 1 024
+    // 31.2, 22.9; 1 024 of 1 024 23.5, 29.8; four references, 64 positions behind 448 20.1, 14.9).
     constexpr int64_t L2_BYTES = (int64_t)64 << 20;
-    const int64_t sms = sm_count(a.device), units = p.all_units, flat = groups * group_tiles, average = (flat + units - 1) / units;
+    const int64_t sms = sm_count(a.device);
     const bool settled = groups * a.T * a.D * 4 <= L2_BYTES;
-    const int64_t rounds = (units + sms - 1) / sms;
-    const bool even = least * 4 >= most * 3 && rounds <= CT_MAX_SEGMENTS;
-    const int64_t waves = settled ? 0 : units / sms;
-    const int64_t tail = settled ? flat : (units - waves * sms) * average, per = std::max<int64_t>(4, (tail + sms - 1) / sms);   // (exact length below)
-    const int64_t pieces = std::min<int64_t>(sms / units, least / 2);
-    const int64_t set_up = 3 + (parts == 1 ? 3 : 2);
-    const int64_t whole = even ? 3 + rounds * (average + 1) : std::max<int64_t>(most, rounds * average) + 3 * rounds;
-    const int64_t cut = set_up + waves * (most + 1) + per + 2 * (per / average) + 3 + (most / per + 2) / 2;
-    const int64_t apart = pieces > 1 ? set_up + (most + pieces - 1) / pieces + 2 + pieces / 2 : INT64_MAX;
-    int64_t tail_tiles = 0, ranges = 0;
-    if (apart < whole && apart <= cut) {
-        ranges = units * pieces;
-    } else if (cut < whole && waves + 2 < CT_MAX_SEGMENTS) {
-        tail_tiles = flat;
-        for (int64_t u = 0; u < waves * sms; ++u) tail_tiles -= ct_unit_tiles(p, (int)(u % p.units));
-        ranges = std::max<int64_t>(1, std::min<int64_t>(sms, tail_tiles / 4));
-        if (tail_tiles < 1 || tail_tiles > (int64_t)1 << 29 || group_tiles > (int64_t)1 << 29 ||
-            tail_tiles / ranges / least + 2 > CT_MAX_SEGMENTS - waves)
-            tail_tiles = ranges = 0;
+    struct Plan {
+        double cost;
+        int64_t units, group_tiles, rounds, waves, pieces, ranges, tail_tiles;
+        int most;
+        bool even;
+    };
+    auto plan_of = [&](int wide) {
+        Plan g = {};
+        p.wide = wide;
+        p.units = (p.row_tiles + wide - 1) / wide;
+        int least = INT_MAX;
+        for (int u = 0; u < p.units; ++u) {
+            const int n = ct_unit_tiles(p, u);
+            g.group_tiles += n;
+            g.most = std::max(g.most, n);
+            least = std::min(least, n);
+        }
+        g.units = groups * p.units;
+        const double tile = wide == 2 ? 1.0 : parts == 1 ? 0.6 : parts == 2 ? 0.8 : 0.9;
+        const int64_t flat = groups * g.group_tiles, average = (flat + g.units - 1) / g.units;
+        g.rounds = (g.units + sms - 1) / sms;
+        g.even = least * 4 >= g.most * 3 && g.rounds <= CT_MAX_SEGMENTS;
+        g.waves = settled ? 0 : g.units / sms;
+        const int64_t tail = settled ? flat : (g.units - g.waves * sms) * average, per = std::max<int64_t>(4, (tail + sms - 1) / sms);   // (exact length below)
+        g.pieces = std::min<int64_t>(sms / g.units, least / 2);
+        const int set_up = 3 + (parts == 1 ? 3 : 2);
+        const double whole = g.even ? 3 + g.rounds * (average * tile + 1) : std::max<int64_t>(g.most, g.rounds * average) * tile + 3 * g.rounds;
+        const double cut = set_up + g.waves * (g.most * tile + 1) + per * tile + 2 * (per / average) + 3 + (g.most / per + 2) / 2;
+        const double apart = g.pieces > 1 ? set_up + (g.most + g.pieces - 1) / g.pieces * tile + 2 + g.pieces / 2 : INFINITY;
+        g.cost = whole;
+        if (apart < whole && apart <= cut) {
+            g.ranges = g.units * g.pieces;
+            g.cost = apart;
+        } else if (cut < whole && g.waves + 2 < CT_MAX_SEGMENTS) {
+            g.tail_tiles = flat;
+            for (int64_t u = 0; u < g.waves * sms; ++u) g.tail_tiles -= ct_unit_tiles(p, (int)(u % p.units));
+            g.ranges = std::max<int64_t>(1, std::min<int64_t>(sms, g.tail_tiles / 4));
+            g.cost = cut;
+            if (g.tail_tiles < 1 || g.tail_tiles > (int64_t)1 << 29 || g.group_tiles > (int64_t)1 << 29 ||
+                g.tail_tiles / g.ranges / least + 2 > CT_MAX_SEGMENTS - g.waves) {
+                g.tail_tiles = g.ranges = 0;
+                g.cost = whole;
+            }
+        }
+        return g;
+    };
+    Plan g = plan_of(1);
+    if (p.row_tiles > 1) {
+        const Plan pairs = plan_of(2);
+        if (pairs.cost <= g.cost) g = pairs;
+        else (void)plan_of(1);
     }
+    p.all_units = (int)g.units;
     int64_t ctas, longest;                                       // ... and the most key tiles of a segment
     size_t o_bytes, ml_bytes, t_bytes, fold_bytes;
     auto lay_out = [&] {
-        if (tail_tiles > 0) {
-            ctas = waves > 0 ? sms : ranges;
-            p.waves = (int)waves;
-            p.ranges = (int)ranges;
-            p.per = (int)(tail_tiles / ranges);
-            p.rem = (int)(tail_tiles % ranges);
-            p.group_tiles = (int)group_tiles;
-            for (int64_t u = waves * sms / p.units * p.units; u < waves * sms; ++u) p.tail_base += ct_unit_tiles(p, (int)u);
-            longest = waves > 0 ? most : std::min(most, p.per + 1);
-        } else if (ranges > 0) {
-            ctas = ranges;
-            p.pieces = (int)pieces;
-            longest = (most + pieces - 1) / pieces;
+        if (g.tail_tiles > 0) {
+            ctas = g.waves > 0 ? sms : g.ranges;
+            p.waves = (int)g.waves;
+            p.ranges = (int)g.ranges;
+            p.per = (int)(g.tail_tiles / g.ranges);
+            p.rem = (int)(g.tail_tiles % g.ranges);
+            p.group_tiles = (int)g.group_tiles;
+            for (int64_t u = g.waves * sms / p.units * p.units; u < g.waves * sms; ++u) p.tail_base += ct_unit_tiles(p, (int)u);
+            longest = g.waves > 0 ? g.most : std::min(g.most, p.per + 1);
+        } else if (g.ranges > 0) {
+            ctas = g.ranges;
+            p.pieces = (int)g.pieces;
+            longest = (g.most + g.pieces - 1) / g.pieces;
         } else {
-            ctas = even ? std::min(units, sms) : units;
-            p.waves = even ? (int)rounds : 1;
-            longest = most;
+            ctas = g.even ? std::min(g.units, sms) : g.units;
+            p.waves = g.even ? (int)g.rounds : 1;
+            longest = g.most;
         }
         // (in memory a fold costs a key tile's time: 512 f16 keys 323 us where no folds take 267, 768 about 300, and the kernel
         // that folded every tile in registers 311; 512 x 8 x 32 heads behind 3 584 keys)
-        p.fold = fold_keys(a.q_dtype) * (a.D == 128 ? 3 : 2) / 2 / TC_KEYS;
-        const size_t part = (size_t)ranges * 4 * TC_ROWS;
+        const bool in_memory = a.D == 128 && p.wide == 2;
+        p.fold = fold_keys(a.q_dtype) * (in_memory ? 3 : 2) / 2 / TC_KEYS;
+        if (in_memory) {                                         // even stretches: no fold for a last tile or two
+            const int64_t stretches = std::max<int64_t>(1, (2 * longest + p.fold) / (2 * p.fold));
+            p.fold = (int)((longest + stretches - 1) / stretches);
+        }
+        const size_t part = (size_t)g.ranges * 4 * TC_ROWS;
         o_bytes = part * a.D * sizeof(float);
         ml_bytes = part * sizeof(float2);
-        t_bytes = ranges > 0 ? (size_t)(tail_tiles > 0 ? units - waves * sms : units) * 2 * sizeof(int) : 0;
-        fold_bytes = a.D == 128 && longest > p.fold ? (size_t)ctas * 2 * TC_ROWS * a.D * sizeof(float) : 0;
+        t_bytes = g.ranges > 0 ? (size_t)(g.tail_tiles > 0 ? g.units - g.waves * sms : g.units) * 2 * sizeof(int) : 0;
+        fold_bytes = in_memory && longest > p.fold ? (size_t)ctas * 2 * TC_ROWS * a.D * sizeof(float) : 0;
         return fold_bytes + o_bytes + ml_bytes + t_bytes;
     };
     const ChunkTcParams uncut = p;
     CallMemory mem(lay_out(), stream);
-    if (!mem.ptr && ranges > 0) {                                // no room: whole units
+    if (!mem.ptr && g.ranges > 0) {                              // no room: whole units
         p = uncut;
-        tail_tiles = ranges = 0;
+        g.tail_tiles = g.ranges = 0;
         lay_out();
     }
     if (!mem.ptr && fold_bytes > 0) return 0;
@@ -848,7 +985,7 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
     p.o_part = (float *)((char *)mem.ptr + fold_bytes);
     p.ml_part = (float2 *)((char *)p.o_part + o_bytes);
     p.tickets = (int *)((char *)p.ml_part + ml_bytes);
-    if (ranges > 0) KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
+    if (g.ranges > 0) KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
     bool taken;
     if (a.D == 128)
         taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 128>(qmap, kmap, vmap, p, (int)ctas, parts, stream)
@@ -857,8 +994,8 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
         taken = a.q_dtype == KVC_BF16 ? launch_tc_typed<__nv_bfloat16, 64>(qmap, kmap, vmap, p, (int)ctas, parts, stream)
                                       : launch_tc_typed<__half, 64>(qmap, kmap, vmap, p, (int)ctas, parts, stream);
     if (taken && trace_dispatch())
-        fprintf(stderr, "[kvc] chunk_tc: %lld units of two row tiles (%d heads x %d positions), %lld CTAs, %d rounds, ranges of %d tiles, %d pieces, %d references a tile\n",
-                (long long)units, p.hb, p.lb, (long long)ctas, p.waves, p.per, p.pieces, parts);
+        fprintf(stderr, "[kvc] chunk_tc: %lld units of %d row tiles (%d heads x %d positions), %lld CTAs, %d rounds, ranges of %d tiles, %d pieces, %d references a tile\n",
+                (long long)g.units, p.wide, p.hb, p.lb, (long long)ctas, p.waves, p.per, p.pieces, parts);
     return taken ? 1 : 0;
 }
 

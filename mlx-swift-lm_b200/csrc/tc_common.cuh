@@ -164,8 +164,7 @@ __device__ __forceinline__ void add4_global(float4 *p, float x, float y, float z
 // The fp32 sums a softmax thread (a row) folds its D columns of O into, in a reference of their own. Behind O in TMEM where
 // there is room, otherwise in memory that only this thread touches: [column / 4][128 rows] of float4, added to where they lie
 // (no load to wait for) unless the reference has left them far behind.
-template <int D> struct FoldedSums {
-    static constexpr bool IN_TMEM = D == 64;
+template <int D, bool IN_TMEM> struct FoldedSums {
     uint32_t o;
     float4 *sums;
     float m = -INFINITY;                 // their reference
