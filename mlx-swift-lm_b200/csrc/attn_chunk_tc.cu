@@ -519,7 +519,8 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
             const int tile_limit = (int)(p.causal ? min(p.T - 1, p.causal_offset + l0) : p.T - 1);
             float m_top = -INFINITY, m_ref = -INFINITY, l_run = 0.f;   // largest score, reference of O and of l_run
             int since = -1;                                            // tiles behind the last fold
-            FoldedSums<D, SINGLE || D == 64> sums(o_addr, (float4 *)p.o_fold + ((int64_t)blockIdx.x * 2 + i) * (D / 4) * TC_ROWS + row);
+            using Sums = FoldedSums<D, SINGLE || D == 64>;
+            Sums sums(o_addr, (float4 *)p.o_fold + ((int64_t)blockIdx.x * 2 + i) * (D / 4) * TC_ROWS + row);
             for (int t = w.t0; t < w.t1; ++t) {
                 ok = warp_wait(&bars[BAR::S_FULL + buf], s_par);
                 if (!ok) break;
@@ -533,10 +534,12 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     tc_fence_after();
                     settled = true;
                 };
+                typename Sums::Form fold = Sums::DONE;
+                float fold_f = 1.f;
                 if (++since == p.fold) {
                     if (!settled) settle();
                     if (!ok) break;
-                    sums.fold(m_ref);
+                    fold = sums.begin(m_ref, fold_f);
                     since = 0;
                 }
                 uint32_t raw[TC_KEYS];
@@ -566,7 +569,8 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                 // O is settled when the scores of a pair are there: they came behind the O products of the tile before
                 auto hand_over = [&](auto which) {
                     constexpr int h = decltype(which)::value, FROM = key_of(h), TO = key_of(h + 1), part = PARTS == 1 ? 0 : h;
-                    const bool first = h == 0, move = (first ? since > 0 : PARTS > 1) && __any_sync(0xffffffffu, alpha[part] != 1.f);
+                    const bool first = h == 0, lay = first && fold != Sums::DONE;
+                    const bool move = (first ? since > 0 : PARTS > 1) && __any_sync(0xffffffffu, alpha[part] != 1.f);
                     const uint64_t alpha2 = pack_f2(alpha[part], alpha[part]);
                     constexpr int CH = PARTS == 1 ? 32 : 16;   // columns of O at a time (16: 3 % slower with one reference)
                     uint32_t o[CH];
@@ -576,6 +580,10 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     };
                     auto o_store = [&](int cb) {
                         tmem_ld_wait();
+                        if (lay) {
+                            sums.put(fold, cb * CH / 4, o, fold_f);
+                            return;
+                        }
 #pragma unroll
                         for (int k = 0; k < CH; k += 2) {
                             float lo, hi;
@@ -592,8 +600,8 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                     if (SINGLE && first && !settled) settle();
 #pragma unroll
                     for (int k0 = FROM; k0 < TO; k0 += CH) {
-                        // a rescale of O runs under the exponentials: they wait for the special-function unit
-                        if (first && move && k0 < D) o_load(k0 / CH);
+                        // a rescale of O, or a fold, runs under the exponentials: they wait for the special-function unit
+                        if (first && (move || lay) && k0 < D) o_load(k0 / CH);
 #pragma unroll
                         for (int k = k0; k < k0 + CH; k += 2) {
                             float e0, e1;
@@ -604,14 +612,14 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
                             // the probabilities as pairs, kept in the registers the scores came in
                             raw[k >> 1] = pack_pair<T>(e0, e1);
                         }
-                        if (first && move && k0 < D) o_store(k0 / CH);
+                        if (first && (move || lay) && k0 < D) o_store(k0 / CH);
                     }
                     if (!first && PARTS > 1) {
                         if (ok) ok = warp_wait(&bars[BAR::O_PART + i], h_par);
                         h_par ^= 1;
                         tc_fence_after();
                     }
-                    if (move)
+                    if (move || lay)
 #pragma unroll
                         for (int cb = first ? TO / CH : 0; cb < D / CH; ++cb) {
                             o_load(cb);
@@ -958,8 +966,8 @@ int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream) {
             p.waves = g.even ? (int)g.rounds : 1;
             longest = g.most;
         }
-        // (in memory a fold costs a key tile's time: 512 f16 keys 323 us where no folds take 267, 768 about 300, and the kernel
-        // that folded every tile in registers 311; 512 x 8 x 32 heads behind 3 584 keys)
+        // (in memory a fold costs half a key tile's time, under the exponentials, a whole one ahead of them: every 768 keys 282 and 300
+        // us where no folds take 262; the kernel that folded every tile in registers took 312. 512 x 8 x 32 f16 heads behind 3 584 keys)
         const bool in_memory = a.D == 128 && p.wide == 2;
         p.fold = fold_keys(a.q_dtype) * (in_memory ? 3 : 2) / 2 / TC_KEYS;
         if (in_memory) {                                         // even stretches: no fold for a last tile or two

@@ -200,8 +200,10 @@ template <int D, bool IN_TMEM> struct FoldedSums {
             for (int c4 = 0; c4 < 8; ++c4) __stcg(&to[(cb * 8 + c4) * TC_ROWS], make_float4(x[c4 * 4], x[c4 * 4 + 1], x[c4 * 4 + 2], x[c4 * 4 + 3]));
         }
     }
-    // All threads of a warp; O is settled, and the product after it starts from nothing.
-    __device__ __forceinline__ void fold(float m_o) {
+    // A fold: all threads of a warp; O is settled, and the product after it starts from nothing. In memory it is begun here and put()
+    // for all columns by the caller, who has work to do it under, unless the reference has moved too far: then it is done at once.
+    enum Form { DONE, STORE, ADD };
+    __device__ __forceinline__ Form begin(float m_o, float &f) {
         if (IN_TMEM) {
 #pragma unroll 1
             for (int cb = 0; cb < D / 32; ++cb) {
@@ -214,20 +216,40 @@ template <int D, bool IN_TMEM> struct FoldedSums {
             }
             tmem_st_wait();
             m = m_o;
-        } else if (!any || __any_sync(0xffffffffu, !(m_o - m <= 64.f))) {
-            leave(m_o, sums);
-            m = m_o;
-        } else {
-            const float f = fast_exp2(m_o - m);
-#pragma unroll 2
-            for (int cb = 0; cb < D / 32; ++cb) {
-                float x[32];
-                tmem_ld32(o + cb * 32, x);
-#pragma unroll
-                for (int c4 = 0; c4 < 8; ++c4) add4_global(&sums[(cb * 8 + c4) * TC_ROWS], x[c4 * 4] * f, x[c4 * 4 + 1] * f, x[c4 * 4 + 2] * f, x[c4 * 4 + 3] * f);
-            }
+            any = true;
+            return DONE;
         }
+        f = 1.f;
+        if (any && !__any_sync(0xffffffffu, !(m_o - m <= 64.f))) {
+            f = fast_exp2(m_o - m);
+            return ADD;
+        }
+        const bool again = any;
+        if (again) leave(m_o, sums);
+        m = m_o;
         any = true;
+        return again ? DONE : STORE;
+    }
+    // N columns of O from column 4 * at on
+    template <int N> __device__ __forceinline__ void put(Form form, int at, const uint32_t (&x)[N], float f) {
+#pragma unroll
+        for (int i = 0; i < N / 4; ++i) {
+            const float4 y = make_float4(__uint_as_float(x[4 * i]) * f, __uint_as_float(x[4 * i + 1]) * f, __uint_as_float(x[4 * i + 2]) * f, __uint_as_float(x[4 * i + 3]) * f);
+            if (form == ADD) add4_global(&sums[(at + i) * TC_ROWS], y.x, y.y, y.z, y.w);
+            else __stcg(&sums[(at + i) * TC_ROWS], y);
+        }
+    }
+    __device__ __forceinline__ void fold(float m_o) {
+        float f;
+        const Form form = begin(m_o, f);
+        if (form == DONE) return;
+#pragma unroll 2
+        for (int cb = 0; cb < D / 32; ++cb) {
+            uint32_t x[32];
+            tmem_ld32_issue(o + cb * 32, x);
+            tmem_ld_wait();
+            put(form, cb * 8, x, f);
+        }
     }
 };
 

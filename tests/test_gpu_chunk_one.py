@@ -1,4 +1,6 @@
 """The tcgen05 chunk kernel that keeps P as pairs: boolean array masks, and head dim 256."""
+import re
+
 import pytest
 import torch
 
@@ -90,4 +92,26 @@ def test_sums_over_long_contexts(kvc, cuda, capfd, monkeypatch, D, mask, B, Hq, 
                        @ v[0, h * Hkv // Hq].double() for h in range(Hq)])
     assert abs(((out[0].double() - ref) * ref.sign()).mean().item()) <= (3e-6 + 4 * 2.2e-4 * out.numel() ** -0.5) * ref.abs().mean().item()
     assert ((out[0].double() - ref).norm() / ref.norm()).item() <= 2.0 ** -11
+    assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,D,L,T,array", [(1, 4, 1, 256, 40, 3000, False), (1, 4, 1, 256, 40, 3000, True), (1, 8, 2, 128, 70, 2000, True)])
+def test_cut_units_can_be_captured(kvc, cuda, capfd, monkeypatch, B, Hq, Hkv, D, L, T, array):
+    """The partials of a captured call belong to its graph: replays on other inputs give the eager call's bits."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    q, k, v = _case(cuda, torch.bfloat16, B, Hq, Hkv, D, L, T)
+    mask = torch.arange(T, device=cuda) <= torch.arange(T - L, T, device=cuda)[:, None] if array else "causal"
+    out = torch.empty_like(q)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, mask, out=out)
+    assert int(re.search(r"chunk_one: .* (\d+) pieces", capfd.readouterr().err)[1]) > 1
+    for seed in (11, 12):
+        q.copy_(_case(cuda, torch.bfloat16, B, Hq, Hkv, D, L, T, seed)[0])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, mask))
     assert kvc.lib().kvc_device_status() == 0

@@ -102,8 +102,8 @@ print(kvc.launch_count())
     (1, 2, 1, 128, 512, 512, "causal"),     # one 512-token chunk from an empty cache
 ])
 def test_chunk_kernel_matches_oracle(kvc, oracle, cuda, dtype, B, Hq, Hkv, D, L, T, mask):
-    """Multi-token chunks (more than 16 rows per KV head): rows split across the warps of the mma.sync chunk
-    kernel; 17 to 64 rows per KV head at head dim 128 go to the tcgen05 verify kernel."""
+    """Multi-token chunks (more than 16 rows per KV head), whichever kernel takes them: the tcgen05 chunk kernels from 65 rows
+    on, the tcgen05 verify kernel up to 64 at head dim 128."""
     q = seeded((B, Hq, L, D), 1, dtype)
     k, v = seeded((B, Hkv, T, D), 2, dtype), seeded((B, Hkv, T, D), 3, dtype)
     n0 = kvc.launch_count(reset=True)
@@ -115,6 +115,32 @@ def test_chunk_kernel_matches_oracle(kvc, oracle, cuda, dtype, B, Hq, Hkv, D, L,
         assert launches == 1            # one kernel: partial + merge in one launch
     ref = oracle.sdpa(to_oracle(q), to_oracle(k), to_oracle(v), D ** -0.5, mask)
     assert max_abs_diff(out, ref) <= TOL[dtype]
+    assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("mask", ["causal", "none", "window", "added"])
+@pytest.mark.parametrize("B,Hq,Hkv,D,L,T", [
+    (1, 32, 8, 64, 8, 5000),     # verify rounds at head dims the tcgen05 verify kernel does not have: splits and their merge
+    (2, 32, 8, 64, 6, 5001),     # 24 rows, a last tile of nine keys
+    (1, 4, 1, 256, 8, 3000),
+    (3, 4, 1, 256, 5, 70),       # 20 rows, two tiles
+    (2, 4, 2, 64, 64, 64),       # 128 rows over one tile
+])
+def test_mma_sync_chunk_kernel(kvc, cuda, capfd, monkeypatch, dtype, mask, B, Hq, Hkv, D, L, T):
+    """What the tcgen05 kernels leave for the mma.sync chunk kernel: up to 64 rows of a group, up to 64 keys, added masks."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    q, k, v = (seeded((B, h, n, D), i, dtype).to(cuda) for i, (h, n) in enumerate(((Hq, L), (Hkv, T), (Hkv, T))))
+    i, j = torch.arange(T - L, T, device=cuda)[:, None], torch.arange(T, device=cuda)[None]
+    seen = {"none": j >= 0, "causal": j <= i}.get(mask, (j <= i) & (j > i - 50)).expand(L, T)
+    added = torch.zeros(L, T, device=cuda).masked_fill(~seen, float("-inf"))
+    out = kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, {"window": seen, "added": added.to(dtype)}.get(mask, mask))
+    torch.cuda.synchronize()
+    assert "chunk_mma" in capfd.readouterr().err
+    k, v = (x.double().repeat_interleave(Hq // Hkv, 1) for x in (k, v))
+    ref = torch.softmax(q.double() @ k.transpose(-1, -2) * D ** -0.5 + added, -1) @ v
+    # P and the outputs are each rounded to 16 bits: at most half a spacing of a value each
+    assert (out.double() - ref).norm() <= 2.0 ** (-8 if dtype == torch.bfloat16 else -11) * ref.norm()
     assert kvc.lib().kvc_device_status() == 0
 
 
@@ -212,7 +238,7 @@ def test_batched_decode_steps_over_layers(kvc, oracle, cuda, dtype):
     (5, 16, 16, 129, 257, "causal"),     # one row past a block, one key past a tile
 ])
 def test_tensor_core_chunk_kernel_matches_oracle(kvc, oracle, cuda, capfd, monkeypatch, dtype, B, Hq, Hkv, L, T, mask):
-    """Long chunks over raw K/V at head dim 128 run on the tcgen05 kernel (128 query rows per CTA)."""
+    """Chunks over raw K/V at head dim 128 run on the tcgen05 kernel (two tiles of 128 query rows per CTA)."""
     D = 128
     monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
     q = seeded((B, Hq, L, D), 1, dtype)
