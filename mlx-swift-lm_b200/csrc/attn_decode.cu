@@ -998,8 +998,9 @@ flat_list_merge_kernel(const __grid_constant__ FlatList list, const __grid_const
 // accumulation rounds towards zero, and errors against 64-bit sums grew with the number of keys, by 0.02 % for f16
 // outputs at 30 000 (for bf16, whose store is eight times coarser, by 0.0006 % at 16 000: no fold there, it costs a fifth
 // of the time at D 256).
-// Six 512-token chunks of the Gemma-3-1B shape (4 x 4 heads, D 256, five rings of 512 and a global layer): 20.4 ms
-// on the general kernel, 0.407 ms here (0.487 with one 16-token block at a time).
+// Boolean masks come here only with up to 64 rows of a group or up to 64 keys (else attn_chunk_one_tc.cu), masks that are added
+// with any number. Six 512-token chunks of the Gemma-3-1B shape (4 x 4 heads, D 256, five rings of 512 and a global layer) under
+// boolean masks took 20.4 ms on the general kernel, 0.407 ms here (0.487 with one 16-token block at a time) and take 0.233 there.
 //
 // PAIRS takes q, K and V as pairs of arrays, high and low halves of fp32 values that were brought into the range of f16
 // by powers of two: products of 22 significant bits (hi hi + lo hi + hi lo; the small ones are summed apart), for rows
@@ -1874,6 +1875,9 @@ int launch_rows(const AttnArgs &a, const ChunkLow *low, cudaStream_t stream) {
 
     if (chunk) {
         const int ctas = (int)(bh * row_blocks * splits);
+        if (trace_dispatch())
+            fprintf(stderr, "[kvc] chunk_mma: %lld row blocks in %lld splits%s%s\n", (long long)(bh * row_blocks), (long long)splits,
+                    masked ? ", array mask" : "", low ? ", pairs" : "");
         if (low) {
             ChunkPairMaps pm;
             KVSource kl = a.k, vl = a.v;
