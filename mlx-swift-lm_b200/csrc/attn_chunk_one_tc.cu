@@ -20,6 +20,9 @@
 // Every `fold` tiles O goes on in fp32 sums, as in attn_chunk_tc.cu (masked f16 outputs: errors against 64 bits + 0.5 % at 32 000
 // keys without it, in eight pieces).
 //
+// A hidden key has weight zero, which an infinite or NaN value turns into NaN: in all rows of a tile that some row sees, as in
+// softmax times V.
+//
 // What bounds it: the chain S -> softmax -> O of one row tile; the two products take 1 800 cycles of a tile at head dim
 // 256 (768 for S, whose 64 columns are bound by shared-memory reads, 1 024 for both halves of P).
 //
@@ -91,7 +94,7 @@ template <typename T> __device__ __forceinline__ float2 unpack_pair(uint32_t w);
 template <> __device__ __forceinline__ float2 unpack_pair<__half>(uint32_t w) { return MmaType<__half>::unpack(w); }
 template <> __device__ __forceinline__ float2 unpack_pair<__nv_bfloat16>(uint32_t w) { return MmaType<__nv_bfloat16>::unpack(w); }
 
-template <typename T, int D, bool MASKED>
+template <typename T, int D, bool MASKED, bool FOLDS>
 __global__ void __launch_bounds__(ON_THREADS, D == 256 ? 1 : 2)
 attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                       const __grid_constant__ CUtensorMap vmap, const __grid_constant__ ChunkOneParams p) {
@@ -244,7 +247,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 umma_commit(&bars[BAR::RING_EMPTY + slot]);
             }
             __syncwarp();
-            since = since == p.fold - 1 ? 0 : since + 1;
+            since = FOLDS && since == p.fold - 1 ? 0 : since + 1;
             next();
         };
         for (int c = 0; ok && c < mine; ++c) {
@@ -284,8 +287,8 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         uint32_t n = 0;
         int since = -1;                      // tiles behind the last fold
         bool ok = true;
-        float4 *part = (float4 *)p.o_part + ((int64_t)unit * p.pieces + piece) * (D / 4) * TC_ROWS + row;
-        FoldedSums<D, D == 64> sums(o_addr, part);
+        auto own_part = [&] { return (float4 *)p.o_part + ((int64_t)unit * p.pieces + piece) * (D / 4) * TC_ROWS + row; };
+        FoldedSums<D, D == 64> sums(o_addr, FOLDS ? own_part() : nullptr);
         for (int c = 0; c < mine; ++c) {
             if (!live(c)) continue;
             const int key0 = (piece + c * p.pieces) * ON_KEYS;
@@ -334,7 +337,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 low[k >> 1] = pack_pair<T>(e0 * P_UP - f.x, e1 * P_UP - f.y);
                 raw[k >> 1] = high;
             }
-            const bool fold = ++since == p.fold;
+            const bool fold = FOLDS && ++since == p.fold;
             if (n > 0 && (fold || __any_sync(0xffffffffu, alpha != 1.f))) {
                 ok = warp_wait(&bars[BAR::O_DONE], (n - 1) & 1);   // (not a phase too early: the product before
                                                                      // it was done when these scores came)
@@ -368,7 +371,8 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
             T *dst = (T *)p.out + b * p.o_sb + (int64_t)(hk * p.rep + h) * p.o_sh + (int64_t)l * p.o_sl;
             auto o_of = [&](int cb, float (&o)[32]) {
                 if (n > 0) {
-                    sums.total(cb, m_run, o);
+                    if constexpr (FOLDS) sums.total(cb, m_run, o);
+                    else tmem_ld32(o_addr + cb * 32, o);
                 } else {
 #pragma unroll
                     for (int k = 0; k < 32; ++k) o[k] = 0.f;
@@ -384,12 +388,13 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                 }
             } else {
                 // ---- leave a partial; the CTA that leaves the last one of the unit merges them ----
+                float4 *part = own_part();
 #pragma unroll 1
                 for (int cb = 0; cb < D / 32; ++cb) {
                     float o[32];
                     o_of(cb, o);
 #pragma unroll
-                    for (int c4 = 0; c4 < 8; ++c4) __stcg(&part[(cb * 8 + c4) * TC_ROWS], make_float4(o[c4 * 4], o[c4 * 4 + 1], o[c4 * 4 + 2], o[c4 * 4 + 3]));
+                    for (int c4 = 0; c4 < 8; ++c4) part[(cb * 8 + c4) * TC_ROWS] = make_float4(o[c4 * 4], o[c4 * 4 + 1], o[c4 * 4 + 2], o[c4 * 4 + 3]);
                 }
                 p.ml_part[((int64_t)unit * p.pieces + piece) * TC_ROWS + row] = make_float2(m_run, l_run);
                 __threadfence();
@@ -447,7 +452,7 @@ attn_chunk_one_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     }
 }
 
-template <typename T, int D, bool MASKED>
+template <typename T, int D, bool MASKED, bool FOLDS>
 bool launch_one_as(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkOneParams &p, int ctas,
                    cudaStream_t stream) {
     constexpr size_t smem = (size_t)(D / 64) * (TC_BOX + on_stages<D>() * ON_BOX) + OneBars<on_stages<D>()>::COUNT * sizeof(uint64_t) + 8 +
@@ -459,27 +464,27 @@ bool launch_one_as(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUten
     if (dev < 0 || dev >= 64) return false;
     int state = configured[dev].load(std::memory_order_acquire);
     if (state == 0) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_chunk_one_kernel<T, D, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_chunk_one_kernel<T, D, MASKED, FOLDS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) (void)cudaGetLastError();
         state = e == cudaSuccess ? 1 : -1;
         configured[dev].store(state, std::memory_order_release);
     }
     if (state < 0) return false;
     KernelTimer timer(stream);
-    KVC_CUDA(launch_pdl(attn_chunk_one_kernel<T, D, MASKED>, dim3(ctas), dim3(ON_THREADS), smem, stream, qmap, kmap, vmap, p));
+    KVC_CUDA(launch_pdl(attn_chunk_one_kernel<T, D, MASKED, FOLDS>, dim3(ctas), dim3(ON_THREADS), smem, stream, qmap, kmap, vmap, p));
     timer.stop();
     ++g_launch_count;
     return true;
 }
 
-template <typename T>
+template <typename T, bool FOLDS>
 bool launch_one(const CUtensorMap &qmap, const CUtensorMap &kmap, const CUtensorMap &vmap, const ChunkOneParams &p, int D, bool masked,
                 int ctas, cudaStream_t stream) {
     if (D == 256)
-        return masked ? launch_one_as<T, 256, true>(qmap, kmap, vmap, p, ctas, stream)
-                      : launch_one_as<T, 256, false>(qmap, kmap, vmap, p, ctas, stream);
-    return D == 128 ? launch_one_as<T, 128, true>(qmap, kmap, vmap, p, ctas, stream)
-                    : launch_one_as<T, 64, true>(qmap, kmap, vmap, p, ctas, stream);
+        return masked ? launch_one_as<T, 256, true, FOLDS>(qmap, kmap, vmap, p, ctas, stream)
+                      : launch_one_as<T, 256, false, FOLDS>(qmap, kmap, vmap, p, ctas, stream);
+    return D == 128 ? launch_one_as<T, 128, true, FOLDS>(qmap, kmap, vmap, p, ctas, stream)
+                    : launch_one_as<T, 64, true, FOLDS>(qmap, kmap, vmap, p, ctas, stream);
 }
 
 }  // namespace
@@ -564,8 +569,13 @@ int launch_attention_chunk_one(const AttnArgs &a, cudaStream_t stream) {
         KVC_CUDA(cudaMemsetAsync(p.tickets, 0, t_bytes, stream));
     }
     const int ctas = (int)(units * p.pieces);
-    const bool taken = a.q_dtype == KVC_BF16 ? launch_one<__nv_bfloat16>(qmap, kmap, vmap, p, a.D, masked, ctas, stream)
-                                             : launch_one<__half>(qmap, kmap, vmap, p, a.D, masked, ctas, stream);
+    // (the test for a fold costs a call of ten tiles 0.7 %)
+    const bool long_sums = (n + pieces - 1) / pieces > p.fold;
+    const bool taken = a.q_dtype == KVC_BF16
+        ? (long_sums ? launch_one<__nv_bfloat16, true>(qmap, kmap, vmap, p, a.D, masked, ctas, stream)
+                     : launch_one<__nv_bfloat16, false>(qmap, kmap, vmap, p, a.D, masked, ctas, stream))
+        : (long_sums ? launch_one<__half, true>(qmap, kmap, vmap, p, a.D, masked, ctas, stream)
+                     : launch_one<__half, false>(qmap, kmap, vmap, p, a.D, masked, ctas, stream));
     if (taken && trace_dispatch())
         fprintf(stderr, "[kvc] chunk_one: %lld row tiles (%d heads x %d positions), %d pieces%s\n", (long long)units, p.hb, p.lb, p.pieces,
                 masked ? ", array mask" : "");

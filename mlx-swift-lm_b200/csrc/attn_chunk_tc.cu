@@ -307,6 +307,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
             if (!ok) {
                 atomicExch(p.status, 21);
                 drain_copies(&bars[BAR::RING_FULL], STAGES, slot, round);
+#pragma unroll 1
                 for (int i = 0; i < 2; ++i)
                     if (q_used[i] > 0) (void)mbar_wait(&bars[BAR::Q_FULL + i], (q_used[i] - 1) & 1);
             }

@@ -140,6 +140,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
 // After a wait that ran out. Producer lane: the copies into a ring whose next entry is `slot` in its use number `round` have
 // arrived (the last use of every entry).
 __device__ __forceinline__ void drain_copies(uint64_t *full, uint32_t stages, uint32_t slot, uint32_t round) {
+#pragma unroll 1
     for (uint32_t s = 0; s < stages; ++s) {
         const uint32_t uses = round + (s < slot ? 1u : 0u);
         if (uses > 0) (void)mbar_wait(&full[s], (uses - 1) & 1);
