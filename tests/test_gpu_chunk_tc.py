@@ -1,7 +1,6 @@
 """The tcgen05 chunk kernel over the ways its work is cut, and under stream capture."""
 import re
 
-import numpy as np
 import pytest
 import torch
 
@@ -115,12 +114,16 @@ def test_chunk_scores_that_move_the_reference(kvc, cuda, capfd, monkeypatch, gro
     _check(out[some], *_reference(q[some], k[some], v[some], D ** -0.5, True, parts))
 
 
-def test_chunk_with_cut_units_can_be_captured(kvc, cuda, capfd, monkeypatch):
-    """The partials of a captured call belong to its graph: replays on other inputs give the eager call's bits."""
-    B, Hq, Hkv, D, L, T = 1, 32, 8, 128, 96, 3000
-    q, k, v = (seeded((B, h, n, D), s, torch.bfloat16).to(cuda) for h, n, s in ((Hq, L, 1), (Hkv, T, 2), (Hkv, T, 3)))
+@pytest.mark.parametrize("dtype,B,L,T,cut", [
+    (torch.bfloat16, 1, 96, 3000, True),      # partials of cut units
+    (torch.float16, 8, 128, 2000, False),     # sums that are folded into memory
+])
+def test_chunk_with_memory_of_its_own_can_be_captured(kvc, cuda, capfd, monkeypatch, dtype, B, L, T, cut):
+    """The memory of a captured call belongs to its graph: replays on other inputs give the eager call's bits."""
+    Hq, Hkv, D = 32, 8, 128
+    q, k, v = (seeded((B, h, n, D), s, dtype).to(cuda) for h, n, s in ((Hq, L, 1), (Hkv, T, 2), (Hkv, T, 3)))
     monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
-    assert _run(kvc, capfd, q, k, v, D ** -0.5, "causal")[-1]
+    assert _run(kvc, capfd, q, k, v, D ** -0.5, "causal")[-1] == cut
     out = torch.empty_like(q)
     side = torch.cuda.Stream()
     with torch.cuda.stream(side):
@@ -128,10 +131,10 @@ def test_chunk_with_cut_units_can_be_captured(kvc, cuda, capfd, monkeypatch):
         with torch.cuda.graph(graph, stream=side):
             kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, "causal", out=out)
     for seed in (11, 12):
-        q.copy_(seeded(tuple(q.shape), seed, torch.bfloat16))
+        q.copy_(seeded(tuple(q.shape), seed, dtype))
         graph.replay()
         torch.cuda.synchronize()
-        assert np.array_equal(out.view(torch.int16).cpu(), kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, "causal").view(torch.int16).cpu())
+        assert torch.equal(out, kvc.scaled_dot_product_attention(q, k, v, D ** -0.5, "causal"))
 
 
 def _bias(out, ref):
