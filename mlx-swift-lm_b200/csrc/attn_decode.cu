@@ -428,11 +428,6 @@ __device__ __forceinline__ void flat_locate(FlatSeg &g, const DecodeParams &p, i
     g.unit = u;
 }
 
-__device__ __forceinline__ int flat_cta_of32(const FlatPlan &f, uint32_t x) {
-    const uint32_t big = (uint32_t)f.rem * (f.per + 1);
-    return x < big ? (int)(x / (uint32_t)(f.per + 1)) : f.rem + (int)((x - big) / (uint32_t)f.per);
-}
-
 // What the consumers need of a segment.
 struct FlatWork {
     const unsigned char *q, *new_k, *new_v;   // the unit's query rows, and its new rows (null: stored already)
@@ -568,7 +563,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                         FlatWork w = flat_work<T>(gs, p);
                         if (gs.new_k) flat_new_rows<T>(w, gs);
                         w.nslots = gs.plan.nslots;
-                        w.part = gs.part_first + ((int64_t)b * p.Hq + hk * rep) * w.nslots + gs.cta - flat_cta_of32(gs.plan, (uint32_t)(x - t0));
+                        w.part = gs.part_first + ((int64_t)b * p.Hq + hk * rep) * w.nslots + gs.cta - flat_cta_of(gs.plan, x - t0);
                         works[qb] = w;
                     }
                     if (p.q_bulk) mbar_expect_tx(&qfull[qb], q_bytes);

@@ -97,7 +97,7 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
         while (si + 1 < list.n && list.seq[si + 1].tile_first <= x) ++si;
         const F32Seq &sq = list.seq[si];
         const int64_t in = x - sq.tile_first;
-        const int u_in = (int)(in / sq.tiles), tile = (int)(in % sq.tiles);
+        const int u_in = flat_div(in, sq.tiles), tile = flat_mod(in, sq.tiles, u_in);
         const int chunk = u_in % p.chunks, hk = (u_in / p.chunks) % p.Hkv, b = u_in / p.chunks / p.Hkv;
         const int tiles = (int)min((int64_t)(sq.tiles - tile), x_end - x);
         const int row0 = chunk * RN, R = min(RN, rows_all - row0), T = sq.T;

@@ -612,8 +612,8 @@ template <bool VARLEN, int TILE>
 __device__ __forceinline__ void resolve_unit(const AffineParams &p, const VarlenAttnTable &vt, int64_t x, int tiles,
                                              int &unit, int &tile, int &utiles, int &hk, int &b) {
     if (!VARLEN) {
-        unit = (int)(x / tiles);
-        tile = (int)(x % tiles);
+        unit = flat_div(x, tiles);
+        tile = flat_mod(x, tiles, unit);
         utiles = tiles;
         const int bh = unit / p.chunks;   // a group of more than eight query rows is cut into units of eight
         hk = bh % p.Hkv;
@@ -625,8 +625,8 @@ __device__ __forceinline__ void resolve_unit(const AffineParams &p, const Varlen
         if (i + step < vt.n && (int64_t)p.Hkv * vt.seq[i + step].tile_prefix <= x) i += step;
     const int64_t base = (int64_t)p.Hkv * vt.seq[i].tile_prefix;
     utiles = (vt.seq[i].T + TILE - 1) / TILE;
-    hk = (int)((x - base) / utiles);
-    tile = (int)((x - base) % utiles);
+    hk = flat_div(x - base, utiles);
+    tile = flat_mod(x - base, utiles, hk);
     b = i;
     unit = i * p.Hkv + hk;
 }
@@ -1223,7 +1223,7 @@ int launch_attention_affine_varlen(const AttnArgs *args, int n, cudaStream_t str
     }
     if (a0.D / a0.k.group > 4 || (a0.k.group * a0.k.bits) / 32 < 4) return 0;
     const int64_t units = (int64_t)n * a0.Hkv;
-    if (units * (int64_t)sizeof(int) > PK_COUNTER_BYTES) return 0;
+    if (units * (int64_t)sizeof(int) > PK_COUNTER_BYTES || !flat_fits(prefix * a0.Hkv)) return 0;
     int *status = device_status_word(a0.device);
     if (!status) return 0;
     int *counters = counters_get(a0.device, stream, PK_COUNTER_BYTES);
@@ -1308,6 +1308,7 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     const bool decode8 = (rep * a.L <= 8 || chunks > 1) && pairs_fit;
     const int64_t tile8 = affine8_warps(a.D, a.k.bits, false) * 16;
     const int64_t tiles = decode8 ? (a.T + tile8 - 1) / tile8 : (a.T + PK_TILE - 1) / PK_TILE;
+    if (!flat_fits(bh * tiles)) return 0;
     // resident CTAs per SM (a fourth CTA fits the 4-bit kernels at 94 registers but measured slower)
     const int slots = sm_count(a.device) * (decode8 ? 3 : 2);
     int64_t best_s = 1;

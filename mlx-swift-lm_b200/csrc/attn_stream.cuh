@@ -300,9 +300,9 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
             sg.unit_tiles = list.seq[sg.seq].tiles;
             sg.unit = sg.seq * p.B * p.Hkv * p.chunks;
         }
-        const int u_in = (int)(in / sg.unit_tiles);
+        const int u_in = flat_div(in, sg.unit_tiles);
         sg.unit += u_in;
-        sg.tile = (int)(in % sg.unit_tiles);
+        sg.tile = flat_mod(in, sg.unit_tiles, u_in);
         sg.chunk = u_in % p.chunks;
         sg.hk = (u_in / p.chunks) % p.Hkv;
         sg.b = u_in / p.chunks / p.Hkv;
@@ -897,7 +897,7 @@ struct StreamPick {
 // The flat plan over `work` tiles, `max_tiles` in the longest unit; false when the partials need too many slots.
 inline bool stream_plan(const AttnArgs &a, int64_t units, int64_t work, int64_t max_tiles, int resident, int rows, StreamParams *p,
                  int64_t qrows, cudaStream_t stream, int *ctas) {
-    if (units * (int64_t)sizeof(int) > ST_COUNTER_BYTES) return false;
+    if (units * (int64_t)sizeof(int) > ST_COUNTER_BYTES || !flat_fits(work)) return false;
     const int64_t n = std::min<int64_t>((int64_t)sm_count(a.device) * resident, work);
     p->flat.tiles = (int)max_tiles;
     p->flat.per = (int)(work / n);

@@ -175,7 +175,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
         if (lane == 0) {
             int it = 0, sg = 0;
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
-                const int unit = (int)(x / tiles), tb = (int)(x % tiles);
+                const int unit = flat_div(x, tiles), tb = flat_mod(x, tiles, unit);
                 const int n = (int)min((int64_t)(tiles - tb), x_hi - x);
                 const int hk = unit % p.Hkv, b = unit / p.Hkv;
                 if (p.q_bulk) {
@@ -215,7 +215,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
     uint32_t st_ph = 0;
     int sg = 0;
     for (int64_t x = x_lo; x < x_hi; ++sg) {
-        const int unit = (int)(x / tiles), tile_begin = (int)(x % tiles);
+        const int unit = flat_div(x, tiles), tile_begin = flat_mod(x, tiles, unit);
         const int ntiles = (int)min((int64_t)(tiles - tile_begin), x_hi - x);
         const int hk = unit % p.Hkv, b = unit / p.Hkv;
         // ---- rotated queries of this unit: q' = H(signs * q) / sqrt(D) * scale * log2(e), rows past R zero ----
@@ -542,6 +542,7 @@ int launch_attention_turbo(const AttnArgs &a, cudaStream_t stream) {
     const size_t per_cta = fixed + turbo_red_smem(plan) + 1024;
     const int resident = (int)std::max<size_t>(1, std::min<size_t>(2, (size_t)227 * 1024 / per_cta));
     const int64_t work_tiles = bh * tiles;
+    if (!flat_fits(work_tiles)) return 0;
     const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a.device) * resident, work_tiles);
     plan.per = (int)(work_tiles / ctas);
     plan.rem = (int)(work_tiles % ctas);

@@ -123,14 +123,6 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&dst)[N]) {
     }
 }
 
-// The 8x8 b16 transpose without `volatile`: every lane of the warp reaches it (it is never under a
-// divergent branch here) and it has no side effect, so the compiler may schedule it among the lookups.
-__device__ __forceinline__ uint32_t movmatrix_free(uint32_t x) {
-    uint32_t r;
-    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
-    return r;
-}
-
 // Address of value-table entry `byte BYTE of x` for this lane: one byte permute. `lane_const`
 // holds (table base | lane << 2) with the table base a multiple of 64 KB.
 template <int BYTE>
@@ -258,7 +250,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
         if (issuer && !(KVC_SKIP_BITS(p) & 2)) {   // measurement bit 2: no loads at all (consumers compute on stale stages)
             int it = 0, sg = 0;
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
-                const int unit = (int)(x / tiles), tb = (int)(x % tiles);
+                const int unit = flat_div(x, tiles), tb = flat_mod(x, tiles, unit);
                 const int n = (int)min((int64_t)(tiles - tb), x_hi - x);
                 const int bh = CHUNKED ? unit / p.chunks : unit;
                 const int hk = bh % p.Hkv, b = bh / p.Hkv;
@@ -312,7 +304,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
     uint32_t g_ph = 0;
     int sg = 0;
     for (int64_t x = x_lo; x < x_hi; ++sg) {
-        const int unit = (int)(x / tiles), tile_begin = (int)(x % tiles);
+        const int unit = flat_div(x, tiles), tile_begin = flat_mod(x, tiles, unit);
         const int ntiles = (int)min((int64_t)(tiles - tile_begin), x_hi - x);
         const int bh = CHUNKED ? unit / p.chunks : unit, row0 = CHUNKED ? (unit % p.chunks) * 8 : 0;
         const int hk = bh % p.Hkv, b = bh / p.Hkv;
@@ -671,6 +663,7 @@ int launch_attention_turbo_v4(const AttnArgs &a, cudaStream_t stream) {
     plan.tiles = (int)tiles;
     plan.red_rows = std::min(8, rep * a.L);
     const int64_t work_tiles = bh * tiles;
+    if (!flat_fits(work_tiles)) return 0;
     const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a.device), work_tiles);
     plan.per = (int)(work_tiles / ctas);
     plan.rem = (int)(work_tiles % ctas);
