@@ -85,10 +85,11 @@ void stream_params(const AttnArgs &a, const StreamPick &pk, StreamParams *p) {
     const bool k_turbo = pk.kk >= SK_T2, v_turbo = pk.vk >= SK_T2;
     bool shared = k_turbo && v_turbo && pk.kk == pk.vk;
     for (int i = 0; shared && i < (1 << a.k.bits); ++i) shared = a.k.codebook[i] == a.v.codebook[i];
-    p->v_table = (k_turbo && v_turbo && !shared) ? 2 * (1 << (2 * a.k.bits)) * 128 : 0;   // behind the keys' high and low halves
+    p->v_table = (k_turbo && v_turbo && !shared && a.v.bits <= a.k.bits) ? (1 << (2 * a.k.bits)) * 256 : 0;   // behind the keys' table, which is no smaller
     p->B = a.B; p->Hq = a.Hq; p->Hkv = a.Hkv; p->L = a.L; p->T = (int32_t)a.T;
     p->causal = a.mask.mode == KVC_MASK_CAUSAL ? 1 : 0;
     p->causal_offset = a.mask.causal_offset;
+    p->status = device_status_word(a.device);
     p->scale_log2 = a.scale * 1.4426950408889634f;
 }
 
@@ -109,6 +110,7 @@ int launch_attention_stream(const AttnArgs &a, cudaStream_t stream) {
     if (!stream_pick(a, &pk) || (int64_t)(a.Hq / a.Hkv) * a.L > 64) return 0;
     StreamParams p = {};
     stream_params(a, pk, &p);
+    if (!p.status) return 0;
     return run_stream_any(a, pk, p, nullptr, stream);
 }
 
@@ -120,6 +122,7 @@ int launch_attention_stream_list(const AttnArgs *args, int n, cudaStream_t strea
     if (!stream_pick(a0, &pk) || (int64_t)(a0.Hq / a0.Hkv) * a0.L > 64) return 0;
     StreamParams p = {};
     stream_params(a0, pk, &p);
+    if (!p.status) return 0;
     static thread_local StreamList list;
     list.n = n;
     for (int i = 0; i < n; ++i) {

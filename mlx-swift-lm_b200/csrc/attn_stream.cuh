@@ -16,14 +16,19 @@
 //     g and g + 8. Affine codes enter as exact integers around zero and the scale / bias of a group is applied to the
 //     group's fp32 score (s * (q . (c - m)) + (b + m s) * sum q); index keys enter as centroids (pair lookups in a table
 //     replicated per lane, no bank conflicts) and the row norm multiplies the fp32 score.
-//   * Values are unpacked 64 dims at a time into a private [16][64] f16 tile (16-byte chunks swizzled by the
-//     token) and read back transposed with ldmatrix. The row norm / group scale goes into P in fp32, the affine
-//     bias is accumulated beside the MMAs in fp32.
+//   * Values need no transpose either: a register of the A operand of O^T = V^T P^T holds one dim of two tokens, so
+//     a lane reads the same run of dims of its four tokens and interleaves the codes of two tokens with a few logic
+//     operations; the pair is an index of the same table (codebook indices) or one logic operation away from two f16
+//     (affine codes). The row norm / group scale goes into P in fp32, the affine bias is accumulated beside the MMAs
+//     in fp32. Before, the rows went through a private f16 tile and came back with ldmatrix: two thirds
+//     of the shared-memory wavefronts of the value side, and a wait between the lookups and the products.
+//   * A table entry holds the high and the low halves of a centroid pair, eight bytes a lane: one load for both.
 //   * Nothing fp32 is cut to one f16: P * factor, rotated queries and centroids are pairs (high half, low half, 22
 //     bits) and a product is the three MMAs hi hi + lo hi + hi lo (two where one side is exact). The MMAs are not what
 //     bounds the kernel; the second table lookup of each centroid pair is the price.
 //     8 layers x 4 sequences x 4099 tokens, 32/8 heads, D 128, 8-bit keys / 4-bit values, f16: 2521 us on the general
-//     kernel, 114 us here; 80 us with single f16 operands, which no longer err by the store's rounding alone.
+//     kernel, 89 us here (114 with the values through the tile and a load for each half); with single f16 operands the
+//     outputs no longer err by the store's rounding alone.
 //   * The running reference is only moved when a score (with its value factor) passes it by more than 2^3.
 // Work is cut into equal ranges of 64-token tiles per resident CTA (FlatPlan), units that cross a CTA boundary
 // are merged by segment_epilogue.
@@ -58,8 +63,7 @@ struct Kind {
     static constexpr int BLOCK = 16 * RB;                         // bytes per 16-token block
     static constexpr int SIDE = RAW ? 0 : AFFINE ? 16 * (D / 32) * 2 : 64;   // scales (and as much again for biases) or norms
     static constexpr int STAGE = BLOCK + (AFFINE ? 2 : 1) * SIDE;
-    static constexpr int TABLE = TURBO ? (1 << (2 * BITS)) * 128 : 0;   // of the centroids' high halves; the low ones follow
-    static constexpr int TABLES = 2 * TABLE;
+    static constexpr int TABLE = TURBO ? (1 << (2 * BITS)) * 256 : 0;   // high and low halves of a centroid pair, per lane
     static constexpr int CH = RB / 16;                            // 16-byte chunks per row (where whole)
     static constexpr bool POW2 = RB % 16 == 0 && (CH & (CH - 1)) == 0;
 };
@@ -101,7 +105,8 @@ struct StreamParams {
     int32_t B, Hq, Hkv, L, T;
     int32_t groups_k, groups_v;           // affine groups per row
     int32_t chunks;                       // row blocks per KV head
-    int32_t v_table;                      // byte offset of the value table (equal to the key table's when shared)
+    int32_t v_table;                      // byte offset of the value table (0: first, or the keys' own)
+    int *status;
     int32_t out_dtype, causal;
     int64_t causal_offset;
     float scale_log2;
@@ -118,6 +123,11 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
     return r;
 }
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+    uint16_t r;
+    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(r) : "r"(a) : "memory");
+    return r;
+}
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 r;
     asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a) : "memory");
@@ -127,6 +137,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     uint4 r;
     asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a) : "memory");
     return r;
+}
+__device__ __forceinline__ void sts64(uint32_t a, uint2 v) {
+    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v.x), "r"(v.y) : "memory");
 }
 __device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -156,23 +169,61 @@ __device__ __forceinline__ int key_xor(int tok) {
     if (KIND == SK_T4 && CH == 8) return tok & 1;
     return 0;
 }
+// Values are read by lanes (run of dims g, tokens 2c and 2c + 1, then 8 tokens on): the four tokens of a load lie
+// next to each other, their chunks turned so that the runs of eight (sixteen byte loads: two) lanes fill all banks.
 template <int KIND, int D>
-__device__ __forceinline__ int value_xor(int tok) {
+__device__ __forceinline__ int value_xor(int c) {
     constexpr int CH = Kind<KIND, D>::CH;
     if (!Kind<KIND, D>::POW2) return 0;
-    return CH >= 8 ? tok & 7 : CH == 4 ? (tok >> 1) & 3 : CH == 2 ? (tok >> 2) & 1 : 0;
+    return CH >= 8 ? 2 * c : CH == 4 ? c & 2 : 0;
+}
+template <int KIND, int D>
+__device__ __forceinline__ int value_slot(int tok) {
+    return Kind<KIND, D>::POW2 ? (tok & 8) | (tok & 1) << 2 | ((tok >> 1) & 3) : tok;
 }
 
-// The 2 * BITS bits of pair j of a run of words, shifted to bits 7 and up: the byte offset of the pair's entry.
+// Byte offset of the table entry that field n (2 * BITS bits) of a run of words names; `lane_const` holds the lane's
+// place in the entry and, above the fields' bits, which table it is.
 template <int BITS, int NW>
-__device__ __forceinline__ uint32_t pair_offset(const uint32_t (&w)[NW], int j, uint32_t lane_bits) {
+__device__ __forceinline__ uint32_t entry_offset(const uint32_t (&w)[NW], int n, uint32_t lane_const) {
     constexpr int B2 = 2 * BITS;
-    constexpr uint32_t MASK = ((1u << B2) - 1u) << 7;
-    const int bit = B2 * j, k = bit >> 5, s = bit & 31;
+    if constexpr (BITS == 4) return __byte_perm(w[n >> 2], lane_const, 0x7604 | ((n & 3) << 4));
+    constexpr uint32_t MASK = ((1u << B2) - 1u) << 8;
+    const int bit = B2 * n, k = bit >> 5, s = bit & 31;
     uint32_t x;
-    if (s + B2 <= 32) x = (s >= 7) ? (w[k] >> (s - 7)) : (w[k] << (7 - s));
-    else x = __funnelshift_r(w[k], w[(k + 1 < NW) ? k + 1 : k], s - 7);
-    return (x & MASK) | lane_bits;
+    if (s + B2 <= 32) x = (s >= 8) ? (w[k] >> (s - 8)) : (w[k] << (8 - s));
+    else x = __funnelshift_r(w[k], w[(k + 1 < NW) ? k + 1 : k], s - 8);
+    return (x & MASK) | lane_const;
+}
+// Dynamic shared memory starts here in a block's window (what the driver reserves lies in front; checked at the start),
+// so that the tables' place is part of the load.
+constexpr uint32_t ST_WINDOW = 1024;
+// Tables do not change after the barrier behind their making: these loads may be moved freely.
+__device__ __forceinline__ uint2 table_entry(uint32_t offset) {
+    uint2 r;
+    asm("ld.shared.v2.b32 {%0,%1}, [%2+%3];" : "=r"(r.x), "=r"(r.y) : "r"(offset), "n"(ST_WINDOW));
+    return r;
+}
+
+// Bits of word k of a run of 3-bit codes that belong to codes of even places.
+__host__ __device__ constexpr uint32_t even3(int k) {
+    uint32_t m = 0;
+    for (int i = 0; i < 32; ++i)
+        if ((32 * k + i) % 6 < 3) m |= 1u << i;
+    return m;
+}
+// The codes of one run of dims of tokens a and b as pairs: field n of `even` (`odd`) has dim 2n (2n + 1) of a in its
+// lower BITS bits and of b in its upper ones.
+template <int BITS, int NW>
+__device__ __forceinline__ void pair_tokens(const uint32_t (&a)[NW], const uint32_t (&b)[NW], uint32_t (&even)[NW], uint32_t (&odd)[NW]) {
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+        const uint32_t m = BITS == 4 ? 0x0F0F0F0Fu : BITS == 2 ? 0x33333333u : even3(k);
+        const uint32_t up = BITS == 3 && k > 0 ? __funnelshift_l(b[k > 0 ? k - 1 : 0], b[k], BITS) : b[k] << BITS;
+        const uint32_t down = BITS == 3 && k + 1 < NW ? __funnelshift_r(a[k], a[k + 1 < NW ? k + 1 : k], BITS) : a[k] >> BITS;
+        even[k] = (a[k] & m) | (up & ~m);
+        odd[k] = (down & m) | (b[k] & ~m);
+    }
 }
 
 // Two codes n as the f16 pair n - 8 or n - 128, exact: 1024 + n (+ 16 n for the upper nibble of a byte) by one logic
@@ -191,8 +242,6 @@ __device__ __forceinline__ uint32_t code4(uint32_t w, int i) {
 }
 __device__ __forceinline__ uint32_t code8(uint32_t w, int i) { return h2_fma(__byte_perm(w, 0x64646464u, i ? 0x4342 : 0x4140), 1.f, -1152.f); }
 template <int KIND> constexpr float code_middle() { return KIND == SK_A4 ? 8.f : 128.f; }
-// dim within its chunk of eight that column j of an unpacked chunk holds
-template <int KIND> __device__ __forceinline__ constexpr int chunk_dim(int j) { return KIND == SK_A4 ? (j & 1) * 4 + (j >> 1) : j; }
 
 template <typename T> __device__ __forceinline__ float ld16(uint32_t a) {
     uint16_t r;
@@ -205,8 +254,7 @@ struct StreamShape {
     using K = Kind<KK, D>;
     using V = Kind<VK, D>;
     static constexpr int STAGE = K::STAGE + V::STAGE;
-    static constexpr int VTILE = (V::TURBO ? 2 : 1) * 16 * 64 * 2;   // centroids: a tile of high, one of low halves
-    static constexpr int WARP_BYTES = ST_STAGES * STAGE + VTILE;
+    static constexpr int WARP_BYTES = ST_STAGES * STAGE;
     static constexpr int ROWS = 8 * NB;
     static constexpr int RED_STRIDE = D + 4;
     static constexpr int QS = ROWS * D * 4;                       // staged query rows
@@ -216,9 +264,9 @@ struct StreamShape {
         return (rings > red ? rings : red) + QS + HEAD;           // the merge buffers reuse the ring
     }
     // Eight warps where two CTAs fit an SM; where the tables leave room for one, twelve that share them if they fit:
-    // 168 registers keep a step's loads in flight (sixteen warps of 128 registers, with one value tile each that the
-    // halves take in turn: 118 us where this takes 111, the shape above).
-    static constexpr int MOST_TABLES = K::TABLES + V::TABLES;
+    // 168 registers keep a step's loads in flight (sixteen warps of 128 registers: 99 us
+    // where this takes 90, the shape above).
+    static constexpr int MOST_TABLES = K::TABLE + V::TABLE;
     static constexpr bool WIDE = NB == 1 && D <= 128;
     static constexpr bool PAIR = WIDE && 2 * (MOST_TABLES + fixed(8) + 1024) <= 228 * 1024;
     static constexpr bool fits(int warps) { return MOST_TABLES + fixed(warps) <= ST_SMEM; }
@@ -227,6 +275,13 @@ struct StreamShape {
     static constexpr int RESIDENT = PAIR ? 2 : 1;
     static constexpr int THREADS = WARPS * 32;
     static constexpr int FIXED = fixed(WARPS);
+    // A table lies at a multiple of its size, so that an entry's offset and the table's are joined by a logic operation:
+    // the larger one first.
+    static constexpr int K_AT = K::TURBO && V::TABLE > K::TABLE ? V::TABLE : 0;
+    static constexpr int tables(int v_table) {
+        const int k = K_AT + K::TABLE, v = V::TURBO ? v_table + V::TABLE : 0;
+        return k > v ? k : v;
+    }
 };
 
 // Token range and place of one segment: `x` flat tiles in, at most `left` tiles.
@@ -244,44 +299,45 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
     using V = Kind<VK, D>;
     using KT = std::conditional_t<K::RAW, T, __half>;             // operand type of the score MMAs
     static_assert(!V::RAW, "raw values have kernels of their own");
-    using VT = __half;
     constexpr int ST_WARPS = SH::WARPS, ST_THREADS = SH::THREADS;
-    constexpr int KSTEPS = D / 16, MT = D / 16, PASSES = D / 64;
+    constexpr int KSTEPS = D / 16, MT = D / 16;
     constexpr int KU = K::AFFINE ? UNIT : K::RAW ? 32 : D;        // dims that share a fragment order
     constexpr int NU = D / KU, UK = KU / 16;                      // units, k-steps per unit
     constexpr int NG = V::AFFINE ? D / UNIT : 1;                  // value groups kept apart (128-wide ones twice)
+    constexpr int VU = V::AFFINE ? UNIT : D, VM = VU / 16;        // value dims under one factor, their MMAs
+    constexpr int VRUN = VU / 8, VRB = VRUN * V::BITS, VW = (VRB + 31) / 32;   // a lane's run of them: dims, bits, words
     constexpr int QP = K::TURBO ? 2 : 1;                          // query fragments: high and low halves where the rows are rotated
 
     extern __shared__ __align__(1024) unsigned char smem[];
     // tables first (constant offsets), then the merge flag, the query rows and the rings
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
     const uint32_t s0 = smem_u32(smem);
-    const int table_bytes = K::TABLE || V::TABLE ? p.v_table + V::TABLES : 0;
-    const int tab_end = max(table_bytes, K::TABLES);
+    if (s0 != ST_WINDOW) {                                        // uniform over the grid
+        if (tid == 0) atomicExch(p.status, 36);
+        return;
+    }
+    const int tab_end = SH::tables(p.v_table);
     int *flag = (int *)(smem + tab_end);
     float *rowf = (float *)(smem + tab_end + 32);                 // what a score of the row is multiplied by in the end
     float *qs = (float *)(smem + tab_end + SH::HEAD);
     unsigned char *body = smem + tab_end + SH::HEAD + SH::QS;
     const uint32_t ring = smem_u32(body) + warp * SH::WARP_BYTES;
-    const uint32_t vtile = ring + ST_STAGES * SH::STAGE;
-    const uint32_t lane_bits = (uint32_t)lane << 2;
+    const uint32_t k_lane_bits = (uint32_t)lane << 3 | SH::K_AT, v_lane_bits = (uint32_t)lane << 3 | (uint32_t)p.v_table;
 
-    // Pair tables, one 128-byte line (32 equal words) per entry: a warp takes an entry, the centroids sit in its lanes.
-    auto build_table = [&](auto bits, const float *cb, uint32_t *dst) {
+    // Pair tables, 32 equal (high, low) pairs of words per entry: a warp takes an entry, the centroids sit in its lanes.
+    auto build_table = [&](auto bits, const float *cb, uint2 *dst) {
         constexpr int BITS = decltype(bits)::value;
         const float mine = lane < (1 << BITS) ? cb[lane] : 0.f;
 #pragma unroll 4
         for (int j = warp; j < (1 << (2 * BITS)); j += ST_WARPS) {
             const float a = __shfl_sync(0xffffffffu, mine, j & ((1 << BITS) - 1)), b = __shfl_sync(0xffffffffu, mine, j >> BITS);
             const uint32_t hi = pack_h2(a, b);
-            dst[j * 32 + lane] = hi;
-            dst[(1 << (2 * BITS)) * 32 + j * 32 + lane] = low_half2(hi, a, b);
+            dst[j * 32 + lane] = make_uint2(hi, low_half2(hi, a, b));
         }
     };
-    if constexpr (K::TURBO) build_table(std::integral_constant<int, K::BITS>{}, p.kcb, (uint32_t *)smem);
+    if constexpr (K::TURBO) build_table(std::integral_constant<int, K::BITS>{}, p.kcb, (uint2 *)(smem + SH::K_AT));
     if constexpr (V::TURBO)
-        if (!K::TURBO || p.v_table) build_table(std::integral_constant<int, V::BITS>{}, p.vcb, (uint32_t *)(smem + p.v_table));
-    const uint32_t vtab = s0 + (uint32_t)p.v_table;
+        if (!K::TURBO || SH::K_AT || p.v_table) build_table(std::integral_constant<int, V::BITS>{}, p.vcb, (uint2 *)(smem + p.v_table));
     pdl_wait();
     pdl_trigger();
 
@@ -345,8 +401,8 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
         auto value_place = [](int i) {
             if constexpr (!V::POW2) return i << 4;
             else {
-                const int tok = i / V::CH, ch = i % V::CH;
-                return (tok * V::CH + (ch ^ value_xor<VK, D>(tok))) << 4;
+                const int tok = i / V::CH, ch = i % V::CH, slot = value_slot<VK, D>(tok);
+                return (slot * V::CH + (ch ^ value_xor<VK, D>(slot & 3))) << 4;
             }
         };
         constexpr int KC = K::BLOCK / 16, VC = V::BLOCK / 16, KI = (KC + 31) / 32, VI = (VC + 31) / 32;
@@ -635,10 +691,10 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                 }
 #pragma unroll
                 for (int q = 0; q < KSTEPS; ++q) {
-                    const uint32_t o0 = s0 + pair_offset<K::BITS, QW>(w[0], 2 * q, lane_bits), o1 = s0 + pair_offset<K::BITS, QW>(w[1], 2 * q, lane_bits);
-                    const uint32_t o2 = s0 + pair_offset<K::BITS, QW>(w[0], 2 * q + 1, lane_bits), o3 = s0 + pair_offset<K::BITS, QW>(w[1], 2 * q + 1, lane_bits);
-                    mma_k(s, q, lds32(o0), lds32(o1), lds32(o2), lds32(o3));
-                    const uint32_t lo[4] = {lds32(o0 + K::TABLE), lds32(o1 + K::TABLE), lds32(o2 + K::TABLE), lds32(o3 + K::TABLE)};
+                    const uint2 x0 = table_entry(entry_offset<K::BITS, QW>(w[0], 2 * q, k_lane_bits)), x1 = table_entry(entry_offset<K::BITS, QW>(w[1], 2 * q, k_lane_bits));
+                    const uint2 x2 = table_entry(entry_offset<K::BITS, QW>(w[0], 2 * q + 1, k_lane_bits)), x3 = table_entry(entry_offset<K::BITS, QW>(w[1], 2 * q + 1, k_lane_bits));
+                    mma_k(s, q, x0.x, x1.x, x2.x, x3.x);
+                    const uint32_t lo[4] = {x0.y, x1.y, x2.y, x3.y};
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb) MmaType<KT>::mma(s2[nb], lo, qb[nb][0][q][0], qb[nb][0][q][1]);
                 }
@@ -728,77 +784,93 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                     for (int i = 0; i < 2; ++i) {
                         const float f = i ? f1 : f0, x = s[nb][2 * i] * f, y = s[nb][2 * i + 1] * f;
                         const uint32_t hi = pack_h2(x, y);
-                        pb[nb][0][i] = movmatrix_trans(hi);
-                        pb[nb][1][i] = movmatrix_trans(low_half2(hi, x, y));
+                        pb[nb][0][i] = movmatrix_free(hi);
+                        pb[nb][1][i] = movmatrix_free(low_half2(hi, x, y));
                     }
             };
-            if constexpr (V::TURBO) pack_p(vf[0][0], vf[1][0]);
-            const int vt = lane & 15, vh = lane >> 4;     // unpacking: token, 32-dim half of the pass
-            const int frow = (lane >> 4) * 8 + (lane & 7), fch = (lane >> 3) & 1;   // ldmatrix row and chunk parity
-#pragma unroll
-            for (int ps = 0; ps < PASSES; ++ps) {
-                constexpr int W = V::BITS;            // words of 32 codes
-                uint32_t w[W];
-                const int off = (ps * 2 + vh) * 4 * W;
-                if constexpr (W == 4 || W == 8) {
-#pragma unroll
-                    for (int j = 0; j < W / 4; ++j) {
-                        const int ch = (off >> 4) + j;
-                        const uint4 v = lds128(vst + vt * V::RB + ((ch ^ value_xor<VK, D>(vt)) << 4));
-                        w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
-                    }
-                } else if constexpr (W == 2) {
-                    const uint2 v = lds64(vst + vt * V::RB + ((((off >> 4) ^ value_xor<VK, D>(vt)) << 4) | (off & 15)));
-                    w[0] = v.x; w[1] = v.y;
-                } else {
-#pragma unroll
-                    for (int j = 0; j < W; ++j) w[j] = lds32(vst + vt * V::RB + off + 4 * j);
-                }
-                __syncwarp();                         // the tiles' previous contents have been read
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t at = vtile + vt * 128 + (((vh * 4 + j) ^ (vt & 7)) << 4);
-                    if constexpr (VK == SK_A4) {
-                        sts128(at, make_uint4(code4(w[j], 0), code4(w[j], 1), code4(w[j], 2), code4(w[j], 3)));
-                    } else if constexpr (VK == SK_A8) {
-                        sts128(at, make_uint4(code8(w[2 * j], 0), code8(w[2 * j], 1), code8(w[2 * j + 1], 0), code8(w[2 * j + 1], 1)));
-                    } else {
-                        uint32_t o[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) o[i] = vtab + pair_offset<V::BITS, W>(w, 4 * j + i, lane_bits);
-                        sts128(at, make_uint4(lds32(o[0]), lds32(o[1]), lds32(o[2]), lds32(o[3])));
-                        sts128(at + 2048, make_uint4(lds32(o[0] + V::TABLE), lds32(o[1] + V::TABLE), lds32(o[2] + V::TABLE), lds32(o[3] + V::TABLE)));
+            // this lane's run of unit u of token 2c + j + 8h
+            auto load_run = [&](int u, int j, int h, uint32_t (&w)[VW]) {
+                if constexpr (V::POW2) {
+                    const int off = u * (VU * V::BITS / 8) + g * (VRB / 8);
+                    const uint32_t ad = vst + (8 * h + 4 * j + c) * V::RB + ((((off >> 4) ^ value_xor<VK, D>(c)) << 4) | (off & 15));
+                    if constexpr (VRB == 16) w[0] = lds16(ad);
+                    else if constexpr (VRB == 32) w[0] = lds32(ad);
+                    else if constexpr (VRB == 64) { const uint2 v = lds64(ad); w[0] = v.x; w[1] = v.y; }
+                    else { const uint4 v = lds128(ad); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
+                } else {                              // 3-bit indices: runs of 24, 48 and 96 bits
+                    const int byte = g * (VRB / 8);
+                    const uint32_t ad = vst + (2 * c + j + 8 * h) * V::RB + (byte & ~3);
+                    if constexpr (VRB == 96) {
+                        w[0] = lds32(ad); w[1] = lds32(ad + 4); w[2] = lds32(ad + 8);
+                    } else {                          // (the word behind a run may be the next row's: its bits are not used)
+                        const uint32_t lo = lds32(ad), hi = lds32(ad + 4);
+                        w[0] = __funnelshift_r(lo, hi, 8 * (byte & 3));
+                        if constexpr (VRB == 48) w[1] = hi >> (8 * (byte & 3));
                     }
                 }
-                __syncwarp();
+            };
+            // the high halves of the centroids (or the exact codes) meet both halves of P, the low ones the high half
+            auto mma_v = [&](int mt, const uint32_t (&a)[4]) {
 #pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    if constexpr (V::AFFINE) {
-                        if (mt * 16 % UNIT == 0) {
-                            const int u = (ps * 64 + mt * 16) / UNIT, gr = (u * p.groups_v) / NG;
-                            const uint32_t a0 = vst + V::BLOCK + V::SIDE + (g * p.groups_v + gr) * 2, a1 = a0 + 16 * p.groups_v;
-                            pack_p(vf[0][u], vf[1][u]);
-                            const float b0 = fmaf(vf[0][u], code_middle<VK>(), ld16<T>(a0)), b1 = fmaf(vf[1][u], code_middle<VK>(), ld16<T>(a1));
+                for (int nb = 0; nb < NB; ++nb) {
+                    mma_f16(acc[nb][mt], a, pb[nb][0][0], pb[nb][0][1]);
+                    mma_f16(acc[nb][mt], a, pb[nb][1][0], pb[nb][1][1]);
+                }
+            };
+            if constexpr (V::TURBO) {
+                uint32_t even[2][VW], odd[2][VW];
 #pragma unroll
-                            for (int nb = 0; nb < NB; ++nb)
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t wa[VW], wb[VW];
+                    load_run(0, 0, h, wa);
+                    load_run(0, 1, h, wb);
+                    pair_tokens<V::BITS, VW>(wa, wb, even[h], odd[h]);
+                }
+                pack_p(vf[0][0], vf[1][0]);
 #pragma unroll
-                                for (int h = 0; h < 2; ++h)
-                                    vbias[nb][u][h] = fmaf(s[nb][h], b0, fmaf(s[nb][2 + h], b1, vbias[nb][u][h]));
+                for (int n = 0; n < VM; ++n) {
+                    const uint2 x0 = table_entry(entry_offset<V::BITS, VW>(even[0], n, v_lane_bits)), x1 = table_entry(entry_offset<V::BITS, VW>(odd[0], n, v_lane_bits));
+                    const uint2 x2 = table_entry(entry_offset<V::BITS, VW>(even[1], n, v_lane_bits)), x3 = table_entry(entry_offset<V::BITS, VW>(odd[1], n, v_lane_bits));
+                    const uint32_t hi[4] = {x0.x, x1.x, x2.x, x3.x}, lo[4] = {x0.y, x1.y, x2.y, x3.y};
+                    mma_v(n, hi);
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb) mma_f16(acc[nb][n], lo, pb[nb][0][0], pb[nb][0][1]);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < NG; ++u) {
+                    uint32_t w[2][2][VW];             // [token pair][token]
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        load_run(u, 0, h, w[h][0]);
+                        load_run(u, 1, h, w[h][1]);
+                    }
+                    const int gr = (u * p.groups_v) / NG;
+                    const uint32_t a0 = vst + V::BLOCK + V::SIDE + (g * p.groups_v + gr) * 2, a1 = a0 + 16 * p.groups_v;
+                    pack_p(vf[0][u], vf[1][u]);
+                    const float b0 = fmaf(vf[0][u], code_middle<VK>(), ld16<T>(a0)), b1 = fmaf(vf[1][u], code_middle<VK>(), ld16<T>(a1));
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            vbias[nb][u][h] = fmaf(s[nb][h], b0, fmaf(s[nb][2 + h], b1, vbias[nb][u][h]));
+#pragma unroll
+                    for (int n = 0; n < VM; n += 2) { // four dims: half a word of 4-bit codes, a word of 8-bit ones
+                        uint32_t a[2][4];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            if constexpr (VK == SK_A4) {
+                                const uint32_t x = __byte_perm(w[h][0][0], w[h][1][0], (n & 2) ? 0x7632 : 0x5410);
+                                a[0][2 * h] = code4(x, 0); a[0][2 * h + 1] = code4(x, 1);
+                                a[1][2 * h] = code4(x, 2); a[1][2 * h + 1] = code4(x, 3);
+                            } else {
+                                const uint32_t x = __byte_perm(w[h][0][n >> 1], w[h][1][n >> 1], 0x5140), y = __byte_perm(w[h][0][n >> 1], w[h][1][n >> 1], 0x7362);
+                                a[0][2 * h] = code8(x, 0); a[0][2 * h + 1] = code8(x, 1);
+                                a[1][2 * h] = code8(y, 0); a[1][2 * h + 1] = code8(y, 1);
+                            }
                         }
-                    }
-                    // the high halves of the centroids (or the exact codes) meet both halves of P, the low ones the high half
-                    uint32_t a[4];
-                    const uint32_t at = vtile + frow * 128 + (((2 * mt + fch) ^ (frow & 7)) << 4);
-                    ldmatrix_x4_trans(a, at);
-#pragma unroll
-                    for (int nb = 0; nb < NB; ++nb) {
-                        MmaType<VT>::mma(acc[nb][ps * 4 + mt], a, pb[nb][0][0], pb[nb][0][1]);
-                        MmaType<VT>::mma(acc[nb][ps * 4 + mt], a, pb[nb][1][0], pb[nb][1][1]);
-                    }
-                    if constexpr (V::TURBO) {
-                        ldmatrix_x4_trans(a, at + 2048);
-#pragma unroll
-                        for (int nb = 0; nb < NB; ++nb) MmaType<VT>::mma(acc[nb][ps * 4 + mt], a, pb[nb][0][0], pb[nb][0][1]);
+                        mma_v(u * VM + n, a[0]);
+                        mma_v(u * VM + n + 1, a[1]);
                     }
                 }
             }
@@ -814,8 +886,6 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
         float *work = red_ml + ST_WARPS * rr_n * 2;
         __syncthreads();        // every warp has left the ring that the merge buffers overlay
         const float undo = (V::AFFINE ? 1.f : p.vcb_undo) / ST_PSCALE;
-        // lane g holds columns g of the chunks of eight: its dim
-        const int gd = chunk_dim<VK>(g);
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
@@ -838,9 +908,9 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
                     float *dst = red_o + (warp * rr_n + r) * SH::RED_STRIDE;
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt) {
-                        const float b = vb[V::AFFINE ? mt * 16 / UNIT : 0];
-                        dst[16 * mt + gd] = fmaf(acc[nb][mt][h], undo, b);
-                        dst[16 * mt + 8 + gd] = fmaf(acc[nb][mt][2 + h], undo, b);
+                        const int u = mt / VM;
+                        const float b = vb[V::AFFINE ? u : 0];
+                        *(float2 *)&dst[u * VU + g * VRUN + 2 * (mt % VM)] = make_float2(fmaf(acc[nb][mt][h], undo, b), fmaf(acc[nb][mt][2 + h], undo, b));
                     }
                     if (g == 0) {
                         red_ml[(warp * rr_n + r) * 2] = l > 0.f ? m_run[nb][h] : -INFINITY;
@@ -873,7 +943,7 @@ void launch_stream_typed(const StreamParams &p, const void *list, int ctas, cuda
     using SH = StreamShape<T, D, KK, VK, UNIT, NB, LIST>;
     using LT = std::conditional_t<LIST, StreamList, StreamNoList>;
     auto kernel = attn_stream_kernel<T, D, KK, VK, UNIT, NB, LIST>;
-    const size_t tables = std::max<size_t>(Kind<KK, D>::TABLES, (size_t)p.v_table + Kind<VK, D>::TABLES);
+    const size_t tables = SH::tables(p.v_table);
     const size_t smem = tables + SH::FIXED;
     static size_t configured[64] = {0};
     const int dev = current_device();
