@@ -1,16 +1,18 @@
 // Decode attention over affine-quantised caches of single-precision callers (4- / 8-bit codes, f32 scales and
 // biases), head dims 64 / 128 / 256, up to eight query rows per unit, one call or a list of calls of one shape.
 //
-// Everything is fp32 (the codes become scale * code + bias before they are multiplied), so the work sits on the
-// FMA pipe: about 34 warp instructions per cached row of a 4-row group at D 64. What bounds the shapes it serves
-// (a few MB of codes per step) is latency. Split as in attn_stream.cuh: a warp walks 16-token blocks on its own,
-// with a private two-stage ring filled by 16-byte cp.async copies; no barrier before a segment's end.
+// Everything is fp32 (the codes become scale * code + bias before they are multiplied), two dims an instruction
+// (f32x2.cuh). A unit holds two, four or eight rows, as many as the group has: rows that are not there cost as much as
+// those that are (2 layers x 3 sequences x 7 876 tokens, 16/8 heads, D 128, 4 bits: 55 us with four rows and single
+// products, 43 with two). What bounds small shapes (a few MB of codes per step) is latency. Split as in
+// attn_stream.cuh: a warp walks 16-token blocks on its own, with a private two-stage ring filled by 16-byte cp.async copies; no barrier before a segment's end.
 //   * scores: lane = (token, half of the head dims); a lane reads its row's chunks (swizzled by the token) and the
 //     query rows as broadcasts, the two halves meet in one shuffle.
 //   * values: lane = D / 32 neighbouring dims; probabilities are read back as broadcasts.
 // Work is cut into equal ranges of 64-token tiles over the resident CTAs, partials merged by segment_epilogue.
 // Before (general kernel + merge kernel): 34 us per layer of the Llama-3.2-1B shape at 1024 tokens.
 #include "attn_stream.cuh"
+#include "f32x2.cuh"
 
 namespace kvc {
 
@@ -61,19 +63,40 @@ template <int CH> __device__ __forceinline__ int row_xor(int tok) {
     return CH >= 8 ? tok & 7 : CH == 4 ? (tok >> 1) & 3 : CH == 2 ? (tok >> 2) & 1 : 0;
 }
 
-// Code k of a word as a float: the exact integer.
-template <int BITS> __device__ __forceinline__ float code_f32(uint32_t w, int k) {
-    if (BITS == 8) return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + k)) - 8388608.f;
-    return (float)((w >> (4 * k)) & 15u);
-}
+// Codes k and k + 1 (k even) of a word under a group's scale and bias. A 4-bit code stays where it lies in its half word, so
+// it is its integer times 16^(k % 4), of which the scale is rid by a power of two: the products are those of the integers.
+template <int BITS> struct GroupScale {
+    uint64_t s[BITS == 4 ? 2 : 1], bias;
+    __device__ __forceinline__ GroupScale(float scale, float b) {
+        if (BITS == 4) {
+            s[0] = pack_f2(scale, scale * 0.0625f);
+            s[BITS == 4 ? 1 : 0] = pack_f2(scale * 0.00390625f, scale * 0.000244140625f);
+        } else {
+            s[0] = pack_f2(scale, scale);
+        }
+        bias = pack_f2(b, b);
+    }
+    __device__ __forceinline__ uint64_t pair(uint32_t w, int k) const {
+        uint32_t a, b;
+        if (BITS == 8) {
+            a = __byte_perm(w, 0x4B000000u, 0x7440 + k);
+            b = __byte_perm(w, 0x4B000000u, 0x7441 + k);
+        } else {
+            const uint32_t h = k >= 4 ? w >> 16 : w;
+            a = (h & (15u << (4 * (k & 3)))) | 0x4B000000u;
+            b = (h & (15u << (4 * (k & 3) + 4))) | 0x4B000000u;
+        }
+        const uint64_t code = add_f2(pack_f2(__uint_as_float(a), __uint_as_float(b)), pack_f2(-8388608.f, -8388608.f));
+        return fma_f2(s[BITS == 4 ? (k >> 1) & 1 : 0], code, bias);
+    }
+};
 
 __device__ __forceinline__ float lds_f32(uint32_t a) { return __uint_as_float(lds32(a)); }
-__device__ __forceinline__ float4 lds_f32x4(uint32_t a) {
-    const uint4 v = lds128(a);
-    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+__device__ __forceinline__ void lds_f2x2(uint32_t a, uint64_t &x, uint64_t &y) {
+    asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory");
 }
 
-// RN: query rows a unit carries (4 or 8).
+// RN: query rows a unit carries (2, 4 or 8).
 template <int D, int BITS, int RN>
 __global__ void __launch_bounds__(ST_THREADS, D <= 128 ? 2 : 1)
 attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32List list) {
@@ -140,7 +163,8 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
         __syncthreads();
 
         const int tok = lane & 15, half = lane >> 4;
-        float m_run[RN], l_run[RN], acc[RN][E];
+        float m_run[RN], l_run[RN];
+        uint64_t acc[RN][E / 2];
         int lim[RN];
 #pragma unroll
         for (int r = 0; r < RN; ++r) {
@@ -149,7 +173,7 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
             lim[r] = T - 1;
             if (p.causal && row0 + r < rows_all) lim[r] = (int)min((int64_t)(T - 1), sq.causal_offset + (row0 + r) % p.L);
 #pragma unroll
-            for (int e = 0; e < E; ++e) acc[r][e] = 0.f;
+            for (int e = 0; e < E / 2; ++e) acc[r][e] = 0;
         }
         int stage = 0;
         for (int blk = warp; blk < nblk; blk += ST_WARPS) {
@@ -160,32 +184,34 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
             const uint32_t st = ring + stage * SH::STAGE, sides = st + 2 * SH::BLOCK;
             const int t0 = t_lo + blk * 16;
 
-            float s[RN];
+            uint64_t dot[RN];                                      // even and odd dims
 #pragma unroll
-            for (int r = 0; r < RN; ++r) s[r] = 0.f;
-            constexpr int PER = 128 / BITS;                        // dims per chunk
+            for (int r = 0; r < RN; ++r) dot[r] = 0;
+            constexpr int PER = 128 / BITS, CPW = 32 / BITS;       // dims per chunk, per word
 #pragma unroll
             for (int j = 0; j < CH / 2; ++j) {
                 const int ch = half * (CH / 2) + j;
                 const uint4 w4 = lds128(st + ((tok * CH + (ch ^ row_xor<CH>(tok))) << 4));
                 const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
                 const int gr = ch * PER * p.groups / D;
-                const float sc = lds_f32(sides + (tok * p.groups + gr) * 4), bi = lds_f32(sides + SH::SIDE + (tok * p.groups + gr) * 4);
+                const GroupScale<BITS> gs(lds_f32(sides + (tok * p.groups + gr) * 4), lds_f32(sides + SH::SIDE + (tok * p.groups + gr) * 4));
 #pragma unroll
-                for (int i = 0; i < PER / 4; ++i) {
-                    float kv[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int at = 4 * i + e;
-                        kv[e] = fmaf(sc, code_f32<BITS>(w[at * BITS / 32], at % (32 / BITS)), bi);
-                    }
+                for (int i = 0; i < PER; i += 4) {
+                    const uint64_t k0 = gs.pair(w[i / CPW], i % CPW), k1 = gs.pair(w[i / CPW], i % CPW + 2);
 #pragma unroll
                     for (int r = 0; r < RN; ++r) {
-                        const float4 q = lds_f32x4(q0 + (r * SH::QROW + half * (HALF + 4) + j * PER + 4 * i) * 4);
-                        s[r] = fmaf(q.x, kv[0], s[r]); s[r] = fmaf(q.y, kv[1], s[r]);
-                        s[r] = fmaf(q.z, kv[2], s[r]); s[r] = fmaf(q.w, kv[3], s[r]);
+                        uint64_t q01, q23;
+                        lds_f2x2(q0 + (r * SH::QROW + half * (HALF + 4) + j * PER + i) * 4, q01, q23);
+                        dot[r] = fma_f2(q23, k1, fma_f2(q01, k0, dot[r]));
                     }
                 }
+            }
+            float s[RN];
+#pragma unroll
+            for (int r = 0; r < RN; ++r) {
+                float even, odd;
+                unpack_f2(dot[r], even, odd);
+                s[r] = even + odd;
             }
             bool moved = false;
 #pragma unroll
@@ -205,7 +231,7 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
                     m_run[r] = mx;
                     l_run[r] *= alpha;
 #pragma unroll
-                    for (int e = 0; e < E; ++e) acc[r][e] *= alpha;
+                    for (int e = 0; e < E / 2; ++e) acc[r][e] = mul_f2(acc[r][e], pack_f2(alpha, alpha));
                 }
             }
 #pragma unroll
@@ -213,11 +239,16 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
                 s[r] = exp2f(s[r] - m_run[r]);
                 if (half == 0) l_run[r] += s[r];
             }
-            if (half == 0)
+            if (half == 0) {
+                if constexpr (RN == 2) {
+                    sts64(prob + tok * 8, make_uint2(__float_as_uint(s[0]), __float_as_uint(s[1])));
+                } else {
 #pragma unroll
-                for (int r = 0; r < RN; r += 4)
-                    sts128(prob + (tok * RN + r) * 4, make_uint4(__float_as_uint(s[r]), __float_as_uint(s[r + 1]),
-                                                                 __float_as_uint(s[r + 2]), __float_as_uint(s[r + 3])));
+                    for (int r = 0; r < RN; r += 4)
+                        sts128(prob + (tok * RN + r) * 4, make_uint4(__float_as_uint(s[r]), __float_as_uint(s[r + 1]),
+                                                                     __float_as_uint(s[r + 2]), __float_as_uint(s[r + 3])));
+                }
+            }
             __syncwarp();
             // ---- values: this lane's E dims of every token ----
             const int off = lane * E * BITS / 8, ch = off >> 4, gr = lane * E * p.groups / D;
@@ -228,18 +259,24 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
                 uint32_t w[(E * BITS + 31) / 32];
                 if constexpr (E * BITS == 64) { const uint2 v = lds64(ad); w[0] = v.x; w[1] = v.y; }
                 else w[0] = lds32(ad) >> ((off & 3) * 8);
-                const float sc = lds_f32(sides + 2 * SH::SIDE + (t * p.groups + gr) * 4), bi = lds_f32(sides + 3 * SH::SIDE + (t * p.groups + gr) * 4);
+                const GroupScale<BITS> gs(lds_f32(sides + 2 * SH::SIDE + (t * p.groups + gr) * 4), lds_f32(sides + 3 * SH::SIDE + (t * p.groups + gr) * 4));
                 float pr[RN];
+                if constexpr (RN == 2) {
+                    const uint2 v = lds64(prob + t * 8);
+                    pr[0] = __uint_as_float(v.x); pr[1] = __uint_as_float(v.y);
+                } else {
 #pragma unroll
-                for (int r = 0; r < RN; r += 4) {
-                    const float4 v = lds_f32x4(prob + (t * RN + r) * 4);
-                    pr[r] = v.x; pr[r + 1] = v.y; pr[r + 2] = v.z; pr[r + 3] = v.w;
+                    for (int r = 0; r < RN; r += 4) {
+                        const uint4 v = lds128(prob + (t * RN + r) * 4);
+                        pr[r] = __uint_as_float(v.x); pr[r + 1] = __uint_as_float(v.y);
+                        pr[r + 2] = __uint_as_float(v.z); pr[r + 3] = __uint_as_float(v.w);
+                    }
                 }
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const float v = fmaf(sc, code_f32<BITS>(w[e * BITS / 32], e % (32 / BITS)), bi);
+                for (int e = 0; e < E / 2; ++e) {
+                    const uint64_t v = gs.pair(w[2 * e * BITS / 32], 2 * e % (32 / BITS));
 #pragma unroll
-                    for (int r = 0; r < RN; ++r) acc[r][e] = fmaf(pr[r], v, acc[r][e]);
+                    for (int r = 0; r < RN; ++r) acc[r][e] = fma_f2(pack_f2(pr[r], pr[r]), v, acc[r][e]);
                 }
             }
             __syncwarp();   // this stage and the probabilities may be overwritten
@@ -258,7 +295,7 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
             for (int o = 16; o >= 1; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
             if (r < R) {
 #pragma unroll
-                for (int e = 0; e < E; ++e) red_o[(warp * rr_n + r) * (D + 4) + lane * E + e] = acc[r][e];
+                for (int e = 0; e < E / 2; ++e) *(uint64_t *)&red_o[(warp * rr_n + r) * (D + 4) + lane * E + 2 * e] = acc[r][e];
                 if (lane == 0) {
                     red_ml[(warp * rr_n + r) * 2] = l > 0.f ? m_run[r] : -INFINITY;
                     red_ml[(warp * rr_n + r) * 2 + 1] = l;
@@ -327,7 +364,7 @@ StreamSource f32_stream_source(const KVSource &s) {
 int launch_attention_f32_list(const AttnArgs *args, int n, cudaStream_t stream) {
     if (n < 1 || n > KVC_LIST_MAX || !f32_call(args[0])) return 0;
     const AttnArgs &a0 = args[0];
-    const int rows = a0.Hq / a0.Hkv * a0.L, rn = rows <= 4 ? 4 : 8;
+    const int rows = a0.Hq / a0.Hkv * a0.L, rn = rows <= 2 ? 2 : rows <= 4 ? 4 : 8;
     F32Params p = {};
     p.chunks = (rows + rn - 1) / rn;
     const int64_t units = (int64_t)a0.B * a0.Hkv * p.chunks;
@@ -364,7 +401,8 @@ int launch_attention_f32_list(const AttnArgs *args, int n, cudaStream_t stream) 
     p.scale_log2 = a0.scale * 1.4426950408889634f;
 #define KVC_F32K(DD, BB)                                                    \
     if (a0.D == DD && a0.k.bits == BB) {                                    \
-        if (rn == 4) launch_f32_typed<DD, BB, 4>(p, list, ctas, stream);    \
+        if (rn == 2) launch_f32_typed<DD, BB, 2>(p, list, ctas, stream);    \
+        else if (rn == 4) launch_f32_typed<DD, BB, 4>(p, list, ctas, stream);    \
         else launch_f32_typed<DD, BB, 8>(p, list, ctas, stream);            \
         return 1;                                                           \
     }
