@@ -1019,44 +1019,80 @@ turbo_encode_vec_kernel(TurboEncodeArgs ka, TurboEncodeArgs va, float inv_sqrt_d
 // The same encode for many rows: 16 dims per lane, so a warp holds 32 / (D / 16) rows. Issue-bound like the
 // one-row-per-warp form above, with a third of its instructions per row: the Walsh-Hadamard stages that pair
 // dims less than 16 apart need no shuffle, the shuffles left carry several rows each, a lane's codes fill whole
-// words, and a code is found with one table read and one comparison: a monotone map sends the value to one of
-// 64 cells that hold at most one boundary each, so the boundaries of lower cells are passed and those of higher
-// cells are not, whatever the rounding of the map (the host builds the cells with the same fused multiply-add).
+// words, and a code is found with one table read and one subtraction, whose sign counts the cell's boundary: a monotone
+// map (bits of one fused multiply-add) sends the value to one of 256 cells that hold at most one boundary each, so the
+// boundaries of lower cells are passed and those of higher cells are not, whatever the rounding of the map. The cells
+// span [-1, 1], so a coordinate of a unit vector needs no clamp; other codebooks, calibrated rows and signs that are
+// not +-1 clamp. Signs of one turn the sign bits of the packed elements. A block walks neighbouring row groups, so
+// that places move by strides, with the next row's loads in flight.
 // Sums run over the fixed tree (D / 32 neighbouring dims left to right, then the exchanges 16, 8, 4, 2, 1, of
 // which the last ones stay inside a lane), so norms and codes are the bits of turbo_encode_kernel.
-// 2 x 131072 rows of D 128 bf16, 4 bits: 96 us before. Products and sums take two dims an instruction (f32x2.cuh): keys with
-// the calibration statistic 43.3 -> 41.1 us, values 33 -> 30.
+// 131072 rows of D 128 bf16, 4 bits (27 instructions an element, 66 % of the issue rate): 22 us; 30 with 64 clamped
+// cells, products by signs and a place computed per row. Keys with the calibration statistic (128 registers, two
+// blocks an SM): 34 us, 41 before.
 // ---------------------------------------------------------------------
+constexpr int CELLS = 256;
 struct EncodeCells {
-    float scale, shift;      // cell = round(x * scale) + shift, as the low bits of fma(x, scale, shift)
-    float2 cell[64];         // boundary of the cell (+inf: none), number of boundaries below it
+    float scale, shift;      // cell = floor(x * scale) + a constant: bits 7 .. 14 of fma(x, scale, shift)
+    int32_t clamp;           // 0: the cells span [-1, 1], which no coordinate of a unit vector leaves
 };
-constexpr float CELL_MAGIC = 12582912.f;   // 1.5 * 2^23
+constexpr float CELL_MAGIC = 98304.f;      // 1.5 * 2^16: a unit in the last place is 2^-7
+constexpr float CELL_TOP = CELL_MAGIC + 254.9921875f;
+constexpr float SUM_MAGIC = 12582912.f;    // 1.5 * 2^23: a unit in the last place is 1
 
+// The cell of a value (the host and the kernels agree to the bit: one fused multiply-add, exact comparisons).
+__host__ __device__ inline int cell_of(const EncodeCells &c, float x) {
+    const float u = fminf(fmaxf(fmaf(x, c.scale, c.shift), CELL_MAGIC), CELL_TOP);
+#ifdef __CUDA_ARCH__
+    const uint32_t bits = __float_as_uint(u);
+#else
+    uint32_t bits;
+    std::memcpy(&bits, &u, sizeof bits);
+#endif
+    return (int)((bits >> 7) & (CELLS - 1));
+}
+
+// No two boundaries in a cell, and none in the first and last one, where values that are no numbers go.
+bool cells_hold(const TurboEncodeArgs &a, const EncodeCells &c) {
+    int before = 0;
+    for (int i = 0; i < (1 << a.bits) - 1; ++i) {
+        const int at = cell_of(c, a.boundaries[i]);
+        if (at <= before || at >= CELLS - 1) return false;
+        before = at;
+    }
+    return true;
+}
+
+// Cell `i` of a codebook's boundaries: the boundary in it (+inf: none) and the number of boundaries below it. The last cell
+// holds what is no number, all of whose bits are set, and no number: nothing is passed.
+template <int BITS>
+__device__ __forceinline__ float2 make_cell(const TurboEncodeArgs &a, const EncodeCells &c, int i) {
+    float bound = INFINITY;
+    uint32_t below = 0;
+#pragma unroll
+    for (int j = 0; j < (1 << BITS) - 1; ++j) {
+        const int at = cell_of(c, a.boundaries[j]);
+        below += at < i ? 1u : 0u;
+        if (at == i) bound = a.boundaries[j];
+    }
+    return make_float2(bound, __uint_as_float(i == CELLS - 1 ? 0u : below));
+}
+
+// Cells that need no clamp where the boundaries lie within (-1, 1) and no two share a cell, else cells between the outer boundaries.
 bool build_cells(const TurboEncodeArgs &a, EncodeCells *c) {
     const int n = (1 << a.bits) - 1;
     const float lo = a.boundaries[0], hi = a.boundaries[n - 1];
     for (int i = 0; i < n; ++i)
         if (!(fabsf(a.boundaries[i]) < 1e4f) || (i && !(a.boundaries[i - 1] < a.boundaries[i]))) return false;
-    c->scale = n == 1 ? 1.f : 61.f / (hi - lo);
+    c->clamp = 0;
+    c->scale = 126.f;
+    c->shift = CELL_MAGIC + 128.f;
+    if (!a.calib && lo > -1.f && hi < 1.f && cells_hold(a, *c)) return true;
+    c->clamp = 1;
+    c->scale = n == 1 ? 1.f : 253.f / (hi - lo);
     if (!(c->scale < 1e6f)) return false;
-    c->shift = CELL_MAGIC + 1.f - rintf(lo * c->scale);
-    auto place = [&](float x) {
-        const float u = fmaf(x, c->scale, c->shift);
-        return (int)(fminf(fmaxf(u, CELL_MAGIC), CELL_MAGIC + 63.f) - CELL_MAGIC);
-    };
-    int next = 0;
-    for (int i = 0; i < 64; ++i) {
-        c->cell[i] = make_float2(INFINITY, 0.f);
-        const int below = next;
-        if (next < n && place(a.boundaries[next]) == i) {
-            if (i == 0) return false;            // cell 0 is where values that are no numbers go
-            c->cell[i].x = a.boundaries[next++];
-        }
-        if (next < n && place(a.boundaries[next]) <= i) return false;
-        std::memcpy(&c->cell[i].y, &below, sizeof below);
-    }
-    return next == n;
+    c->shift = CELL_MAGIC + 1.5f - rintf(lo * c->scale);
+    return cells_hold(a, *c);
 }
 
 template <int D> __device__ __forceinline__ float tree_sum(float (&p)[16 / (D / 32)]) {
@@ -1074,9 +1110,39 @@ template <int D> __device__ __forceinline__ float tree_sum(float (&p)[16 / (D / 
     return p[0];
 }
 
-// This lane's dims `v` of a row, rotated in place (before 1 / sqrt(D)); the row's norm.
-template <int D>
-__device__ __forceinline__ float rotate_wide(const float (&sg)[16], int l, float (&v)[16]) {
+// 16 neighbouring elements of a row as they lie in memory, and times their signs. Signs of one turn over the sign bits
+// (`flip`: the bits to turn), which is the product to the bit.
+template <typename T> struct RawRun {
+    static constexpr int WORDS = 16 * sizeof(T) / 4;
+    uint32_t w[WORDS];
+    __device__ __forceinline__ void load(const T *src) {
+#pragma unroll
+        for (int i = 0; i < WORDS / 4; ++i) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint32_t *>(src) + 4 * i);
+            w[4 * i] = x.x; w[4 * i + 1] = x.y; w[4 * i + 2] = x.z; w[4 * i + 3] = x.w;
+        }
+    }
+    __device__ __forceinline__ void signed_by(const RawRun &flip, float (&v)[16]) const {
+#pragma unroll
+        for (int i = 0; i < WORDS; ++i) {
+            const uint32_t x = w[i] ^ flip.w[i];
+            if constexpr (std::is_same<T, float>::value) {
+                v[i] = __uint_as_float(x);
+            } else if constexpr (std::is_same<T, __half>::value) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&x));
+                v[2 * i] = f.x; v[2 * i + 1] = f.y;
+            } else {
+                v[2 * i] = __uint_as_float(x << 16);
+                v[2 * i + 1] = __uint_as_float(x & 0xFFFF0000u);
+            }
+        }
+    }
+};
+
+// This lane's dims `v` of a row, signs applied, rotated in place (before 1 / sqrt(D)); the row's norm. SCALED: `scale_by` may
+// point at the magnitudes of signs that are not one.
+template <int D, bool SCALED>
+__device__ __forceinline__ float rotate_wide(int l, const float *scale_by, float (&v)[16]) {
     constexpr int E = D / 32, RUNS = 16 / E, LPR = D / 16;
     using namespace dev;
     uint64_t x[8];                                   // dims 2i and 2i + 1
@@ -1096,7 +1162,9 @@ __device__ __forceinline__ float rotate_wide(const float (&sg)[16], int l, float
     const uint64_t inv2 = pack_f2(inv_norm, inv_norm), minus = pack_f2(-1.f, -1.f);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        x[i] = mul_f2(x[i], mul_f2(inv2, pack_f2(sg[2 * i], sg[2 * i + 1])));
+        uint64_t f = inv2;
+        if (SCALED && scale_by) f = mul_f2(inv2, pack_f2(fabsf(scale_by[2 * i]), fabsf(scale_by[2 * i + 1])));
+        x[i] = mul_f2(x[i], f);
         float lo, hi;
         unpack_f2(x[i], lo, hi);
         x[i] = pack_f2(__fadd_rn(lo, hi), __fsub_rn(lo, hi));
@@ -1131,16 +1199,16 @@ template <int D> struct WideRows {
     static constexpr int LPR = D / 16, RPW = 32 / LPR, GROUP = 8 * RPW;
 };
 
-template <typename T, int D, int BITS, bool CAL>
-__device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a, const EncodeCells &cells, const float2 *cell,
-                                                       const float (&sg)[16], int b, int h, int s, int l, float inv_sqrt_dim,
-                                                       float (&rot)[16]) {
+// One row: 16 of its dims, its words to `dst`, its norm to `norm_at`. CLAMP: the value's cell is brought into
+// the table first. `lane_at`: where this lane's copy of a cell lies in its 128 bytes.
+template <typename T, int D, int BITS, bool CAL, bool CLAMP>
+__device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a, const EncodeCells &cells, const unsigned char *cells_mem, uint32_t lane_at,
+                                                       const RawRun<T> &raw, const RawRun<T> &flip, const float *scale_by, uint32_t *dst, float *norm_at, bool live,
+                                                       int l, float inv_sqrt_dim, float (&rot)[16]) {
     constexpr int E = D / 32, RUNS = 16 / E;
-    const bool live = s < a.S;
-    const T *src = (const T *)a.src + b * a.s_sb + h * a.s_sh + (int64_t)(live ? s : a.S - 1) * a.s_ss + l * 16;
     float (&v)[16] = rot;
-    load_row_elems<T, 16>(src, v);
-    const float norm = rotate_wide<D>(sg, l, v);
+    raw.signed_by(flip, v);
+    const float norm = rotate_wide<D, CLAMP>(l, scale_by, v);
     float place[16];                                 // cell of a value, before it is brought into the table
     {
         using namespace dev;
@@ -1154,8 +1222,7 @@ __device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a,
     }
     float stored = norm;
     uint32_t w[2] = {0u, 0u};
-    constexpr int PER = BITS * 16 > 32 ? 32 / BITS : 16;    // codes per word (3 bits: ten, and the straddling one below)
-    uint64_t bits3 = 0;
+    constexpr int PER = BITS > 2 ? 8 : 16;           // codes per word here (3 bits: joined below)
     float p[RUNS];
 #pragma unroll
     for (int i = 15; i >= 0; --i) {
@@ -1164,14 +1231,20 @@ __device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a,
             cal = a.calib[l * 16 + i];
             x = __fdiv_rn(x, cal);
         }
-        const float u = fminf(fmaxf(CAL ? __fmaf_rn(x, cells.scale, cells.shift) : place[i], CELL_MAGIC), CELL_MAGIC + 63.f);
-        const float2 e = cell[(__float_as_uint(u) & 63u) * 16];
-        const uint32_t idx = __float_as_uint(e.y) + (x > e.x ? 1u : 0u);
-        if constexpr (BITS == 3) bits3 = (bits3 << 3) | idx;
-        else w[i / PER] = (w[i / PER] << BITS) | idx;
+        float u = CAL ? __fmaf_rn(x, cells.scale, cells.shift) : place[i];
+        if (CLAMP) u = fminf(fmaxf(u, CELL_MAGIC), CELL_TOP);
+        const float2 e = *reinterpret_cast<const float2 *>(cells_mem + ((__float_as_uint(u) & ((CELLS - 1) << 7)) | lane_at));
+        const float bound = e.x;
+        const uint32_t below = __float_as_uint(e.y);
+        uint32_t &word = w[i / PER];
         if (CAL) {
+            const uint32_t idx = below + (x > bound ? 1u : 0u);
+            word = (word << BITS) | idx;
             const float cv = __fmul_rn(a.centroids[idx], cal);
             v[i] = __fmul_rn(cv, cv);
+        } else {
+            // the sign of the difference: set where x is above the boundary (equal: +0; no number, no boundary: clear)
+            word = (word << BITS) + below + (__float_as_uint(__fsub_rn(bound, x)) >> 31);
         }
     }
     if (CAL) {
@@ -1184,28 +1257,30 @@ __device__ __forceinline__ void turbo_encode_wide_body(const TurboEncodeArgs &a,
         const float recon = __fsqrt_rn(tree_sum<D>(p));
         if (recon > 1e-8f) stored = __fdiv_rn(norm, recon);
     }
-    uint32_t *dst = a.packed + b * a.p_sb + h * a.p_sh + (a.pos + s) * a.p_st;
     if constexpr (BITS == 4) {
-        if (live) *(uint2 *)(dst + 2 * l) = make_uint2(w[0], w[1]);
+        if (live) *(uint2 *)dst = make_uint2(w[0], w[1]);
     } else if constexpr (BITS == 2) {
-        if (live) dst[l] = w[0];
+        if (live) *dst = w[0];
     } else if constexpr (BITS == 3) {
         // two lanes hold 96 bits: the even one writes the first two words, the odd one the third
-        const uint32_t lo = (uint32_t)bits3, hi = (uint32_t)(bits3 >> 32), odd_lo = __shfl_down_sync(0xffffffffu, lo, 1);
-        uint32_t *pair = dst + (l >> 1) * 3;
+        const uint32_t lo = w[0] | (w[1] << 24), hi = w[1] >> 8, odd_lo = __shfl_down_sync(0xffffffffu, lo, 1);
         if (live) {
             if (l & 1) {
-                pair[2] = (lo >> 16) | (hi << 16);
+                *dst = (lo >> 16) | (hi << 16);
             } else {
-                pair[0] = lo;
-                pair[1] = hi | (odd_lo << 16);
+                dst[0] = lo;
+                dst[1] = hi | (odd_lo << 16);
             }
         }
     } else {
         const uint32_t other = __shfl_down_sync(0xffffffffu, w[0], 1);
-        if (live && !(l & 1)) dst[l >> 1] = w[0] | (other << 16);
+        if (live && !(l & 1)) *dst = w[0] | (other << 16);
     }
-    if (live && l == 0) a.norms[b * a.n_sb + h * a.n_sh + (a.pos + s) * a.n_st] = stored;
+    if (live && l == 0) *norm_at = stored;
+}
+// Words of a row in front of those that lane l writes.
+template <int BITS> __device__ __forceinline__ int wide_word(int l) {
+    return BITS == 4 ? 2 * l : BITS == 2 ? l : BITS == 3 ? (l >> 1) * 3 + (l & 1) * 2 : l >> 1;
 }
 
 // The calibration statistic of the keys, taken from the rotated rows while they are encoded (uncalibrated; when the
@@ -1228,8 +1303,8 @@ struct CalibSums {
         using namespace dev;
         auto both = [](float x) { return pack_f2(x, x); };
         auto add = [&](int w, int i, uint64_t y, float down, float up) {
-            const uint64_t t = fma_f2(y, both(down), both(CELL_MAGIC));
-            const uint64_t r = add_f2(fma_f2(add_f2(t, both(-CELL_MAGIC)), both(up), y), both(CELL_MAGIC));
+            const uint64_t t = fma_f2(y, both(down), both(SUM_MAGIC));
+            const uint64_t r = add_f2(fma_f2(add_f2(t, both(-SUM_MAGIC)), both(up), y), both(SUM_MAGIC));
             float t0, t1, r0, r1;
             unpack_f2(t, t0, t1);
             unpack_f2(r, r0, r1);
@@ -1250,32 +1325,79 @@ constexpr int CALIB_ROWS = 1024;      // rows a lane may add up before a part co
 
 // y = keys or values; the row groups of a tensor are dealt to the blocks of x, so a launch is one wave.
 template <typename T, int D, int KB, int VB, bool STATS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, STATS ? 2 : 3)
 turbo_encode_wide_kernel(const __grid_constant__ TurboEncodeArgs ka, const __grid_constant__ TurboEncodeArgs va,
                          const __grid_constant__ EncodeCells kc, const __grid_constant__ EncodeCells vc, int groups, int groups_per_plane,
                          float inv_sqrt_dim, unsigned long long *sums) {
     using W = WideRows<D>;
     asm volatile("griddepcontrol.launch_dependents;");
-    __shared__ float2 table[64 * 16];
+    __shared__ __align__(128) float2 table[CELLS * 16];
     const bool is_v = blockIdx.y != 0;
     const TurboEncodeArgs &a = is_v ? va : ka;
-    for (int i = threadIdx.x; i < 64 * 16; i += blockDim.x) table[i] = is_v ? vc.cell[i >> 4] : kc.cell[i >> 4];
     const int lane = threadIdx.x & 31, l = lane % W::LPR, warp = threadIdx.x >> 5;
-    float sg[16];
-    load_row_elems<float, 16>(a.signs + l * 16, sg);
+    RawRun<T> flip;
+    RawRun<float> signs;
+    signs.load(a.signs + l * 16);
+    {   // a thread takes a cell; the lanes start at different copies of theirs, so that they meet no bank twice
+        static_assert(CELLS == 256, "a thread a cell");
+        const float2 c = is_v ? make_cell<VB>(va, vc, threadIdx.x) : make_cell<KB>(ka, kc, threadIdx.x);
+        const float4 cc = make_float4(c.x, c.y, c.x, c.y);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) reinterpret_cast<float4 *>(table)[threadIdx.x * 8 + ((j + lane) & 7)] = cc;
+    }
+    bool unit = true;
+#pragma unroll
+    for (int i = 0; i < RawRun<T>::WORDS; ++i) flip.w[i] = 0u;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const uint32_t sg = signs.w[i];
+        unit = unit && (sg & 0x7FFFFFFFu) == 0x3F800000u;
+        if (sizeof(T) == 4) flip.w[i % RawRun<T>::WORDS] = sg & 0x80000000u;
+        else flip.w[i / 2] |= (sg >> 31) << ((i & 1) ? 31 : 15);
+    }
+    unit = __all_sync(0xffffffffu, unit);
     __syncthreads();
-    const float2 *cell = table + (lane & 15);     // this lane's copy of the cells: a half warp meets no bank twice
+    const unsigned char *cells_mem = reinterpret_cast<const unsigned char *>(table);
+    const uint32_t lane_at = (lane & 15) * 8;            // a half warp meets no bank twice
     CalibSums cs;
     if (STATS) cs.clear();
-    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
-        const int plane = g / groups_per_plane, h = plane % a.H, b = plane / a.H;
-        const int s0 = (g % groups_per_plane) * W::GROUP + warp * W::RPW, s = s0 + lane / W::LPR;
-        if (s0 >= a.S) continue;      // whole warp
-        float rot[16];
-        if (is_v) turbo_encode_wide_body<T, D, VB, false>(va, vc, cell, sg, b, h, s, l, inv_sqrt_dim, rot);
-        else if (!STATS && ka.calib) turbo_encode_wide_body<T, D, KB, true>(ka, kc, cell, sg, b, h, s, l, inv_sqrt_dim, rot);
-        else turbo_encode_wide_body<T, D, KB, false>(ka, kc, cell, sg, b, h, s, l, inv_sqrt_dim, rot);
-        if (STATS && s < a.S) cs.add_row(rot);
+    const bool cal = !is_v && !STATS && ka.calib, clamp = (is_v ? vc.clamp : kc.clamp) || !unit;
+    const float *scale_by = unit ? nullptr : a.signs + l * 16;
+    // Row groups in runs of neighbours: the place of a group is found once a plane, then moved on by a stride.
+    const int share = groups / (int)gridDim.x, extra = groups % (int)gridDim.x, first = blockIdx.x * share + min((int)blockIdx.x, extra);
+    int left = share + ((int)blockIdx.x < extra), plane = first / groups_per_plane, in = first % groups_per_plane;
+    while (left > 0) {
+        const int h = plane % a.H, b = plane / a.H, n = min(left, groups_per_plane - in);
+        int s = in * W::GROUP + warp * W::RPW + lane / W::LPR;
+        const T *src = (const T *)a.src + b * a.s_sb + h * a.s_sh + (int64_t)s * a.s_ss + l * 16;
+        uint32_t *dst = a.packed + b * a.p_sb + h * a.p_sh + (a.pos + s) * a.p_st + (is_v ? wide_word<VB>(l) : wide_word<KB>(l));
+        float *norm_at = a.norms + b * a.n_sb + h * a.n_sh + (a.pos + s) * a.n_st;
+        const int64_t src_step = W::GROUP * a.s_ss, dst_step = W::GROUP * a.p_st, norm_step = W::GROUP * a.n_st;
+        // the row after this one is on its way while this one is encoded (the sums leave no registers for it)
+        constexpr bool AHEAD = !STATS && sizeof(T) == 2;
+        auto row = [&](const T *at, int t) { return t < a.S ? at : at - (int64_t)(t - (a.S - 1)) * a.s_ss; };
+        RawRun<T> raw, next;
+        if (AHEAD) next.load(row(src, s));
+        for (int k = 0; k < n; ++k, s += W::GROUP, src += src_step, dst += dst_step, norm_at += norm_step) {
+            if (s - lane / W::LPR >= a.S) break;      // whole warp
+            const bool live = s < a.S;
+            if (AHEAD) raw = next;
+            else raw.load(row(src, s));
+            if (AHEAD && k + 1 < n) next.load(row(src + src_step, s + W::GROUP));
+            float rot[16];
+#define KVC_EWROW(BITS, CAL, CLAMP, A, C) turbo_encode_wide_body<T, D, BITS, CAL, CLAMP>(A, C, cells_mem, lane_at, raw, flip, scale_by, dst, norm_at, live, l, inv_sqrt_dim, rot)
+            if (is_v) {
+                if (clamp) KVC_EWROW(VB, false, true, va, vc);
+                else KVC_EWROW(VB, false, false, va, vc);
+            } else if (cal) KVC_EWROW(KB, true, true, ka, kc);
+            else if (clamp) KVC_EWROW(KB, false, true, ka, kc);
+            else KVC_EWROW(KB, false, false, ka, kc);
+#undef KVC_EWROW
+            if (STATS && live) cs.add_row(rot);
+        }
+        left -= n;
+        in = 0;
+        ++plane;
     }
     if constexpr (STATS) {
         long long(*part)[D] = (long long(*)[D])table;      // [warps at a time][D]: the cells are no longer read

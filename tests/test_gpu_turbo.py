@@ -72,6 +72,33 @@ def _pair(kvc, oracle, **kw):
     return g, kb, vb
 
 
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_many_rows_encode_like_few(kvc, oracle, cuda, dtype, bits, D):
+    """Rows of 16 and more a head take the kernel of cells; eight at a time take the search. The same words and norms for
+    rows of zeros, of infinities, of NaN and of one dim, for boundaries closer than a cell of [-1, 1] and beyond it, and
+    for signs that are no signs."""
+    S = 333
+    x = seeded((S, D), 3, dtype)
+    x[1] = 0
+    x[2, 5] = float("inf")
+    x[3, 7] = float("nan")
+    x[4] = 0
+    x[4, 9] = -3.0
+    x[5] = torch.from_numpy(oracle.wht_signs(D, 42)).to(dtype)          # one coordinate of the rotated row holds all of it
+    x[100:200] *= 1e-4 if dtype == torch.float16 else 1e-6
+    x = x.to(cuda)
+    table = oracle.boundaries_of(oracle.codebook(D, bits))
+    signs = oracle.wht_signs(D, 42)
+    scaled = signs * np.linspace(0.25, 8.0, D, dtype=np.float32)
+    for sg, bounds in ((signs, table), (signs, table * 0.02), (signs, table * 8.0), (scaled, table)):
+        packed, norms = kvc.turbo_encode(x, sg, bounds, bits)
+        for s in range(0, S, 8):
+            few, few_norms = kvc.turbo_encode(x[s:s + 8], sg, bounds, bits)
+            assert torch.equal(packed[s:s + 8], few) and torch.equal(norms[s:s + 8].view(torch.int32), few_norms.view(torch.int32))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("kw", [dict(bits=4), dict(bits=4, key_bits=3, value_bits=4), dict(bits=3),
                                 dict(bits=4, key_bits=0, value_bits=4), dict(bits=4, key_bits=8, value_bits=3),
