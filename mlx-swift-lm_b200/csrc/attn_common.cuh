@@ -5,6 +5,7 @@
 
 #include "common.h"
 
+#include <algorithm>
 #include <cstdlib>
 #include <utility>
 
@@ -365,6 +366,54 @@ __device__ __forceinline__ int flat_cta_of(const FlatPlan &f, int64_t x) {
     return (uint32_t)x < big ? flat_div(x, f.per + 1) : f.rem + flat_div((uint32_t)x - big, f.per);
 }
 
+// The same for units of one length, with the ends of the ranges where they cost least. A range that leaves one unit for the
+// next pays for another segment: queries turned and packed, warps folded, a partial, a ticket (v4 kernel, 64 units of nine
+// tiles on 148 CTAs: 11 000 .. 17 000 cycles, where a tile takes 2 050). So ranges are multiples of `step` tiles: 1
+// where equal ranges are the best, a piece of a unit (its tiles rounded up to whole pieces; a CTA stops at the `real`
+// ones) or a whole unit.
+struct UnitPlan {
+    int32_t tiles;     // tiles per unit, rounded up to whole steps
+    int32_t per, rem;  // CTA c owns (per + (c < rem)) * step tiles
+    int32_t nslots, red_rows;
+    int32_t step, real;
+};
+
+__device__ __forceinline__ int64_t flat_lo(const UnitPlan &f, int c) { return ((int64_t)c * f.per + min(c, f.rem)) * f.step; }
+__device__ __forceinline__ int flat_cta_of(const UnitPlan &f, int64_t x) {
+    const uint32_t xs = f.step == 1 ? (uint32_t)x : (uint32_t)x / (uint32_t)f.step, big = (uint32_t)f.rem * (uint32_t)(f.per + 1);
+    return xs < big ? flat_div(xs, f.per + 1) : f.rem + flat_div(xs - big, f.per);
+}
+
+// Plans `units` of `tiles` tiles over at most `slots` CTAs; `segment`: what a segment costs beside its tiles, in tiles.
+inline int64_t plan_units(UnitPlan *f, int64_t units, int64_t tiles, int64_t slots, int64_t segment) {
+    const int64_t work = units * tiles, n = std::min(slots, work), most = (work + n - 1) / n;
+    const bool even = work % n == 0;
+    const int64_t touched = even && tiles % most == 0 ? 1 : even && most % tiles == 0 ? most / tiles : (most + tiles - 2) / tiles + 1;
+    const int64_t cost = most + segment * touched;
+    f->real = (int32_t)tiles;
+    f->tiles = (int32_t)tiles;
+    f->step = 1;
+    f->per = (int32_t)(work / n);
+    f->rem = (int32_t)(work % n);
+    f->nslots = (int32_t)((tiles + f->per - 1) / f->per + 1);
+    if (units <= slots) {
+        const int64_t piece = (tiles + slots / units - 1) / (slots / units), pieces = (tiles + piece - 1) / piece;
+        if (piece + segment >= cost) return n;
+        f->tiles = (int32_t)(pieces * piece);
+        f->step = (int32_t)piece;
+        f->per = 1;
+        f->rem = 0;
+        f->nslots = (int32_t)pieces;
+        return units * pieces;
+    }
+    if ((units + slots - 1) / slots * (tiles + segment) >= cost) return n;
+    f->step = (int32_t)tiles;
+    f->per = (int32_t)(units / slots);
+    f->rem = (int32_t)(units % slots);
+    f->nslots = 1;
+    return slots;
+}
+
 // Barrier among the NW consumer warps only (the producer warp never joins it). Every consumer
 // warp reaches every one of these whether or not one of its bounded waits has run out.
 template <int NW>
@@ -423,8 +472,8 @@ __device__ __forceinline__ void rotate_out_rows(const UnitOut &u, const float *r
 // 64/8 heads, 4 bits: 145 us -> 130.
 // NBUF (default NW) is the number of warps that wrote cross-warp buffers: a kernel that has already
 // folded its NW warps down to NBUF of them passes the smaller count, all NW warps still take part.
-template <int D, int NW, int NBUF = NW>
-__device__ void segment_epilogue(const UnitOut &u, const FlatPlan &f, const float *red_o, const float *red_ml,
+template <int D, int NW, int NBUF = NW, typename Plan>
+__device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *red_o, const float *red_ml,
                                  int red_stride, float *work, int *flag, int unit, int b, int hk, int rep, int R,
                                  int64_t x_unit = -1, int unit_tiles = 0, int row0 = 0) {
     // row0: the unit covers the query rows row0 .. row0 + R - 1 of its (batch, kv head) group (a group

@@ -40,7 +40,7 @@ struct F32Params {
     float *o_part;
     float2 *ml_part;
     int *counters;
-    FlatPlan flat;
+    UnitPlan flat;
     int32_t B, Hq, Hkv, L, chunks, groups, causal;
     float scale_log2;
 };
@@ -111,7 +111,7 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
     pdl_wait();
     pdl_trigger();
 
-    const FlatPlan fp = p.flat;
+    const UnitPlan fp = p.flat;
     const int rep = p.Hq / p.Hkv, rows_all = rep * p.L, side = 4 * p.groups;   // scale bytes per token
     int64_t x = flat_lo(fp, blockIdx.x);
     const int64_t x_end = flat_lo(fp, blockIdx.x + 1);
@@ -393,6 +393,7 @@ int launch_attention_f32_list(const AttnArgs *args, int n, cudaStream_t stream) 
     if (!stream_plan(a0, n * units, work, most, a0.D <= 128 ? 2 : 1, std::min(rows, rn), &plan, (int64_t)n * a0.B * a0.Hq * a0.L, stream, &ctas))
         return 0;
     p.flat = plan.flat;
+    stream_list_tiles(list.seq, n, units, p.flat);
     p.o_part = plan.o_part; p.ml_part = plan.ml_part; p.counters = plan.counters;
     p.q_sh = a0.q_sh; p.q_sl = a0.q_sl; p.o_sh = a0.o_sh; p.o_sl = a0.o_sl;
     p.B = a0.B; p.Hq = a0.Hq; p.Hkv = a0.Hkv; p.L = a0.L;

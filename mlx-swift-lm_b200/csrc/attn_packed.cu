@@ -65,7 +65,7 @@ struct AffineParams {
     int32_t debug_skip;  // measurement aid: 1 = consumers release tiles without computing
     int64_t causal_offset;
     float scale_log2;
-    FlatPlan flat;  // decode8 kernel: flat tile decomposition
+    UnitPlan flat;  // decode8 kernel: flat tile decomposition
     int32_t q_bulk; // decode8 kernel: a unit's query rows are one contiguous 16-byte aligned block
     int32_t chunks; // decode8 kernel: units per (batch, kv head) = ceil(query rows of the group / 8); 1 for decode
 };
@@ -658,7 +658,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     // pointer + offset (no integer round trip) so that loads through it stay ld.shared
     unsigned char *stages = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     constexpr int RING = NSTAGE * STAGE_BYTES;
-    const FlatPlan &fp = p.flat;
+    const UnitPlan &fp = p.flat;
     uint64_t *full = (uint64_t *)(stages + ((RING + 15) / 16) * 16);
     uint64_t *empty = full + NSTAGE;
     int *is_last = (int *)(empty + NSTAGE);
@@ -710,7 +710,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
                 int unit, tb, utiles, hk, b;
                 resolve_unit<VARLEN, P8_TILE>(p, vt, x, tiles, unit, tb, utiles, hk, b);
-                const int n = (int)min((int64_t)(utiles - tb), x_hi - x);
+                const int own = (int)min((int64_t)(utiles - tb), x_hi - x), n = VARLEN ? own : min(own, fp.real - tb);
                 if (p.q_bulk) {
                     const int qb = sg & 1;
                     if (sg >= 2) ok = mbar_wait(&qempty[qb], ((sg >> 1) - 1) & 1);
@@ -753,7 +753,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                     bulk_load(st + 2 * CODE_TILE + 2 * SC_TILE, vs + t0 * G, rows * SB, &full[s]);
                     bulk_load(st + 2 * CODE_TILE + 3 * SC_TILE, vb + t0 * G, rows * SB, &full[s]);
                 }
-                x += n;
+                x += own;
             }
             if (!ok) atomicExch(p.status, 5);
         }
@@ -767,7 +767,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     for (int64_t x = x_lo; x < x_hi; ++sg) {
         int unit, tile_begin, utiles, hk, b;
         resolve_unit<VARLEN, P8_TILE>(p, vt, x, tiles, unit, tile_begin, utiles, hk, b);
-        const int ntiles = (int)min((int64_t)(utiles - tile_begin), x_hi - x);
+        const int own = (int)min((int64_t)(utiles - tile_begin), x_hi - x), ntiles = VARLEN ? own : min(own, fp.real - tile_begin);
         const int64_t T_seq = VARLEN ? (int64_t)vt.seq[b].T : p.T;   // tokens of this unit's sequence
         const int row0 = VARLEN ? 0 : (unit % p.chunks) * 8;         // first query row of the group this unit carries
         const int R = min(8, R_all - row0);
@@ -1092,7 +1092,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
         u.splits = 0; u.Hq = p.Hq; u.L = p.L;
         segment_epilogue<D, P8_WARPS>(u, fp, red_o, red_ml, RED_STRIDE, work, is_last, unit, b, hk, rep, R,
                                       x - tile_begin, utiles, row0);
-        x += ntiles;
+        x += own;
     }
 }
 
@@ -1167,6 +1167,9 @@ bool affine_source_fits(const KVSource &s, int D, int64_t T) {
 namespace {
 const VarlenAttnTable kNoVarlen = {};
 
+// What a segment of the decode8 kernel costs beside its tiles, in tiles (of 64 or 240 tokens).
+constexpr int P8_SEGMENT = 4;
+
 constexpr int affine8_stages(int D, int bits, bool varlen) {
     if (affine8_warps(D, bits, varlen) == 15) return 4;
     return bits == 4 ? (D == 128 ? 5 : 8) : (D == 128 ? 4 : 6);
@@ -1233,6 +1236,7 @@ int launch_attention_affine_varlen(const AttnArgs *args, int n, cudaStream_t str
     const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a0.device) * resident, work_tiles);
     AffineParams p = {};
     p.flat.tiles = (int)max_tiles;
+    p.flat.step = 1;
     p.flat.per = (int)(work_tiles / ctas);
     p.flat.rem = (int)(work_tiles % ctas);
     p.flat.nslots = (int)((max_tiles + p.flat.per - 1) / p.flat.per + 1);
@@ -1308,7 +1312,7 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     const bool decode8 = (rep * a.L <= 8 || chunks > 1) && pairs_fit;
     const int64_t tile8 = affine8_warps(a.D, a.k.bits, false) * 16;
     const int64_t tiles = decode8 ? (a.T + tile8 - 1) / tile8 : (a.T + PK_TILE - 1) / PK_TILE;
-    if (!flat_fits(bh * tiles)) return 0;
+    if (!flat_fits(2 * bh * tiles)) return 0;
     // resident CTAs per SM (a fourth CTA fits the 4-bit kernels at 94 registers but measured slower)
     const int slots = sm_count(a.device) * (decode8 ? 3 : 2);
     int64_t best_s = 1;
@@ -1329,11 +1333,10 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     }
     // decode8: flat decomposition over one wave of resident CTAs (every CTA streams the same number
     // of tiles); the partial slots per unit take the place of the splits
-    const int64_t work_tiles = bh * tiles;
     const int flat_resident = affine_resident_ctas(a.D, a.k.bits, a.k.group, std::min(8, rep * a.L), false);
-    const int64_t flat_ctas = std::min<int64_t>((int64_t)sm_count(a.device) * flat_resident, work_tiles);
-    const int64_t flat_per = work_tiles / flat_ctas, flat_rem = work_tiles % flat_ctas;
-    const int64_t flat_slots = (tiles + flat_per - 1) / flat_per + 1;
+    UnitPlan plan;
+    const int64_t flat_ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * flat_resident, P8_SEGMENT);
+    const int64_t flat_slots = plan.nslots;
     if (decode8 && flat_slots > 64) return 0;
     const int64_t splits = decode8 ? flat_slots : best_s;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
@@ -1360,9 +1363,8 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     p.debug_skip = measure_skip_bits();
     p.causal_offset = a.mask.causal_offset;
     p.scale_log2 = a.scale * 1.4426950408889634f;
-    p.flat.tiles = (int)tiles;
-    p.flat.per = (int)flat_per; p.flat.rem = (int)flat_rem;
-    p.flat.nslots = (int)flat_slots; p.flat.red_rows = decode8 ? std::min(8, rep * a.L) : rep * a.L;
+    p.flat = plan;
+    p.flat.red_rows = decode8 ? std::min(8, rep * a.L) : rep * a.L;
     p.chunks = chunks;
     p.q_bulk = (chunks == 1 && a.L == 1 && a.q_sh == a.D && ((uintptr_t)a.q & 15) == 0 && (a.q_sb * 2) % 16 == 0) ? 1 : 0;
     const int units = decode8 ? (int)flat_ctas : (int)(bh * splits);

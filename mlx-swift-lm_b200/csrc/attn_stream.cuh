@@ -30,7 +30,7 @@
 //     kernel, 89 us here (114 with the values through the tile and a load for each half); with single f16 operands the
 //     outputs no longer err by the store's rounding alone.
 //   * The running reference is only moved when a score (with its value factor) passes it by more than 2^3.
-// Work is cut into equal ranges of 64-token tiles per resident CTA (FlatPlan), units that cross a CTA boundary
+// Work is cut into equal ranges of 64-token tiles per resident CTA (UnitPlan), units that cross a CTA boundary
 // are merged by segment_epilogue.
 #pragma once
 
@@ -47,6 +47,7 @@ using namespace dev;
 
 constexpr int ST_TILE = 64;        // tokens per tile of the flat plan
 constexpr int ST_STAGES = 2;       // packed 16-token blocks per warp: one in use, one on its way
+constexpr int ST_SEGMENT = 8;      // what a segment costs beside its tiles, in tiles
 constexpr int ST_COUNTER_BYTES = 64 * 1024;
 constexpr float ST_LAZY = 3.f;     // log2 of how far a score may pass the running maximum
 constexpr float ST_PSCALE = 1024.f;  // P * factor (at most 2^3) is carried 2^10 up: its low half stays clear of f16 subnormals
@@ -101,7 +102,7 @@ struct StreamParams {
     float *o_part;
     float2 *ml_part;
     int *counters;
-    FlatPlan flat;
+    UnitPlan flat;
     int32_t B, Hq, Hkv, L, T;
     int32_t groups_k, groups_v;           // affine groups per row
     int32_t chunks;                       // row blocks per KV head
@@ -341,7 +342,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
     pdl_wait();
     pdl_trigger();
 
-    const FlatPlan fp = p.flat;
+    const UnitPlan fp = p.flat;
     const int rep = p.Hq / p.Hkv, rows_all = rep * p.L;
     int64_t x = flat_lo(fp, blockIdx.x);
     const int64_t x_end = flat_lo(fp, blockIdx.x + 1);
@@ -967,12 +968,19 @@ struct StreamPick {
 // The flat plan over `work` tiles, `max_tiles` in the longest unit; false when the partials need too many slots.
 inline bool stream_plan(const AttnArgs &a, int64_t units, int64_t work, int64_t max_tiles, int resident, int rows, StreamParams *p,
                  int64_t qrows, cudaStream_t stream, int *ctas) {
-    if (units * (int64_t)sizeof(int) > ST_COUNTER_BYTES || !flat_fits(work)) return false;
-    const int64_t n = std::min<int64_t>((int64_t)sm_count(a.device) * resident, work);
-    p->flat.tiles = (int)max_tiles;
-    p->flat.per = (int)(work / n);
-    p->flat.rem = (int)(work % n);
-    p->flat.nslots = (int)((max_tiles + p->flat.per - 1) / p->flat.per + 1);
+    if (units * (int64_t)sizeof(int) > ST_COUNTER_BYTES || !flat_fits(2 * units * max_tiles)) return false;
+    const int64_t slots = (int64_t)sm_count(a.device) * resident;
+    int64_t n;
+    if (work == units * max_tiles) {
+        n = plan_units(&p->flat, units, max_tiles, slots, ST_SEGMENT);
+    } else {
+        n = std::min(slots, work);
+        p->flat.tiles = (int)max_tiles;
+        p->flat.step = 1;
+        p->flat.per = (int)(work / n);
+        p->flat.rem = (int)(work % n);
+        p->flat.nslots = (int)((max_tiles + p->flat.per - 1) / p->flat.per + 1);
+    }
     p->flat.red_rows = rows;
     const size_t o_bytes = (size_t)qrows * p->flat.nslots * a.D * sizeof(float);
     char *scratch = (char *)scratch_get(a.device, o_bytes + (size_t)qrows * p->flat.nslots * sizeof(float2) + 256, stream);
@@ -981,6 +989,16 @@ inline bool stream_plan(const AttnArgs &a, int64_t units, int64_t work, int64_t 
     p->counters = counters_get(a.device, stream, ST_COUNTER_BYTES);
     *ctas = (int)n;
     return true;
+}
+
+// The tiles of a list's calls where the plan has rounded them up (then all calls have as many).
+template <typename Seq>
+inline void stream_list_tiles(Seq *seq, int n, int64_t units, const UnitPlan &f) {
+    if (f.step == 1) return;
+    for (int i = 0; i < n; ++i) {
+        seq[i].tiles = f.tiles;
+        seq[i].tile_first = i * units * f.tiles;
+    }
 }
 
 // One call (list null) or a list of calls of one shape in one launch.
@@ -1004,6 +1022,7 @@ int run_stream(const AttnArgs &a, StreamParams p, StreamList *list, cudaStream_t
     if (!stream_plan(a, n * units, work, most, StreamShape<T, D, KK, VK, UNIT, NB, false>::RESIDENT, std::min(rows, 8 * NB), &p,
                      (int64_t)n * a.B * a.Hq * a.L, stream, &ctas))
         return 0;
+    if (list) stream_list_tiles(list->seq, n, units, p.flat);
     if (list) launch_stream_typed<T, D, KK, VK, UNIT, NB, true>(p, list, ctas, stream);
     else launch_stream_typed<T, D, KK, VK, UNIT, NB, false>(p, nullptr, ctas, stream);
     return 1;

@@ -40,6 +40,7 @@ using namespace dev;
 constexpr int TQ_WARPS = 4;
 constexpr int TQ_THREADS = (TQ_WARPS + 1) * 32;
 constexpr int TQ_TILE = 64;
+constexpr int TQ_SEGMENT = 6;            // what a segment costs beside its tiles, in tiles
 constexpr int TQ_D = 128;
 constexpr int TQ_COUNTER_BYTES = 64 * 1024;
 
@@ -66,7 +67,7 @@ struct TurboParams {
     int32_t debug_skip;  // measurement aid: 1 = consumers release tiles without computing
     int64_t causal_offset;
     float scale_log2;
-    FlatPlan flat;  // flat tile decomposition (one wave of CTAs, segments per unit)
+    UnitPlan flat;  // flat tile decomposition (one wave of CTAs, segments per unit)
     int32_t q_bulk; // a unit's query rows are one contiguous 16-byte aligned block
 };
 
@@ -123,7 +124,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
     float *qrot = (float *)(vtab + VTAB);               // [8][D]
     unsigned char *stages = (unsigned char *)(qrot + 8 * D);
     constexpr int RING = NSTAGE * STAGE_BYTES;
-    const FlatPlan &fp = p.flat;
+    const UnitPlan &fp = p.flat;
     uint64_t *full = (uint64_t *)(stages + ((RING + 15) / 16) * 16);
     uint64_t *empty = full + NSTAGE;
     int *is_last = (int *)(empty + NSTAGE);
@@ -176,7 +177,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
             int it = 0, sg = 0;
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
                 const int unit = flat_div(x, tiles), tb = flat_mod(x, tiles, unit);
-                const int n = (int)min((int64_t)(tiles - tb), x_hi - x);
+                const int own = (int)min((int64_t)(tiles - tb), x_hi - x), n = min(own, fp.real - tb);
                 const int hk = unit % p.Hkv, b = unit / p.Hkv;
                 if (p.q_bulk) {
                     const int qb = sg & 1;
@@ -202,7 +203,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
                     bulk_load(st + K_TILE + V_TILE, kn + t0, N_TILE, &full[s]);
                     bulk_load(st + K_TILE + V_TILE + N_TILE, vn + t0, N_TILE, &full[s]);
                 }
-                x += n;
+                x += own;
             }
             if (!ok) atomicExch(p.status, 7);
         }
@@ -216,7 +217,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
     int sg = 0;
     for (int64_t x = x_lo; x < x_hi; ++sg) {
         const int unit = flat_div(x, tiles), tile_begin = flat_mod(x, tiles, unit);
-        const int ntiles = (int)min((int64_t)(tiles - tile_begin), x_hi - x);
+        const int own = (int)min((int64_t)(tiles - tile_begin), x_hi - x), ntiles = min(own, fp.real - tile_begin);
         const int hk = unit % p.Hkv, b = unit / p.Hkv;
         // ---- rotated queries of this unit: q' = H(signs * q) / sqrt(D) * scale * log2(e), rows past R zero ----
         const T *q_stage = nullptr;
@@ -439,7 +440,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
         u.o_signs = p.o_signs;
         u.splits = 0; u.Hq = p.Hq; u.L = p.L;
         segment_epilogue<D, TQ_WARPS>(u, fp, red_o, red_ml, RED_STRIDE, work, is_last, unit, b, hk, rep, R);
-        x += ntiles;
+        x += own;
     }
 }
 
@@ -452,7 +453,7 @@ constexpr size_t turbo_fixed_smem() {
     return (size_t)KTAB + VTAB + 8 * D * 4 + (size_t)NSTAGE * STAGE_BYTES + 16 + 2 * NSTAGE * sizeof(uint64_t) + 64 + 128;
 }
 
-inline size_t turbo_red_smem(const FlatPlan &f) {
+inline size_t turbo_red_smem(const UnitPlan &f) {
     return (size_t)TQ_WARPS * f.red_rows * (TQ_D + 8) * 4 + (size_t)TQ_WARPS * f.red_rows * 8 +
            (size_t)f.red_rows * f.nslots * 4 + (size_t)f.red_rows * TQ_D * 4 + 4 * sizeof(uint64_t) +
            (size_t)2 * f.red_rows * TQ_D * 2 + 16;
@@ -535,18 +536,13 @@ int launch_attention_turbo(const AttnArgs &a, cudaStream_t stream) {
     else if (kb == 4 && vb == 2) fixed = turbo_fixed_smem<4, 2, 7>();
     else if (kb == 3 && vb == 3) fixed = turbo_fixed_smem<3, 3, 7>();
     else fixed = turbo_fixed_smem<2, 2, 10>();
-    FlatPlan plan;
-    plan.tiles = (int)tiles;
+    UnitPlan plan;
     plan.red_rows = rep * a.L;
     plan.nslots = 64;
     const size_t per_cta = fixed + turbo_red_smem(plan) + 1024;
     const int resident = (int)std::max<size_t>(1, std::min<size_t>(2, (size_t)227 * 1024 / per_cta));
-    const int64_t work_tiles = bh * tiles;
-    if (!flat_fits(work_tiles)) return 0;
-    const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a.device) * resident, work_tiles);
-    plan.per = (int)(work_tiles / ctas);
-    plan.rem = (int)(work_tiles % ctas);
-    plan.nslots = (int)((tiles + plan.per - 1) / plan.per + 1);
+    if (!flat_fits(2 * bh * tiles)) return 0;
+    const int64_t ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * resident, TQ_SEGMENT);
     if (plan.nslots > 64) return 0;
     const int64_t splits = plan.nslots;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;

@@ -56,6 +56,7 @@ constexpr int V4_GROUPS = 1;                       // warp groups; group i takes
 constexpr int V4_PRODUCERS = KVC_V4_PRODUCERS;     // producer warps: 4 = one per array of a stage, 1 = lanes 0..3 issue them
 constexpr int V4_THREADS = (V4_WARPS + V4_PRODUCERS) * 32;
 constexpr int V4_TILE = 16 * V4_GW;                // tokens per ring stage
+constexpr int V4_SEGMENT = 5;                     // what a segment costs beside its tiles, in tiles
 constexpr int V4_D = 128;
 constexpr int V4_VW = 16;                         // value words per row (4 bits)
 constexpr int V4_MAX_STAGES = 12;                 // of 64 tokens; fewer when a stage is larger
@@ -87,7 +88,7 @@ struct TurboV4Params {
     int32_t out_dtype;
     int64_t causal_offset;
     float scale_log2;
-    FlatPlan flat;
+    UnitPlan flat;
     int32_t q_bulk;      // a unit's query rows are one contiguous 16-byte aligned block
     uint32_t smem_bytes; // dynamic shared memory of the launch
     int32_t debug_skip;  // measurement builds only (KVC_SKIP_BITS): 1 = consumers release stages without computing
@@ -155,7 +156,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
     static_assert(K_TILE % 16 == 0 && STAGE_BYTES % 128 == 0, "bulk copies need 16-byte multiples");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const FlatPlan &fp = p.flat;
+    const UnitPlan &fp = p.flat;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     // ---- shared-memory plan: the table sits on the first 64 KB boundary of the shared window at or
@@ -251,7 +252,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
             int it = 0, sg = 0;
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
                 const int unit = flat_div(x, tiles), tb = flat_mod(x, tiles, unit);
-                const int n = (int)min((int64_t)(tiles - tb), x_hi - x);
+                const int own = (int)min((int64_t)(tiles - tb), x_hi - x), n = min(own, fp.real - tb);
                 const int bh = CHUNKED ? unit / p.chunks : unit;
                 const int hk = bh % p.Hkv, b = bh / p.Hkv;
                 if (p.q_bulk && pw == 0) {
@@ -281,7 +282,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
                     mbar_expect_tx(&full[s], bytes);
                     bulk_load(stages + (size_t)s * STAGE_BYTES + dst_off, src + t0 * per_token, bytes, &full[s]);
                 }
-                x += n;
+                x += own;
             }
             if (!ok) atomicExch(p.status, 32);
         }
@@ -305,7 +306,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
     int sg = 0;
     for (int64_t x = x_lo; x < x_hi; ++sg) {
         const int unit = flat_div(x, tiles), tile_begin = flat_mod(x, tiles, unit);
-        const int ntiles = (int)min((int64_t)(tiles - tile_begin), x_hi - x);
+        const int own = (int)min((int64_t)(tiles - tile_begin), x_hi - x), ntiles = min(own, fp.real - tile_begin);
         const int bh = CHUNKED ? unit / p.chunks : unit, row0 = CHUNKED ? (unit % p.chunks) * 8 : 0;
         const int hk = bh % p.Hkv, b = bh / p.Hkv;
         const int R = CHUNKED ? min(8, R_all - row0) : R_all;
@@ -600,7 +601,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
         u.o_signs = p.o_signs;
         u.splits = 0; u.Hq = p.Hq; u.L = p.L;
         segment_epilogue<D, V4_WARPS, 4>(u, fp, red_o, red_ml, V4_RED_STRIDE, work, is_last, unit, b, hk, rep, R, -1, 0, row0);
-        x += ntiles;
+        x += own;
     }
 }
 
@@ -659,15 +660,10 @@ int launch_attention_turbo_v4(const AttnArgs &a, cudaStream_t stream) {
     int *counters = counters_get(a.device, stream, V4_COUNTER_BYTES);
 
     const int64_t tiles = (a.T + V4_TILE - 1) / V4_TILE;
-    FlatPlan plan;
-    plan.tiles = (int)tiles;
+    UnitPlan plan;
     plan.red_rows = std::min(8, rep * a.L);
-    const int64_t work_tiles = bh * tiles;
-    if (!flat_fits(work_tiles)) return 0;
-    const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a.device), work_tiles);
-    plan.per = (int)(work_tiles / ctas);
-    plan.rem = (int)(work_tiles % ctas);
-    plan.nslots = (int)((tiles + plan.per - 1) / plan.per + 1);
+    if (!flat_fits(2 * bh * tiles)) return 0;
+    const int64_t ctas = plan_units(&plan, bh, tiles, sm_count(a.device), V4_SEGMENT);
     if (plan.nslots > 64) return 0;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
     const size_t o_bytes = (size_t)qrows * plan.nslots * a.D * sizeof(float);
