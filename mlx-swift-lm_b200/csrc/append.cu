@@ -24,8 +24,8 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
 template <typename V>
 __global__ void append_kernel(AppendArgs a, int64_t k_units, int64_t total_units,
                               int k_upr, int v_upr /* units per row */) {
-    // lets a dependent kernel launched with programmatic serialization begin its prologue now
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total_units) return;
     const bool is_v = i >= k_units;
@@ -58,7 +58,8 @@ struct AppendList {
     AppendArgs a[KVC_LIST_MAX];
 };
 __global__ void append_list_kernel(const __grid_constant__ AppendList l, int k_units, int total_units, int k_upr, int v_upr) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const AppendArgs &a = l.a[blockIdx.y];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total_units) return;
@@ -80,6 +81,8 @@ __global__ void append_list_kernel(const __grid_constant__ AppendList l, int k_u
 // are not 16-byte aligned.
 template <typename E>
 __global__ void append_strided_kernel(AppendArgs a, int64_t k_elems, int64_t total) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const bool is_v = i >= k_elems;
@@ -173,6 +176,8 @@ template <typename V> __device__ __forceinline__ void gather_unit(const GatherAr
 
 template <typename V>
 __global__ void gather_kernel(GatherArgs a, int64_t total_units, int upr, int64_t rows_per_bh) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total_units) return;
     const int u = (int)(i % upr);
@@ -186,6 +191,8 @@ __global__ void gather_kernel(GatherArgs a, int64_t total_units, int upr, int64_
 // 4 x 1 heads x 512 rows of D 256, a launch each.
 __global__ void gather_pair_kernel(const __grid_constant__ GatherArgs k, const __grid_constant__ GatherArgs v, uint32_t total_units,
                                    uint32_t upr, uint32_t rows_per_bh) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total_units) return;
     const uint32_t u = i % upr, row = i / upr, j = row % rows_per_bh, bh = row / rows_per_bh;
@@ -193,6 +200,8 @@ __global__ void gather_pair_kernel(const __grid_constant__ GatherArgs k, const _
 }
 
 __global__ void causal_mask_kernel(uint8_t *out, int64_t n, int64_t offset, int64_t window) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     // createCausalMask (KVCache.swift:253-275): rows are absolute positions
     // offset..offset+n-1, columns 0..offset+n-1; keep when row >= col and,
     // with a window, row < col + window.
@@ -210,6 +219,8 @@ __global__ void causal_mask_kernel(uint8_t *out, int64_t n, int64_t offset, int6
 // (createCausalMask's `lengths` argument, KVCache.swift:268-271). out: [batch, 1, n, offset + n].
 __global__ void causal_mask_lengths_kernel(uint8_t *out, int64_t n, int64_t offset, int64_t window,
                                            const int32_t *lengths, int64_t total) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const int64_t cols = offset + n;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
@@ -223,6 +234,8 @@ __global__ void causal_mask_lengths_kernel(uint8_t *out, int64_t n, int64_t offs
 }
 
 __global__ void rolled_mask_kernel(uint8_t *out, int64_t size, int64_t window, int64_t shift) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     // RotatingKVCache.makeMask single-token branch (KVCache.swift:861-865):
     // mask[i] = i >= size - window, rolled right by `shift`.
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -258,7 +271,7 @@ bool launch_append_list(const AppendArgs *args, int n, cudaStream_t stream) {
         if (a.B != a0.B || a.H != a0.H || a.S != a0.S || a.Dk != a0.Dk || a.Dv != a0.Dv || a.esize != a0.esize || !append_vectors(a)) return false;
         l.a[i] = a;
     }
-    append_list_kernel<<<dim3((unsigned)((total + 255) / 256), (unsigned)n), 256, 0, stream>>>(l, (int)(rows * k_upr), (int)total, (int)k_upr, (int)v_upr);
+    KVC_CUDA(launch_pdl(append_list_kernel, dim3((unsigned)((total + 255) / 256), (unsigned)n), dim3(256), 0, stream, l, (int)(rows * k_upr), (int)total, (int)k_upr, (int)v_upr));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
     return true;
@@ -274,14 +287,14 @@ void launch_append(const AppendArgs &a, cudaStream_t stream) {
         const int k_upr = (int)(kb / 16), v_upr = (int)(vb / 16);
         const int64_t k_units = rows * k_upr, total = k_units + rows * v_upr;
         const int64_t blocks = (total + threads - 1) / threads;
-        append_kernel<uint4><<<(unsigned)blocks, threads, 0, stream>>>(a, k_units, total, k_upr, v_upr);
+        KVC_CUDA(launch_pdl(append_kernel<uint4>, dim3((unsigned)blocks), dim3(threads), 0, stream, a, k_units, total, k_upr, v_upr));
     } else {
         const int64_t k_elems = rows * a.Dk, total = k_elems + rows * a.Dv;
         const int64_t blocks = (total + threads - 1) / threads;
         if (a.esize == 2)
-            append_strided_kernel<uint16_t><<<(unsigned)blocks, threads, 0, stream>>>(a, k_elems, total);
+            KVC_CUDA(launch_pdl(append_strided_kernel<uint16_t>, dim3((unsigned)blocks), dim3(threads), 0, stream, a, k_elems, total));
         else if (a.esize == 4)
-            append_strided_kernel<uint32_t><<<(unsigned)blocks, threads, 0, stream>>>(a, k_elems, total);
+            KVC_CUDA(launch_pdl(append_strided_kernel<uint32_t>, dim3((unsigned)blocks), dim3(threads), 0, stream, a, k_elems, total));
         else
             fail(KVC_ERR_INVALID_ARG, "append: unsupported element size");
     }
@@ -292,6 +305,8 @@ void launch_append(const AppendArgs &a, cudaStream_t stream) {
 namespace {
 // y = array, x = 16-byte pieces of the tails of its planes; pieces that straddle an end go by half words
 __global__ void zero_tails_kernel(const __grid_constant__ ZeroTails z) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const auto &t = z.tail[blockIdx.y];
     const int64_t first = t.from & ~(int64_t)15, per_plane = (t.pitch - first + 15) >> 4;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per_plane * t.planes; i += (int64_t)gridDim.x * blockDim.x) {
@@ -306,6 +321,8 @@ __global__ void zero_tails_kernel(const __grid_constant__ ZeroTails z) {
 }
 struct Floats { float v[1024 - 16]; };
 __global__ void store_floats_kernel(float *dst, const __grid_constant__ Floats f, int n) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = f.v[i];
 }
 }  // namespace
@@ -315,7 +332,7 @@ void launch_zero_tails(const ZeroTails &z, cudaStream_t stream) {
     int64_t most = 0;
     for (int i = 0; i < z.n; ++i) most = std::max<int64_t>(most, (z.tail[i].pitch - z.tail[i].from + 31) / 16 * z.tail[i].planes);
     if (most <= 0) return;
-    zero_tails_kernel<<<dim3((unsigned)std::min<int64_t>((most + 255) / 256, 1184), (unsigned)z.n), 256, 0, stream>>>(z);
+    KVC_CUDA(launch_pdl(zero_tails_kernel, dim3((unsigned)std::min<int64_t>((most + 255) / 256, 1184), (unsigned)z.n), dim3(256), 0, stream, z));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }
@@ -326,7 +343,7 @@ void launch_store_floats(float *dst, const float *src, int n, cudaStream_t strea
         Floats f;
         const int m = std::min(n - at, MOST);
         std::memcpy(f.v, src + at, (size_t)m * sizeof(float));
-        store_floats_kernel<<<1, 256, 0, stream>>>(dst + at, f, m);
+        KVC_CUDA(launch_pdl(store_floats_kernel, dim3(1), dim3(256), 0, stream, dst + at, f, m));
         KVC_CUDA(cudaGetLastError());
         ++g_launch_count;
     }
@@ -355,7 +372,7 @@ void launch_gather_pair(const GatherArgs &k, const GatherArgs &v, cudaStream_t s
         launch_gather(v, stream);
         return;
     }
-    gather_pair_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, stream>>>(k, v, (uint32_t)total, (uint32_t)upr, (uint32_t)tokens);
+    KVC_CUDA(launch_pdl(gather_pair_kernel, dim3((unsigned)((total + 255) / 256), 2), dim3(256), 0, stream, k, v, (uint32_t)total, (uint32_t)upr, (uint32_t)tokens));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }
@@ -370,20 +387,20 @@ void launch_gather(const GatherArgs &a, cudaStream_t stream) {
     if (vec) {
         const int upr = (int)(rb / 16);
         const int64_t total = rows * upr;
-        gather_kernel<uint4><<<(unsigned)((total + threads - 1) / threads), threads, 0, stream>>>(
-            a, total, upr, rows_per_bh);
+        KVC_CUDA(launch_pdl(gather_kernel<uint4>, dim3((unsigned)((total + threads - 1) / threads)), dim3(threads), 0, stream, 
+            a, total, upr, rows_per_bh));
     } else if (rb % 4 == 0 && ((uintptr_t)a.src & 3) == 0 && ((uintptr_t)a.dst & 3) == 0 &&
                (a.esize == 4 || (a.s_sb % 2 == 0 && a.s_sh % 2 == 0 && a.s_st % 2 == 0 &&
                                  a.d_sb % 2 == 0 && a.d_sh % 2 == 0 && a.d_st % 2 == 0))) {
         const int upr = (int)(rb / 4);
         const int64_t total = rows * upr;
-        gather_kernel<uint32_t><<<(unsigned)((total + threads - 1) / threads), threads, 0, stream>>>(
-            a, total, upr, rows_per_bh);
+        KVC_CUDA(launch_pdl(gather_kernel<uint32_t>, dim3((unsigned)((total + threads - 1) / threads)), dim3(threads), 0, stream, 
+            a, total, upr, rows_per_bh));
     } else if (a.esize == 2) {
         const int upr = (int)(rb / 2);
         const int64_t total = rows * upr;
-        gather_kernel<uint16_t><<<(unsigned)((total + threads - 1) / threads), threads, 0, stream>>>(
-            a, total, upr, rows_per_bh);
+        KVC_CUDA(launch_pdl(gather_kernel<uint16_t>, dim3((unsigned)((total + threads - 1) / threads)), dim3(threads), 0, stream, 
+            a, total, upr, rows_per_bh));
     } else {
         fail(KVC_ERR_INVALID_ARG, "gather: unsupported row layout");
     }
@@ -413,7 +430,7 @@ void launch_rope(const RopeArgs &a, cudaStream_t s) {
 void launch_causal_mask(uint8_t *out, int64_t n, int64_t offset, int64_t window, cudaStream_t s) {
     const int64_t total = n * (offset + n);
     if (total <= 0) return;
-    causal_mask_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(out, n, offset, window);
+    KVC_CUDA(launch_pdl(causal_mask_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, out, n, offset, window));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }
@@ -422,14 +439,14 @@ void launch_causal_mask_lengths(uint8_t *out, int64_t n, int64_t offset, int64_t
                                 int64_t batch, cudaStream_t s) {
     const int64_t total = batch * n * (offset + n);
     if (total <= 0) return;
-    causal_mask_lengths_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(out, n, offset, window, lengths, total);
+    KVC_CUDA(launch_pdl(causal_mask_lengths_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, out, n, offset, window, lengths, total));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }
 
 void launch_rolled_mask(uint8_t *out, int64_t size, int64_t window, int64_t shift, cudaStream_t s) {
     if (size <= 0) return;
-    rolled_mask_kernel<<<(unsigned)((size + 255) / 256), 256, 0, s>>>(out, size, window, shift);
+    KVC_CUDA(launch_pdl(rolled_mask_kernel, dim3((unsigned)((size + 255) / 256)), dim3(256), 0, s, out, size, window, shift));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }

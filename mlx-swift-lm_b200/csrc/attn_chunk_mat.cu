@@ -75,6 +75,8 @@ struct MatParams {
 constexpr int MAT_ROWS = 4;
 template <typename T, typename TO, int D, bool TURBO>
 __global__ void __launch_bounds__(256) materialize_kernel(const __grid_constant__ MatParams p) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     constexpr int PER_ROW = D / 8, STEP = 256 / PER_ROW;
     __shared__ float table[TURBO ? 16 * 32 : 1];
     const int which = blockIdx.z & 1, b = blockIdx.z >> 1, h = blockIdx.y;
@@ -134,8 +136,8 @@ __global__ void __launch_bounds__(256) materialize_kernel(const __grid_constant_
 template <typename T, bool TURBO> void materialize(const MatParams &p, cudaStream_t stream) {
     const int per_block = 256 / (p.D / 8) * MAT_ROWS;
     const dim3 grid((unsigned)((p.T + per_block - 1) / per_block), (unsigned)p.H, (unsigned)(2 * p.B));
-    if (p.D == 128) materialize_kernel<T, T, 128, TURBO><<<grid, 256, 0, stream>>>(p);
-    else materialize_kernel<T, T, 64, TURBO><<<grid, 256, 0, stream>>>(p);
+    if (p.D == 128) KVC_CUDA(launch_pdl(materialize_kernel<T, T, 128, TURBO>, grid, dim3(256), 0, stream, p));
+    else KVC_CUDA(launch_pdl(materialize_kernel<T, T, 64, TURBO>, grid, dim3(256), 0, stream, p));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }
@@ -153,6 +155,8 @@ struct RotParams {
 // out[row] = post * H(pre * in[row]) / sqrt(D), one warp per row, lane l holds dims E*l .. E*l + E - 1.
 template <typename TI, typename TO, int D>
 __global__ void __launch_bounds__(256) rotate_rows_kernel(const __grid_constant__ RotParams p) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     constexpr int E = D / 32;
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -220,8 +224,8 @@ template <typename TI, typename TO>
 void rotate_rows(const RotParams &p, int D, cudaStream_t stream) {
     const int64_t rows = (int64_t)p.B * p.H * p.L;
     const unsigned blocks = (unsigned)((rows + 7) / 8);
-    if (D == 128) rotate_rows_kernel<TI, TO, 128><<<blocks, 256, 0, stream>>>(p);
-    else rotate_rows_kernel<TI, TO, 64><<<blocks, 256, 0, stream>>>(p);
+    if (D == 128) KVC_CUDA(launch_pdl(rotate_rows_kernel<TI, TO, 128>, dim3(blocks), dim3(256), 0, stream, p));
+    else KVC_CUDA(launch_pdl(rotate_rows_kernel<TI, TO, 64>, dim3(blocks), dim3(256), 0, stream, p));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }

@@ -594,7 +594,12 @@ __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *r
 }  // namespace dev
 
 // Launch with programmatic stream serialization (see dev::pdl_wait). KVC_NO_PDL=1 falls
-// back to a plain launch.
+// back to a plain launch. The small kernels in front of an attention kernel (appends, quantisers, encoders, gathers) are
+// launched so too, wait first and release their successors after the wait: a plain launch behind a programmatic one
+// started at multiples of 2.05 us behind the one before (steps of an affine or compressed cache took n * 2.05 us a layer),
+// a chain of programmatic ones starts at once: 18.5 -> 14.6 us for rotary, append and attention of 64/8 heads over 64 .. 300
+// tokens, 8 bits. Kernels that hold TMEM release nobody early: the successor's CTAs could take columns that a CTA
+// of theirs has yet to allocate, and wait for it.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args &&...args) {

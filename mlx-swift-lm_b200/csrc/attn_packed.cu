@@ -174,6 +174,7 @@ attn_affine_kernel(const AffineParams p) {
     }
     __syncthreads();
     pdl_wait();  // everything below reads what earlier kernels on the stream wrote
+    pdl_trigger();
 
     bool ok = true;
     const int g = lane >> 2, c = lane & 3;
@@ -699,6 +700,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     }
     __syncthreads();
     pdl_wait();  // everything below reads what earlier kernels on the stream wrote
+    pdl_trigger();
 
     bool ok = true;
     const int g = lane >> 2, c = lane & 3;

@@ -167,6 +167,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
     }
     __syncthreads();
     pdl_wait();  // the tables came from kernel parameters; everything below reads global memory
+    pdl_trigger();
 
     bool ok = true;
     const int g = lane >> 2, c = lane & 3;

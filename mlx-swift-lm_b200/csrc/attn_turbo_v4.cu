@@ -235,6 +235,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
     }
     __syncthreads();
     pdl_wait();  // the tables came from kernel parameters; everything below reads global memory
+    pdl_trigger();
 
     bool ok = true;
 

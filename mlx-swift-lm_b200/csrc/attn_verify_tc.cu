@@ -740,6 +740,8 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 
 // Units cut by a CTA boundary: out[row] = sum_s o_s 2^(m_s - m) / sum_s l_s 2^(m_s - m) over the unit's pieces.
 __global__ void __launch_bounds__(128) verify_merge_kernel(const __grid_constant__ VerifyParams p) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const int unit = blockIdx.x / p.R, row = blockIdx.x % p.R, d = threadIdx.x;
     const int hk = unit % p.Hkv, b = unit / p.Hkv, rep = p.Hq / p.Hkv;
     const int n_all = (int)((p.T + TC_KEYS - 1) / TC_KEYS);
@@ -780,6 +782,8 @@ struct QPadParams {
 // position r % L; out = calib * H(signs * q) / sqrt(D) in f16, rows past R zero. One warp per row.
 template <typename T>
 __global__ void __launch_bounds__(256) verify_q_kernel(const __grid_constant__ QPadParams p) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     constexpr int D = VT_D, E = D / 32;
     const int lane = threadIdx.x & 31;
     const int64_t gr = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -821,6 +825,8 @@ __global__ void __launch_bounds__(256) verify_q_kernel(const __grid_constant__ Q
 // tiles (affine_dim_of; p.perm_bits = the code bits). One thread per eight dims.
 template <typename T>
 __global__ void __launch_bounds__(256) verify_q_plain_kernel(const __grid_constant__ QPadParams p) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     constexpr int D = VT_D;
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t units = (int64_t)p.B * p.Hkv;
@@ -929,8 +935,8 @@ int launch_attention_verify_tc(const AttnArgs &a, cudaStream_t stream) {
     qp.B = a.B; qp.Hq = a.Hq; qp.Hkv = a.Hkv; qp.L = a.L; qp.R = R;
     qp.signs = a.q_signs; qp.calib = a.q_calib;
     const unsigned qblocks = (unsigned)((units * TC_ROWS + 7) / 8);
-    if (a.q_dtype == KVC_BF16) verify_q_kernel<__nv_bfloat16><<<qblocks, 256, 0, stream>>>(qp);
-    else verify_q_kernel<__half><<<qblocks, 256, 0, stream>>>(qp);
+    if (a.q_dtype == KVC_BF16) KVC_CUDA(launch_pdl(verify_q_kernel<__nv_bfloat16>, dim3(qblocks), dim3(256), 0, stream, qp));
+    else KVC_CUDA(launch_pdl(verify_q_kernel<__half>, dim3(qblocks), dim3(256), 0, stream, qp));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
     int launches = 1;
@@ -968,7 +974,7 @@ int launch_attention_verify_tc(const AttnArgs &a, cudaStream_t stream) {
     if (!taken) fail(KVC_ERR_INTERNAL, "verify kernel: the device refused its shared memory");
     ++launches;
     if (merge) {
-        verify_merge_kernel<<<(unsigned)(units * R), VT_D, 0, stream>>>(p);
+        KVC_CUDA(launch_pdl(verify_merge_kernel, dim3((unsigned)(units * R)), dim3(VT_D), 0, stream, p));
         KVC_CUDA(cudaGetLastError());
         ++g_launch_count;
         ++launches;
@@ -987,6 +993,8 @@ int launch_attention_verify_tc(const AttnArgs &a, cudaStream_t stream) {
 // One thread per eight dims.
 template <typename T>
 __global__ void __launch_bounds__(256) verify_q_raw_kernel(const QPadParams p) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     constexpr int D = VT_D;
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t units = (int64_t)p.B * p.Hkv;
@@ -1071,8 +1079,8 @@ int launch_attention_verify_tc_affine(const AttnArgs &a, cudaStream_t stream) {
     qp.B = a.B; qp.Hq = a.Hq; qp.Hkv = a.Hkv; qp.L = a.L; qp.R = R;
     qp.perm_bits = a.k.bits;
     const unsigned qblocks = (unsigned)((units * TC_ROWS * (VT_D / 8) + 255) / 256);
-    if (a.q_dtype == KVC_BF16) verify_q_plain_kernel<__nv_bfloat16><<<qblocks, 256, 0, stream>>>(qp);
-    else verify_q_plain_kernel<__half><<<qblocks, 256, 0, stream>>>(qp);
+    if (a.q_dtype == KVC_BF16) KVC_CUDA(launch_pdl(verify_q_plain_kernel<__nv_bfloat16>, dim3(qblocks), dim3(256), 0, stream, qp));
+    else KVC_CUDA(launch_pdl(verify_q_plain_kernel<__half>, dim3(qblocks), dim3(256), 0, stream, qp));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
     int launches = 1;
@@ -1114,7 +1122,7 @@ int launch_attention_verify_tc_affine(const AttnArgs &a, cudaStream_t stream) {
     if (!taken) fail(KVC_ERR_INTERNAL, "verify kernel: the device refused its shared memory");
     ++launches;
     if (merge) {
-        verify_merge_kernel<<<(unsigned)(units * R), VT_D, 0, stream>>>(p);
+        KVC_CUDA(launch_pdl(verify_merge_kernel, dim3((unsigned)(units * R)), dim3(VT_D), 0, stream, p));
         KVC_CUDA(cudaGetLastError());
         ++g_launch_count;
         ++launches;
@@ -1175,8 +1183,8 @@ int launch_attention_verify_tc_raw(const AttnArgs &a, cudaStream_t stream) {
     qp.q_sb = a.q_sb; qp.q_sh = a.q_sh; qp.q_sl = a.q_sl;
     qp.B = a.B; qp.Hq = a.Hq; qp.Hkv = a.Hkv; qp.L = a.L; qp.R = R;
     const unsigned qblocks = (unsigned)((units * TC_ROWS * (VT_D / 8) + 255) / 256);
-    if (a.q_dtype == KVC_BF16) verify_q_raw_kernel<__nv_bfloat16><<<qblocks, 256, 0, stream>>>(qp);
-    else verify_q_raw_kernel<__half><<<qblocks, 256, 0, stream>>>(qp);
+    if (a.q_dtype == KVC_BF16) KVC_CUDA(launch_pdl(verify_q_raw_kernel<__nv_bfloat16>, dim3(qblocks), dim3(256), 0, stream, qp));
+    else KVC_CUDA(launch_pdl(verify_q_raw_kernel<__half>, dim3(qblocks), dim3(256), 0, stream, qp));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
     int launches = 1;
@@ -1202,7 +1210,7 @@ int launch_attention_verify_tc_raw(const AttnArgs &a, cudaStream_t stream) {
     if (!taken) fail(KVC_ERR_INTERNAL, "verify kernel: the device refused its shared memory");
     ++launches;
     if (merge) {
-        verify_merge_kernel<<<(unsigned)(units * R), VT_D, 0, stream>>>(p);
+        KVC_CUDA(launch_pdl(verify_merge_kernel, dim3((unsigned)(units * R)), dim3(VT_D), 0, stream, p));
         KVC_CUDA(cudaGetLastError());
         ++g_launch_count;
         ++launches;

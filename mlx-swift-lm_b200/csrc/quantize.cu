@@ -8,6 +8,7 @@
 //     contiguous elements [l*E, l*E+E);
 //   * sums run sequentially over a lane's own elements, then over the xor
 //     butterfly 16, 8, 4, 2, 1 across lanes.
+#include "attn_common.cuh"
 #include "common.h"
 #include "f32x2.cuh"
 
@@ -113,8 +114,8 @@ __device__ __forceinline__ void quantize_row_warp(const T *src, int64_t s_sd, ui
 template <typename T, int E>
 __global__ void affine_quantize_warp_kernel(QuantAppendArgs ka, QuantAppendArgs va, int64_t k_rows,
                                             int64_t total_rows) {
-    // lets a dependent kernel launched with programmatic serialization begin its prologue now
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= total_rows) return;
@@ -249,7 +250,8 @@ __device__ __forceinline__ void affine_quantize_vec_body(const QuantAppendArgs &
 template <typename T, int LPR, int BITS, int U>
 __global__ void __launch_bounds__(256)
 affine_quantize_vec_kernel(QuantAppendArgs ka, QuantAppendArgs va, int lpg_log2) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     // keys and values share B, H and S; the branch is uniform over the block
     if ((int)blockIdx.z >= ka.B) affine_quantize_vec_body<T, LPR, BITS, U>(va, (int)blockIdx.z - ka.B, lpg_log2);
     else affine_quantize_vec_body<T, LPR, BITS, U>(ka, (int)blockIdx.z, lpg_log2);
@@ -259,7 +261,8 @@ affine_quantize_vec_kernel(QuantAppendArgs ka, QuantAppendArgs va, int lpg_log2)
 // head); every pointer of the table already addresses head 0 at the sequence's append position.
 template <typename T, int E>
 __global__ void affine_quantize_varlen_kernel(const __grid_constant__ VarlenQuantArgs a) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= a.n * 2 * a.H) return;
@@ -278,6 +281,8 @@ __global__ void affine_quantize_varlen_kernel(const __grid_constant__ VarlenQuan
 template <typename T>
 __global__ void affine_quantize_group_kernel(QuantAppendArgs ka, QuantAppendArgs va,
                                              int64_t k_groups, int64_t total_groups) {
+    dev::pdl_wait();
+    dev::pdl_trigger();
     int64_t gidx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gidx >= total_groups) return;
     const bool is_v = gidx >= k_groups;
@@ -339,7 +344,8 @@ struct QuantList {
 };
 template <typename T, int LPR, int BITS>
 __global__ void __launch_bounds__(256) affine_quantize_list_kernel(const __grid_constant__ QuantList l, int lpg_log2) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     const int B = l.a[0][0].B, b = blockIdx.z % B, w = blockIdx.z / B;
     affine_quantize_vec_body<T, LPR, BITS, 1>(l.a[w / l.tensors][w % l.tensors], b, lpg_log2);
 }
@@ -378,9 +384,9 @@ bool quantize_list(const QuantAppendArgs *k, const QuantAppendArgs *v, int n, cu
     const dim3 grid((unsigned)((k0.S + warps * rpp - 1) / (warps * rpp)), (unsigned)k0.H, (unsigned)z);
 #define KVC_QL(LPR)                                                                                                  \
     switch (k0.bits) {                                                                                               \
-        case 2: affine_quantize_list_kernel<T, LPR, 2><<<grid, warps * 32, 0, stream>>>(l, lpg_log2); break;         \
-        case 4: affine_quantize_list_kernel<T, LPR, 4><<<grid, warps * 32, 0, stream>>>(l, lpg_log2); break;         \
-        default: affine_quantize_list_kernel<T, LPR, 8><<<grid, warps * 32, 0, stream>>>(l, lpg_log2); break;        \
+        case 2: KVC_CUDA(launch_pdl(affine_quantize_list_kernel<T, LPR, 2>, grid, dim3(warps * 32), 0, stream, l, lpg_log2)); break;         \
+        case 4: KVC_CUDA(launch_pdl(affine_quantize_list_kernel<T, LPR, 4>, grid, dim3(warps * 32), 0, stream, l, lpg_log2)); break;         \
+        default: KVC_CUDA(launch_pdl(affine_quantize_list_kernel<T, LPR, 8>, grid, dim3(warps * 32), 0, stream, l, lpg_log2)); break;        \
     }
     switch (lpr) {
         case 8: KVC_QL(8); break;
@@ -424,8 +430,8 @@ void quantize_dispatch(const QuantAppendArgs &k, const QuantAppendArgs &v, bool 
                         (unsigned)(k.B * (have_v ? 2 : 1)));
 #define KVC_QVEC(LPR, BITS)                                                                                   \
     do {                                                                                                      \
-        if (deep) affine_quantize_vec_kernel<T, LPR, BITS, 4><<<grid, warps * 32, 0, stream>>>(k, vv, lpg_log2); \
-        else affine_quantize_vec_kernel<T, LPR, BITS, 1><<<grid, warps * 32, 0, stream>>>(k, vv, lpg_log2);      \
+        if (deep) KVC_CUDA(launch_pdl(affine_quantize_vec_kernel<T, LPR, BITS, 4>, grid, dim3(warps * 32), 0, stream, k, vv, lpg_log2)); \
+        else KVC_CUDA(launch_pdl(affine_quantize_vec_kernel<T, LPR, BITS, 1>, grid, dim3(warps * 32), 0, stream, k, vv, lpg_log2));      \
     } while (0)
 #define KVC_QVEC_B(LPR)                                            \
     switch (k.bits) {                                              \
@@ -445,17 +451,17 @@ void quantize_dispatch(const QuantAppendArgs &k, const QuantAppendArgs &v, bool 
         const int warps = 8;
         const unsigned blocks = (unsigned)((total + warps - 1) / warps);
         switch (k.D / 32) {
-            case 1: affine_quantize_warp_kernel<T, 1><<<blocks, warps * 32, 0, stream>>>(k, vv, k_rows, total); break;
-            case 2: affine_quantize_warp_kernel<T, 2><<<blocks, warps * 32, 0, stream>>>(k, vv, k_rows, total); break;
-            case 4: affine_quantize_warp_kernel<T, 4><<<blocks, warps * 32, 0, stream>>>(k, vv, k_rows, total); break;
-            case 8: affine_quantize_warp_kernel<T, 8><<<blocks, warps * 32, 0, stream>>>(k, vv, k_rows, total); break;
+            case 1: KVC_CUDA(launch_pdl(affine_quantize_warp_kernel<T, 1>, dim3(blocks), dim3(warps * 32), 0, stream, k, vv, k_rows, total)); break;
+            case 2: KVC_CUDA(launch_pdl(affine_quantize_warp_kernel<T, 2>, dim3(blocks), dim3(warps * 32), 0, stream, k, vv, k_rows, total)); break;
+            case 4: KVC_CUDA(launch_pdl(affine_quantize_warp_kernel<T, 4>, dim3(blocks), dim3(warps * 32), 0, stream, k, vv, k_rows, total)); break;
+            case 8: KVC_CUDA(launch_pdl(affine_quantize_warp_kernel<T, 8>, dim3(blocks), dim3(warps * 32), 0, stream, k, vv, k_rows, total)); break;
         }
     } else {
         const int64_t k_groups = k_rows * (k.D / k.group);
         const int64_t v_groups = have_v ? v_rows * (v.D / v.group) : 0;
         const int64_t total = k_groups + v_groups;
-        affine_quantize_group_kernel<T><<<(unsigned)((total + 127) / 128), 128, 0, stream>>>(
-            k, vv, k_groups, total);
+        KVC_CUDA(launch_pdl(affine_quantize_group_kernel<T>, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, stream,
+            k, vv, k_groups, total));
     }
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
@@ -475,10 +481,10 @@ bool launch_affine_quantize_varlen(const VarlenQuantArgs &a, cudaStream_t stream
     const unsigned blocks = (unsigned)((total + warps - 1) / warps);
 #define KVC_QV(TT)                                                                                      \
     switch (E) {                                                                                        \
-        case 1: affine_quantize_varlen_kernel<TT, 1><<<blocks, warps * 32, 0, stream>>>(a); break;     \
-        case 2: affine_quantize_varlen_kernel<TT, 2><<<blocks, warps * 32, 0, stream>>>(a); break;     \
-        case 4: affine_quantize_varlen_kernel<TT, 4><<<blocks, warps * 32, 0, stream>>>(a); break;     \
-        default: affine_quantize_varlen_kernel<TT, 8><<<blocks, warps * 32, 0, stream>>>(a); break;    \
+        case 1: KVC_CUDA(launch_pdl(affine_quantize_varlen_kernel<TT, 1>, dim3(blocks), dim3(warps * 32), 0, stream, a)); break;     \
+        case 2: KVC_CUDA(launch_pdl(affine_quantize_varlen_kernel<TT, 2>, dim3(blocks), dim3(warps * 32), 0, stream, a)); break;     \
+        case 4: KVC_CUDA(launch_pdl(affine_quantize_varlen_kernel<TT, 4>, dim3(blocks), dim3(warps * 32), 0, stream, a)); break;     \
+        default: KVC_CUDA(launch_pdl(affine_quantize_varlen_kernel<TT, 8>, dim3(blocks), dim3(warps * 32), 0, stream, a)); break;    \
     }
     if (a.dtype == KVC_BF16) { KVC_QV(__nv_bfloat16) }
     else if (a.dtype == KVC_F16) { KVC_QV(__half) }
@@ -549,8 +555,8 @@ namespace {
 template <typename T, int E>
 __global__ void turbo_encode_kernel(TurboEncodeArgs ka, TurboEncodeArgs va, int64_t k_rows,
                                     int64_t total_rows, float inv_sqrt_dim) {
-    // lets a dependent kernel launched with programmatic serialization begin its prologue now
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     extern __shared__ uint32_t s_words[];  // [warps][PWmax]
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1008,7 +1014,8 @@ __device__ __forceinline__ void turbo_encode_vec_body(const TurboEncodeArgs &a, 
 template <typename T, int E, int R>
 __global__ void __launch_bounds__(256)
 turbo_encode_vec_kernel(TurboEncodeArgs ka, TurboEncodeArgs va, float inv_sqrt_dim, int sorted) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     __shared__ float s_bnd[16];
     // keys and values share B, H and S; the branch is uniform over the block
     if ((int)blockIdx.z >= ka.B) turbo_encode_vec_body<T, E, R>(va, (int)blockIdx.z - ka.B, inv_sqrt_dim, sorted, s_bnd);
@@ -1330,14 +1337,10 @@ turbo_encode_wide_kernel(const __grid_constant__ TurboEncodeArgs ka, const __gri
                          const __grid_constant__ EncodeCells kc, const __grid_constant__ EncodeCells vc, int groups, int groups_per_plane,
                          float inv_sqrt_dim, unsigned long long *sums) {
     using W = WideRows<D>;
-    asm volatile("griddepcontrol.launch_dependents;");
     __shared__ __align__(128) float2 table[CELLS * 16];
     const bool is_v = blockIdx.y != 0;
     const TurboEncodeArgs &a = is_v ? va : ka;
     const int lane = threadIdx.x & 31, l = lane % W::LPR, warp = threadIdx.x >> 5;
-    RawRun<T> flip;
-    RawRun<float> signs;
-    signs.load(a.signs + l * 16);
     {   // a thread takes a cell; the lanes start at different copies of theirs, so that they meet no bank twice
         static_assert(CELLS == 256, "a thread a cell");
         const float2 c = is_v ? make_cell<VB>(va, vc, threadIdx.x) : make_cell<KB>(ka, kc, threadIdx.x);
@@ -1345,6 +1348,11 @@ turbo_encode_wide_kernel(const __grid_constant__ TurboEncodeArgs ka, const __gri
 #pragma unroll
         for (int j = 0; j < 8; ++j) reinterpret_cast<float4 *>(table)[threadIdx.x * 8 + ((j + lane) & 7)] = cc;
     }
+    dev::pdl_wait();      // the cells came from the parameters
+    dev::pdl_trigger();
+    RawRun<T> flip;
+    RawRun<float> signs;
+    signs.load(a.signs + l * 16);
     bool unit = true;
 #pragma unroll
     for (int i = 0; i < RawRun<T>::WORDS; ++i) flip.w[i] = 0u;
@@ -1451,7 +1459,7 @@ bool launch_encode_wide(const TurboEncodeArgs &k, const TurboEncodeArgs &v, bool
     if (groups > (int64_t)1 << 30) return false;
     const int64_t slots = std::max<int64_t>(1, (int64_t)sm_count(current_device()) * resident / (have_v ? 2 : 1));
     if (STATS && (groups + slots - 1) / slots > CALIB_ROWS) return false;
-    kernel<<<dim3((unsigned)std::min(groups, slots), have_v ? 2 : 1), 256, 0, stream>>>(k, v, kc, vc, (int)groups, (int)per_plane, 1.0f / sqrtf((float)D), sums);
+    KVC_CUDA(launch_pdl(kernel, dim3((unsigned)std::min(groups, slots), have_v ? 2 : 1), dim3(256), 0, stream, k, v, kc, vc, (int)groups, (int)per_plane, 1.0f / sqrtf((float)D), sums));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
     return true;
@@ -1486,7 +1494,8 @@ struct EncodeList {
 };
 template <typename T, int E>
 __global__ void __launch_bounds__(256) turbo_encode_list_kernel(const __grid_constant__ EncodeList l, float inv_sqrt_dim, int sorted) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    dev::pdl_wait();
+    dev::pdl_trigger();
     __shared__ float s_bnd[16];
     const int B = l.a[0][0].B, b = blockIdx.z % B, w = blockIdx.z / B;
     turbo_encode_vec_body<T, E, 1>(l.a[w / l.tensors][w % l.tensors], b, inv_sqrt_dim, sorted, s_bnd);
@@ -1522,7 +1531,7 @@ bool encode_list(const TurboEncodeArgs *k, const TurboEncodeArgs *v, int n, cuda
     if (k0.H > 65535 || z > 65535) return false;
     const int vw = std::max(1, std::min(8, k0.S));
     const dim3 grid((unsigned)((k0.S + vw - 1) / vw), (unsigned)k0.H, (unsigned)z);
-    turbo_encode_list_kernel<T, E><<<grid, vw * 32, 0, stream>>>(l, 1.0f / sqrtf((float)k0.D), sorted ? 1 : 0);
+    KVC_CUDA(launch_pdl(turbo_encode_list_kernel<T, E>, grid, dim3(vw * 32), 0, stream, l, 1.0f / sqrtf((float)k0.D), sorted ? 1 : 0));
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
     return true;
@@ -1558,8 +1567,8 @@ void turbo_dispatch(const TurboEncodeArgs &k, const TurboEncodeArgs &v, bool hav
         const dim3 grid((unsigned)((k.S + vw * rpw - 1) / (vw * rpw)), (unsigned)k.H, (unsigned)(k.B * (have_v ? 2 : 1)));
 #define KVC_TV(EE)                                                                                        \
     do {                                                                                                  \
-        if (deep) turbo_encode_vec_kernel<T, EE, 2><<<grid, vw * 32, 0, stream>>>(k, v, inv_sqrt_dim, sorted); \
-        else turbo_encode_vec_kernel<T, EE, 1><<<grid, vw * 32, 0, stream>>>(k, v, inv_sqrt_dim, sorted);      \
+        if (deep) KVC_CUDA(launch_pdl(turbo_encode_vec_kernel<T, EE, 2>, grid, dim3(vw * 32), 0, stream, k, v, inv_sqrt_dim, sorted)); \
+        else KVC_CUDA(launch_pdl(turbo_encode_vec_kernel<T, EE, 1>, grid, dim3(vw * 32), 0, stream, k, v, inv_sqrt_dim, sorted));      \
     } while (0)
         switch (E) {
             case 1: KVC_TV(1); break;
@@ -1573,7 +1582,7 @@ void turbo_dispatch(const TurboEncodeArgs &k, const TurboEncodeArgs &v, bool hav
         return;
     }
 #define KVC_TE(EE)                                                                               \
-    turbo_encode_kernel<T, EE><<<blocks, warps * 32, smem, stream>>>(k, v, k_rows, total, inv_sqrt_dim)
+    KVC_CUDA(launch_pdl(turbo_encode_kernel<T, EE>, dim3(blocks), dim3(warps * 32), smem, stream, k, v, k_rows, total, inv_sqrt_dim))
     switch (k.D / 32) {
         case 1: KVC_TE(1); break;
         case 2: KVC_TE(2); break;
