@@ -132,6 +132,12 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return r;
 }
 
+__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
 // Bits of 32 mask bytes starting at p (any alignment), the first n of them inside the row.
 __device__ __forceinline__ uint32_t mask_bits32(const uint8_t *p, int n) {
     if (n <= 0) return 0;
@@ -240,6 +246,23 @@ __device__ __forceinline__ void store_out(void *p, int32_t dtype, int64_t i, flo
         case KVC_F32: ((float *)p)[i] = v; break;
         case KVC_F16: ((__half *)p)[i] = __float2half_rn(v); break;
         default: ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(v); break;
+    }
+}
+
+// Four neighbouring elements, in one store where they lie on its boundary.
+__device__ __forceinline__ void store_out4(void *p, int32_t dtype, int64_t i, float4 v) {
+    const uintptr_t at = (uintptr_t)p + (uintptr_t)(i * (dtype == KVC_F32 ? 4 : 2));
+    if (at & (dtype == KVC_F32 ? 15 : 7)) {
+        store_out(p, dtype, i, v.x);
+        store_out(p, dtype, i + 1, v.y);
+        store_out(p, dtype, i + 2, v.z);
+        store_out(p, dtype, i + 3, v.w);
+    } else if (dtype == KVC_F32) {
+        *(float4 *)at = v;
+    } else if (dtype == KVC_F16) {
+        *(uint2 *)at = make_uint2(pack_h2(v.x, v.y), pack_h2(v.z, v.w));
+    } else {
+        *(uint2 *)at = make_uint2(pack_bf2(v.x, v.y), pack_bf2(v.z, v.w));
     }
 }
 
@@ -467,15 +490,16 @@ __device__ __forceinline__ void rotate_out_rows(const UnitOut &u, const float *r
 // red_ml[(warp * red_rows + r) * 2 + {0, 1}] = (max, sum): merges the warps and, where the segment is the whole unit,
 // writes the output rows; else writes the segment's partial, takes a ticket and, in the CTA that completes the unit,
 // merges all partials (log-sum-exp) and writes the rows (through signs * H(.) / sqrt(D) when
-// o_signs is set; `work` then holds red_rows * D floats and is unused otherwise). Lists of short units are mostly
+// o_signs is set; `work` then holds red_rows * D floats, and is not touched otherwise). Lists of short units are mostly
 // whole ones, and the divisions behind a segment's place took 64 bits before: 4 layers of 32 sequences of 425 .. 1 761 tokens,
 // 64/8 heads, 4 bits: 145 us -> 130.
 // NBUF (default NW) is the number of warps that wrote cross-warp buffers: a kernel that has already
-// folded its NW warps down to NBUF of them passes the smaller count, all NW warps still take part.
-template <int D, int NW, int NBUF = NW, typename Plan>
+// folded its NW warps down to NBUF of them passes the smaller count, all NW warps still take part; `live`: as many
+// of these as had tokens (the first ones).
+template <int D, int NW, int NBUF = NW, int FLY = 16, typename Plan>
 __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *red_o, const float *red_ml,
                                  int red_stride, float *work, int *flag, int unit, int b, int hk, int rep, int R,
-                                 int64_t x_unit = -1, int unit_tiles = 0, int row0 = 0) {
+                                 int64_t x_unit = -1, int unit_tiles = 0, int row0 = 0, int live = NBUF) {
     // row0: the unit covers the query rows row0 .. row0 + R - 1 of its (batch, kv head) group (a group
     // of more rows than one unit carries is cut into several units)
     const int tid = threadIdx.x;
@@ -490,33 +514,51 @@ __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *r
     const int expected = flat_cta_of(f, x_unit + unit_tiles - 1) - first_cta + 1;
     const int slot = (int)blockIdx.x - first_cta;
     const int64_t qrow0 = ((int64_t)b * u.Hq + hk * rep) * u.L + row0;
-    // One element of the segment's rows, the warps merged; its maximum and sum.
+    // A thread takes four neighbouring dims of a row at a time: the weights of the row are worked out once for them, and
+    // where partials are merged, loads of sixteen slots are in flight. (One dim at a time and eight slots, the CTA that
+    // merged 17 slots of four rows at D 128 spent 7 us on it, a third of what a decode step of a chat takes in all.)
+    constexpr int D4 = D / 4;
+    // Four dims of the segment's rows, the warps merged; their row's maximum and sum.
     auto merged = [&](int r, int d, float &m, float &l) {
         m = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < NBUF; ++w) m = fmaxf(m, red_ml[(w * f.red_rows + r) * 2]);
-        float o = 0.f;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
         l = 0.f;
 #pragma unroll
-        for (int w = 0; w < NBUF; ++w) {
-            const float mw = red_ml[(w * f.red_rows + r) * 2];
-            const float fw = (mw == -INFINITY) ? 0.f : fast_exp2(mw - m);
-            o += red_o[(w * f.red_rows + r) * red_stride + d] * fw;
-            l += red_ml[(w * f.red_rows + r) * 2 + 1] * fw;
+        for (int w0 = 0; w0 < NBUF; w0 += 4) {
+            if (w0 >= live) break;
+#pragma unroll
+            for (int w = w0; w < w0 + 4 && w < NBUF; ++w) m = fmaxf(m, red_ml[(w * f.red_rows + r) * 2]);
+        }
+#pragma unroll
+        for (int w0 = 0; w0 < NBUF; w0 += 4) {
+            if (w0 >= live) break;
+#pragma unroll
+            for (int w = w0; w < w0 + 4 && w < NBUF; ++w) {
+                const float mw = red_ml[(w * f.red_rows + r) * 2];
+                const float fw = (mw == -INFINITY) ? 0.f : fast_exp2(mw - m);
+                const float4 x = *(const float4 *)&red_o[(w * f.red_rows + r) * red_stride + d];
+                o.x += x.x * fw; o.y += x.y * fw; o.z += x.z * fw; o.w += x.w * fw;
+                l += red_ml[(w * f.red_rows + r) * 2 + 1] * fw;
+            }
         }
         return o;
     };
+    // The finished dims of a row: to the output, or to `work` where they have to be rotated back first.
+    auto finish = [&](int r, int d, float4 o, float l) {
+        o = l > 0.f ? make_float4(o.x / l, o.y / l, o.z / l, o.w / l) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (u.o_signs) {
+            *(float4 *)&work[r * D + d] = o;
+        } else {
+            const int hq = hk * rep + (row0 + r) / u.L, lq = (row0 + r) % u.L;
+            store_out4(u.out, u.out_dtype, b * u.o_sb + hq * u.o_sh + lq * u.o_sl + d, o);
+        }
+    };
     if (expected == 1) {   // the segment is the whole unit: its rows go straight to the output
-        for (int i = tid; i < R * D; i += NT) {
-            const int r = i / D, d = i % D;
-            float m, l, o = merged(r, d, m, l);
-            o = l > 0.f ? o / l : 0.f;
-            if (u.o_signs) {
-                work[i] = o;
-            } else {
-                const int hq = hk * rep + (row0 + r) / u.L, lq = (row0 + r) % u.L;
-                store_out(u.out, u.out_dtype, b * u.o_sb + hq * u.o_sh + lq * u.o_sl + d, o);
-            }
+        for (int i = tid; i < R * D4; i += NT) {
+            const int r = i / D4, d = i % D4 * 4;
+            float m, l;
+            const float4 o = merged(r, d, m, l);
+            finish(r, d, o, l);
         }
         consumer_bar<NW>();
         if (u.o_signs) {
@@ -525,12 +567,12 @@ __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *r
         }
         return;   // the buffers are free again
     }
-    for (int i = tid; i < R * D; i += NT) {
-        const int r = i / D, d = i % D;
+    for (int i = tid; i < R * D4; i += NT) {
+        const int r = i / D4, d = i % D4 * 4;
         float m, l;
-        const float o = merged(r, d, m, l);
+        const float4 o = merged(r, d, m, l);
         const int64_t base = (qrow0 + r) * f.nslots + slot;
-        __stcg(&u.o_part[base * D + d], o);
+        __stcg((float4 *)&u.o_part[base * D + d], o);
         if (d == 0) __stcg(&u.ml_part[base], make_float2(m, l));
     }
     __threadfence();
@@ -543,49 +585,47 @@ __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *r
     consumer_bar<NW>();
     if (*flag) {
         __threadfence();
-        // Every thread merges its own (row, dim) elements: the (max, sum) pairs and the partial
-        // values of all slots are loaded together (one round trip), the weights are recomputed per
-        // element (a unit has a handful of slots).
-        float *rows = work;  // [R][D], only for the rotated (TurboQuant) output
-        for (int i = tid; i < R * D; i += NT) {
-            const int r = i / D, d = i % D;
+        // The (max, sum) pairs and the partial values of FLY slots are loaded together (eight where the kernel has no
+        // registers for more), the weights are recomputed per thread; slots are merged eight at a time.
+        for (int i = tid; i < R * D4; i += NT) {
+            const int r = i / D4, d = i % D4 * 4;
             const float2 *mlp = u.ml_part + (qrow0 + r) * f.nslots;
             const float *src = u.o_part + ((qrow0 + r) * f.nslots) * D + d;
-            float m = -INFINITY, o = 0.f, lsum = 0.f;
-            for (int s0 = 0; s0 < expected; s0 += 8) {   // all loads of a batch of 8 slots are issued together
-                float2 ml[8];
-                float ov[8];
+            float m = -INFINITY, lsum = 0.f;
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int s0 = 0; s0 < expected; s0 += FLY) {
+                float2 ml[FLY];
+                float4 ov[FLY];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < FLY; ++j) {
                     const bool in = s0 + j < expected;
                     ml[j] = in ? __ldcg(&mlp[s0 + j]) : make_float2(-INFINITY, 0.f);
-                    ov[j] = in ? __ldcg(src + (int64_t)(s0 + j) * D) : 0.f;
+                    ov[j] = in ? __ldcg((const float4 *)(src + (int64_t)(s0 + j) * D)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
-                float mb = m;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) mb = fmaxf(mb, (ml[j].y > 0.f) ? ml[j].x : -INFINITY);
-                const float keep = (m == -INFINITY) ? 0.f : fast_exp2(m - mb);   // rescale what earlier batches gave
-                o *= keep;
-                lsum *= keep;
-                m = mb;
+                for (int half = 0; half < FLY; half += 8) {
+                    if (s0 + half >= expected) break;
+                    float mb = m;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float fw = (ml[j].x == -INFINITY || ml[j].y <= 0.f) ? 0.f : fast_exp2(ml[j].x - m);
-                    lsum = fmaf(ml[j].y, fw, lsum);
-                    o = fmaf(ov[j], fw, o);
+                    for (int j = half; j < half + 8; ++j) mb = fmaxf(mb, (ml[j].y > 0.f) ? ml[j].x : -INFINITY);
+                    const float keep = (m == -INFINITY) ? 0.f : fast_exp2(m - mb);   // rescale what earlier slots gave
+                    o.x *= keep; o.y *= keep; o.z *= keep; o.w *= keep;
+                    lsum *= keep;
+                    m = mb;
+#pragma unroll
+                    for (int j = half; j < half + 8; ++j) {
+                        const float fw = (ml[j].x == -INFINITY || ml[j].y <= 0.f) ? 0.f : fast_exp2(ml[j].x - m);
+                        lsum = fmaf(ml[j].y, fw, lsum);
+                        o.x = fmaf(ov[j].x, fw, o.x); o.y = fmaf(ov[j].y, fw, o.y);
+                        o.z = fmaf(ov[j].z, fw, o.z); o.w = fmaf(ov[j].w, fw, o.w);
+                    }
                 }
             }
-            o = lsum > 0.f ? o / lsum : 0.f;
-            if (!u.o_signs) {
-                const int hq = hk * rep + (row0 + r) / u.L, lq = (row0 + r) % u.L;
-                store_out(u.out, u.out_dtype, b * u.o_sb + hq * u.o_sh + lq * u.o_sl + d, o);
-            } else {
-                rows[i] = o;
-            }
+            finish(r, d, o, lsum);
         }
         if (u.o_signs) {
             consumer_bar<NW>();
-            rotate_out_rows<D, NW>(u, rows, b, hk, rep, R, row0);
+            rotate_out_rows<D, NW>(u, work, b, hk, rep, R, row0);
         }
     }
     consumer_bar<NW>();  // buffers and flag are reused by the next segment

@@ -477,14 +477,13 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
     const FlatPlan &fp = p.flat;
     float *red_o = (float *)(is_last + 4);                                   // [4][red_rows][RED_STRIDE]
     float *red_ml = red_o + CONSUMER_WARPS * fp.red_rows * RED_STRIDE;       // [4][red_rows][2]
-    float *work = red_ml + CONSUMER_WARPS * fp.red_rows * 2;                 // [red_rows][nslots]
     // Query rows of a segment's unit, brought in by the producer with one bulk copy (two buffers):
     // plain loads issued by the consumers while the tile stream saturates the memory system cost
     // several microseconds per segment.
     // Lists have no cross-warp buffer, and the producer hands the consumers a segment's descriptor with its query rows:
     // worked out by every warp at a segment's start it was constant-cache misses and divisions between two tiles.
     constexpr int NQ = LIST ? FLAT_AHEAD : 2;
-    uint64_t *qfull = LIST ? (uint64_t *)red_o : (uint64_t *)(work + ((fp.red_rows * fp.nslots + 3) & ~3));   // keeps qbuf 16-byte aligned
+    uint64_t *qfull = LIST ? (uint64_t *)red_o : (uint64_t *)(red_ml + CONSUMER_WARPS * fp.red_rows * 2);   // (qbuf stays 16-byte aligned)
     uint64_t *qempty = qfull + NQ;
     unsigned char *qbuf = (unsigned char *)(qempty + NQ);                     // [NQ][red_rows][D] elements
     FlatWork *works = (FlatWork *)(qbuf + (size_t)NQ * (p.Hq / p.Hkv) * p.L * D * 2);   // [NQ] (lists)
@@ -904,7 +903,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             u.o_signs = nullptr;
             u.splits = 0; u.Hq = p.Hq; u.L = p.L;
             if (!(KVC_SKIP_BITS(p) & 16))
-                segment_epilogue<D, CONSUMER_WARPS>(u, fp, red_o, red_ml, RED_STRIDE, work, is_last, w.unit, w.b, w.hk, rep, R);
+                segment_epilogue<D, CONSUMER_WARPS>(u, fp, red_o, red_ml, RED_STRIDE, nullptr, is_last, w.unit, w.b, w.hk, rep, R);
         }
         x += n;
     }
@@ -1602,10 +1601,9 @@ FlatShape flat_shape(int sms, int D, int R, int64_t work, int64_t most_tiles) {
     f.nslots = (most_tiles + f.per - 1) / f.per + 1;
     f.nstage = D == 64 ? 6 : 3;
     const size_t ring = (size_t)f.nstage * 2 * (TILE_T * D * 2);
-    const size_t red = (size_t)CONSUMER_WARPS * R * (D + 8) * 4 + (size_t)CONSUMER_WARPS * R * 8 + (size_t)R * f.nslots * 4 +
-                       16 + 4 * sizeof(uint64_t) + (size_t)2 * R * D * 2;
+    const size_t red = (size_t)CONSUMER_WARPS * R * (D + 8) * 4 + (size_t)CONSUMER_WARPS * R * 8 + 16 + 4 * sizeof(uint64_t) + (size_t)2 * R * D * 2;
     f.smem = ring + 2 * f.nstage * sizeof(uint64_t) + 64 + red + 1024;
-    f.fits = f.smem <= (size_t)(D <= 128 ? 112 : 224) * 1024 && f.nslots <= 64;
+    f.fits = f.smem <= (size_t)(D <= 128 ? 112 : 224) * 1024;
     return f;
 }
 

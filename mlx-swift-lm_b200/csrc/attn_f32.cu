@@ -310,7 +310,7 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
         uo.o_signs = nullptr;
         uo.splits = 0; uo.Hq = p.Hq; uo.L = p.L;
         segment_epilogue<D, ST_WARPS>(uo, fp, red_o, red_ml, D + 4, nullptr, flag, si * p.B * p.Hkv * p.chunks + u_in, si * p.B + b, hk,
-                                      rep, R, x - tile, sq.tiles, row0);
+                                      rep, R, x - tile, sq.tiles, row0, min(ST_WARPS, nblk));
         x += tiles;
     }
 }

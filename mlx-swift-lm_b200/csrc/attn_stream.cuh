@@ -884,7 +884,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
         const int rr_n = fp.red_rows;
         float *red_o = (float *)body;
         float *red_ml = red_o + ST_WARPS * rr_n * SH::RED_STRIDE;
-        float *work = red_ml + ST_WARPS * rr_n * 2;
+        float *work = red_ml + ((ST_WARPS * rr_n * 2 + 3) & ~3);      // 16-byte aligned for any row count
         __syncthreads();        // every warp has left the ring that the merge buffers overlay
         const float undo = (V::AFFINE ? 1.f : p.vcb_undo) / ST_PSCALE;
 #pragma unroll
@@ -934,7 +934,7 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
         }
         uo.splits = 0; uo.Hq = p.Hq; uo.L = p.L;
         segment_epilogue<D, ST_WARPS>(uo, fp, red_o, red_ml, SH::RED_STRIDE, work, flag, sg.unit, b_row, sg.hk, rep, R,
-                                      sg.unit_x, sg.unit_tiles, row0);
+                                      sg.unit_x, sg.unit_tiles, row0, min(ST_WARPS, nblk));
         x += sg.tiles;
     }
 }

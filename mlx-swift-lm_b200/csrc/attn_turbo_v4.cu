@@ -601,7 +601,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
         u.o_sb = p.o_sb; u.o_sh = p.o_sh; u.o_sl = p.o_sl;
         u.o_signs = p.o_signs;
         u.splits = 0; u.Hq = p.Hq; u.L = p.L;
-        segment_epilogue<D, V4_WARPS, 4>(u, fp, red_o, red_ml, V4_RED_STRIDE, work, is_last, unit, b, hk, rep, R, -1, 0, row0);
+        segment_epilogue<D, V4_WARPS, 4, 8>(u, fp, red_o, red_ml, V4_RED_STRIDE, work, is_last, unit, b, hk, rep, R, -1, 0, row0);
         x += own;
     }
 }
