@@ -131,20 +131,16 @@ __global__ void rope_kernel(RopeArgs a, int64_t q_items, int64_t total_items) {
     T *dst = (T *)t.dst + b * t.d_sb + h * t.d_sh + l * t.d_sl;
     const int rp = a.dims / 2;           // rotated pairs
     float sn = 0.f, cs = 1.f;
-    if (p < rp) {
-        // the frequency in double precision, rounded once: at positions in the tens of thousands a float32
-        // exp2 would already move the angle by 1e-3
-        const float inv_freq = (float)exp2(-(double)p * a.log2_base_over_half);
-        sincosf(__fmul_rn(__fmul_rn((float)(a.offset + l), a.scale), inv_freq), &sn, &cs);
-    }
+    if (p < rp) dev::rope_angle(p, a.log2_base_over_half, a.offset + l, a.scale, cs, sn);
     dev::pdl_wait();
     dev::pdl_trigger();
     if (!live) return;
     if (p < rp) {
         const int i0 = a.traditional ? 2 * p : p, i1 = a.traditional ? 2 * p + 1 : p + rp;
-        const float x0 = to_float<T>(src[i0]), x1 = to_float<T>(src[i1]);
-        dst[i0] = from_float<T>(x0 * cs - x1 * sn);
-        dst[i1] = from_float<T>(x0 * sn + x1 * cs);
+        float y0, y1;
+        dev::rope_turn(to_float<T>(src[i0]), to_float<T>(src[i1]), cs, sn, y0, y1);
+        dst[i0] = from_float<T>(y0);
+        dst[i1] = from_float<T>(y1);
     } else {
         // the features past `dims`, two per item
         const int j = a.dims + 2 * (p - rp);

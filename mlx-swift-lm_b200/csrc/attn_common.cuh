@@ -218,6 +218,27 @@ template <> struct MmaType<__half> {
 };
 
 
+// A tile's lines towards L2, where every kernel's writes meet: may run ahead of the wait on the kernel before, whatever that
+// one writes.
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap *map, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
+                 ::"l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(w)
+                 : "memory");
+}
+
+// Rotary positions: cosine and sine of pair `p` at a position (MLX's published RoPE: p turns by
+// position * scale * base^(-2p / dims)). The frequency in double precision, rounded once: at positions in the tens of
+// thousands a float32 exp2 would already move the angle by 1e-3.
+__device__ __forceinline__ void rope_angle(int p, double log2_base_over_half, int64_t position, float scale, float &cs, float &sn) {
+    const float inv_freq = (float)exp2(-(double)p * log2_base_over_half);
+    sincosf(__fmul_rn(__fmul_rn((float)position, scale), inv_freq), &sn, &cs);
+}
+// A pair turned (in float32, one product rounded, one fused).
+__device__ __forceinline__ void rope_turn(float x0, float x1, float cs, float sn, float &y0, float &y1) {
+    y0 = __fmaf_rn(x0, cs, -__fmul_rn(x1, sn));
+    y1 = __fmaf_rn(x0, sn, __fmul_rn(x1, cs));
+}
+
 // Untiled bulk copy global -> shared (both 16-byte aligned, size a multiple of 16).
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile(

@@ -71,6 +71,11 @@ struct DecodeParams {
     // fused append: the new rows [B, Hkv, D] of this step (null = the cache already holds them)
     const void *new_k, *new_v;
     int32_t early_tiles;  // flat kernel: the stored rows may be streamed before the preceding kernel has finished
+    // flat kernel, fused append of unturned rows: pairs that turn (0: rows come turned), their layout and the position
+    int32_t rope_pairs, rope_traditional;
+    double rope_log2;
+    float rope_scale;
+    int64_t rope_position;
     int64_t new_slot;     // flat kernel, fused append: token index the new row is stored at (T - 1, or a ring slot)
     int64_t nk_sb, nk_sh, nv_sb, nv_sh;  // element strides
     int64_t causal_offset;
@@ -459,7 +464,20 @@ __device__ __forceinline__ FlatWork flat_work(const FlatSeg &g, const DecodePara
     return w;
 }
 
-template <typename T, int D, int NSTAGE, bool LIST>
+// The queries of a chat step come unturned (ROPE): a launch of its own for their rotary positions cost more than the turns.
+// The angles are worked out before the wait on the kernel before; the consumers turn the unit's query rows where the bulk
+// copy puts them, the warp that appends turns the new key row, and the tiles are drawn towards L2 before the wait. A layer
+// of 32/8 heads, D 128, 1 031 tokens: 8.8 us in two launches, 8.1 in one. The bits are those of the two launches.
+template <typename T, int D>
+__device__ __forceinline__ void rope_row(T *row, const float2 *tab, const DecodeParams &p, int i) {
+    const int i0 = p.rope_traditional ? 2 * i : i, i1 = p.rope_traditional ? 2 * i + 1 : i + p.rope_pairs;
+    float y0, y1;
+    rope_turn(to_f32<T>(row[i0]), to_f32<T>(row[i1]), tab[i].x, tab[i].y, y0, y1);
+    MmaType<T>::store(row, i0, y0);
+    MmaType<T>::store(row, i1, y1);
+}
+
+template <typename T, int D, int NSTAGE, bool LIST, bool ROPE>
 __global__ void __launch_bounds__(DEC_THREADS, (D <= 128 ? 2 : 1))
 attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatList, FlatSingle> list,
                         const __grid_constant__ DecodeParams p) {
@@ -486,6 +504,8 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
     uint64_t *qfull = LIST ? (uint64_t *)red_o : (uint64_t *)(red_ml + CONSUMER_WARPS * fp.red_rows * 2);   // (qbuf stays 16-byte aligned)
     uint64_t *qempty = qfull + NQ;
     unsigned char *qbuf = (unsigned char *)(qempty + NQ);                     // [NQ][red_rows][D] elements
+    float2 *rope_tab = (float2 *)(qbuf + (size_t)NQ * (p.Hq / p.Hkv) * p.L * D * 2);   // [D / 2] cosines and sines (ROPE), then
+    T *rope_k = (T *)(rope_tab + D / 2);                                      // [D] the new key row
     FlatWork *works = (FlatWork *)(qbuf + (size_t)NQ * (p.Hq / p.Hkv) * p.L * D * 2);   // [NQ] (lists)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -507,14 +527,19 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    if (ROPE && tid < p.rope_pairs) {
+        float cs, sn;
+        rope_angle(tid, p.rope_log2, p.rope_position, p.rope_scale, cs, sn);
+        rope_tab[tid] = make_float2(cs, sn);
+    }
     __syncthreads();
     // Everything read below was written by earlier kernels on the stream, so it comes after the wait
     // on the preceding kernel. One exception, early_tiles: the producer streams its first tiles of
     // stored rows before that wait. The host vouches that the preceding kernel does not write them (it
     // is a layer of the same batched call, working on another cache), and every kernel before that one
     // has completed, because kernels release their successor only after their own wait.
-    const bool early = p.early_tiles != 0 && warp == CONSUMER_WARPS;
-    if (!early) {
+    const bool early = p.early_tiles != 0 && warp == CONSUMER_WARPS, ahead = early || (ROPE && warp == CONSUMER_WARPS);
+    if (!ahead) {
         pdl_wait();
         pdl_trigger();
     }
@@ -524,7 +549,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
         // ---------------- producer: one stream of tiles across the segments ----------------
         if (lane == 0) {
             int it = 0, sg = 0;
-            bool waited = !early;
+            bool waited = !ahead;
             FlatSeg gs;
             gs.layer = 0;
             int r = blockIdx.x;
@@ -537,6 +562,17 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 flat_locate(gs, p, x, x_hi);
                 const int t0 = gs.t0, n = gs.n, hk = gs.hk, b = gs.b;
                 int j_first = 0;
+                if (ROPE && !waited && !early) {
+                    for (int j = 0; j < n && j < NSTAGE; ++j)
+#pragma unroll
+                        for (int bx = 0; bx < BOXES; ++bx) {
+                            tma_prefetch_4d(gs.kmap, bx * 64, (t0 + j) * TILE_T, hk, b);
+                            tma_prefetch_4d(gs.vmap, bx * 64, (t0 + j) * TILE_T, hk, b);
+                        }
+                    pdl_wait();
+                    pdl_trigger();
+                    waited = true;
+                }
                 if (!waited) {
                     // the ring is empty: up to NSTAGE tiles go out before the wait
                     for (; j_first < n && j_first < NSTAGE; ++j_first, ++it) {
@@ -664,6 +700,15 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             const int l = r % p.L;
             row_limit[half] = (r < R) ? (p.causal ? min(t_cached, p.causal_offset + l) : t_cached) : -1;
         }
+        if (ROPE && fused && warp == 0 && w.last) {
+            // the new key row, turned as the queries are; its last reads lie behind the barriers of the segment before
+            FlatWork rows;
+            flat_new_rows<T>(rows, gs);
+            if (lane < D / 8) *(uint4 *)(rope_k + 8 * lane) = *(const uint4 *)(rows.new_k + 16 * lane);
+            __syncwarp();
+            for (int i = lane; i < p.rope_pairs; i += 32) rope_row<T, D>(rope_k, rope_tab, p, i);
+            __syncwarp();
+        }
         if (fused && warp == 0 && w.last && lane < 4) {
             // the new rows are consumed at the end of the segment: pull them towards L2 now
             FlatWork rows;
@@ -679,6 +724,14 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                 if (!ok && lane == 0) atomicExch(p.status, 13);
             }
             const unsigned char *qs = qbuf + (size_t)qb * q_bytes;
+            if constexpr (ROPE) {
+                // (consumer threads alone; every one of them is here for every segment)
+                for (int i = tid; i < R * p.rope_pairs; i += CONSUMER_WARPS * 32) {
+                    const int r = i / p.rope_pairs;
+                    rope_row<T, D>((T *)(qbuf + (size_t)qb * q_bytes) + (size_t)r * D, rope_tab, p, i - r * p.rope_pairs);
+                }
+                consumer_bar<CONSUMER_WARPS>();
+            }
 #pragma unroll
             for (int ks = 0; ks < KSTEPS; ++ks) {
                 const int bx = ks / 4, ps = (ks >> 1) & 1, h = ks & 1;
@@ -817,7 +870,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             FlatWork rows;
             if constexpr (!LIST) flat_new_rows<T>(rows, gs);
             const FlatWork &nr = LIST ? w : rows;
-            const T *kn = (const T *)nr.new_k, *vn = (const T *)nr.new_v;
+            const T *kn = ROPE ? rope_k : (const T *)nr.new_k, *vn = (const T *)nr.new_v;
             float dot[2] = {0.f, 0.f};
 #pragma unroll
             for (int ks = 0; ks < KSTEPS; ++ks) {
@@ -1525,20 +1578,20 @@ void launch_typed(const CUtensorMap &kmap, const CUtensorMap &vmap, const Decode
     ++g_launch_count;
 }
 
-template <typename T, int D, int NSTAGE, bool LIST>
+template <typename T, int D, int NSTAGE, bool LIST, bool ROPE>
 void launch_flat_typed(const std::conditional_t<LIST, FlatList, FlatSingle> &list, const DecodeParams &p, int ctas, size_t smem,
                        cudaStream_t stream) {
     static size_t configured[64] = {0};
     const int dev = current_device();
     if (dev >= 0 && dev < 64 && configured[dev] < smem) {
-        KVC_CUDA(cudaFuncSetAttribute(attn_decode_flat_kernel<T, D, NSTAGE, LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        KVC_CUDA(cudaFuncSetAttribute(attn_decode_flat_kernel<T, D, NSTAGE, LIST, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-        KVC_CUDA(cudaFuncSetAttribute(attn_decode_flat_kernel<T, D, NSTAGE, LIST>,
+        KVC_CUDA(cudaFuncSetAttribute(attn_decode_flat_kernel<T, D, NSTAGE, LIST, ROPE>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         configured[dev] = smem;
     }
     KernelTimer timer(stream);
-    KVC_CUDA(launch_pdl(attn_decode_flat_kernel<T, D, NSTAGE, LIST>, dim3(ctas), dim3(DEC_THREADS), smem, stream, list, p));
+    KVC_CUDA(launch_pdl(attn_decode_flat_kernel<T, D, NSTAGE, LIST, ROPE>, dim3(ctas), dim3(DEC_THREADS), smem, stream, list, p));
     if constexpr (LIST) {
         const int elems = p.Hq / p.Hkv * D;
         KVC_CUDA(launch_pdl(flat_list_merge_kernel<T, D>, dim3(list.n * p.B * p.Hkv, (elems + 127) / 128), dim3(128), 0, stream, list, p));
@@ -1705,7 +1758,7 @@ int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t strea
         char *scratch = (char *)scratch_get(a0.device, o_bytes + (size_t)row_slots * CONSUMER_WARPS * sizeof(float2) + 256, stream);
         p.o_part = (float *)scratch;
         p.ml_part = (float2 *)(scratch + ((o_bytes + 255) / 256) * 256);
-#define KVC_FLATL(TT, DD, NS) launch_flat_typed<TT, DD, NS, true>(list, p, ctas, smem, stream)
+#define KVC_FLATL(TT, DD, NS) launch_flat_typed<TT, DD, NS, true, false>(list, p, ctas, smem, stream)
         if (a0.q_dtype == KVC_BF16) {
             if (a0.D == 64) KVC_FLATL(__nv_bfloat16, 64, 6);
             else if (a0.D == 128) KVC_FLATL(__nv_bfloat16, 128, 3);
@@ -1798,9 +1851,22 @@ int launch_rows(const AttnArgs &a, const ChunkLow *low, cudaStream_t stream) {
             p.flat.per = (int)per; p.flat.rem = (int)rem;
             p.flat.nslots = (int)nslots; p.flat.red_rows = R;
             p.q_bulk = (a.L == 1 && a.q_sh == a.D && ((uintptr_t)a.q & 15) == 0 && (a.q_sb * 2) % 16 == 0) ? 1 : 0;
+            size_t bytes = smem;
+            if (a.rope) {
+                // the query rows have to come by the bulk copy, and the row and the table need room behind them
+                if (!p.q_bulk || !a.new_k || a.rope->D != a.D || a.rope->dims > a.D) return 0;
+                p.rope_pairs = a.rope->dims / 2;
+                p.rope_traditional = a.rope->traditional;
+                p.rope_log2 = a.rope->log2_base_over_half;
+                p.rope_scale = a.rope->scale;
+                p.rope_position = a.rope->offset;
+                bytes += (size_t)a.D / 2 * sizeof(float2) + (size_t)a.D * 2;
+            }
             FlatSingle maps;
             maps.kmap = kmap; maps.vmap = vmap;
-#define KVC_FLAT(TT, DD, NS) launch_flat_typed<TT, DD, NS, false>(maps, p, (int)ctas, smem, stream)
+#define KVC_FLAT(TT, DD, NS)                                                                                       \
+    (a.rope ? launch_flat_typed<TT, DD, NS, false, true>(maps, p, (int)ctas, bytes, stream)                         \
+            : launch_flat_typed<TT, DD, NS, false, false>(maps, p, (int)ctas, bytes, stream))
             if (a.q_dtype == KVC_BF16) {
                 if (a.D == 64) KVC_FLAT(__nv_bfloat16, 64, 6);
                 else if (a.D == 128) KVC_FLAT(__nv_bfloat16, 128, 3);

@@ -1194,9 +1194,59 @@ static bool fused_append_off() {
     return off;
 }
 
+// Whether cache_attention will hand unturned rows to the decode kernel: its own conditions, and those of the kernel that
+// do not depend on what it allocates.
+bool cache_takes_rope(const kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v, int32_t mask_mode) {
+    if (fused_append_off() || c->open_round || mask_mode != KVC_MASK_NONE) return false;
+    if (c->cfg.kind != KVC_KIND_SIMPLE && c->cfg.kind != KVC_KIND_ROTATING) return false;
+    if (k.dtype != KVC_BF16 && k.dtype != KVC_F16) return false;
+    if (q.ndim != 4 || k.ndim != 4 || v.ndim != 4 || q.shape[2] != 1 || k.shape[2] != 1 || v.shape[2] != 1) return false;
+    if (v.dtype != k.dtype || q.dtype != k.dtype || k.stride[3] != 1 || v.stride[3] != 1 || q.stride[3] != 1) return false;
+    if (k.shape[0] != v.shape[0] || k.shape[1] != v.shape[1] || q.shape[0] != k.shape[0] || q.shape[3] != k.shape[3]) return false;
+    const int64_t D = q.shape[3], rep = k.shape[1] > 0 ? q.shape[1] / k.shape[1] : 0;
+    if ((D != 64 && D != 128 && D != 256) || rep < 1 || rep > 16 || q.shape[1] % k.shape[1]) return false;
+    auto rows = [](const kvc_tensor &t) { return !((uintptr_t)t.data & 15) && (t.stride[0] * 2) % 16 == 0 && (t.stride[1] * 2) % 16 == 0; };
+    return rows(q) && rows(k) && rows(v) && q.stride[1] == D;
+}
+
+namespace {
+// Queries and keys turned into memory of their own, where the decode kernel did not take them as they are.
+struct TurnedRows {
+    kvc_tensor q, k;
+    char *buf = nullptr;
+    cudaStream_t stream;
+    TurnedRows(const kvc_tensor &q_, const kvc_tensor &k_, const RopeArgs *rope, cudaStream_t s) : q(q_), k(k_), stream(s) {
+        if (!rope) return;
+        const size_t es = dtype_size(q.dtype);
+        auto elems = [](const kvc_tensor &t) { return (size_t)(t.shape[0] * t.shape[1] * t.shape[2] * t.shape[3]); };
+        const size_t q_bytes = (elems(q) * es + 255) / 256 * 256;
+        buf = (char *)dev_alloc(q_bytes + elems(k) * es, s);
+        RopeArgs a = *rope;
+        auto place = [&](kvc_tensor &t, char *at, RopeTensor &r) {
+            r.src = t.data; r.dst = at;
+            r.s_sb = t.stride[0]; r.s_sh = t.stride[1]; r.s_sl = t.stride[2];
+            r.B = (int32_t)t.shape[0]; r.H = (int32_t)t.shape[1]; r.L = (int32_t)t.shape[2];
+            t.data = at;
+            t.stride[3] = 1; t.stride[2] = t.shape[3]; t.stride[1] = t.shape[2] * t.stride[2]; t.stride[0] = t.shape[1] * t.stride[1];
+            r.d_sb = t.stride[0]; r.d_sh = t.stride[1]; r.d_sl = t.stride[2];
+        };
+        place(q, buf, a.q);
+        place(k, buf + q_bytes, a.k);
+        launch_rope(a, s);
+    }
+    TurnedRows(const TurnedRows &) = delete;
+    ~TurnedRows() { if (buf) dev_free(buf, stream); }
+    void queries_of(AttnArgs &a) const {
+        a.q = q.data;
+        a.q_sb = q.stride[0]; a.q_sh = q.stride[1]; a.q_sl = q.stride[2];
+        a.rope = nullptr;
+    }
+};
+}  // namespace
+
 void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v,
                      float scale, int32_t mask_mode, const kvc_tensor *mask, const kvc_tensor &out,
-                     cudaStream_t s) {
+                     cudaStream_t s, const RopeArgs *rope) {
     c->last_stream = s;
     require4(q, "queries");
     require4(k, "keys");
@@ -1256,8 +1306,11 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
                 a.stored_rows_settled = previous_spares(c) && k_before == ck.data;
                 a.nk_sb = k.stride[0]; a.nk_sh = k.stride[1];
                 a.nv_sb = v.stride[0]; a.nv_sh = v.stride[1];
+                a.rope = rope;
                 if (launch_attention_decode(a, s) > 0) return;
-                append_pair(c->k, c->v, k, v, prev, s);
+                const TurnedRows t(q, k, rope, s);
+                append_pair(c->k, c->v, t.k, v, prev, s);
+                t.queries_of(a);
                 a.new_k = a.new_v = nullptr;
                 launch_attention(a, s);
                 return;
@@ -1285,8 +1338,11 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
                 // no growth copy and no ring rebuild in this call: the stored rows are as the last step left them
                 a.stored_rows_settled = previous_spares(c) && k_before == ck.data &&
                                         launches_before == g_launch_count;
+                a.rope = rope;
                 if (slot >= 0 && slot < ck.shape[2] && launch_attention_decode(a, s) > 0) return;
-                append_pair(c->k, c->v, k, v, slot, s);
+                const TurnedRows t(q, k, rope, s);
+                append_pair(c->k, c->v, t.k, v, slot, s);
+                t.queries_of(a);
                 a.new_k = a.new_v = nullptr;
                 a.new_slot = -1;
                 a.stored_rows_settled = false;

@@ -151,7 +151,9 @@ void cache_attention_varlen(kvc_cache *const *caches, int n, const kvc_tensor *q
                             const kvc_tensor *v, float scale, const kvc_tensor *outs, cudaStream_t s);
 void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v,
                      float scale, int32_t mask_mode, const kvc_tensor *mask, const kvc_tensor &out,
-                     cudaStream_t s);
+                     cudaStream_t s, const RopeArgs *rope = nullptr);
+// Whether that call turns unturned queries and keys itself (`rope`).
+bool cache_takes_rope(const kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v, int32_t mask_mode);
 int64_t cache_trim(kvc_cache *c, int64_t n);
 bool cache_is_trimmable_after(const kvc_cache *c, int64_t positions);
 int cache_state_count(const kvc_cache *c);

@@ -1302,6 +1302,11 @@ kvc_status kvc_attention_rope(kvc_cache *cache, const kvc_tensor *q, const kvc_t
         DeviceGuard dg(cache ? cache->device : -1);
         // cache?.ropeOffset: the scalar cache offset (KVCache.swift:107-109), 0 without a cache
         const int64_t offset = cache ? cache->offset : 0;
+        if (cache && kvc::cache_takes_rope(cache, *q, *k, *v, mask_mode)) {
+            const kvc::RopeArgs a = rope_args(*rope, q->dtype, (int)q->shape[3], offset);
+            kvc::cache_attention(cache, *q, *k, *v, scale, mask_mode, mask, *out, s, &a);
+            return;
+        }
         const size_t es = kvc::dtype_size(q->dtype);
         const int64_t D = q->shape[3], L = q->shape[2];
         const size_t qn = (size_t)(q->shape[0] * q->shape[1] * L * D), kn = (size_t)(k->shape[0] * k->shape[1] * L * D);

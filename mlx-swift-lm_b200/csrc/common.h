@@ -129,6 +129,8 @@ struct AttnArgs {
     // written to the cache yet; the kernel scores them from here and stores them at token T - 1 itself.
     const void *new_k = nullptr, *new_v = nullptr;
     int64_t nk_sb = 0, nk_sh = 0, nv_sb = 0, nv_sh = 0;  // element strides (inner stride 1)
+    // With a fused append: the queries and the new key row are not turned yet (one position); the kernel turns both.
+    const struct RopeArgs *rope = nullptr;
     // Token index the new row is stored at: T - 1 (append at the end) unless the cache is a wrapped
     // ring, where it replaces the oldest row somewhere in the middle; that row is not attended.
     int64_t new_slot = -1;
