@@ -270,6 +270,16 @@ __device__ __forceinline__ void store_out(void *p, int32_t dtype, int64_t i, flo
     }
 }
 
+// Query row n of a group as head and position: a decode step has one position and needs no division.
+__device__ __forceinline__ void split_row(int n, int L, int &head, int &pos) {
+    head = n;
+    pos = 0;
+    if (L != 1) {
+        head = n / L;
+        pos = n - head * L;
+    }
+}
+
 // Four neighbouring elements, in one store where they lie on its boundary.
 __device__ __forceinline__ void store_out4(void *p, int32_t dtype, int64_t i, float4 v) {
     const uintptr_t at = (uintptr_t)p + (uintptr_t)(i * (dtype == KVC_F32 ? 4 : 2));
@@ -497,7 +507,9 @@ __device__ __forceinline__ void rotate_out_rows(const UnitOut &u, const float *r
                 x[j] = upper ? y - x[j] : x[j] + y;
             }
         }
-        const int hq = hk * rep + (row0 + r) / u.L, lq = (row0 + r) % u.L;
+        int hq, lq;
+        split_row(row0 + r, u.L, hq, lq);
+        hq += hk * rep;
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             const int d = E * lane + j;
@@ -570,7 +582,9 @@ __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *r
         if (u.o_signs) {
             *(float4 *)&work[r * D + d] = o;
         } else {
-            const int hq = hk * rep + (row0 + r) / u.L, lq = (row0 + r) % u.L;
+            int hq, lq;
+            split_row(row0 + r, u.L, hq, lq);
+            hq += hk * rep;
             store_out4(u.out, u.out_dtype, b * u.o_sb + hq * u.o_sh + lq * u.o_sl + d, o);
         }
     };
@@ -608,6 +622,41 @@ __device__ void segment_epilogue(const UnitOut &u, const Plan &f, const float *r
         __threadfence();
         // The (max, sum) pairs and the partial values of FLY slots are loaded together (eight where the kernel has no
         // registers for more), the weights are recomputed per thread; slots are merged eight at a time.
+        if (expected <= 4) {
+            // Few slots: two of a thread's elements at a time, so that their loads meet.
+            for (int i0 = tid; i0 < R * D4; i0 += 2 * NT) {
+                float2 ml[2][4];
+                float4 ov[2][4];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int i = i0 + e * NT, r = i / D4, d = i % D4 * 4;
+                    const int64_t at = (qrow0 + r) * f.nslots;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const bool in = i < R * D4 && j < expected;
+                        ml[e][j] = in ? __ldcg(&u.ml_part[at + j]) : make_float2(-INFINITY, 0.f);
+                        ov[e][j] = in ? __ldcg((const float4 *)&u.o_part[(at + j) * D + d]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int i = i0 + e * NT;
+                    if (i >= R * D4) break;
+                    float m = -INFINITY, lsum = 0.f;
+                    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) m = fmaxf(m, (ml[e][j].y > 0.f) ? ml[e][j].x : -INFINITY);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float fw = (ml[e][j].x == -INFINITY || ml[e][j].y <= 0.f) ? 0.f : fast_exp2(ml[e][j].x - m);
+                        lsum = fmaf(ml[e][j].y, fw, lsum);
+                        o.x = fmaf(ov[e][j].x, fw, o.x); o.y = fmaf(ov[e][j].y, fw, o.y);
+                        o.z = fmaf(ov[e][j].z, fw, o.z); o.w = fmaf(ov[e][j].w, fw, o.w);
+                    }
+                    finish(i / D4, i % D4 * 4, o, lsum);
+                }
+            }
+        } else
         for (int i = tid; i < R * D4; i += NT) {
             const int r = i / D4, d = i % D4 * 4;
             const float2 *mlp = u.ml_part + (qrow0 + r) * f.nslots;

@@ -155,8 +155,9 @@ attn_f32_kernel(const __grid_constant__ F32Params p, const __grid_constant__ F32
             const int r = i / D, d = i % D;
             float v = 0.f;
             if (r < R) {
-                const int rr = row0 + r, h = hk * rep + rr / p.L, l = rr % p.L;
-                v = sq.q[b * sq.q_sb + h * p.q_sh + l * p.q_sl + d];
+                int h, l;
+                split_row(row0 + r, p.L, h, l);
+                v = sq.q[b * sq.q_sb + (hk * rep + h) * p.q_sh + l * p.q_sl + d];
             }
             qs[r * SH::QROW + d + (d >= HALF ? 4 : 0)] = v;
         }

@@ -608,9 +608,10 @@ __device__ __forceinline__ void load_words(const uint32_t *src, uint32_t (&dst)[
 }
 
 // Flat tile x -> the unit (batch or sequence `b`, KV head `hk`) it belongs to, the tile index inside
-// the unit and the unit's tile count.
+// the unit and the unit's tile count. Lists: `first` holds the sequences' first flat tiles, `len` their tokens, both
+// in shared memory (looked up in the launch's parameters, the search cost 1 000 cycles a segment, 180 here).
 template <bool VARLEN, int TILE>
-__device__ __forceinline__ void resolve_unit(const AffineParams &p, const VarlenAttnTable &vt, int64_t x, int tiles,
+__device__ __forceinline__ void resolve_unit(const AffineParams &p, int n, const int *first, const int *len, int64_t x, int tiles,
                                              int &unit, int &tile, int &utiles, int &hk, int &b) {
     if (!VARLEN) {
         unit = flat_div(x, tiles);
@@ -622,12 +623,12 @@ __device__ __forceinline__ void resolve_unit(const AffineParams &p, const Varlen
         return;
     }
     int i = 0;
-    for (int step = 16; step >= 1; step >>= 1)   // largest i with Hkv * tile_prefix[i] <= x
-        if (i + step < vt.n && (int64_t)p.Hkv * vt.seq[i + step].tile_prefix <= x) i += step;
-    const int64_t base = (int64_t)p.Hkv * vt.seq[i].tile_prefix;
-    utiles = (vt.seq[i].T + TILE - 1) / TILE;
-    hk = flat_div(x - base, utiles);
-    tile = flat_mod(x - base, utiles, hk);
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1)   // largest i with first[i] <= x
+        if (i + step < n && first[i + step] <= (int)x) i += step;
+    utiles = (len[i] + TILE - 1) / TILE;
+    hk = flat_div((int)x - first[i], utiles);
+    tile = flat_mod((int)x - first[i], utiles, hk);
     b = i;
     unit = i * p.Hkv + hk;
 }
@@ -672,7 +673,14 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     uint64_t *qempty = qfull + 2;
     unsigned char *qbuf = (unsigned char *)(qempty + 2);                  // [2][red_rows][D] elements
 
+    int *seq_first = (int *)(qbuf + (size_t)2 * fp.red_rows * D * 2);    // lists: [32] first flat tiles
+    int *seq_len = seq_first + KVC_VARLEN_MAX;                           // and [32] tokens
+
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (VARLEN && tid < vt.n) {
+        seq_first[tid] = p.Hkv * vt.seq[tid].tile_prefix;
+        seq_len[tid] = vt.seq[tid].T;
+    }
     const int rep = p.Hq / p.Hkv;
     const int R_all = rep * p.L;   // query rows of a (batch, kv head) group; a unit carries up to eight of them
     const int tiles = fp.tiles;
@@ -711,7 +719,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             int it = 0, sg = 0;
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
                 int unit, tb, utiles, hk, b;
-                resolve_unit<VARLEN, P8_TILE>(p, vt, x, tiles, unit, tb, utiles, hk, b);
+                resolve_unit<VARLEN, P8_TILE>(p, vt.n, seq_first, seq_len, x, tiles, unit, tb, utiles, hk, b);
                 const int own = (int)min((int64_t)(utiles - tb), x_hi - x), n = VARLEN ? own : min(own, fp.real - tb);
                 if (p.q_bulk) {
                     const int qb = sg & 1;
@@ -739,7 +747,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                 }
                 // tokens of this unit that copies may touch: the stored rows rounded up to 256 (inside the
                 // slab by the launch checks); a tile of 240 tokens may end past them and is then cut short
-                const int64_t t_pad = ((VARLEN ? (int64_t)vt.seq[b].T : p.T) + 255) / 256 * 256;
+                const int64_t t_pad = ((VARLEN ? (int64_t)seq_len[b] : p.T) + 255) / 256 * 256;
                 for (int j = 0; j < n && ok; ++j, ++it) {
                     const int s = it % NSTAGE;
                     if (it >= NSTAGE) ok = mbar_wait(&empty[s], ((it / NSTAGE) - 1) & 1);
@@ -768,9 +776,9 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     int sg = 0;
     for (int64_t x = x_lo; x < x_hi; ++sg) {
         int unit, tile_begin, utiles, hk, b;
-        resolve_unit<VARLEN, P8_TILE>(p, vt, x, tiles, unit, tile_begin, utiles, hk, b);
+        resolve_unit<VARLEN, P8_TILE>(p, vt.n, seq_first, seq_len, x, tiles, unit, tile_begin, utiles, hk, b);
         const int own = (int)min((int64_t)(utiles - tile_begin), x_hi - x), ntiles = VARLEN ? own : min(own, fp.real - tile_begin);
-        const int64_t T_seq = VARLEN ? (int64_t)vt.seq[b].T : p.T;   // tokens of this unit's sequence
+        const int64_t T_seq = VARLEN ? (int64_t)seq_len[b] : p.T;   // tokens of this unit's sequence
         const int row0 = VARLEN ? 0 : (unit % p.chunks) * 8;         // first query row of the group this unit carries
         const int R = min(8, R_all - row0);
         // per-lane state for query rows 2c and 2c+1
@@ -798,6 +806,31 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             }
             q_stage = (const T *)(qbuf + (size_t)qslot * q_bytes);
         }
+        // a lane's dims of a group are neighbours: as 16-byte loads of the staged rows, else one by one
+        constexpr int LD = GROUP / 4;                 // dims
+        uint32_t qraw[G][LD / 2];
+#pragma unroll
+        for (int gr = 0; gr < G; ++gr) {
+#pragma unroll
+            for (int i = 0; i < LD / 2; ++i) qraw[gr][i] = 0u;
+            if (g >= R || !ok) continue;
+            const int d0 = gr * GROUP + c * LD;
+            if (q_stage) {
+#pragma unroll
+                for (int i = 0; i < LD / 8; ++i) {
+                    const uint4 v = *(const uint4 *)(q_stage + g * D + d0 + 8 * i);
+                    qraw[gr][4 * i] = v.x; qraw[gr][4 * i + 1] = v.y; qraw[gr][4 * i + 2] = v.z; qraw[gr][4 * i + 3] = v.w;
+                }
+            } else {
+                int hq, l;
+                split_row(row0 + g, p.L, hq, l);
+                hq += hk * rep;
+                const uint16_t *qp = VARLEN ? (const uint16_t *)vt.seq[b].q + hq * p.q_sh + l * p.q_sl
+                                            : (const uint16_t *)p.q + b * p.q_sb + hq * p.q_sh + l * p.q_sl;
+#pragma unroll
+                for (int i = 0; i < LD / 2; ++i) qraw[gr][i] = (uint32_t)qp[d0 + 2 * i] | (uint32_t)qp[d0 + 2 * i + 1] << 16;
+            }
+        }
         uint32_t qb[G][MPG][2];
         float qsum_own[G];
 #pragma unroll
@@ -807,16 +840,12 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
 #pragma unroll
             for (int m = 0; m < MPG; ++m) {
                 int dd[4];
-                kslot_dims<BITS>(gr * WPG + c * WPL + m / MPW, m % MPW, dd);
-                float x[4] = {0.f, 0.f, 0.f, 0.f};
-                if (g < R && ok) {
-                    const int hq = hk * rep + (row0 + g) / p.L, l = (row0 + g) % p.L;
-                    const T *qp = q_stage ? q_stage + g * D
-                                  : VARLEN ? (const T *)vt.seq[b].q + hq * p.q_sh + l * p.q_sl
-                                           : (const T *)p.q + b * p.q_sb + hq * p.q_sh + l * p.q_sl;
+                kslot_dims<BITS>(m / MPW, m % MPW, dd);   // relative to the lane's first dim of the group
+                float x[4];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        x[k] = __half2float(__float2half_rn(to_f32<T>(qp[dd[k]]) * p.scale_log2));
+                for (int k = 0; k < 4; ++k) {
+                    const float2 two = MmaType<T>::unpack(qraw[gr][dd[k] / 2]);
+                    x[k] = __half2float(__float2half_rn(((dd[k] & 1) ? two.y : two.x) * p.scale_log2));
                 }
                 qb[gr][m][0] = pack_h2(x[0] * LOWMUL, x[1] * LOWMUL);   // k-slots 2c, 2c+1
                 qb[gr][m][1] = pack_h2(x[2], x[3]);                     // k-slots 2c+8, 2c+9
@@ -846,7 +875,8 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int r = 2 * c + k;
-            const int l = (r < R) ? (row0 + r) % p.L : 0;
+            int hq, l = 0;
+            if (r < R) split_row(row0 + r, p.L, hq, l);
             row_limit[k] = p.causal ? (int)min((int64_t)t_last, p.causal_offset + l) : t_last;
         }
         const int min_limit = p.causal ? (int)min((int64_t)t_last, p.causal_offset) : t_last;
@@ -1130,7 +1160,7 @@ void launch_affine8_typed(const AffineParams &p, const VarlenAttnTable &vt, int 
     constexpr int STAGE_BYTES = 2 * P8_TILE * RB + 4 * P8_TILE * G * 2;
     const size_t red = (size_t)P8_WARPS * p.flat.red_rows * (D + 8) * 4 + (size_t)P8_WARPS * p.flat.red_rows * 8 + 32 +
                        16 + 4 * sizeof(uint64_t) +
-                       (size_t)2 * p.flat.red_rows * D * 2;
+                       (size_t)2 * p.flat.red_rows * D * 2 + (VARLEN ? 2 * KVC_VARLEN_MAX * sizeof(int) : 0);
     const size_t smem = (size_t)NSTAGE * STAGE_BYTES + 16 + 2 * NSTAGE * sizeof(uint64_t) + 64 + red + 128;
     static size_t configured[64] = {0};
     const int dev = current_device();

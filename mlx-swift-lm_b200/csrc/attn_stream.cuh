@@ -471,8 +471,9 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
             const int r = i / D, d = i % D;
             float v = 0.f;
             if (r < R) {
-                const int rr = row0 + r, h = sg.hk * rep + rr / p.L, l = rr % p.L;
-                v = to_f32<T>(qp[h * p.q_sh + l * p.q_sl + d]);
+                int h, l;
+                split_row(row0 + r, p.L, h, l);
+                v = to_f32<T>(qp[(sg.hk * rep + h) * p.q_sh + l * p.q_sl + d]);
                 if (K::TURBO) v *= q_signs[d];
             }
             qs[i] = v;

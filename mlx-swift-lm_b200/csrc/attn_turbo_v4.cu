@@ -328,7 +328,9 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
             const int r = warp;
             float x[4] = {0.f, 0.f, 0.f, 0.f};
             if (r < R && ok) {
-                const int hq = hk * rep + (row0 + r) / p.L, l = (row0 + r) % p.L;
+                int hq, l;
+                split_row(row0 + r, p.L, hq, l);
+                hq += hk * rep;
                 const T *src = q_stage ? q_stage + r * D : (const T *)p.q + b * p.q_sb + hq * p.q_sh + l * p.q_sl;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) x[j] = to_f32<T>(src[4 * lane + j]) * p.q_signs[4 * lane + j];
@@ -377,7 +379,8 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int r = 2 * c + k;
-            const int l = (r < R) ? (row0 + r) % p.L : 0;
+            int hq, l = 0;
+            if (r < R) split_row(row0 + r, p.L, hq, l);
             row_limit[k] = p.causal ? (int)min((int64_t)t_last, p.causal_offset + l) : t_last;
         }
         const int min_limit = p.causal ? (int)min((int64_t)t_last, p.causal_offset) : t_last;
