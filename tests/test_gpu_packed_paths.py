@@ -384,6 +384,28 @@ def test_decode_at_every_context_length_around_the_stage_boundaries(kvc, oracle,
     assert kvc.lib().kvc_device_status() == 0
 
 
+@pytest.mark.parametrize("dtype,B,Hq,Hkv,kb,vb,P,L,written", [
+    (torch.bfloat16, 1, 32, 8, 3, 4, 47, 17, False),      # 64 keys: one tile, decoded in the tile loop
+    (torch.bfloat16, 1, 32, 8, 3, 4, 48, 17, True),       # 65
+    (torch.float16, 2, 28, 4, 2, 2, 111, 10, True),       # 70 rows of a group
+    (torch.float16, 3, 8, 8, 4, 2, 130, 65, True),        # one head a group, 65 positions
+    (torch.bfloat16, 1, 64, 8, 3, 3, 1000, 33, True),
+])
+def test_short_turbo_chunk_with_rows_written_out(kvc, oracle, cuda, capfd, monkeypatch, dtype, B, Hq, Hkv, kb, vb, P, L, written):
+    """Short chunks over TurboQuant caches: which kernels take them, and the stated 2e-2 plus one spacing of the store."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    D = 128
+    g, o = _caches(kvc, oracle, cuda, dtype, dict(key_bits=kb, value_bits=vb), B, Hkv, D, P)
+    q, k1, v1 = seeded((B, Hq, L, D), 3, dtype), seeded((B, Hkv, L, D), 4, dtype), seeded((B, Hkv, L, D), 5, dtype)
+    capfd.readouterr()
+    out = g.attention(q.to(cuda), k1.to(cuda), v1.to(cuda), D ** -0.5, "causal")
+    torch.cuda.synchronize()
+    assert ("rows written out" in capfd.readouterr().err) == written
+    ref = oracle.attention_with_cache_update(to_oracle(q), to_oracle(k1), to_oracle(v1), o, D ** -0.5, "causal")
+    assert worst_excess(out, ref, dtype) <= 0
+    assert kvc.lib().kvc_device_status() == 0
+
+
 @pytest.mark.parametrize("dtype,kw,Hq,Hkv,D,P,L", [
     (torch.float16, dict(key_bits=8, value_bits=4), 8, 2, 128, 1, 1),       # a single cached row
     (torch.bfloat16, dict(key_bits=8, value_bits=3), 28, 4, 128, 61, 1),    # 62 rows: the last block is short
