@@ -72,8 +72,6 @@ __device__ __forceinline__ void store_pair(__half *high, __half *low, const floa
 // The largest finite magnitude the decoded rows of a (batch, KV head) can hold; z as in pair_rows_kernel.
 template <typename T>
 __global__ void __launch_bounds__(256) pair_top_kernel(const __grid_constant__ PairRows p) {
-    dev::pdl_wait();
-    dev::pdl_trigger();
     const int per = 2 - p.first, which = p.first + blockIdx.z % per, b = blockIdx.z / per, h = blockIdx.y;
     const PairSource &s = p.s[which];
     if (s.kind == SRC_RAW) return;
@@ -103,8 +101,6 @@ __global__ void __launch_bounds__(256) pair_top_kernel(const __grid_constant__ P
 // One thread = eight consecutive head dims of one token of K or V. T: type of scales and biases.
 template <typename T>
 __global__ void __launch_bounds__(256) pair_rows_kernel(const __grid_constant__ PairRows p) {
-    dev::pdl_wait();
-    dev::pdl_trigger();
     const int per = 2 - p.first, which = p.first + blockIdx.z % per, b = blockIdx.z / per, h = blockIdx.y;
     const PairSource &s = p.s[which];
     const int per_row = p.D / 8;
@@ -159,8 +155,6 @@ struct PairTurn {
 };
 template <typename TI, typename TO, int D>
 __global__ void __launch_bounds__(256) pair_turn_kernel(const __grid_constant__ PairTurn p) {
-    dev::pdl_wait();
-    dev::pdl_trigger();
     constexpr int E = D / 32;
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -218,9 +212,9 @@ __global__ void __launch_bounds__(256) pair_turn_kernel(const __grid_constant__ 
 template <typename TI, typename TO>
 void pair_turn(const PairTurn &p, int D, cudaStream_t stream) {
     const unsigned blocks = (unsigned)(((int64_t)p.B * p.H * p.L + 7) / 8);
-    if (D == 256) KVC_CUDA(launch_pdl(pair_turn_kernel<TI, TO, 256>, dim3(blocks), dim3(256), 0, stream, p));
-    else if (D == 128) KVC_CUDA(launch_pdl(pair_turn_kernel<TI, TO, 128>, dim3(blocks), dim3(256), 0, stream, p));
-    else KVC_CUDA(launch_pdl(pair_turn_kernel<TI, TO, 64>, dim3(blocks), dim3(256), 0, stream, p));
+    if (D == 256) pair_turn_kernel<TI, TO, 256><<<blocks, 256, 0, stream>>>(p);
+    else if (D == 128) pair_turn_kernel<TI, TO, 128><<<blocks, 256, 0, stream>>>(p);
+    else pair_turn_kernel<TI, TO, 64><<<blocks, 256, 0, stream>>>(p);
     KVC_CUDA(cudaGetLastError());
     ++g_launch_count;
 }
@@ -320,11 +314,11 @@ int launch_attention_chunk_packed_pairs(const AttnArgs &a, cudaStream_t stream) 
         const dim3 grid((unsigned)((a.T * (a.D / 8) + 255) / 256), (unsigned)a.Hkv, planes);
         const dim3 tops((unsigned)std::min<int64_t>((a.T + 255) / 256, 64), (unsigned)a.Hkv, planes);
         if (bf16) {
-            KVC_CUDA(launch_pdl(pair_top_kernel<__nv_bfloat16>, tops, dim3(256), 0, stream, pr));
-            KVC_CUDA(launch_pdl(pair_rows_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, pr));
+            pair_top_kernel<__nv_bfloat16><<<tops, 256, 0, stream>>>(pr);
+            pair_rows_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(pr);
         } else {
-            KVC_CUDA(launch_pdl(pair_top_kernel<__half>, tops, dim3(256), 0, stream, pr));
-            KVC_CUDA(launch_pdl(pair_rows_kernel<__half>, grid, dim3(256), 0, stream, pr));
+            pair_top_kernel<__half><<<tops, 256, 0, stream>>>(pr);
+            pair_rows_kernel<__half><<<grid, 256, 0, stream>>>(pr);
         }
         KVC_CUDA(cudaGetLastError());
         g_launch_count += 2;

@@ -259,7 +259,7 @@ struct StreamShape {
     static constexpr int ROWS = 8 * NB;
     static constexpr int RED_STRIDE = D + 4;
     static constexpr int QS = ROWS * D * 4;                       // staged query rows
-    static constexpr int HEAD = 128;                              // merge flag, one factor per query row
+    static constexpr int HEAD = 32 + ROWS * 4 > 128 ? 256 : 128;  // merge flag, one factor per query row
     static constexpr int fixed(int warps) {
         const int red = warps * ROWS * (RED_STRIDE + 2) * 4 + ROWS * D * 4, rings = warps * WARP_BYTES;
         return (rings > red ? rings : red) + QS + HEAD;           // the merge buffers reuse the ring
@@ -1030,9 +1030,16 @@ int run_stream(const AttnArgs &a, StreamParams p, StreamList *list, cudaStream_t
 }
 
 // Up to eight rows per KV head: one column block. More: two column blocks share one unpacking where the
-// accumulators fit the registers (D <= 128), else units of eight rows.
+// accumulators fit the registers (D <= 128), else units of eight rows. At head dim 64 four blocks, but only where a CTA
+// walks many tiles (the line: 128 an SM): a verify round of 28 rows over 30 x 17 642 tokens, 3-bit keys and 4-bit values, takes
+// 460 us in units of sixteen rows and 399 in units of 32; over 4 x 1 500 tokens the longer start of a segment costs more
+// than the second unpacking (two layers: 38 us and 45).
 template <typename T, int D, int KK, int VK, int UNIT>
 int run_stream_rows(const AttnArgs &a, const StreamParams &p, StreamList *list, cudaStream_t stream) {
+    if constexpr (D == 64) {
+        const int64_t tiles = (int64_t)(list ? list->n : 1) * a.B * a.Hkv * ((a.T + ST_TILE - 1) / ST_TILE);
+        if (a.Hq / a.Hkv * a.L > 16 && tiles >= 128 * (int64_t)sm_count(a.device)) return run_stream<T, D, KK, VK, UNIT, 4>(a, p, list, stream);
+    }
     if constexpr (D <= 128)
         if (a.Hq / a.Hkv * a.L > 8) return run_stream<T, D, KK, VK, UNIT, 2>(a, p, list, stream);
     return run_stream<T, D, KK, VK, UNIT, 1>(a, p, list, stream);

@@ -313,6 +313,11 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
         const int R = CHUNKED ? min(8, R_all - row0) : R_all;
         // ---- rotated queries of this unit: q' = H(signs * q) / sqrt(D) * scale * log2(e), rows past R zero ----
         const T *q_stage = nullptr;
+        float sgn[4] = {0.f, 0.f, 0.f, 0.f};      // on their way while the rows are waited for
+        if (warp < 8) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sgn[j] = p.q_signs[4 * lane + j];
+        }
         if (p.q_bulk) {
             if (ok && !(KVC_SKIP_BITS(p) & 2)) {
                 ok = mbar_wait(&qfull[sg & 1], (sg >> 1) & 1);
@@ -333,7 +338,7 @@ attn_turbo_v4_kernel(const __grid_constant__ TurboV4Params p) {
                 hq += hk * rep;
                 const T *src = q_stage ? q_stage + r * D : (const T *)p.q + b * p.q_sb + hq * p.q_sh + l * p.q_sl;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) x[j] = to_f32<T>(src[4 * lane + j]) * p.q_signs[4 * lane + j];
+                for (int j = 0; j < 4; ++j) x[j] = to_f32<T>(src[4 * lane + j]) * sgn[j];
             }
             {
                 const float a0 = x[0] + x[1], a1 = x[0] - x[1], a2 = x[2] + x[3], a3 = x[2] - x[3];
