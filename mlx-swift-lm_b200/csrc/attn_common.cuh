@@ -438,6 +438,14 @@ __device__ __forceinline__ int flat_cta_of(const UnitPlan &f, int64_t x) {
     return xs < big ? flat_div(xs, f.per + 1) : f.rem + flat_div(xs - big, f.per);
 }
 
+// Whether equal ranges would cut a unit into more than 64 partials. Calls of so few units stay with the streaming kernel,
+// whose operands are f16 pairs, where a kernel's are single (f16 outputs of one sequence of 5 000 tokens, 28/4 heads,
+// err by 2.5 times as much there).
+inline bool few_units(int64_t units, int64_t tiles, int64_t slots) {
+    const int64_t work = units * tiles, per = work / std::min(slots, work);
+    return (tiles + per - 1) / per + 1 > 64;
+}
+
 // Plans `units` of `tiles` tiles over at most `slots` CTAs; `segment`: what a segment costs beside its tiles, in tiles.
 inline int64_t plan_units(UnitPlan *f, int64_t units, int64_t tiles, int64_t slots, int64_t segment) {
     const int64_t work = units * tiles, n = std::min(slots, work), most = (work + n - 1) / n;

@@ -1272,6 +1272,7 @@ int launch_attention_affine_varlen(const AttnArgs *args, int n, cudaStream_t str
     p.flat.per = (int)(work_tiles / ctas);
     p.flat.rem = (int)(work_tiles % ctas);
     p.flat.nslots = (int)((max_tiles + p.flat.per - 1) / p.flat.per + 1);
+    if (p.flat.nslots > 64) return 0;
     p.flat.red_rows = rep;
     p.q_bulk = a0.q_sh == a0.D ? 1 : 0;
     for (int i = 0; i < n; ++i)
@@ -1368,6 +1369,11 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     UnitPlan plan;
     const int64_t flat_ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * flat_resident, P8_SEGMENT);
     const int64_t flat_slots = plan.nslots;
+    // 8-bit codes in one group a row and at most two query rows: three CTAs an SM, and outputs that differ from run to run by up
+    // to 13 % of a row (4 sequences of 5 000 tokens, 16/8 heads; other row counts and groups agree with 64-bit sums). The
+    // cause is not found, so the streaming kernel takes these calls.
+    if (decode8 && a.k.bits == 8 && a.k.group == 128 && a.D == 128 && rep * a.L <= 2) return 0;
+    if (decode8 && few_units(bh, tiles, (int64_t)sm_count(a.device) * flat_resident)) return 0;
     const int64_t splits = decode8 ? flat_slots : best_s;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
     const size_t o_bytes = (size_t)qrows * splits * a.D * sizeof(float);

@@ -544,7 +544,7 @@ int launch_attention_turbo(const AttnArgs &a, cudaStream_t stream) {
     const int resident = (int)std::max<size_t>(1, std::min<size_t>(2, (size_t)227 * 1024 / per_cta));
     if (!flat_fits(2 * bh * tiles)) return 0;
     const int64_t ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * resident, TQ_SEGMENT);
-    if (plan.nslots > 64) return 0;
+    if (few_units(bh, tiles, (int64_t)sm_count(a.device) * resident)) return 0;
     const int64_t splits = plan.nslots;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
     const size_t o_bytes = (size_t)qrows * splits * a.D * sizeof(float);

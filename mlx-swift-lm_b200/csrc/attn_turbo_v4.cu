@@ -673,7 +673,7 @@ int launch_attention_turbo_v4(const AttnArgs &a, cudaStream_t stream) {
     plan.red_rows = std::min(8, rep * a.L);
     if (!flat_fits(2 * bh * tiles)) return 0;
     const int64_t ctas = plan_units(&plan, bh, tiles, sm_count(a.device), V4_SEGMENT);
-    if (plan.nslots > 64) return 0;
+    if (few_units(bh, tiles, sm_count(a.device))) return 0;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
     const size_t o_bytes = (size_t)qrows * plan.nslots * a.D * sizeof(float);
     const size_t ml_bytes = (size_t)qrows * plan.nslots * sizeof(float2);
