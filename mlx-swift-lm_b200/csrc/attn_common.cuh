@@ -91,6 +91,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     return false;
 }
 
+// A consumer warp gives ring entry `bar` back to the copies that fill it. An arrival orders this warp's reads before other
+// threads' loads and stores, but not before a bulk or TMA copy (the async proxy): loads whose values are still on their way
+// were overtaken by the copy of a later tile (8-bit codes in one group a row, three CTAs an SM: every run gave other outputs,
+// off by up to 20 % of a row). So the reads are either fenced off ...
+__device__ __forceinline__ void release_fenced(uint64_t *bar, int lane) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+// ... or the arrival's address is made to need them: `read` joins words that came out of the last loads (those before came back
+// before them), `none` is zero and not known to the compiler. A kernel whose later shared loads or stores need every value
+// that it took from the entry has waited for them already, and arrives as it is.
+__device__ __forceinline__ void release_after(uint64_t *bar, int lane, uint32_t read, uint32_t none) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive((uint64_t *)((unsigned char *)bar + (read & none)));
+}
+
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y,
                                             int z, int w) {
     asm volatile(

@@ -293,8 +293,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                     MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa, vf[2], vf[3]);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            release_fenced(&empty[s], lane);
         }
         if (!ok && lane == 0) atomicExch(p.status, 2);
     }
@@ -861,8 +860,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                     MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa, vf[2], vf[3]);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            release_fenced(&empty[s], lane);
         }
 
         if (fused && warp == 0 && w.last && !(KVC_SKIP_BITS(p) & 32)) {
@@ -1429,8 +1427,7 @@ attn_chunk_kernel(const __grid_constant__ std::conditional_t<PAIRS, ChunkPairMap
                     }
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            release_fenced(&empty[s], lane);
         }
         if (!ok && lane == 0) atomicExch(p.status, 4);
 

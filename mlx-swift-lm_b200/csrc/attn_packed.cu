@@ -405,8 +405,7 @@ attn_affine_kernel(const AffineParams p) {
                     }
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            release_fenced(&empty[s], lane);
         }
         if (!ok && lane == 0) atomicExch(p.status, 4);
     }
@@ -712,6 +711,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
 
     bool ok = true;
     const int g = lane >> 2, c = lane & 3;
+    const uint32_t none = gridDim.y - 1;
 
     if (warp == P8_WARPS) {
         // ---------------- producer: one stream of tiles across the segments ----------------
@@ -864,10 +864,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             qsum[0][gr] = __shfl_sync(0xffffffffu, v, (2 * c) * 4);
             qsum[1][gr] = __shfl_sync(0xffffffffu, v, (2 * c + 1) * 4);
         }
-        if (p.q_bulk) {
-            __syncwarp();
-            if (ok && lane == 0) mbar_arrive(&qempty[sg & 1]);
-        }
+        if (p.q_bulk && ok) release_fenced(&qempty[sg & 1], lane);
         // Last visible token per row. Rows past R hold zero queries and are never written
         // out; they take the limit of a real row so that they do not force the mask path.
         int row_limit[2];
@@ -1050,10 +1047,12 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             }
             // ---- O^T += codes^T . P'^T (subnormal operands; the 2^24 / 2^20 leaves in the epilogue) ----
             const uint32_t v_row = smem_u32(vct + v_off);
+            uint32_t read = __float_as_uint(bsum[0][G - 1]) | __float_as_uint(bsum[1][G - 1]);
 #pragma unroll
             for (int cp = 0; cp < CH / 2; ++cp) {
                 uint32_t vf[4];
                 ldmatrix_x4_trans(vf, v_row + cp * 32);
+                read |= vf[3];
                 constexpr int dims_per_pair = 2 * 8 * EPU;
                 const int gr = (cp * dims_per_pair) / GROUP;
                 const UnitPair<BITS> u0(vf[0]), u1(vf[1]), u2(vf[2]), u3(vf[3]);
@@ -1067,8 +1066,10 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                     mma_f16(o_acc[cp * EPU + i], a, pb[gr][0], pb[gr][1]);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            // 8-bit codes: waiting for the values costs less than the fence, 4-bit ones: more (layer of 16 x 12 000 tokens,
+            // 64/8 heads, 8 bits: 89.6 us and 94.2; 4 bits: 53.4 and 52.6, where arrivals that may be overtaken take 52.2)
+            if constexpr (BITS == 8) release_after(&empty[s], lane, read, none);
+            else release_fenced(&empty[s], lane);
         }
         // a warp whose tokens were all masked reports "no maximum"
         if (m_run[0] <= M_INIT) m_run[0] = -INFINITY;
@@ -1369,9 +1370,8 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     UnitPlan plan;
     const int64_t flat_ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * flat_resident, P8_SEGMENT);
     const int64_t flat_slots = plan.nslots;
-    // 8-bit codes in one group a row and at most two query rows: three CTAs an SM, and outputs that differ from run to run by up
-    // to 13 % of a row (4 sequences of 5 000 tokens, 16/8 heads; other row counts and groups agree with 64-bit sums). The
-    // cause is not found, so the streaming kernel takes these calls.
+    // 8-bit codes in one group a row and at most two query rows: the streaming kernel's operand pairs err by a third as much and
+    // take as long (4 sequences of 5 000 tokens, 16/8 heads: 2.1e-4 and 6.7e-4 of the output, 19.9 us and 19.2).
     if (decode8 && a.k.bits == 8 && a.k.group == 128 && a.D == 128 && rep * a.L <= 2) return 0;
     if (decode8 && few_units(bh, tiles, (int64_t)sm_count(a.device) * flat_resident)) return 0;
     const int64_t splits = decode8 ? flat_slots : best_s;

@@ -503,6 +503,46 @@ def _caches(kvc, oracle, cuda, dtype, kw, B, Hkv, D, P, gain=1.0):
     return g, o
 
 
+@pytest.mark.parametrize("dtype,kw,Hq,lists", [
+    *[(torch.float16, dict(bits=b, group=gr), Hq, False) for b, gr in ((8, 128), (8, 64), (8, 32), (4, 64), (4, 128)) for Hq in (8, 16, 24, 32)],
+    (torch.bfloat16, dict(bits=8, group=128), 24, False),
+    (torch.float16, dict(bits=4, group=64), 80, False),         # ten rows a group
+    (torch.float16, dict(bits=8, group=64), 24, True),          # independent sequences
+    (torch.float16, dict(bits=4, group=64), 24, True),
+    (torch.float16, dict(key_bits=3, value_bits=4), 24, False),
+    (torch.float16, dict(key_bits=4, value_bits=2), 24, False),
+])
+def test_ring_entries_are_read_before_they_are_filled_again(kvc, oracle, cuda, dtype, kw, Hq, lists):
+    """Contexts that walk the rings of packed tiles several times, out of L2, where a copy is back soonest: run after run
+    the same bits, and every row within 2^-7 of the oracle's sums (a 16-bit query, weight and store err by up to 2^-11
+    each for f16, a bf16 store by 2^-9; sums over 9 000 tokens keep the ratio; a lost tile of 64 tokens is 2^-3.6)."""
+    B, Hkv, D, P = 2, 8, 128, 9000
+    n = B if lists else 1
+    g, o = [], []
+    for i in range(n):
+        a, b = _caches(kvc, oracle, cuda, dtype, kw, B // n, Hkv, D, P - i)
+        g.append(a)
+        o.append(b)
+    q, k1, v1 = seeded((B, Hq, 1, D), 3, dtype), seeded((B, Hkv, 1, D), 4, dtype), seeded((B, Hkv, 1, D), 5, dtype)
+    dq, dk, dv = ([t.to(cuda)[i:i + B // n] for i in range(n)] for t in (q, k1, v1))
+    runs = []
+    for _ in range(12):
+        outs = [torch.empty_like(t) for t in dq]
+        if lists:
+            kvc.DecodeStep(g, dq, dk, dv, outs, D ** -0.5).run_varlen()
+        else:
+            outs[0].copy_(g[0].attention(dq[0], dk[0], dv[0], D ** -0.5))
+        runs.append(torch.cat(outs).cpu())
+        kvc.trim_prompt_cache(g, 1)
+    assert all(torch.equal(r, runs[0]) for r in runs[1:])
+    for i in range(n):
+        at = slice(i * (B // n), (i + 1) * (B // n))
+        ref = torch.from_numpy(oracle_f32(oracle.attention_with_cache_update(
+            to_oracle(q.float()[at]), to_oracle(k1[at]), to_oracle(v1[at]), o[i], D ** -0.5))).double()
+        assert float(((runs[0][at].double() - ref).norm(dim=-1) / ref.norm(dim=-1)).max()) <= 2.0 ** -7
+    assert kvc.lib().kvc_device_status() == 0
+
+
 @pytest.mark.parametrize("dtype,kw,Hq,Hkv,D,P,L,mask", [
     (torch.float16, dict(key_bits=8, value_bits=4), 32, 8, 128, 700, 1, "none"),       # stream kernel: two MMAs a key, three a value
     (torch.float16, dict(key_bits=0, value_bits=3), 8, 4, 256, 700, 1, "none"),
