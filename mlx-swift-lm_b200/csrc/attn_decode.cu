@@ -744,8 +744,8 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                     qa[ks][2 + half] = w.y;
                 }
             }
-            __syncwarp();
-            if (!LIST && ok && lane == 0) mbar_arrive(&qempty[qb]);
+            // (the rows turned in place above are stores that the next copy into the slot comes after, too)
+            if (!LIST && ok) release_fenced(&qempty[qb], lane);
         } else
 #pragma unroll
         for (int ks = 0; ks < KSTEPS; ++ks) {

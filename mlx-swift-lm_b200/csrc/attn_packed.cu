@@ -1047,7 +1047,9 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             }
             // ---- O^T += codes^T . P'^T (subnormal operands; the 2^24 / 2^20 leaves in the epilogue) ----
             const uint32_t v_row = smem_u32(vct + v_off);
-            uint32_t read = __float_as_uint(bsum[0][G - 1]) | __float_as_uint(bsum[1][G - 1]);
+            uint32_t read = 0;
+#pragma unroll
+            for (int gr = 0; gr < G; ++gr) read |= __float_as_uint(bsum[0][gr]) | __float_as_uint(bsum[1][gr]);
 #pragma unroll
             for (int cp = 0; cp < CH / 2; ++cp) {
                 uint32_t vf[4];

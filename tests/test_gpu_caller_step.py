@@ -185,26 +185,32 @@ def test_chained_rope_steps_are_rope_then_attention(kvc, cuda, ring, P, D):
         assert s.offset == t.offset and all(torch.equal(m, n) for m, n in zip(s.state, t.state))
 
 
-@pytest.mark.parametrize("dtype,Hq,Hkv,D,dims,traditional,rope_scale,B,shift", [
-    (torch.bfloat16, 8, 2, 128, 128, True, 1.0, 2, 0),
-    (torch.float16, 4, 4, 64, 32, False, 0.5, 3, 0),        # half the dims turn
-    (torch.bfloat16, 16, 1, 256, 2, True, 1.0, 1, 0),       # a single pair, the most rows of a group
-    (torch.float16, 20, 1, 128, 128, False, 1.0, 1, 0),     # more rows than the decode kernel takes
-    (torch.bfloat16, 8, 2, 128, 96, False, 8.0, 2, 4),      # queries off a 16-byte boundary
+@pytest.mark.parametrize("dtype,Hq,Hkv,D,dims,traditional,rope_scale,B,P,shift,one", [
+    (torch.bfloat16, 8, 2, 128, 128, True, 1.0, 2, 70, 0, True),
+    (torch.float16, 4, 4, 64, 32, False, 0.5, 3, 70, 0, True),        # half the dims turn
+    (torch.bfloat16, 4, 1, 256, 2, True, 1.0, 1, 70, 0, True),        # a single pair
+    (torch.bfloat16, 16, 8, 128, 128, False, 1.0, 128, 50, 0, True),  # CTAs of several units: the slots of the query rows come round
+    (torch.float16, 8, 4, 256, 256, False, 1.0, 128, 50, 0, True),
+    (torch.bfloat16, 16, 1, 256, 2, True, 1.0, 1, 70, 0, False),       # more rows than shared memory holds
+    (torch.float16, 20, 1, 128, 128, False, 1.0, 1, 70, 0, False),     # more rows than the decode kernel takes
+    (torch.bfloat16, 8, 2, 128, 96, False, 8.0, 2, 70, 4, False),      # queries off a 16-byte boundary: turned into memory of their own
 ])
-def test_rope_inside_the_decode_kernel(kvc, cuda, dtype, Hq, Hkv, D, dims, traditional, rope_scale, B, shift):
+def test_rope_inside_the_decode_kernel(kvc, cuda, dtype, Hq, Hkv, D, dims, traditional, rope_scale, B, P, shift, one):
     """One launch that turns its own rows, or the launches it replaces: the bits of turning q and k first."""
     a, b = kvc.KVCacheSimple(), kvc.KVCacheSimple()
     for c in (a, b):
-        c.update(seeded((B, Hkv, 70, D), 1, dtype).to(cuda), seeded((B, Hkv, 70, D), 2, dtype).to(cuda))
+        c.update(seeded((B, Hkv, P, D), 1, dtype).to(cuda), seeded((B, Hkv, P, D), 2, dtype).to(cuda))
     for step in range(3):
         q = torch.empty(B * Hq * D + 8, dtype=dtype, device=cuda)[shift:shift + B * Hq * D].view(B, Hq, 1, D)
         q.copy_(seeded((B, Hq, 1, D), 10 + step, dtype).to(cuda))
         k, v = seeded((B, Hkv, 1, D), 20 + step, dtype).to(cuda), seeded((B, Hkv, 1, D), 30 + step, dtype).to(cuda)
         kept = q.clone(), k.clone()
+        kvc.launch_count(reset=True)
         x = kvc.attention_rope(q, k, v, a, {"dims": dims, "base": 10000.0, "traditional": traditional, "scale": rope_scale}, D ** -0.5)
+        assert (kvc.launch_count() == 1) == one
         assert torch.equal(q, kept[0]) and torch.equal(k, kept[1])
         rope = lambda t: kvc.rope(t, b.offset, dims, traditional=traditional, base=10000.0, scale=rope_scale)
         y = b.attention(rope(q), rope(k), v, D ** -0.5)
         assert torch.equal(x, y)
     assert a.offset == b.offset and all(torch.equal(m, n) for m, n in zip(a.state, b.state))
+    assert kvc.lib().kvc_device_status() == 0
