@@ -31,7 +31,6 @@
 namespace kvc {
 
 int launch_attention_chunk_tc(const AttnArgs &a, cudaStream_t stream);
-int launch_attention_decode(const AttnArgs &a, cudaStream_t stream);
 bool attention_chunk_tc_accepts(const AttnArgs &a);
 
 namespace {
@@ -39,6 +38,7 @@ namespace {
 using namespace dev;
 
 constexpr size_t MAT_SCRATCH_LIMIT = (size_t)3 << 30;   // bytes of materialised K + V (+ Q') per slice
+constexpr size_t MAT_ARENA_LIMIT = (size_t)64 << 20;    // up to here they lie in the stream's scratch arena
 
 template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
@@ -269,9 +269,12 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
     // 117 -> 37) and no less exact than the kernel that decodes the same f16 rows in its tile loop (errors against
     // 64-bit sums 0.64 .. 0.76 times its for f16 callers, 0.93 .. 0.97 for bf16, 108 shapes of all schemes). Affine
     // rows would be rounded to bf16, and chunks at head dim 64 keep operand pairs: for less work than this the kernels that
-    // decode in their tile loop. Asked of every slice too, so that all sequences of a call are computed alike.
+    // decode in their tile loop. Asked of every slice too, so that all sequences of a call are computed alike. Long contexts keep
+    // the order: 9 .. 63 positions of 64/8 heads behind 32 768 tokens of 16 sequences, 2.1 GB written out and read, 1 164 .. 2 262 us
+    // where that kernel takes 2 494 .. 8 976; of one sequence of 32/8 heads 119 .. 161 and 247 .. 483.
+    const bool always = turbo && a.D == 128 && a.T > 64;
     auto enough = [&](int64_t B) {
-        if (turbo && a.D == 128 && a.T > 64) return true;
+        if (always) return true;
         return a.L >= 64 && B * a.Hq * ((a.L + 127) / 128) >= sm_count(a.device) / 2;
     };
     if (!enough(a.B)) return 0;
@@ -300,7 +303,7 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
     // whole sequences per slice, the slices as even as they come
     const int fit = (int)std::min<size_t>((size_t)a.B, MAT_SCRATCH_LIMIT / per_b);
     const int nslices = (a.B + fit - 1) / fit;
-    const int slice = (a.B + nslices - 1) / nslices;
+    int slice = (a.B + nslices - 1) / nslices;
     {
         AttnArgs probe = r;
         probe.B = a.B - (nslices - 1) * slice;   // the last, smallest slice
@@ -308,7 +311,25 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
         probe.B = slice;
         if (!attention_chunk_tc_accepts(probe)) return 0;
     }
-    char *scratch = (char *)scratch_get(a.device, (size_t)slice * per_b + 1024, stream);
+    // Large rows come from the pool, where their memory serves the caches again; small ones from the arena (the pool's two calls
+    // are 2 us of host time: 30 us a call behind 300 tokens, 32). A device without room for them gets smaller slices where
+    // every slice is worth it, else the kernels that decode in their tile loop.
+    struct Rows {
+        cudaStream_t stream;
+        char *at = nullptr;
+        ~Rows() { dev_free(at, stream); }
+    } rows{stream};
+    auto room = [&] {
+        const size_t bytes = (size_t)slice * per_b + 1024;
+        if (bytes <= MAT_ARENA_LIMIT) return (char *)scratch_try(a.device, bytes, stream);
+        return rows.at = (char *)dev_try_alloc(bytes, stream);
+    };
+    char *scratch = room();
+    while (!scratch && always && slice > 1) {
+        slice = (slice + 1) / 2;
+        scratch = room();
+    }
+    if (!scratch) return 0;
     int launches = 0;
     for (int b0 = 0; b0 < a.B; b0 += slice) {
         const int nb = std::min(slice, a.B - b0);
@@ -345,8 +366,7 @@ int launch_attention_chunk_materialized(const AttnArgs &a, cudaStream_t stream) 
             call.q_sb = rp.o_sb; call.q_sh = rp.o_sh; call.q_sl = rp.o_sl;
         }
         int n = launch_attention_chunk_tc(call, stream);
-        if (n <= 0) n = launch_attention_decode(call, stream);   // no memory for its sums: the mma.sync chunk kernel
-        if (n <= 0) fail(KVC_ERR_INTERNAL, "the tensor-core chunk kernel refused a call it had accepted");
+        if (n <= 0) return 0;   // no memory for its sums: as if there were none for the rows
         launches += n;
         if (turbo) {
             RotParams rp = {};

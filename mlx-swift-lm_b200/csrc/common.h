@@ -65,6 +65,7 @@ void dev_free(void *ptr, cudaStream_t stream);
 // Scratch that grows on demand, one arena per (device, stream), reused by every
 // attention call enqueued on that stream (split-K partials).
 void *scratch_get(int device, size_t bytes, cudaStream_t stream);
+void *scratch_try(int device, size_t bytes, cudaStream_t stream);   // null where the device has no room
 // Zero-initialised ticket counters of the same (device, stream) arena; fixed size.
 int *counters_get(int device, cudaStream_t stream, size_t bytes);
 int current_device();

@@ -98,7 +98,7 @@ struct Arena {
 std::map<std::pair<int, cudaStream_t>, Arena> g_arenas;
 }  // namespace
 
-void *scratch_get(int device, size_t bytes, cudaStream_t stream) {
+void *scratch_try(int device, size_t bytes, cudaStream_t stream) {
     std::lock_guard<std::mutex> lock(g_mu);
     Arena &ar = g_arenas[{device, stream}];
     if (ar.bytes >= bytes) return ar.ptr;
@@ -116,10 +116,17 @@ void *scratch_get(int device, size_t bytes, cudaStream_t stream) {
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        fail(KVC_ERR_OUT_OF_MEMORY, std::string("scratch cudaMalloc: ") + cudaGetErrorString(e));
+        if (e == cudaErrorMemoryAllocation) return nullptr;
+        fail(KVC_ERR_CUDA, std::string("scratch cudaMalloc: ") + cudaGetErrorString(e));
     }
     ar.ptr = p;
     ar.bytes = want;
+    return p;
+}
+
+void *scratch_get(int device, size_t bytes, cudaStream_t stream) {
+    void *p = scratch_try(device, bytes, stream);
+    if (!p) fail(KVC_ERR_OUT_OF_MEMORY, std::string("scratch cudaMalloc: ") + cudaGetErrorString(cudaErrorMemoryAllocation));
     return p;
 }
 

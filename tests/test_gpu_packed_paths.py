@@ -816,6 +816,42 @@ assert float((outs[0].float() - outs[1].float()).abs().max()) < 2e-3
     subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
 
 
+@pytest.mark.parametrize("B,room,slices", [(2, 250, [1, 2]), (1, 90, [0, 1])])
+def test_short_turbo_chunk_on_a_full_device(kvc, cuda, B, room, slices):
+    """Rows of 164 MB a sequence that the device has no room for: sequence by sequence, or in the kernel that decodes in its
+    tile loop, instead of failing; and all at once when there is room again (`slices`: sequences per slice, 0: not written out)."""
+    code = f"""
+import torch, kvcache_b200 as kvc
+torch.manual_seed(0)
+B = {B}
+c = kvc.TurboQuantKVCache(bits=4, key_bits=3, value_bits=4, reserve_tokens=40960)
+for _ in range(10):
+    k, v = torch.randn(2, B, 8, 4000, 128, dtype=torch.half, device="cuda")
+    c.encode_new_token(k, v)
+q, k, v = (torch.randn(B, h, 17, 128, dtype=torch.half, device="cuda") for h in (32, 8, 8))
+out = torch.empty_like(q)
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+hold = torch.empty(torch.cuda.mem_get_info()[0] - ({room} << 20), dtype=torch.uint8, device="cuda")
+outs = []
+for step in range(2):
+    c.attention(q, k, v, 128 ** -0.5, "causal", out=out)
+    torch.cuda.synchronize()
+    print("step", file=__import__("sys").stderr, flush=True)
+    outs.append(out.cpu().double())
+    c.trim(17)
+    hold = None
+    torch.cuda.empty_cache()
+assert c.offset == 40000
+assert float((outs[0] - outs[1]).norm()) < 2.0 ** -8 * float(outs[1].norm())
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.path.join(root, "mlx-swift-lm_b200", "python"), KVC_TRACE_DISPATCH="1")
+    err = subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300, stderr=subprocess.PIPE, text=True).stderr
+    for part, n in zip(err.split("step"), slices):
+        assert ("rows written out" in part) == (n > 0) and (n == 0 or f"{n} sequences per slice" in part), err
+
+
 def test_sequences_of_a_call_take_one_kernel(kvc, cuda, capfd, monkeypatch):
     """Rows written out for a chunk are limited to a few GB at a time. Where a last slice of the batch would be too small to be worth it,
     no sequence of the call is treated that way: equal sequences have equal outputs."""
