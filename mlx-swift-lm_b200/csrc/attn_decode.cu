@@ -1679,6 +1679,12 @@ bool flat_off() {
 
 }  // namespace
 
+// Whether one launch may turn, append and attend a step of `rows` query rows per KV head: what the flat kernel asks that
+// does not depend on the context's length.
+bool attention_decode_takes_rope(int device, int D, int64_t rows, int64_t units) {
+    return !flat_off() && rows <= 16 && units * (int64_t)sizeof(int) <= COUNTER_BYTES && flat_shape(sm_count(device), D, (int)rows, 1, 1).fits;
+}
+
 // The single-token steps of up to KVC_LIST_MAX raw caches of one shape (new rows not yet stored, or all stored)
 // in one launch. Returns launches made, 0 when they do not fit.
 int launch_attention_decode_list(const AttnArgs *args, int n, cudaStream_t stream) {

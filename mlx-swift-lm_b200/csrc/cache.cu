@@ -1194,6 +1194,8 @@ static bool fused_append_off() {
     return off;
 }
 
+bool attention_decode_takes_rope(int device, int D, int64_t rows, int64_t units);   // attn_decode.cu
+
 // Whether cache_attention will hand unturned rows to the decode kernel: its own conditions, and those of the kernel that
 // do not depend on what it allocates.
 bool cache_takes_rope(const kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, const kvc_tensor &v, int32_t mask_mode) {
@@ -1206,10 +1208,22 @@ bool cache_takes_rope(const kvc_cache *c, const kvc_tensor &q, const kvc_tensor 
     const int64_t D = q.shape[3], rep = k.shape[1] > 0 ? q.shape[1] / k.shape[1] : 0;
     if ((D != 64 && D != 128 && D != 256) || rep < 1 || rep > 16 || q.shape[1] % k.shape[1]) return false;
     auto rows = [](const kvc_tensor &t) { return !((uintptr_t)t.data & 15) && (t.stride[0] * 2) % 16 == 0 && (t.stride[1] * 2) % 16 == 0; };
-    return rows(q) && rows(k) && rows(v) && q.stride[1] == D;
+    return rows(q) && rows(k) && rows(v) && q.stride[1] == D && attention_decode_takes_rope(current_device(), (int)D, rep, k.shape[0] * k.shape[1]);
 }
 
 namespace {
+// A step whose row the attention kernel stores: where nothing has stored it in the end (no memory, a refused launch), the cache
+// does not count it.
+struct UnstoredRow {
+    kvc_cache *c;
+    bool stored = false;
+    ~UnstoredRow() {
+        if (stored) return;
+        c->offset -= 1;
+        if (c->cfg.kind == KVC_KIND_ROTATING) c->idx -= 1;
+    }
+};
+
 // Queries and keys turned into memory of their own, where the decode kernel did not take them as they are.
 struct TurnedRows {
     kvc_tensor q, k;
@@ -1296,6 +1310,7 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
                 const int64_t prev = c->offset;
                 const void *k_before = c->k.allocated() ? c->k.view(c->offset).data : nullptr;
                 linear_update(c, k, v, s, /*defer_append=*/true);
+                UnstoredRow row{c};
                 kvc_tensor ck = c->k.view(c->offset), cv = c->v.view(c->offset);
                 AttnArgs a = make_attn_args(q, out, scale, KVC_MASK_NONE, nullptr, ck.shape[2], Hkv);
                 a.k = raw_source(ck);
@@ -1307,9 +1322,11 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
                 a.nk_sb = k.stride[0]; a.nk_sh = k.stride[1];
                 a.nv_sb = v.stride[0]; a.nv_sh = v.stride[1];
                 a.rope = rope;
-                if (launch_attention_decode(a, s) > 0) return;
+                row.stored = launch_attention_decode(a, s) > 0;
+                if (row.stored) return;
                 const TurnedRows t(q, k, rope, s);
                 append_pair(c->k, c->v, t.k, v, prev, s);
+                row.stored = true;
                 t.queries_of(a);
                 a.new_k = a.new_v = nullptr;
                 launch_attention(a, s);
@@ -1328,6 +1345,7 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
                 kvc_tensor ck, cv;
                 int64_t slot = -1;
                 rotating_update_in_place(c, k, v, s, &ck, &cv, &slot);
+                UnstoredRow row{c};
                 AttnArgs a = make_attn_args(q, out, scale, KVC_MASK_NONE, nullptr, ck.shape[2], Hkv);
                 a.k = raw_source(ck);
                 a.v = raw_source(cv);
@@ -1339,9 +1357,11 @@ void cache_attention(kvc_cache *c, const kvc_tensor &q, const kvc_tensor &k, con
                 a.stored_rows_settled = previous_spares(c) && k_before == ck.data &&
                                         launches_before == g_launch_count;
                 a.rope = rope;
-                if (slot >= 0 && slot < ck.shape[2] && launch_attention_decode(a, s) > 0) return;
+                row.stored = slot >= 0 && slot < ck.shape[2] && launch_attention_decode(a, s) > 0;
+                if (row.stored) return;
                 const TurnedRows t(q, k, rope, s);
                 append_pair(c->k, c->v, t.k, v, slot, s);
+                row.stored = true;
                 t.queries_of(a);
                 a.new_k = a.new_v = nullptr;
                 a.new_slot = -1;

@@ -2,6 +2,10 @@
 attentionWithCacheUpdate (MLXLLM/Models/Llama.swift:58-69, MLXLMCommon/RoPEApplication.swift:58-69) and
 the cache traffic of a speculative round over a model's layer list (Evaluate.swift:1179-1286,
 KVCachePlan.swift:219-300), against the oracle."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -214,3 +218,54 @@ def test_rope_inside_the_decode_kernel(kvc, cuda, dtype, Hq, Hkv, D, dims, tradi
         assert torch.equal(x, y)
     assert a.offset == b.offset and all(torch.equal(m, n) for m, n in zip(a.state, b.state))
     assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("ring", [False, True])
+@pytest.mark.parametrize("rope", [False, True])
+def test_step_without_memory_leaves_the_cache_as_it_was(ring, rope):
+    """A full device refuses a step's buffers (turned rows of 9 MB, or a new stream's partials): the cache does not count a row that
+    was never stored, and goes on when there is room again."""
+    code = f"""
+import torch, kvcache_b200 as kvc
+torch.manual_seed(0)
+B, Hq, D, P = 1024, 16, 256, 100
+make = (lambda: kvc.RotatingKVCache(max_size=100, keep=4)) if {ring} else kvc.KVCacheSimple
+a, b = make(), make()
+for c in (a, b):
+    torch.manual_seed(1)
+    for n in (90, 17, 1, 1):
+        c.update(*torch.randn(2, B, 1, n, D, dtype=torch.half, device="cuda"))
+q = torch.randn(B, Hq, 1, D, dtype=torch.half, device="cuda")
+k, v = torch.randn(2, B, 1, 1, D, dtype=torch.half, device="cuda")
+out = torch.empty_like(q)
+turn = {{"dims": D, "base": 10000.0}}
+if {rope}:
+    warm = make()
+    warm.attention(q, k, v, 0.0625, out=out)        # the partials of this stream are there; the turned rows are not
+    step = lambda c: kvc.attention_rope(q, k, v, c, turn, 0.0625, out=out)
+    stream = torch.cuda.current_stream()
+else:
+    step = lambda c: c.attention(q, k, v, 0.0625, out=out)
+    stream = torch.cuda.Stream()
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+before = a.offset, a.meta_state
+hold = torch.empty(torch.cuda.mem_get_info()[0] - (5 << 20), dtype=torch.uint8, device="cuda")
+with torch.cuda.stream(stream):
+    try:
+        step(a)
+        raise SystemExit("there was memory")
+    except kvc.KVCError:
+        pass
+assert (a.offset, a.meta_state) == before, (a.offset, a.meta_state, before)
+del hold
+torch.cuda.empty_cache()
+step(a)
+x = out.clone()
+step(b)
+assert torch.equal(x, out) and a.offset == b.offset and a.meta_state == b.meta_state
+assert all(torch.equal(s, t) for s, t in zip(a.state, b.state))
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.path.join(root, "mlx-swift-lm_b200", "python"))
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
