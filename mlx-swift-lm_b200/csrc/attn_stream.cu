@@ -2,6 +2,8 @@
 #include "attn_stream.cuh"
 
 #include <cmath>
+#include <cstdlib>
+#include <mutex>
 
 namespace kvc {
 
@@ -15,6 +17,41 @@ int run_stream_f16_128(const AttnArgs &a, const StreamPick &pk, const StreamPara
 int run_stream_f16_256(const AttnArgs &a, const StreamPick &pk, const StreamParams &p, StreamList *list, cudaStream_t stream);
 
 namespace {
+
+__global__ void window_kernel(uint32_t *start) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    *start = smem_u32(smem);
+}
+
+// Whether dynamic shared memory starts where the kernel's table loads expect it. Asked once per device, on a stream of its
+// own (a stream that is being captured cannot be waited for); where it starts elsewhere, or nobody can tell, the calls
+// stay with the kernels behind this one. KVC_STREAM=0 says no.
+bool window_fits(int device) {
+    static std::mutex mu;
+    static int known[64] = {0};   // 1: yes, 2: no
+    if (device < 0 || device >= 64) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[device]) return known[device] == 1;
+    known[device] = 2;
+    const char *e = std::getenv("KVC_STREAM");
+    if (e && e[0] == '0') return false;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    KVC_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaStream_t own = nullptr;
+    uint32_t *start = nullptr;
+    bool asked = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess && cudaMallocHost(&start, sizeof *start) == cudaSuccess;
+    if (asked) {
+        *start = 0;
+        window_kernel<<<1, 1, 1024, own>>>(start);
+        asked = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess;
+    }
+    if (asked && *start == ST_WINDOW) known[device] = 1;
+    if (start) (void)cudaFreeHost(start);
+    if (own) (void)cudaStreamDestroy(own);
+    (void)cudaGetLastError();
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    return known[device] == 1;
+}
 
 int source_kind(const KVSource &s, const AttnArgs &a) {
     if (s.kind == SRC_RAW) return s.dtype == a.q_dtype ? SK_RAW : -1;
@@ -53,7 +90,7 @@ bool stream_pick(const AttnArgs &a, StreamPick *out) {
     const int kk = source_kind(a.k, a), vk = source_kind(a.v, a);
     if (kk < 0 || vk < 0 || (kk == SK_RAW && vk == SK_RAW)) return false;
     if ((kk >= SK_T2) != (a.q_signs != nullptr) || (vk >= SK_T2) != (a.o_signs != nullptr)) return false;
-    if (!source_streams(a.k, a.D) || !source_streams(a.v, a.D)) return false;
+    if (!source_streams(a.k, a.D) || !source_streams(a.v, a.D) || !window_fits(a.device)) return false;
     const int kg = a.k.kind == SRC_AFFINE ? a.k.group : 64, vg = a.v.kind == SRC_AFFINE ? a.v.group : 64;
     out->kk = kk; out->vk = vk;
     out->unit = std::min(kg, vg) == 32 ? 32 : 64;

@@ -196,8 +196,8 @@ __device__ __forceinline__ uint32_t entry_offset(const uint32_t (&w)[NW], int n,
     else x = __funnelshift_r(w[k], w[(k + 1 < NW) ? k + 1 : k], s - 8);
     return (x & MASK) | lane_const;
 }
-// Dynamic shared memory starts here in a block's window (what the driver reserves lies in front; checked at the start),
-// so that the tables' place is part of the load.
+// Dynamic shared memory starts here in a block's window (what the driver reserves lies in front; the host asks the device
+// before it launches), so that the tables' place is part of the load.
 constexpr uint32_t ST_WINDOW = 1024;
 // Tables do not change after the barrier behind their making: these loads may be moved freely.
 __device__ __forceinline__ uint2 table_entry(uint32_t offset) {
@@ -313,7 +313,8 @@ attn_stream_kernel(const __grid_constant__ StreamParams p,
     // tables first (constant offsets), then the merge flag, the query rows and the rings
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
     const uint32_t s0 = smem_u32(smem);
-    if (s0 != ST_WINDOW) {                                        // uniform over the grid
+    if (s0 != ST_WINDOW) {                                        // (asked before; uniform over the grid)
+        pdl_wait();
         if (tid == 0) atomicExch(p.status, 36);
         return;
     }

@@ -879,7 +879,8 @@ class DecodeStep:
 
 
 def device_status() -> int:
-    """0 unless a bounded device-side wait has run out since the last reset (kvc_device_status)."""
+    """0 unless a kernel has given up since the last reset: a bounded wait that ran out, or (36) shared memory that does not
+    start where it did when the device was asked (kvc_device_status)."""
     return int(_lib.kvc_device_status())
 
 

@@ -4,6 +4,7 @@ way attentionWithCacheUpdate drives them."""
 import os
 import subprocess
 import sys
+import tempfile
 
 import numpy as np
 import pytest
@@ -616,6 +617,40 @@ def test_stream_kernel_values_of_every_width(kvc, oracle, cuda, kw, D):
         ideal = float((ref.to(dtype).double() - ref.double()).norm())
         assert float((out.cpu().double() - ref.double()).norm()) <= (1.05 if P == 31 else 1.2) * ideal, (P, L, Hq)
     assert kvc.lib().kvc_device_status() == 0
+
+
+def test_calls_without_the_stream_kernel(kvc, cuda):
+    """On a device where the stream kernel cannot run (KVC_STREAM=0 stands for one) its calls and lists have other kernels, which differ by
+    the operands' rounding: 2^-9 of the result in f16."""
+    code = """
+import sys, torch, kvcache_b200 as kvc
+torch.manual_seed(0)
+outs = []
+for make in (lambda: kvc.TurboQuantKVCache(bits=8, key_bits=8, value_bits=4), lambda: kvc.TurboQuantKVCache(bits=4, key_bits=0, value_bits=4),
+             lambda: kvc.QuantizedKVCache(32, 4)):
+    cs = [make(), make()]
+    for c in cs:
+        k, v = torch.randn(2, 2, 2, 300, 128, dtype=torch.half, device="cuda")
+        (c.update_quantized if isinstance(c, kvc.QuantizedKVCache) else c.encode_new_token)(k, v)
+    q, k, v = (torch.randn(2, h, 1, 128, dtype=torch.half, device="cuda") for h in (8, 2, 2))
+    one = cs[0].attention(q, k, v, 0.09)
+    kvc.trim_prompt_cache(cs[:1], 1)
+    two = [torch.empty_like(q) for _ in cs]
+    kvc.DecodeStep(cs, [q, q], [k, k], [v, v], two, 0.09).run()
+    outs += [one, *two]
+assert kvc.device_status() == 0
+torch.save(torch.stack(outs).cpu(), sys.argv[1])
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    both = []
+    for on in "10":
+        env = dict(os.environ, PYTHONPATH=os.path.join(root, "mlx-swift-lm_b200", "python"), KVC_STREAM=on)
+        with tempfile.NamedTemporaryFile() as out:
+            subprocess.run([sys.executable, "-c", code, out.name], check=True, env=env, timeout=300)
+            both.append(torch.load(out.name).double())
+    assert not torch.equal(*both)
+    for x, y in zip(*both):
+        assert float((x - y).norm()) <= 2.0 ** -9 * float(y.norm())
 
 
 @pytest.mark.parametrize("kw,D,L", [(dict(key_bits=8, value_bits=4), 128, 1), (dict(key_bits=4, value_bits=4), 64, 1),
