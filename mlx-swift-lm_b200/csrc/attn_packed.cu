@@ -65,7 +65,7 @@ struct AffineParams {
     int32_t debug_skip;  // measurement aid: 1 = consumers release tiles without computing
     int64_t causal_offset;
     float scale_log2;
-    UnitPlan flat;  // decode8 kernel: flat tile decomposition
+    FlatPlan flat;  // decode8 kernel: flat tile decomposition
     int32_t q_bulk; // decode8 kernel: a unit's query rows are one contiguous 16-byte aligned block
     int32_t chunks; // decode8 kernel: units per (batch, kv head) = ceil(query rows of the group / 8); 1 for decode
 };
@@ -659,7 +659,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     // pointer + offset (no integer round trip) so that loads through it stay ld.shared
     unsigned char *stages = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     constexpr int RING = NSTAGE * STAGE_BYTES;
-    const UnitPlan &fp = p.flat;
+    const FlatPlan &fp = p.flat;
     uint64_t *full = (uint64_t *)(stages + ((RING + 15) / 16) * 16);
     uint64_t *empty = full + NSTAGE;
     int *is_last = (int *)(empty + NSTAGE);
@@ -720,7 +720,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
                 int unit, tb, utiles, hk, b;
                 resolve_unit<VARLEN, P8_TILE>(p, vt.n, seq_first, seq_len, x, tiles, unit, tb, utiles, hk, b);
-                const int own = (int)min((int64_t)(utiles - tb), x_hi - x), n = VARLEN ? own : min(own, fp.real - tb);
+                const int n = (int)min((int64_t)(utiles - tb), x_hi - x);
                 if (p.q_bulk) {
                     const int qb = sg & 1;
                     if (sg >= 2) ok = mbar_wait(&qempty[qb], ((sg >> 1) - 1) & 1);
@@ -763,7 +763,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                     bulk_load(st + 2 * CODE_TILE + 2 * SC_TILE, vs + t0 * G, rows * SB, &full[s]);
                     bulk_load(st + 2 * CODE_TILE + 3 * SC_TILE, vb + t0 * G, rows * SB, &full[s]);
                 }
-                x += own;
+                x += n;
             }
             if (!ok) atomicExch(p.status, 5);
         }
@@ -777,7 +777,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     for (int64_t x = x_lo; x < x_hi; ++sg) {
         int unit, tile_begin, utiles, hk, b;
         resolve_unit<VARLEN, P8_TILE>(p, vt.n, seq_first, seq_len, x, tiles, unit, tile_begin, utiles, hk, b);
-        const int own = (int)min((int64_t)(utiles - tile_begin), x_hi - x), ntiles = VARLEN ? own : min(own, fp.real - tile_begin);
+        const int ntiles = (int)min((int64_t)(utiles - tile_begin), x_hi - x);
         const int64_t T_seq = VARLEN ? (int64_t)seq_len[b] : p.T;   // tokens of this unit's sequence
         const int row0 = VARLEN ? 0 : (unit % p.chunks) * 8;         // first query row of the group this unit carries
         const int R = min(8, R_all - row0);
@@ -1127,7 +1127,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
         u.splits = 0; u.Hq = p.Hq; u.L = p.L;
         segment_epilogue<D, P8_WARPS, P8_WARPS, (NW > 8 ? 8 : 16)>(u, fp, red_o, red_ml, RED_STRIDE, nullptr, is_last, unit, b, hk, rep, R,
                                       x - tile_begin, utiles, row0);
-        x += own;
+        x += ntiles;
     }
 }
 
@@ -1202,9 +1202,6 @@ bool affine_source_fits(const KVSource &s, int D, int64_t T) {
 namespace {
 const VarlenAttnTable kNoVarlen = {};
 
-// What a segment of the decode8 kernel costs beside its tiles, in tiles (of 64 or 240 tokens).
-constexpr int P8_SEGMENT = 4;
-
 constexpr int affine8_stages(int D, int bits, bool varlen) {
     if (affine8_warps(D, bits, varlen) == 15) return 4;
     return bits == 4 ? (D == 128 ? 5 : 8) : (D == 128 ? 4 : 6);
@@ -1271,7 +1268,6 @@ int launch_attention_affine_varlen(const AttnArgs *args, int n, cudaStream_t str
     const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a0.device) * resident, work_tiles);
     AffineParams p = {};
     p.flat.tiles = (int)max_tiles;
-    p.flat.step = 1;
     p.flat.per = (int)(work_tiles / ctas);
     p.flat.rem = (int)(work_tiles % ctas);
     p.flat.nslots = (int)((max_tiles + p.flat.per - 1) / p.flat.per + 1);
@@ -1347,7 +1343,7 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     const bool decode8 = (rep * a.L <= 8 || chunks > 1) && pairs_fit;
     const int64_t tile8 = affine8_warps(a.D, a.k.bits, false) * 16;
     const int64_t tiles = decode8 ? (a.T + tile8 - 1) / tile8 : (a.T + PK_TILE - 1) / PK_TILE;
-    if (!flat_fits(2 * bh * tiles)) return 0;
+    if (!flat_fits(bh * tiles)) return 0;
     // resident CTAs per SM (a fourth CTA fits the 4-bit kernels at 94 registers but measured slower)
     const int slots = sm_count(a.device) * (decode8 ? 3 : 2);
     int64_t best_s = 1;
@@ -1367,15 +1363,18 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
         }
     }
     // decode8: flat decomposition over one wave of resident CTAs (every CTA streams the same number
-    // of tiles); the partial slots per unit take the place of the splits
+    // of tiles); the partial slots per unit take the place of the splits. Equal ranges, not ranges that end where units end: probabilities
+    // are single f16 here, exact only for the largest one of a range's warp, so that longer ranges err by more (up to 1.3 times
+    // at 4 sequences of 1 100 tokens, 16/8 heads, 4 bits), whatever they would save in segments.
+    const int64_t work_tiles = bh * tiles;
     const int flat_resident = affine_resident_ctas(a.D, a.k.bits, a.k.group, std::min(8, rep * a.L), false);
-    UnitPlan plan;
-    const int64_t flat_ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * flat_resident, P8_SEGMENT);
-    const int64_t flat_slots = plan.nslots;
+    const int64_t flat_ctas = std::min<int64_t>((int64_t)sm_count(a.device) * flat_resident, work_tiles);
+    const int64_t flat_per = work_tiles / flat_ctas, flat_rem = work_tiles % flat_ctas;
+    const int64_t flat_slots = (tiles + flat_per - 1) / flat_per + 1;
     // 8-bit codes in one group a row and at most two query rows: the streaming kernel's operand pairs err by a third as much and
     // take as long (4 sequences of 5 000 tokens, 16/8 heads: 2.1e-4 and 6.7e-4 of the output, 19.9 us and 19.2).
     if (decode8 && a.k.bits == 8 && a.k.group == 128 && a.D == 128 && rep * a.L <= 2) return 0;
-    if (decode8 && few_units(bh, tiles, (int64_t)sm_count(a.device) * flat_resident)) return 0;
+    if (decode8 && flat_slots > 64) return 0;
     const int64_t splits = decode8 ? flat_slots : best_s;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
     const size_t o_bytes = (size_t)qrows * splits * a.D * sizeof(float);
@@ -1401,7 +1400,8 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     p.debug_skip = measure_skip_bits();
     p.causal_offset = a.mask.causal_offset;
     p.scale_log2 = a.scale * 1.4426950408889634f;
-    p.flat = plan;
+    p.flat.tiles = (int)tiles;
+    p.flat.per = (int)flat_per; p.flat.rem = (int)flat_rem; p.flat.nslots = (int)flat_slots;
     p.flat.red_rows = decode8 ? std::min(8, rep * a.L) : rep * a.L;
     p.chunks = chunks;
     p.q_bulk = (chunks == 1 && a.L == 1 && a.q_sh == a.D && ((uintptr_t)a.q & 15) == 0 && (a.q_sb * 2) % 16 == 0) ? 1 : 0;
