@@ -65,7 +65,7 @@ struct AffineParams {
     int32_t debug_skip;  // measurement aid: 1 = consumers release tiles without computing
     int64_t causal_offset;
     float scale_log2;
-    FlatPlan flat;  // decode8 kernel: flat tile decomposition
+    UnitPlan flat;  // decode8 kernel: flat tile decomposition
     int32_t q_bulk; // decode8 kernel: a unit's query rows are one contiguous 16-byte aligned block
     int32_t chunks; // decode8 kernel: units per (batch, kv head) = ceil(query rows of the group / 8); 1 for decode
 };
@@ -632,7 +632,13 @@ __device__ __forceinline__ void resolve_unit(const AffineParams &p, int n, const
     unit = i * p.Hkv + hk;
 }
 
-template <typename T, int D, int BITS, int GROUP, int NSTAGE, int MINB, bool VARLEN, int NW>
+// What the middles of the codes added to a row, taken off. Weights beyond f16 are infinite, and so is their output without this.
+__device__ __forceinline__ float middle_off(float weights, float middle, float rest) {
+    return fabsf(weights) < INFINITY ? fmaf(weights, -middle, rest) : rest;
+}
+
+// CENTER: codes around their middle, see MIDDLE.
+template <typename T, int D, int BITS, int GROUP, int NSTAGE, int MINB, bool VARLEN, int NW, bool CENTER>
 __global__ void __launch_bounds__((NW + 1) * 32, MINB)
 attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenAttnTable vt) {
     constexpr int P8_WARPS = NW, P8_TILE = NW * 16;
@@ -659,7 +665,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     // pointer + offset (no integer round trip) so that loads through it stay ld.shared
     unsigned char *stages = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     constexpr int RING = NSTAGE * STAGE_BYTES;
-    const FlatPlan &fp = p.flat;
+    const UnitPlan &fp = p.flat;
     uint64_t *full = (uint64_t *)(stages + ((RING + 15) / 16) * 16);
     uint64_t *empty = full + NSTAGE;
     int *is_last = (int *)(empty + NSTAGE);
@@ -720,7 +726,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             for (int64_t x = x_lo; x < x_hi && ok; ++sg) {
                 int unit, tb, utiles, hk, b;
                 resolve_unit<VARLEN, P8_TILE>(p, vt.n, seq_first, seq_len, x, tiles, unit, tb, utiles, hk, b);
-                const int n = (int)min((int64_t)(utiles - tb), x_hi - x);
+                const int own = (int)min((int64_t)(utiles - tb), x_hi - x), n = VARLEN ? own : min(own, fp.real - tb);
                 if (p.q_bulk) {
                     const int qb = sg & 1;
                     if (sg >= 2) ok = mbar_wait(&qempty[qb], ((sg >> 1) - 1) & 1);
@@ -763,7 +769,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                     bulk_load(st + 2 * CODE_TILE + 2 * SC_TILE, vs + t0 * G, rows * SB, &full[s]);
                     bulk_load(st + 2 * CODE_TILE + 3 * SC_TILE, vb + t0 * G, rows * SB, &full[s]);
                 }
-                x += n;
+                x += own;
             }
             if (!ok) atomicExch(p.status, 5);
         }
@@ -777,7 +783,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
     for (int64_t x = x_lo; x < x_hi; ++sg) {
         int unit, tile_begin, utiles, hk, b;
         resolve_unit<VARLEN, P8_TILE>(p, vt.n, seq_first, seq_len, x, tiles, unit, tile_begin, utiles, hk, b);
-        const int ntiles = (int)min((int64_t)(utiles - tile_begin), x_hi - x);
+        const int own = (int)min((int64_t)(utiles - tile_begin), x_hi - x), ntiles = VARLEN ? own : min(own, fp.real - tile_begin);
         const int64_t T_seq = VARLEN ? (int64_t)seq_len[b] : p.T;   // tokens of this unit's sequence
         const int row0 = VARLEN ? 0 : (unit % p.chunks) * 8;         // first query row of the group this unit carries
         const int R = min(8, R_all - row0);
@@ -791,6 +797,9 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int gr = 0; gr < G; ++gr) bsum[h][gr] = 0.f;
+        float psum[G][4];   // [0, 1]: sums of the rounded weights, see MIDDLE (the tile's other rows repeat them)
+#pragma unroll
+        for (int gr = 0; gr < G; ++gr) psum[gr][0] = psum[gr][1] = psum[gr][2] = psum[gr][3] = 0.f;
         // Q^T fragments: B operand column = query row g; k-slots follow the code words.
         // q' = f16(q * scale * log2 e). The code operands are f16 subnormals n * 2^-24 (or
         // n * 2^-20 for the nibbles at bits 4..7): the k-slots fed by the smaller form carry
@@ -878,6 +887,13 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
         }
         const int min_limit = p.causal ? (int)min((int64_t)t_last, p.causal_offset) : t_last;
         constexpr float M_INIT = -1e30f, LAZY = 8.f;
+        // The codes meet weights rounded to f16, p s (1 + e), the biases meet p itself: where the codes count from 0, an e is worth
+        // the code n, and for all but the largest weight of a warp's share of a range (which is s and has no e) n is three times what
+        // it takes from the mean. CENTER, v = s (n - m) + (b + m s): an e is worth n - m, and long ranges err no more than short ones (f16
+        // callers, 350 shapes: 0.74 times the errors of equal ranges without it; longer ranges without it up to 1.29 times). The m
+        // meet the rounded weights in one more MMA a group, with ones for codes: 2 .. 5 % of the time of long contexts, 8 % with four
+        // groups a row, so that equal ranges, which cost no precision, do without.
+        constexpr float MIDDLE = BITS == 4 ? 8.f : 128.f;
         m_run[0] = m_run[1] = M_INIT;
         float m_thr[2] = {M_INIT, M_INIT};  // (m_run + LAZY) / KSCALE once a maximum exists
 
@@ -1021,6 +1037,8 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                     for (int gr = 0; gr < G; ++gr) {
                         bsum[0][gr] *= alpha[0];
                         bsum[1][gr] *= alpha[1];
+                        psum[gr][0] *= alpha[0];
+                        psum[gr][1] *= alpha[1];
                     }
                 }
             }
@@ -1041,8 +1059,15 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
                 for (int gr = 0; gr < G; ++gr) {
                     pb[gr][0] = movmatrix_trans(pack_h2(pr[0] * s0[gr], pr[1] * s0[gr]));  // tokens 0..7 of the block
                     pb[gr][1] = movmatrix_trans(pack_h2(pr[2] * s1[gr], pr[3] * s1[gr]));  // tokens 8..15
-                    bsum[0][gr] = fmaf(pr[0], b0[gr], fmaf(pr[2], b1[gr], bsum[0][gr]));
-                    bsum[1][gr] = fmaf(pr[1], b0[gr], fmaf(pr[3], b1[gr], bsum[1][gr]));
+                    float z0 = b0[gr], z1 = b1[gr];
+                    if constexpr (CENTER) {
+                        z0 = fmaf(s0[gr], MIDDLE, z0);
+                        z1 = fmaf(s1[gr], MIDDLE, z1);
+                        const uint32_t ones[4] = {0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u};
+                        mma_f16(psum[gr], ones, pb[gr][0], pb[gr][1]);
+                    }
+                    bsum[0][gr] = fmaf(pr[0], z0, fmaf(pr[2], z1, bsum[0][gr]));
+                    bsum[1][gr] = fmaf(pr[1], z0, fmaf(pr[3], z1, bsum[1][gr]));
                 }
             }
             // ---- O^T += codes^T . P'^T (subnormal operands; the 2^24 / 2^20 leaves in the epilogue) ----
@@ -1099,12 +1124,14 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
             const int gr = d0 / GROUP;
             const float vs = (BITS == 4 && (i & 1)) ? 1048576.f : 16777216.f;  // undo the subnormal factor
             if (2 * c < R) {
-                wo[(2 * c) * RED_STRIDE + d0] = fmaf(o_acc[mt][0], vs, bsum[0][gr]);
-                wo[(2 * c) * RED_STRIDE + d1] = fmaf(o_acc[mt][2], vs, bsum[0][gr]);
+                const float rest = CENTER ? middle_off(psum[gr][0], MIDDLE, bsum[0][gr]) : bsum[0][gr];
+                wo[(2 * c) * RED_STRIDE + d0] = fmaf(o_acc[mt][0], vs, rest);
+                wo[(2 * c) * RED_STRIDE + d1] = fmaf(o_acc[mt][2], vs, rest);
             }
             if (2 * c + 1 < R) {
-                wo[(2 * c + 1) * RED_STRIDE + d0] = fmaf(o_acc[mt][1], vs, bsum[1][gr]);
-                wo[(2 * c + 1) * RED_STRIDE + d1] = fmaf(o_acc[mt][3], vs, bsum[1][gr]);
+                const float rest = CENTER ? middle_off(psum[gr][1], MIDDLE, bsum[1][gr]) : bsum[1][gr];
+                wo[(2 * c + 1) * RED_STRIDE + d0] = fmaf(o_acc[mt][1], vs, rest);
+                wo[(2 * c + 1) * RED_STRIDE + d1] = fmaf(o_acc[mt][3], vs, rest);
             }
         }
         if (g == 0) {
@@ -1127,7 +1154,7 @@ attn_affine_decode8_kernel(const AffineParams p, const __grid_constant__ VarlenA
         u.splits = 0; u.Hq = p.Hq; u.L = p.L;
         segment_epilogue<D, P8_WARPS, P8_WARPS, (NW > 8 ? 8 : 16)>(u, fp, red_o, red_ml, RED_STRIDE, nullptr, is_last, unit, b, hk, rep, R,
                                       x - tile_begin, utiles, row0);
-        x += ntiles;
+        x += own;
     }
 }
 
@@ -1155,7 +1182,7 @@ void launch_affine_typed(const AffineParams &p, int units, cudaStream_t stream) 
     ++g_launch_count;
 }
 
-template <typename T, int D, int BITS, int GROUP, int NSTAGE, int MINB, bool VARLEN, int NW>
+template <typename T, int D, int BITS, int GROUP, int NSTAGE, int MINB, bool VARLEN, int NW, bool CENTER>
 void launch_affine8_typed(const AffineParams &p, const VarlenAttnTable &vt, int ctas, cudaStream_t stream) {
     constexpr int P8_WARPS = NW, P8_TILE = NW * 16, P8_THREADS = (NW + 1) * 32;
     constexpr int G = D / GROUP;
@@ -1168,14 +1195,14 @@ void launch_affine8_typed(const AffineParams &p, const VarlenAttnTable &vt, int 
     static size_t configured[64] = {0};
     const int dev = current_device();
     if (dev >= 0 && dev < 64 && configured[dev] < smem) {
-        KVC_CUDA(cudaFuncSetAttribute(attn_affine_decode8_kernel<T, D, BITS, GROUP, NSTAGE, MINB, VARLEN, NW>,
+        KVC_CUDA(cudaFuncSetAttribute(attn_affine_decode8_kernel<T, D, BITS, GROUP, NSTAGE, MINB, VARLEN, NW, CENTER>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        KVC_CUDA(cudaFuncSetAttribute(attn_affine_decode8_kernel<T, D, BITS, GROUP, NSTAGE, MINB, VARLEN, NW>,
+        KVC_CUDA(cudaFuncSetAttribute(attn_affine_decode8_kernel<T, D, BITS, GROUP, NSTAGE, MINB, VARLEN, NW, CENTER>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         configured[dev] = smem;
     }
     KernelTimer timer(stream);
-    KVC_CUDA(launch_pdl(attn_affine_decode8_kernel<T, D, BITS, GROUP, NSTAGE, MINB, VARLEN, NW>, dim3(ctas), dim3(P8_THREADS),
+    KVC_CUDA(launch_pdl(attn_affine_decode8_kernel<T, D, BITS, GROUP, NSTAGE, MINB, VARLEN, NW, CENTER>, dim3(ctas), dim3(P8_THREADS),
                         smem, stream, p, vt));
     timer.stop();
     KVC_CUDA(cudaGetLastError());
@@ -1201,6 +1228,11 @@ bool affine_source_fits(const KVSource &s, int D, int64_t T) {
 
 namespace {
 const VarlenAttnTable kNoVarlen = {};
+
+// What a segment of the decode8 kernel costs beside its tiles, in tiles: what plan_units finds the best ranges with, not a
+// measured length. 175 shapes at 0, 1, 2, 4, 7, 12: tiles of 240 tokens 1.16, 1.06, 1.01, 1.01, 1.01, 1.01 times the best time, of 64
+// tokens 1.09, 1.03, 1.00, 1.00, 1.00, 1.00. Four groups a row pay more for codes around their middle: 1.027 at 2, 1.035 at 4.
+int affine8_segment(int D, int group) { return D / group == 4 ? 2 : 4; }
 
 constexpr int affine8_stages(int D, int bits, bool varlen) {
     if (affine8_warps(D, bits, varlen) == 15) return 4;
@@ -1268,6 +1300,7 @@ int launch_attention_affine_varlen(const AttnArgs *args, int n, cudaStream_t str
     const int64_t ctas = std::min<int64_t>((int64_t)sm_count(a0.device) * resident, work_tiles);
     AffineParams p = {};
     p.flat.tiles = (int)max_tiles;
+    p.flat.step = 1;
     p.flat.per = (int)(work_tiles / ctas);
     p.flat.rem = (int)(work_tiles % ctas);
     p.flat.nslots = (int)((max_tiles + p.flat.per - 1) / p.flat.per + 1);
@@ -1292,17 +1325,17 @@ int launch_attention_affine_varlen(const AttnArgs *args, int n, cudaStream_t str
     p.causal_offset = 0;
     p.scale_log2 = a0.scale * 1.4426950408889634f;
     const int bits = a0.k.bits, group = a0.k.group;
-#define KVC_AFFV(TT, DD, BB, GG, NS)                                                        \
+#define KVC_AFFV(TT, DD, BB, GG)                                                        \
     if (a0.D == DD && bits == BB && group == GG) {                                           \
-        launch_affine8_typed<TT, DD, BB, GG, affine8_stages(DD, BB, true), affine8_ctas(DD, BB, true), true, affine8_warps(DD, BB, true)>(p, vt, (int)ctas, stream);         \
+        launch_affine8_typed<TT, DD, BB, GG, affine8_stages(DD, BB, true), affine8_ctas(DD, BB, true), true, affine8_warps(DD, BB, true), false>(p, vt, (int)ctas, stream);         \
         return 1;                                                                            \
     }
     if (a0.q_dtype == KVC_BF16) {
-        KVC_AFFV(__nv_bfloat16, 128, 4, 64, 5)
-        KVC_AFFV(__nv_bfloat16, 128, 8, 64, 4)
+        KVC_AFFV(__nv_bfloat16, 128, 4, 64)
+        KVC_AFFV(__nv_bfloat16, 128, 8, 64)
     } else {
-        KVC_AFFV(__half, 128, 4, 64, 5)
-        KVC_AFFV(__half, 128, 8, 64, 4)
+        KVC_AFFV(__half, 128, 4, 64)
+        KVC_AFFV(__half, 128, 8, 64)
     }
 #undef KVC_AFFV
     return 0;
@@ -1343,7 +1376,7 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     const bool decode8 = (rep * a.L <= 8 || chunks > 1) && pairs_fit;
     const int64_t tile8 = affine8_warps(a.D, a.k.bits, false) * 16;
     const int64_t tiles = decode8 ? (a.T + tile8 - 1) / tile8 : (a.T + PK_TILE - 1) / PK_TILE;
-    if (!flat_fits(bh * tiles)) return 0;
+    if (!flat_fits(2 * bh * tiles)) return 0;
     // resident CTAs per SM (a fourth CTA fits the 4-bit kernels at 94 registers but measured slower)
     const int slots = sm_count(a.device) * (decode8 ? 3 : 2);
     int64_t best_s = 1;
@@ -1363,18 +1396,15 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
         }
     }
     // decode8: flat decomposition over one wave of resident CTAs (every CTA streams the same number
-    // of tiles); the partial slots per unit take the place of the splits. Equal ranges, not ranges that end where units end: probabilities
-    // are single f16 here, exact only for the largest one of a range's warp, so that longer ranges err by more (up to 1.3 times
-    // at 4 sequences of 1 100 tokens, 16/8 heads, 4 bits), whatever they would save in segments.
-    const int64_t work_tiles = bh * tiles;
+    // of tiles); the partial slots per unit take the place of the splits
     const int flat_resident = affine_resident_ctas(a.D, a.k.bits, a.k.group, std::min(8, rep * a.L), false);
-    const int64_t flat_ctas = std::min<int64_t>((int64_t)sm_count(a.device) * flat_resident, work_tiles);
-    const int64_t flat_per = work_tiles / flat_ctas, flat_rem = work_tiles % flat_ctas;
-    const int64_t flat_slots = (tiles + flat_per - 1) / flat_per + 1;
+    UnitPlan plan;
+    const int64_t flat_ctas = plan_units(&plan, bh, tiles, (int64_t)sm_count(a.device) * flat_resident, affine8_segment(a.D, a.k.group));
+    const int64_t flat_slots = plan.nslots;
     // 8-bit codes in one group a row and at most two query rows: the streaming kernel's operand pairs err by a third as much and
     // take as long (4 sequences of 5 000 tokens, 16/8 heads: 2.1e-4 and 6.7e-4 of the output, 19.9 us and 19.2).
     if (decode8 && a.k.bits == 8 && a.k.group == 128 && a.D == 128 && rep * a.L <= 2) return 0;
-    if (decode8 && flat_slots > 64) return 0;
+    if (decode8 && few_units(bh, tiles, (int64_t)sm_count(a.device) * flat_resident)) return 0;
     const int64_t splits = decode8 ? flat_slots : best_s;
     const int64_t qrows = (int64_t)a.B * a.Hq * a.L;
     const size_t o_bytes = (size_t)qrows * splits * a.D * sizeof(float);
@@ -1400,36 +1430,38 @@ int launch_attention_affine(const AttnArgs &a, cudaStream_t stream) {
     p.debug_skip = measure_skip_bits();
     p.causal_offset = a.mask.causal_offset;
     p.scale_log2 = a.scale * 1.4426950408889634f;
-    p.flat.tiles = (int)tiles;
-    p.flat.per = (int)flat_per; p.flat.rem = (int)flat_rem; p.flat.nslots = (int)flat_slots;
+    p.flat = plan;
     p.flat.red_rows = decode8 ? std::min(8, rep * a.L) : rep * a.L;
     p.chunks = chunks;
     p.q_bulk = (chunks == 1 && a.L == 1 && a.q_sh == a.D && ((uintptr_t)a.q & 15) == 0 && (a.q_sb * 2) % 16 == 0) ? 1 : 0;
     const int units = decode8 ? (int)flat_ctas : (int)(bh * splits);
+    const bool longer = plan.step > 1;   // than equal ranges
 
     const int bits = a.k.bits, group = a.k.group;
-#define KVC_AFF8(TT, DD, BB, GG, NS)                                         \
+#define KVC_AFF8(TT, DD, BB, GG)                                         \
     if (a.D == DD && bits == BB && group == GG) {                            \
-        launch_affine8_typed<TT, DD, BB, GG, affine8_stages(DD, BB, false), affine8_ctas(DD, BB, false), false, affine8_warps(DD, BB, false)>(p, kNoVarlen, units, stream); \
+        constexpr int NS = affine8_stages(DD, BB, false), CT = affine8_ctas(DD, BB, false), NW = affine8_warps(DD, BB, false);               \
+        if (longer) launch_affine8_typed<TT, DD, BB, GG, NS, CT, false, NW, true>(p, kNoVarlen, units, stream);                             \
+        else launch_affine8_typed<TT, DD, BB, GG, NS, CT, false, NW, false>(p, kNoVarlen, units, stream);                                   \
         return 1;                                                            \
     }
     if (decode8) {
         if (a.q_dtype == KVC_BF16) {
-            KVC_AFF8(__nv_bfloat16, 128, 4, 64, 5)
-            KVC_AFF8(__nv_bfloat16, 128, 8, 64, 4)
-            KVC_AFF8(__nv_bfloat16, 128, 4, 128, 5)
-            KVC_AFF8(__nv_bfloat16, 128, 8, 128, 4)
-            KVC_AFF8(__nv_bfloat16, 128, 8, 32, 4)
-            KVC_AFF8(__nv_bfloat16, 64, 4, 64, 8)
-            KVC_AFF8(__nv_bfloat16, 64, 8, 64, 6)
+            KVC_AFF8(__nv_bfloat16, 128, 4, 64)
+            KVC_AFF8(__nv_bfloat16, 128, 8, 64)
+            KVC_AFF8(__nv_bfloat16, 128, 4, 128)
+            KVC_AFF8(__nv_bfloat16, 128, 8, 128)
+            KVC_AFF8(__nv_bfloat16, 128, 8, 32)
+            KVC_AFF8(__nv_bfloat16, 64, 4, 64)
+            KVC_AFF8(__nv_bfloat16, 64, 8, 64)
         } else {
-            KVC_AFF8(__half, 128, 4, 64, 5)
-            KVC_AFF8(__half, 128, 8, 64, 4)
-            KVC_AFF8(__half, 128, 4, 128, 5)
-            KVC_AFF8(__half, 128, 8, 128, 4)
-            KVC_AFF8(__half, 128, 8, 32, 4)
-            KVC_AFF8(__half, 64, 4, 64, 8)
-            KVC_AFF8(__half, 64, 8, 64, 6)
+            KVC_AFF8(__half, 128, 4, 64)
+            KVC_AFF8(__half, 128, 8, 64)
+            KVC_AFF8(__half, 128, 4, 128)
+            KVC_AFF8(__half, 128, 8, 128)
+            KVC_AFF8(__half, 128, 8, 32)
+            KVC_AFF8(__half, 64, 4, 64)
+            KVC_AFF8(__half, 64, 8, 64)
         }
     }
 #undef KVC_AFF8

@@ -819,6 +819,25 @@ def test_stream_kernel_keeps_single_precision_over_affine_codes(kvc, oracle, cud
     assert float((out.double() - ref).norm()) <= 1.0003 * ideal
 
 
+@pytest.mark.parametrize("bits,group,B,Hq,Hkv,D,P", [
+    (4, 64, 4, 16, 8, 128, 1100), (4, 128, 4, 16, 8, 128, 1100), (8, 64, 4, 16, 8, 128, 1100), (8, 128, 8, 32, 8, 128, 300),
+    (8, 32, 8, 32, 8, 128, 300), (4, 64, 8, 32, 8, 64, 600), (8, 64, 8, 32, 8, 64, 600),
+])
+def test_affine_ranges_that_end_where_units_end(kvc, oracle, cuda, bits, group, B, Hq, Hkv, D, P):
+    """Units of a few tiles, one or a few whole pieces a CTA. Query, weights and store are f16, `ideal` is what the last of the three
+    errs by; a weight's error meets a code's distance from the middle, so that the three are alike: sqrt(3) * ideal, and 15 %
+    for how alike they are. (Weights that meet the codes themselves: 2.4 .. 2.9 * ideal.)"""
+    c = kvc.QuantizedKVCache(group, bits)
+    c.update_quantized(seeded((B, Hkv, P, D), 1, torch.half).to(cuda), seeded((B, Hkv, P, D), 2, torch.half).to(cuda))
+    q, k1, v1 = (seeded((B, h, 1, D), s, torch.half).to(cuda) for s, h in ((3, Hq), (4, Hkv), (5, Hkv)))
+    out = c.attention(q, k1, v1, D ** -0.5)
+    K, V = _rows64(oracle, c.state, dict(bits=bits, group=group), D)
+    ref = _attention64(q, K, V, D ** -0.5, torch.ones((1, P + 1), dtype=torch.bool, device=cuda))
+    ideal = float((ref.half().double() - ref).norm())
+    assert float((out.double() - ref).norm()) <= 2.0 * ideal
+    assert kvc.lib().kvc_device_status() == 0
+
+
 def test_chunk_on_operand_pairs_on_a_full_device(kvc, cuda):
     """A chunk whose decoded rows the device has no room for runs on the general kernel instead of failing."""
     code = """
