@@ -1024,9 +1024,14 @@ int run_stream(const AttnArgs &a, StreamParams p, StreamList *list, cudaStream_t
     if (!stream_plan(a, n * units, work, most, StreamShape<T, D, KK, VK, UNIT, NB, false>::RESIDENT, std::min(rows, 8 * NB), &p,
                      (int64_t)n * a.B * a.Hq * a.L, stream, &ctas))
         return 0;
-    if (list) stream_list_tiles(list->seq, n, units, p.flat);
-    if (list) launch_stream_typed<T, D, KK, VK, UNIT, NB, true>(p, list, ctas, stream);
-    else launch_stream_typed<T, D, KK, VK, UNIT, NB, false>(p, nullptr, ctas, stream);
+    if constexpr (NB <= 2) {   // lists hold up to sixteen rows
+        if (list) {
+            stream_list_tiles(list->seq, n, units, p.flat);
+            launch_stream_typed<T, D, KK, VK, UNIT, NB, true>(p, list, ctas, stream);
+            return 1;
+        }
+    }
+    launch_stream_typed<T, D, KK, VK, UNIT, NB, false>(p, nullptr, ctas, stream);
     return 1;
 }
 
@@ -1038,8 +1043,9 @@ int run_stream(const AttnArgs &a, StreamParams p, StreamList *list, cudaStream_t
 template <typename T, int D, int KK, int VK, int UNIT>
 int run_stream_rows(const AttnArgs &a, const StreamParams &p, StreamList *list, cudaStream_t stream) {
     if constexpr (D == 64) {
-        const int64_t tiles = (int64_t)(list ? list->n : 1) * a.B * a.Hkv * ((a.T + ST_TILE - 1) / ST_TILE);
-        if (a.Hq / a.Hkv * a.L > 16 && tiles >= 128 * (int64_t)sm_count(a.device)) return run_stream<T, D, KK, VK, UNIT, 4>(a, p, list, stream);
+        const int64_t tiles = (int64_t)a.B * a.Hkv * ((a.T + ST_TILE - 1) / ST_TILE);
+        if (!list && a.Hq / a.Hkv * a.L > 16 && tiles >= 128 * (int64_t)sm_count(a.device))
+            return run_stream<T, D, KK, VK, UNIT, 4>(a, p, nullptr, stream);
     }
     if constexpr (D <= 128)
         if (a.Hq / a.Hkv * a.L > 8) return run_stream<T, D, KK, VK, UNIT, 2>(a, p, list, stream);
