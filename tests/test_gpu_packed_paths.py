@@ -838,6 +838,103 @@ def test_affine_ranges_that_end_where_units_end(kvc, oracle, cuda, bits, group, 
     assert kvc.lib().kvc_device_status() == 0
 
 
+def _packed(kvc, cuda, kw, B, Hkv, D, P, seed=1):
+    """A packed f16 cache of P rows."""
+    c = kvc.QuantizedKVCache(kw["group"], kw["bits"]) if "group" in kw else kvc.TurboQuantKVCache(bits=max(kw["key_bits"], kw["value_bits"]), **kw)
+    k, v = (torch.randn((B, Hkv, P, D), generator=torch.Generator(cuda).manual_seed(seed + i), device=cuda, dtype=torch.half) for i in (0, 100))
+    (c.update_quantized if "group" in kw else c.encode_new_token)(k, v)
+    return c
+
+
+def _err_over_ideal(oracle, out, c, q, kw, D, L=1):
+    """Distance from 64-bit sums over that of their f16 rounding."""
+    K, V = _rows64(oracle, c.state, kw, D)
+    T = K.shape[2]
+    ref = _attention64(q, K, V, D ** -0.5, torch.arange(T, device=q.device) <= torch.arange(T - L, T, device=q.device)[:, None])
+    return float((out.double() - ref).norm() / (ref.half().double() - ref).norm())
+
+
+@pytest.mark.parametrize("kw,rows,D,B,Hkv,P", [
+    # TurboQuant kernels of f16 operands: rotated query, both centroids, weight and store: sqrt(5), and 25 %. Codebooks of two bits have two
+    # magnitudes, whose rounding may be the largest there is, 2.4 times the mean one: sqrt(3 + 2 * 2.4^2)
+    (dict(key_bits=2, value_bits=2), 4, 128, 16, 8, 300),       # tiles of 64: units of five, three pieces or whole ones
+    (dict(key_bits=3, value_bits=3), 4, 128, 4, 8, 1100),
+    (dict(key_bits=4, value_bits=2), 4, 128, 48, 8, 130),
+    (dict(key_bits=3, value_bits=4), 4, 128, 8, 8, 2047),       # tiles of 240: units of nine in pieces of five
+    (dict(key_bits=4, value_bits=4), 4, 128, 32, 8, 300),
+    # operand pairs: the store alone, and 5 %
+    (dict(key_bits=8, value_bits=4), 4, 128, 8, 8, 300),
+    (dict(key_bits=0, value_bits=4), 4, 64, 40, 8, 300),
+    (dict(bits=4, group=32), 4, 256, 16, 8, 300),
+])
+def test_ranges_that_end_where_units_end(kvc, oracle, cuda, kw, rows, D, B, Hkv, P):
+    c = _packed(kvc, cuda, kw, B, Hkv, D, P)
+    q, k1, v1 = (seeded((B, h, 1, D), s, torch.half).to(cuda) for s, h in ((3, rows * Hkv), (4, Hkv), (5, Hkv)))
+    out = c.attention(q, k1, v1, D ** -0.5)
+    pairs = "group" in kw or kw["key_bits"] in (0, 8)
+    assert _err_over_ideal(oracle, out, c, q, kw, D) <= (1.05 if pairs else 3.9 if kw["key_bits"] == 2 or kw["value_bits"] == 2 else 2.8)
+    assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("kw,n,B,Hkv,D,P,L,dtype", [
+    (dict(key_bits=8, value_bits=4), 2, 4, 8, 128, 300, 1, torch.half),      # 64 units of five tiles, rounded up to six
+    (dict(key_bits=8, value_bits=4), 4, 16, 8, 128, 300, 1, torch.half),     # whole units
+    (dict(key_bits=4, value_bits=4), 3, 2, 8, 64, 300, 2, torch.half),
+    (dict(bits=4, group=64), 3, 3, 4, 64, 450, 1, torch.half),
+    (dict(bits=8, group=64), 2, 4, 8, 64, 300, 1, torch.float32),
+    (dict(bits=4, group=64), 4, 20, 8, 64, 300, 1, torch.float32),
+])
+def test_lists_whose_units_are_rounded_up(kvc, oracle, cuda, kw, n, B, Hkv, D, P, L, dtype):
+    """Layers of one length in one launch, whose ranges end where units end. The bounds of the kernels' own tests."""
+    cs = [_packed(kvc, cuda, kw, B, Hkv, D, P, seed=i) for i in range(n)] if dtype == torch.half else []
+    for i in range(n - len(cs)):
+        cs.append(kvc.QuantizedKVCache(kw["group"], kw["bits"]))
+        cs[i].update_quantized(*(seeded((B, Hkv, P, D), 2 * i + j, dtype).to(cuda) for j in (0, 1)))
+    qs, ks, vs = ([seeded((B, h, L, D), s + i, dtype).to(cuda) for i in range(n)] for s, h in ((30, 2 * Hkv), (40, Hkv), (50, Hkv)))
+    outs = [torch.empty_like(q) for q in qs]
+    kvc.launch_count(reset=True)
+    kvc.DecodeStep(cs, qs, ks, vs, outs, D ** -0.5, mask="causal" if L > 1 else "none").run()
+    assert kvc.launch_count() == (3 if kw.get("key_bits") == 8 else 2)          # the rows (of both representations), the attention
+    for c, q, out in zip(cs, qs, outs):
+        if dtype == torch.half:
+            assert _err_over_ideal(oracle, out, c, q, kw, D, L) <= 1.05
+        else:
+            K, V = _rows64(oracle, c.state, kw, D)
+            ref = _attention64(q, K, V, D ** -0.5, torch.ones((1, P + 1), dtype=torch.bool, device=cuda))
+            assert float((out.double() - ref).norm()) <= 2.0 ** -20 * float(ref.norm())
+    assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("kw", [dict(bits=4, group=32), dict(bits=8, group=32), dict(key_bits=4, value_bits=4),
+                                dict(key_bits=3, value_bits=4), dict(key_bits=0, value_bits=2), dict(key_bits=8, value_bits=3)])
+@pytest.mark.parametrize("rep,L,P", [(1, 17, 2305), (4, 7, 2318), (8, 4, 2367), (3, 11, 2304 + 64), (8, 8, 2400)])
+def test_units_of_32_rows(kvc, oracle, cuda, kw, rep, L, P):
+    """Verify rounds of 17, 28, 32, 33 and 64 rows a KV head over enough tokens (128 tiles of 64 an SM) for four column blocks a unit;
+    the last tile of a unit holds 1 .. 64 tokens of the round and before it."""
+    B, Hkv, D = 32, 16, 64
+    c = _packed(kvc, cuda, kw, B, Hkv, D, P)
+    q, k1, v1 = (seeded((B, h, L, D), s, torch.half).to(cuda) for s, h in ((3, rep * Hkv), (4, Hkv), (5, Hkv)))
+    out = c.attention(q, k1, v1, D ** -0.5, "causal")
+    assert _err_over_ideal(oracle, out, c, q, kw, D, L) <= 1.05
+    assert kvc.lib().kvc_device_status() == 0
+
+
+@pytest.mark.parametrize("dtype,Hq,Hkv,D,P", [(torch.bfloat16, 8, 1, 128, 20000), (torch.half, 6, 2, 64, 30011), (torch.half, 4, 1, 256, 12000)])
+def test_raw_units_of_more_than_64_partials(kvc, cuda, dtype, Hq, Hkv, D, P):
+    """One sequence of few heads: every tile of a long context is another CTA's. Weights and store are rounded to the type: two
+    errors of `ideal`, and 15 % for how alike they are."""
+    c = kvc.KVCacheSimple()
+    k, v = (torch.randn((1, Hkv, P, D), generator=torch.Generator(cuda).manual_seed(i), device=cuda).to(dtype) for i in (1, 2))
+    c.update(k, v)
+    q, k1, v1 = (seeded((1, h, 1, D), s, dtype).to(cuda) for s, h in ((3, Hq), (4, Hkv), (5, Hkv)))
+    out = c.attention(q, k1, v1, D ** -0.5)
+    K, V = (torch.cat(t, 2).double() for t in ((k, k1), (v, v1)))
+    ref = _attention64(q, K, V, D ** -0.5, torch.ones((1, P + 1), dtype=torch.bool, device=cuda))
+    ideal = float((ref.to(dtype).double() - ref).norm())
+    assert float((out.double() - ref).norm()) <= 1.15 * 2 ** 0.5 * ideal
+    assert kvc.lib().kvc_device_status() == 0
+
+
 def test_chunk_on_operand_pairs_on_a_full_device(kvc, cuda):
     """A chunk whose decoded rows the device has no room for runs on the general kernel instead of failing."""
     code = """
