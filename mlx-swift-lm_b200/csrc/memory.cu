@@ -140,7 +140,11 @@ int *counters_get(int device, cudaStream_t stream, size_t bytes) {
         (void)cudaGetLastError();
         fail(KVC_ERR_OUT_OF_MEMORY, std::string("counter cudaMalloc: ") + cudaGetErrorString(e));
     }
-    e = cudaMemset(p, 0, bytes);
+    // In the order of the stream that counts: the legacy stream holds nothing back on streams that do not block on it. (A stream that
+    // is being captured would zero them when its graph runs.)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    (void)cudaStreamIsCapturing(stream, &capture);
+    e = capture == cudaStreamCaptureStatusNone ? cudaMemsetAsync(p, 0, bytes, stream) : cudaMemset(p, 0, bytes);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         (void)cudaFree(p);
