@@ -522,7 +522,7 @@ attn_chunk_packed_kernel(const __grid_constant__ ChunkPackedParams p) {
             ok = mbar_wait(&full[s], (it / NSTAGE) & 1);
             if (ok) {
                 SRC::dequant(p, stages + (size_t)s * STAGE_BYTES, tab, dq_tok, dq_half, lane, kdq, vdq);
-                __syncwarp();
+                __syncwarp();   // (the rows just stored have waited for every value of the stage, see release_after)
                 if (lane == 0) mbar_arrive(&empty[s]);
             } else if (lane == 0) {
                 atomicExch(p.status, 12);

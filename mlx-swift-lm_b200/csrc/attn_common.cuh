@@ -101,8 +101,8 @@ __device__ __forceinline__ void release_fenced(uint64_t *bar, int lane) {
     if (lane == 0) mbar_arrive(bar);
 }
 // ... or the arrival's address is made to need them: `read` joins words that came out of the last loads (those before came back
-// before them), `none` is zero and not known to the compiler. A kernel whose later shared loads or stores need every value
-// that it took from the entry has waited for them already, and arrives as it is.
+// before them), `none` is zero and not known to the compiler. A kernel whose later (volatile) shared loads or stores need every
+// value that it took from the entry has waited for them already, and arrives as it is.
 __device__ __forceinline__ void release_after(uint64_t *bar, int lane, uint32_t read, uint32_t none) {
     __syncwarp();
     if (lane == 0) mbar_arrive((uint64_t *)((unsigned char *)bar + (read & none)));

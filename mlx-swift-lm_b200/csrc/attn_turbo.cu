@@ -396,7 +396,7 @@ attn_turbo_decode8_kernel(const __grid_constant__ TurboParams p) {
                     mma_f16(o_acc[mt], a, pb[0], pb[1]);
                 }
             }
-            __syncwarp();
+            __syncwarp();   // (the table lookups above have waited for every value of the stage, see release_after)
             if (lane == 0) mbar_arrive(&empty[s]);
         }
         // a warp whose tokens were all masked reports "no maximum"
