@@ -30,8 +30,8 @@
 //     kernel, 89 us here (114 with the values through the tile and a load for each half); with single f16 operands the
 //     outputs no longer err by the store's rounding alone.
 //   * The running reference is only moved when a score (with its value factor) passes it by more than 2^3.
-// Work is cut into equal ranges of 64-token tiles per resident CTA (UnitPlan), units that cross a CTA boundary
-// are merged by segment_epilogue.
+// Work is cut into ranges of 64-token tiles, equal ones or ones that end where units end (plan_units); units that cross a CTA
+// boundary are merged by segment_epilogue.
 #pragma once
 
 #include "attn_common.cuh"
