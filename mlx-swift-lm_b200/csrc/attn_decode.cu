@@ -662,6 +662,7 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
             v_off[cp] = (uint32_t)((blk * 16 + (mi & 1) * 8 + rr) * 128 + (((2 * cp + (mi >> 1)) ^ rr) << 4));
     }
 
+    const uint32_t none = gridDim.y - 1;
     int it = 0, sg = 0;
     FlatSeg gs;
     gs.layer = 0;
@@ -850,17 +851,20 @@ attn_decode_flat_kernel(const __grid_constant__ std::conditional_t<LIST, FlatLis
                     o_acc[nt][3] *= alpha[1];
                 }
             }
+            uint32_t read = 0;   // the last word of the tile
 #pragma unroll
             for (int bx = 0; bx < BOXES; ++bx) {
 #pragma unroll
                 for (int cp = 0; cp < 4; ++cp) {
                     uint32_t vf[4];
                     ldmatrix_x4_trans(vf, vt_addr + bx * BOX_BYTES + v_off[cp]);
+                    read = vf[3];
                     MmaType<T>::mma(o_acc[bx * 8 + 2 * cp], pa, vf[0], vf[1]);
                     MmaType<T>::mma(o_acc[bx * 8 + 2 * cp + 1], pa, vf[2], vf[3]);
                 }
             }
-            release_fenced(&empty[s], lane);
+            // (6 layers of 13 sequences, 16/16 heads, D 64, 512 and 1 833 tokens: 50.9 us, 51.9 with the fence)
+            release_after(&empty[s], lane, read, none);
         }
 
         if (fused && warp == 0 && w.last && !(KVC_SKIP_BITS(p) & 32)) {

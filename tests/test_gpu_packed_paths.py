@@ -512,6 +512,8 @@ def _caches(kvc, oracle, cuda, dtype, kw, B, Hkv, D, P, gain=1.0):
     (torch.float16, dict(bits=4, group=64), 24, True),
     (torch.float16, dict(key_bits=3, value_bits=4), 24, False),
     (torch.float16, dict(key_bits=4, value_bits=2), 24, False),
+    (torch.float16, None, 24, False),                            # a raw cache
+    (torch.bfloat16, None, 32, False),
 ])
 def test_ring_entries_are_read_before_they_are_filled_again(kvc, oracle, cuda, dtype, kw, Hq, lists):
     """Contexts that walk the rings of packed tiles several times, out of L2, where a copy is back soonest: run after run
