@@ -161,10 +161,10 @@ __device__ __forceinline__ uint32_t mask_bits32(const uint8_t *p, int n) {
     n = min(n, 32);
     const uint32_t *w = (const uint32_t *)((uintptr_t)p & ~(uintptr_t)3);
     const int sh = (int)((uintptr_t)p & 3) * 8, words = (n + (sh >> 3) + 3) >> 2;   // only words that hold a byte of the row
-    uint32_t bits = 0, cur = __ldg(w);
+    uint32_t bits = 0, cur = *w;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const uint32_t nxt = i + 1 < words ? __ldg(w + i + 1) : 0u;
+        const uint32_t nxt = i + 1 < words ? w[i + 1] : 0u;
         const uint32_t b = __vcmpne4(__funnelshift_r(cur, nxt, sh), 0u) & 0x08040201u;
         bits |= ((b | b >> 8 | b >> 16 | b >> 24) & 15u) << (4 * i);
         cur = nxt;

@@ -547,9 +547,9 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                     const int64_t t = (int64_t)(j_lo + j) * TC_KEYS + row;
                     const uint4 *src = (const uint4 *)(cbase + t * KW);
 #pragma unroll
-                    for (int i = 0; i < KW / 4; ++i) nxt[i] = __ldg(src + i);
-                    nsc = __ldg((const uint32_t *)(sbase + t * 2));
-                    nzp = __ldg((const uint32_t *)(zbase + t * 2));
+                    for (int i = 0; i < KW / 4; ++i) nxt[i] = src[i];
+                    nsc = *(const uint32_t *)(sbase + t * 2);
+                    nzp = *(const uint32_t *)(zbase + t * 2);
                 }
             };
 #pragma unroll
@@ -623,8 +623,8 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                     const int64_t t = (int64_t)(j_lo + j) * TC_KEYS + row;
                     const uint4 *src = (const uint4 *)(kbase + t * KW);
 #pragma unroll
-                    for (int i = 0; i < KW / 4; ++i) nk[i] = __ldg(src + i);
-                    nkn = __ldg(knb + t);
+                    for (int i = 0; i < KW / 4; ++i) nk[i] = src[i];
+                    nkn = knb[t];
                 }
             };
             auto fetch_v = [&](int j) {
@@ -632,8 +632,8 @@ attn_verify_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
                     const int64_t t = (int64_t)(j_lo + j) * TC_KEYS + row;
                     const uint4 *src = (const uint4 *)(vbase + t * VW);
 #pragma unroll
-                    for (int i = 0; i < VW / 4; ++i) nv[i] = __ldg(src + i);
-                    nvn = __ldg(vnb + t);
+                    for (int i = 0; i < VW / 4; ++i) nv[i] = src[i];
+                    nvn = vnb[t];
                 }
             };
             // The two halves of a row are a rolled loop and each writer has one call site: unrolled, the roles of

@@ -200,7 +200,7 @@ __device__ __forceinline__ void affine_quantize_vec_body(const QuantAppendArgs &
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int sr = s0 + u * RPP;
-        raw[u] = sr < a.S ? __ldg(reinterpret_cast<const uint4 *>(src + sr * a.s_ss)) : make_uint4(0u, 0u, 0u, 0u);
+        raw[u] = sr < a.S ? *reinterpret_cast<const uint4 *>(src + sr * a.s_ss) : make_uint4(0u, 0u, 0u, 0u);
     }
     const int lpg = 1 << lpg_log2;   // lanes per group
 #pragma unroll
@@ -855,24 +855,25 @@ turbo_calib_stats_kernel(TurboEncodeArgs a, int64_t total_rows, float inv_sqrt_d
         if (s_sum[i]) atomicAdd(&sums[i], s_sum[i]);
 }
 
-// E consecutive elements of a contiguous row in as few loads as their size allows.
+// E consecutive elements of a contiguous row in as few loads as their size allows. (Not through the read-only path: a kernel that
+// starts under the tail of the one before reads what that one writes, if only after its wait.)
 template <typename T, int E>
 __device__ __forceinline__ void load_row_elems(const T *p, float (&v)[E]) {
     constexpr int BYTES = E * (int)sizeof(T);
     if constexpr (BYTES % 16 == 0) {
         uint4 raw[BYTES / 16];
 #pragma unroll
-        for (int i = 0; i < BYTES / 16; ++i) raw[i] = __ldg(reinterpret_cast<const uint4 *>(p) + i);
+        for (int i = 0; i < BYTES / 16; ++i) raw[i] = reinterpret_cast<const uint4 *>(p)[i];
         const T *e = reinterpret_cast<const T *>(raw);
 #pragma unroll
         for (int i = 0; i < E; ++i) v[i] = to_float<T>(e[i]);
     } else if constexpr (BYTES == 8) {
-        const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p));
+        const uint2 raw = *reinterpret_cast<const uint2 *>(p);
         const T *e = reinterpret_cast<const T *>(&raw);
 #pragma unroll
         for (int i = 0; i < E; ++i) v[i] = to_float<T>(e[i]);
     } else if constexpr (BYTES == 4) {
-        const uint32_t raw = __ldg(reinterpret_cast<const uint32_t *>(p));
+        const uint32_t raw = *reinterpret_cast<const uint32_t *>(p);
         const T *e = reinterpret_cast<const T *>(&raw);
 #pragma unroll
         for (int i = 0; i < E; ++i) v[i] = to_float<T>(e[i]);
