@@ -1641,10 +1641,18 @@ bool attention_chunk_rows_accepts(const AttnArgs &a) {
 
 namespace {
 
+// Shared memory of the flat kernel: ring, barriers, cross-warp buffers, two units' query rows.
+constexpr int flat_stages(int D) { return D == 64 ? 6 : 3; }
+constexpr size_t flat_smem(int D, int R) {
+    const size_t ring = (size_t)flat_stages(D) * 2 * (TILE_T * D * 2);
+    const size_t red = (size_t)CONSUMER_WARPS * R * (D + 8) * 4 + (size_t)CONSUMER_WARPS * R * 8 + 16 + 4 * sizeof(uint64_t) + (size_t)2 * R * D * 2;
+    return ring + 2 * flat_stages(D) * sizeof(uint64_t) + 64 + red + 1024;
+}
+constexpr bool flat_fits_sm(int D, int R) { return flat_smem(D, R) <= (size_t)(D <= 128 ? 112 : 224) * 1024; }
+
 // One wave of CTAs over `work` tiles, and the shared memory of the flat kernel for it.
 struct FlatShape {
     int64_t ctas, per, rem, nslots;
-    int nstage;
     size_t smem;
     bool fits;
 };
@@ -1653,11 +1661,8 @@ FlatShape flat_shape(int sms, int D, int R, int64_t work, int64_t most_tiles) {
     f.ctas = std::min<int64_t>((int64_t)sms * (D <= 128 ? 2 : 1), work);
     f.per = work / f.ctas; f.rem = work % f.ctas;
     f.nslots = (most_tiles + f.per - 1) / f.per + 1;
-    f.nstage = D == 64 ? 6 : 3;
-    const size_t ring = (size_t)f.nstage * 2 * (TILE_T * D * 2);
-    const size_t red = (size_t)CONSUMER_WARPS * R * (D + 8) * 4 + (size_t)CONSUMER_WARPS * R * 8 + 16 + 4 * sizeof(uint64_t) + (size_t)2 * R * D * 2;
-    f.smem = ring + 2 * f.nstage * sizeof(uint64_t) + 64 + red + 1024;
-    f.fits = f.smem <= (size_t)(D <= 128 ? 112 : 224) * 1024;
+    f.smem = flat_smem(D, R);
+    f.fits = flat_fits_sm(D, R);
     return f;
 }
 
@@ -1685,8 +1690,8 @@ bool flat_off() {
 
 // Whether one launch may turn, append and attend a step of `rows` query rows per KV head: what the flat kernel asks that
 // does not depend on the context's length.
-bool attention_decode_takes_rope(int device, int D, int64_t rows, int64_t units) {
-    return !flat_off() && rows <= 16 && units * (int64_t)sizeof(int) <= COUNTER_BYTES && flat_shape(sm_count(device), D, (int)rows, 1, 1).fits;
+bool attention_decode_takes_rope(int D, int64_t rows, int64_t units) {
+    return !flat_off() && rows <= 16 && units * (int64_t)sizeof(int) <= COUNTER_BYTES && flat_fits_sm(D, (int)rows);
 }
 
 // The single-token steps of up to KVC_LIST_MAX raw caches of one shape (new rows not yet stored, or all stored)

@@ -1194,7 +1194,7 @@ static bool fused_append_off() {
     return off;
 }
 
-bool attention_decode_takes_rope(int device, int D, int64_t rows, int64_t units);   // attn_decode.cu
+bool attention_decode_takes_rope(int D, int64_t rows, int64_t units);   // attn_decode.cu
 
 // Whether cache_attention will hand unturned rows to the decode kernel: its own conditions, and those of the kernel that
 // do not depend on what it allocates.
@@ -1208,7 +1208,7 @@ bool cache_takes_rope(const kvc_cache *c, const kvc_tensor &q, const kvc_tensor 
     const int64_t D = q.shape[3], rep = k.shape[1] > 0 ? q.shape[1] / k.shape[1] : 0;
     if ((D != 64 && D != 128 && D != 256) || rep < 1 || rep > 16 || q.shape[1] % k.shape[1]) return false;
     auto rows = [](const kvc_tensor &t) { return !((uintptr_t)t.data & 15) && (t.stride[0] * 2) % 16 == 0 && (t.stride[1] * 2) % 16 == 0; };
-    return rows(q) && rows(k) && rows(v) && q.stride[1] == D && attention_decode_takes_rope(current_device(), (int)D, rep, k.shape[0] * k.shape[1]);
+    return rows(q) && rows(k) && rows(v) && q.stride[1] == D && attention_decode_takes_rope((int)D, rep, k.shape[0] * k.shape[1]);
 }
 
 namespace {
