@@ -1005,6 +1005,38 @@ assert float((outs[0] - outs[1]).norm()) < 2.0 ** -8 * float(outs[1].norm())
         assert ("rows written out" in part) == (n > 0) and (n == 0 or f"{n} sequences per slice" in part), err
 
 
+@pytest.mark.parametrize("kw,P,L", [(dict(key_bits=3, value_bits=4), 20000, 17),      # rows from the pool
+                                    (dict(key_bits=3, value_bits=4), 300, 17),        # in the arena
+                                    (dict(bits=4, group=64), 20000, 512)])
+def test_captured_chunk_with_rows_written_out(kvc, cuda, capfd, monkeypatch, kw, P, L):
+    """Replays on other inputs give the eager call's bits, wherever the rows lie."""
+    monkeypatch.setenv("KVC_TRACE_DISPATCH", "1")
+    B, Hq, Hkv, D = 1, 32, 8, 128
+    c = _packed(kvc, cuda, kw, B, Hkv, D, P)
+    q, k1, v1 = (seeded((B, h, L, D), s, torch.half).to(cuda) for s, h in ((3, Hq), (4, Hkv), (5, Hkv)))
+    out = torch.empty_like(q)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        c.attention(q, k1, v1, D ** -0.5, "causal", out=out)        # warm: workspaces of this stream
+    torch.cuda.synchronize()
+    c.trim(L)
+    graph = torch.cuda.CUDAGraph()
+    capfd.readouterr()
+    with torch.cuda.graph(graph, stream=side):
+        c.attention(q, k1, v1, D ** -0.5, "causal", out=out)
+    assert "rows written out" in capfd.readouterr().err
+    for seed in (11, 12):
+        q.copy_(seeded(tuple(q.shape), seed, torch.half))
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        c.trim(L)
+        assert torch.equal(out, c.attention(q, k1, v1, D ** -0.5, "causal"))
+    del graph
+    assert kvc.lib().kvc_device_status() == 0
+
+
 def test_sequences_of_a_call_take_one_kernel(kvc, cuda, capfd, monkeypatch):
     """Rows written out for a chunk are limited to a few GB at a time. Where a last slice of the batch would be too small to be worth it,
     no sequence of the call is treated that way: equal sequences have equal outputs."""
